@@ -49,6 +49,7 @@ CU_SOURCES = (
     "runtime.cu",
     "stencil_setup.cu",
     "init_kernels.cu",
+    "carry3d.cu",
     "binary3d_fast.cu",
     "binary3d_exact.cu",
     "binary2d_fast.cu",

@@ -8,9 +8,9 @@ namespace asets {
 
 static const StencilVariant kVariants[] = {
     // two rows per thread, 240-row tiles, 6 stages, unrolled by 4
-    make_variant<2, 4, 6, EPI_BINARY, true, 4, 4, 2>(),
-    make_variant<2, 8, 4, EPI_BINARY, true>(),
-    make_variant<2, 2, 4, EPI_BINARY, true>(),
+    make_variant<4, 6, EPI_BINARY, true, 4, 4, 2>(),
+    make_variant<8, 4, EPI_BINARY, true>(),
+    make_variant<2, 4, EPI_BINARY, true>(),
     // two iterations per pass, 224-row tiles
     make_variant_t2<4, 5, true, 3, 4>(),
     // square tiles for small images: 32 x 32 (256 threads), 16 x 16 (128)

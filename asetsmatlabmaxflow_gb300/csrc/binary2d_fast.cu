@@ -13,10 +13,10 @@ static const StencilVariant kVariants[] = {
     make_variant_t2<4, 5, false, 3, 4>(),
     // one iteration per pass: two rows per thread, 240-row tiles, 6 stages,
     // the plane loop unrolled by 4
-    make_variant<2, 4, 6, EPI_BINARY, false, 4, 4, 2>(),
-    make_variant<2, 8, 4, EPI_BINARY, false, 4, 4>(),       // 224-row tiles
-    make_variant<2, 2, 4, EPI_BINARY, false>(),             // 56-row tiles (short columns)
-    make_variant<2, 4, 4, EPI_BINARY, false, 4, 4, 2>(),
+    make_variant<4, 6, EPI_BINARY, false, 4, 4, 2>(),
+    make_variant<8, 4, EPI_BINARY, false, 4, 4>(),       // 224-row tiles
+    make_variant<2, 4, EPI_BINARY, false>(),             // 56-row tiles (short columns)
+    make_variant<4, 4, EPI_BINARY, false, 4, 4, 2>(),
     // square tiles for small images: 32 x 32 (256 threads), 16 x 16 (128)
     make_variant_tile<32, 32, 256, false>(),
     make_variant_tile<16, 16, 128, false, 4>(),

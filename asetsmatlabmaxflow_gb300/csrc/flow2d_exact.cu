@@ -7,10 +7,10 @@ namespace asets {
 
 static const StencilVariant kVariants[] = {
     // two rows per thread, 240-row tiles (four and six stages)
-    make_variant<2, 4, 4, EPI_DIV, true, 4, 4, 2>(),
-    make_variant<2, 8, 4, EPI_DIV, true>(),
-    make_variant<2, 2, 4, EPI_DIV, true>(),
-    make_variant<2, 4, 6, EPI_DIV, true, 4, 4, 2>(),
+    make_variant<4, 4, EPI_DIV, true, 4, 4, 2>(),
+    make_variant<8, 4, EPI_DIV, true>(),
+    make_variant<2, 4, EPI_DIV, true>(),
+    make_variant<4, 6, EPI_DIV, true, 4, 4, 2>(),
 };
 
 const StencilVariant *flow2d_exact_variants(int *count)

@@ -9,10 +9,10 @@ namespace asets {
 static const StencilVariant kVariants[] = {
     // default: two rows per thread, 240-row tiles, 4 stages, the plane loop
     // unrolled by 4
-    make_variant<2, 4, 4, EPI_DIV, false, 4, 4, 2>(),
-    make_variant<2, 8, 4, EPI_DIV, false, 4, 4>(),       // 224-row tiles
-    make_variant<2, 2, 4, EPI_DIV, false>(),             // 56-row tiles (short columns)
-    make_variant<2, 4, 6, EPI_DIV, false, 4, 4, 2>(),
+    make_variant<4, 4, EPI_DIV, false, 4, 4, 2>(),
+    make_variant<8, 4, EPI_DIV, false, 4, 4>(),       // 224-row tiles
+    make_variant<2, 4, EPI_DIV, false>(),             // 56-row tiles (short columns)
+    make_variant<4, 6, EPI_DIV, false, 4, 4, 2>(),
 };
 
 const StencilVariant *flow2d_fast_variants(int *count)

@@ -99,6 +99,22 @@ __global__ void validate_alpha_kernel(InitArgs A)
         atomicOr(&A.ctl->alpha_bad, 1);
 }
 
+__global__ void check_range_kernel(InitArgs A)
+{
+    int wide = 0;
+    for (long long g = blockIdx.x * (long long)kInitThreads + threadIdx.x; g < A.cells;
+         g += (long long)gridDim.x * kInitThreads) {
+        if ((int)((unsigned int)g % (unsigned int)A.pitch) >= A.nr)
+            continue;
+        const float m = fmaxf(fmaxf(fabsf(A.cs[g]), fabsf(A.ct[g])), fabsf(A.alpha[g]));
+        // fmaxf drops a NaN: the sum keeps it
+        if (!(m < kColdInputLimit) || !(A.cs[g] + A.ct[g] + A.alpha[g] < INFINITY))
+            wide = 1;
+    }
+    if (__syncthreads_or(wide) && threadIdx.x == 0)
+        atomicOr(&A.ctl->wide, 1);
+}
+
 static int grid_for(long long n, int num_sms)
 {
     long long b = (n + kInitThreads - 1) / kInitThreads;
@@ -123,6 +139,12 @@ cudaError_t launch_init(int model, const InitArgs &a, int num_sms, cudaStream_t 
 cudaError_t launch_validate_alpha(const InitArgs &a, int num_sms, cudaStream_t st)
 {
     validate_alpha_kernel<<<grid_for(a.cells * a.alpha_labels, num_sms), kInitThreads, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_check_range(const InitArgs &a, int num_sms, cudaStream_t st)
+{
+    check_range_kernel<<<grid_for(a.cells, num_sms), kInitThreads, 0, st>>>(a);
     return cudaGetLastError();
 }
 

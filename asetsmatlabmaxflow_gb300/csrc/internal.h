@@ -35,6 +35,8 @@ struct StencilVariant {
     // dynamic shared memory of a launch: smem_bytes + smem_per_fl x flow
     // labels + smem_per_l x labels (label counts known only at run time)
     int smem_per_fl = 0, smem_per_l = 0;
+    const StencilVariant *cold = nullptr;  // fast binary 3D: the form for a cold start
+    int box_cols_s0 = 0;     // 3D: halo box columns of the carried source gk (slot SL_S0)
 };
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
@@ -49,14 +51,14 @@ struct StencilProblem {
     long long pitch, plane, cells;
     int flow_labels;             // labels swept per launch
     float *b[2][3];              // flows [parity][SL_BC, SL_BR, SL_BS]
-    float *src[2][3];            // gk sources s0, s1, s2 per parity
+    float *src[2][3];            // gk sources s0, s1, s2 per parity; 3D: gk, and binary pt, u
     int src_labels[3];           // label extent of each source array
     int lab_mul[NUM_SLOTS], lab_add[NUM_SLOTS];
     float *alpha;
     int alpha_labels;
     const float *cs, *ct;        // binary capacities; Ct of the one-pass multi-label kernel
     int ct_labels;
-    float *dst_s[2][3];          // binary: new ps/pt/u; labelled: [.][0] = divergence
+    float *dst_s[2][3];          // binary: new ps/pt/u (3D: gk/pt/u); labelled: [.][0] = divergence
 };
 
 // Fill the TMA descriptors, destinations and geometry of problem `d` for
@@ -66,6 +68,11 @@ int build_problem_desc(EncodeTiledFn encode, const StencilVariant &v, const Sten
                        ProblemDesc *d);
 // Work split: stream-axis chunks per tile for `slots` resident blocks.
 int choose_zchunks(const StencilProblem &p, const StencilVariant &v, long long slots);
+// Work split of a 3D problem into d->units_a, zchunks_a and zchunks for
+// `slots` resident blocks; returns its length in plane steps.
+double choose_split3(const StencilProblem &p, const StencilVariant &v, long long slots, ProblemDesc *d);
+// Items of a 3D problem with the split of d.
+int split3_items(const StencilProblem &p, const StencilVariant &v, const ProblemDesc &d);
 // Items of one problem with the given chunk count.
 int problem_items(const StencilProblem &p, const StencilVariant &v, int zchunks);
 
@@ -112,6 +119,10 @@ struct LabelArgs {
     float *u;
     float *pt;
     float *ps;           // Potts only
+    // 3D (gk not null): the kernel stores the next iteration's gradient
+    // source; Potts keeps u and ps in two parities (u, ps: even iterations
+    // read, u1, ps1: odd ones) and stores no pt
+    float *u1, *ps1, *gk;
     const float *dv;
     const float *ct;
     IterControl *ctl;
@@ -144,6 +155,9 @@ struct InitArgs {
 };
 
 cudaError_t launch_init(int model, const InitArgs &a, int num_sms, cudaStream_t st);
+// Sets a.ctl->wide if an input of a binary problem is not finite or is
+// beyond the range of the cold start's state.
+cudaError_t launch_check_range(const InitArgs &a, int num_sms, cudaStream_t st);
 cudaError_t launch_validate_alpha(const InitArgs &a, int num_sms, cudaStream_t st);
 cudaError_t launch_wait_selftest(int *d_err, cudaStream_t st);
 
@@ -171,6 +185,26 @@ struct GridGeom {
 struct GridXfer {
     GridGeom f, c;
 };
+// The 3D solvers' carried state (carry3d.cu).
+struct CarryArgs {
+    GridGeom g;
+    int flow_labels, exact;
+    float cc, inv_cc;
+    const float *bc, *br, *bs;       // lower-face flows (br null: zero flows)
+    const float *ps, *pt, *u;
+    const float *cs, *ct, *dv;
+    const float *v;                  // cold binary start: v after the last iteration
+    float *gk;                       // launch_source, launch_cold_source
+    float *out;                      // launch_flows: binary ps, Potts pt
+    float *v_out, *u_out, *pt_out;   // launch_cold_source; launch_cold_state
+};
+// Initial v and gk of the cold binary start, from Cs and Ct.
+cudaError_t launch_cold_source(const CarryArgs &a, int num_sms, cudaStream_t st);
+// u (u_out) or pt (pt_out) of the state v.
+cudaError_t launch_cold_state(const CarryArgs &a, int num_sms, cudaStream_t st);
+cudaError_t launch_source(int model, const CarryArgs &a, int num_sms, cudaStream_t st);
+cudaError_t launch_flows(int model, const CarryArgs &a, int num_sms, cudaStream_t st);
+
 cudaError_t launch_restrict(const GridXfer &X, const float *src, float *dst, int labels,
                             float scale, int num_sms, cudaStream_t st);
 cudaError_t launch_prolong(const GridXfer &X, const float *src, float *dst, int labels,

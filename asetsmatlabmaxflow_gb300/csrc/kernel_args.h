@@ -28,7 +28,8 @@ struct IterControl {
     float denom;        // cvg = (float)erru / denom
     int alpha_bad;      // set by the validation pass
     int rollback;       // two-iteration pass: the solve ended at its first iteration
-    int pad[4];
+    int wide;           // set by the range check (binary 3D)
+    int pad[3];
 };
 
 // Stage slots: which field each TMA box holds.
@@ -36,7 +37,7 @@ enum Slot : int {
     SL_BC = 0,   // flow on faces normal to the column axis (Matlab x in 3D)
     SL_BR = 1,   // flow on faces normal to the row axis (Matlab y)
     SL_BS = 2,   // flow on faces normal to the stream axis (z in 3D, x in 2D)
-    SL_S0 = 3,   // gk source terms: gk = div - ((s0 - s1) + s2/cc)
+    SL_S0 = 3,   // gk source terms: gk = div - ((s0 - s1) + s2/cc); 3D: gk itself
     SL_S1 = 4,
     SL_S2 = 5,
     SL_ALPHA = 6,
@@ -46,6 +47,7 @@ enum Slot : int {
 enum Epilogue : int {
     EPI_BINARY = 0,  // binary model: ps/pt/u update + erriter
     EPI_DIV = 1,     // multi-label models: write the new flow and its divergence
+    EPI_COLD = 3,    // binary 3D from the cold start: pt and u in one array (dst_s: gk, v)
     EPI_FUSED = 2,   // multi-label 2D, one pass: flows of all labels and the label update
 };
 
@@ -63,7 +65,7 @@ struct ProblemDesc {
     CUtensorMap tile[2][NUM_TILE_SLOTS];   // binary; EPI_FUSED: [.][TS_CT] = Ct, all labels,
                                            // halo rows (the same map for both parities)
     float *dst_b[2][3];                    // [source parity][SL_BC, SL_BR, SL_BS]
-    float *dst_s[2][3];                    // binary: ps, pt, u; EPI_DIV: [.][0] = divergence;
+    float *dst_s[2][3];                    // binary: ps (3D: gk), pt, u; EPI_DIV: [.][0] = divergence;
                                            // EPI_FUSED: Potts ps, pt, u; Ishikawa pt, -, u
     const float *alpha, *cs, *ct;          // inputs, for kernels that read them without TMA
     IterControl *ctl;
@@ -76,6 +78,8 @@ struct ProblemDesc {
     int nlab_items;
     int tiles_r, tiles_c;
     int zchunks;                           // stream-axis chunks per tile
+    int units_a, zchunks_a;                // 3D: the first units_a (label, tile) units are split
+                                           // into zchunks_a chunks instead
     int item_begin, n_items;               // this problem's items in the launch
     long long dst_elems;                   // elements of each destination array (bounds checks)
     int lab_mul[NUM_SLOTS];

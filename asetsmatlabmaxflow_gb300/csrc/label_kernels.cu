@@ -9,6 +9,12 @@
 //            then the multipliers (updateU, :578-610).
 //
 // Both accumulate erriter and close the iteration (iteration_end.cuh).
+//
+// CARRY (3D): the kernel also stores the next iteration's gradient source
+// gk = div - ((ps - pt) + u/cc) of every flow label, which it has in
+// registers, for stencil3d_kernel.cuh.  Potts' pt is read by nothing else
+// and is not stored (carry3d.cu forms it on request), and its u and ps go to
+// the other parity, so that the last iteration's inputs stay available for that.
 // Voxels are visited in the padded layout; each label slice is contiguous in
 // rows, so every label access is a coalesced stream.
 #include "internal.h"
@@ -55,7 +61,7 @@ __device__ __forceinline__ float over_cc(float u, float cc, float inv_cc)
 // LFIX > 0: label count known at compile time (register arrays);
 // LFIX == 0: any label count, second pass re-reads dv_k and the new pt_k
 // (same operands, so the same bits).
-template <int LFIX, bool EXACT>
+template <int LFIX, bool EXACT, bool CARRY>
 __global__ void __launch_bounds__(kLabelThreads) potts_label_kernel(LabelArgs A)
 {
     __shared__ double s_red[kLabelThreads / 32];
@@ -69,56 +75,74 @@ __global__ void __launch_bounds__(kLabelThreads) potts_label_kernel(LabelArgs A)
     const float inv_l = 1.0f / (float)L;
     const unsigned int S = (unsigned int)A.label_stride;
     const int lane = threadIdx.x & 31;
+    const bool odd = CARRY && (it & 1);
+    const float *u_in = odd ? A.u1 : A.u, *ps_in = odd ? A.ps1 : A.ps;
+    float *u_out = (CARRY && !odd) ? A.u1 : A.u, *ps_out = (CARRY && !odd) ? A.ps1 : A.ps;
     float erru = 0.0f;
     for (SegWalk w(A.nr); w.row < A.rows; w.next()) {
         const int r = (int)(w.seg << 5) + lane;
         if (r >= A.nr)
             continue;
         const unsigned int g = w.row * (unsigned int)A.pitch + (unsigned int)r;
-        const float ps = A.ps[g];
+        const float ps = ps_in[g];
         float fsum = 0.0f;
+        // the sink flow of a label from its operands
+        auto sink = [&](float uc, float dv, float ctv) {
+            const float pt = (ps + uc) - dv;
+            return (pt < ctv) ? pt : ctv;
+        };
         if constexpr (LFIX > 0) {
-            float ft[LFIX], uu[LFIX];
+            float ft[LFIX], uu[LFIX];              // ft = dv + pt
+            float dd[CARRY ? LFIX : 1], pp[CARRY ? LFIX : 1];
 #pragma unroll
             for (int k = 0; k < LFIX; ++k) {
                 const unsigned int o = g + k * S;
-                const float u = A.u[o];
-                const float uc = over_cc<EXACT>(u, cc, inv_cc);
+                uu[k] = u_in[o];
+                const float uc = over_cc<EXACT>(uu[k], cc, inv_cc);
                 const float dv = A.dv[o];
-                const float ctv = A.ct[o];
-                float pt = (ps + uc) - dv;
-                pt = (pt < ctv) ? pt : ctv;
-                A.pt[o] = pt;
+                const float pt = sink(uc, dv, A.ct[o]);
+                if constexpr (CARRY) {
+                    dd[k] = dv;
+                    pp[k] = pt;
+                } else {
+                    A.pt[o] = pt;
+                }
                 ft[k] = dv + pt;
-                uu[k] = u;
                 fsum += (ft[k] - uc);
             }
             const float ps_n = (EXACT ? __fdiv_rn(fsum, (float)L) : fsum * inv_l) + A.inv_cc_l;
-            A.ps[g] = ps_n;
+            ps_out[g] = ps_n;
 #pragma unroll
             for (int k = 0; k < LFIX; ++k) {
                 const float e = cc * (ft[k] - ps_n);
-                A.u[g + k * S] = uu[k] - e;
+                const float un = uu[k] - e;
+                u_out[g + k * S] = un;
                 erru += abs_ref(e);
+                if constexpr (CARRY)
+                    A.gk[g + k * S] = dd[k] - ((ps_n - pp[k]) + div_cc<EXACT>(un, cc, inv_cc));
             }
         } else {
             for (int k = 0; k < L; ++k) {
                 const unsigned int o = g + k * S;
-                const float uc = over_cc<EXACT>(A.u[o], cc, inv_cc);
+                const float uc = over_cc<EXACT>(u_in[o], cc, inv_cc);
                 const float dv = A.dv[o];
-                const float ctv = A.ct[o];
-                float pt = (ps + uc) - dv;
-                pt = (pt < ctv) ? pt : ctv;
-                A.pt[o] = pt;
+                const float pt = sink(uc, dv, A.ct[o]);
+                if (!CARRY)
+                    A.pt[o] = pt;
                 fsum += ((dv + pt) - uc);
             }
             const float ps_n = (EXACT ? __fdiv_rn(fsum, (float)L) : fsum * inv_l) + A.inv_cc_l;
-            A.ps[g] = ps_n;
+            ps_out[g] = ps_n;
             for (int k = 0; k < L; ++k) {
                 const unsigned int o = g + k * S;
-                const float e = cc * ((A.dv[o] + A.pt[o]) - ps_n);
-                A.u[o] = A.u[o] - e;
+                const float u = u_in[o], dv = A.dv[o];
+                const float pt = CARRY ? sink(over_cc<EXACT>(u, cc, inv_cc), dv, A.ct[o]) : A.pt[o];
+                const float e = cc * ((dv + pt) - ps_n);
+                const float un = u - e;
+                u_out[o] = un;
                 erru += abs_ref(e);
+                if (CARRY)
+                    A.gk[o] = dv - ((ps_n - pt) + div_cc<EXACT>(un, cc, inv_cc));
             }
         }
     }
@@ -174,7 +198,7 @@ __device__ __forceinline__ void st_vec(float *p, const float (&v)[VEC], int n)
 // wider accesses and fewer instructions per voxel.  Rows are padded to a
 // multiple of 4 floats and label slices are whole padded volumes, so every
 // full group is 4*VEC-byte aligned.
-template <int LFIX, bool EXACT, int VEC>
+template <int LFIX, bool EXACT, int VEC, bool CARRY>
 __global__ void __launch_bounds__(kLabelThreads) potts_label_kernel_v(LabelArgs A)
 {
     __shared__ double s_red[kLabelThreads / 32];
@@ -187,6 +211,9 @@ __global__ void __launch_bounds__(kLabelThreads) potts_label_kernel_v(LabelArgs 
     const float inv_l = 1.0f / (float)LFIX;
     const unsigned int S = (unsigned int)A.label_stride;
     const int lane = threadIdx.x & 31;
+    const bool odd = CARRY && (it & 1);
+    const float *u_in = odd ? A.u1 : A.u, *ps_in = odd ? A.ps1 : A.ps;
+    float *u_out = (CARRY && !odd) ? A.u1 : A.u, *ps_out = (CARRY && !odd) ? A.ps1 : A.ps;
     float erru = 0.0f;
     for (SegWalk w(A.nr, 32 * VEC); w.row < A.rows; w.next()) {
         const int r = (int)(w.seg * (32 * VEC)) + lane * VEC;
@@ -195,35 +222,40 @@ __global__ void __launch_bounds__(kLabelThreads) potts_label_kernel_v(LabelArgs 
         const int n = min(VEC, A.nr - r);
         const unsigned int g = w.row * (unsigned int)A.pitch + (unsigned int)r;
         float ps[VEC], fsum[VEC];
-        float ft[LFIX][VEC], uu[LFIX][VEC];
-        ld_vec<VEC>(A.ps + g, ps, n);
+        float ft[LFIX][VEC], uu[LFIX][VEC];        // ft = dv + pt
+        float dd[CARRY ? LFIX : 1][VEC], pp[CARRY ? LFIX : 1][VEC];
+        ld_vec<VEC>(ps_in + g, ps, n);
 #pragma unroll
         for (int i = 0; i < VEC; ++i)
             fsum[i] = 0.0f;
 #pragma unroll
         for (int k = 0; k < LFIX; ++k) {
             const unsigned int o = g + k * S;
-            float u[VEC], dv[VEC], ctv[VEC], pt[VEC];
-            ld_vec<VEC>(A.u + o, u, n);
+            float dv[VEC], ctv[VEC], pt[VEC];
+            ld_vec<VEC>(u_in + o, uu[k], n);
             ld_vec<VEC>(A.dv + o, dv, n);
             ld_vec<VEC>(A.ct + o, ctv, n);
 #pragma unroll
             for (int i = 0; i < VEC; ++i) {
-                const float uc = over_cc<EXACT>(u[i], cc, inv_cc);
+                const float uc = over_cc<EXACT>(uu[k][i], cc, inv_cc);
                 float p = (ps[i] + uc) - dv[i];
                 p = (p < ctv[i]) ? p : ctv[i];
                 pt[i] = p;
                 ft[k][i] = dv[i] + p;
-                uu[k][i] = u[i];
                 fsum[i] += (ft[k][i] - uc);
+                if constexpr (CARRY) {
+                    dd[k][i] = dv[i];
+                    pp[k][i] = p;
+                }
             }
-            st_vec<VEC>(A.pt + o, pt, n);
+            if (!CARRY)
+                st_vec<VEC>(A.pt + o, pt, n);
         }
         float ps_n[VEC];
 #pragma unroll
         for (int i = 0; i < VEC; ++i)
             ps_n[i] = (EXACT ? __fdiv_rn(fsum[i], (float)LFIX) : fsum[i] * inv_l) + A.inv_cc_l;
-        st_vec<VEC>(A.ps + g, ps_n, n);
+        st_vec<VEC>(ps_out + g, ps_n, n);
 #pragma unroll
         for (int k = 0; k < LFIX; ++k) {
             float un[VEC];
@@ -234,13 +266,20 @@ __global__ void __launch_bounds__(kLabelThreads) potts_label_kernel_v(LabelArgs 
                 if (i < n)
                     erru += abs_ref(e);
             }
-            st_vec<VEC>(A.u + g + k * S, un, n);
+            st_vec<VEC>(u_out + g + k * S, un, n);
+            if constexpr (CARRY) {
+                float gk[VEC];
+#pragma unroll
+                for (int i = 0; i < VEC; ++i)
+                    gk[i] = dd[k][i] - ((ps_n[i] - pp[k][i]) + div_cc<EXACT>(un[i], cc, inv_cc));
+                st_vec<VEC>(A.gk + g + k * S, gk, n);
+            }
         }
     }
     finish_iteration<kLabelThreads>(erru, ctl, A.partials, A.cvg, it, s_red, &s_is_last, A.done_count);
 }
 
-template <bool EXACT>
+template <bool EXACT, bool CARRY>
 __global__ void __launch_bounds__(kLabelThreads) ishikawa_label_kernel(LabelArgs A)
 {
     __shared__ double s_red[kLabelThreads / 32];
@@ -285,8 +324,11 @@ __global__ void __launch_bounds__(kLabelThreads) ishikawa_label_kernel(LabelArgs
             if (k >= 1) {
                 // multiplier of layer k-1: cc*(dv + pt_{k} - pt_{k-1}), new pts
                 const float e = cc * ((dv_below + pt_new) - pt_below);
-                A.u[o - S] = u_below - e;
+                const float un = u_below - e;
+                A.u[o - S] = un;
                 erru += abs_ref(e);
+                if (CARRY)
+                    A.gk[o - S] = dv_below - ((pt_below - pt_new) + div_cc<EXACT>(un, cc, inv_cc));
             }
             pt_below = pt_new;
             dv_below = dv_k;
@@ -299,7 +341,7 @@ __global__ void __launch_bounds__(kLabelThreads) ishikawa_label_kernel(LabelArgs
 
 // The Ishikawa update with VEC voxels per thread: the same per-voxel chain
 // as ishikawa_label_kernel (so the same u bits), wider accesses.
-template <bool EXACT, int VEC>
+template <bool EXACT, int VEC, bool CARRY>
 __global__ void __launch_bounds__(kLabelThreads) ishikawa_label_kernel_v(LabelArgs A)
 {
     __shared__ double s_red[kLabelThreads / 32];
@@ -364,6 +406,14 @@ __global__ void __launch_bounds__(kLabelThreads) ishikawa_label_kernel_v(LabelAr
                         erru += abs_ref(e);
                 }
                 st_vec<VEC>(A.u + o - S, un, n);
+                if constexpr (CARRY) {
+                    float gk[VEC];
+#pragma unroll
+                    for (int i = 0; i < VEC; ++i)
+                        gk[i] = dv_below[i] -
+                                ((pt_below[i] - pt_new[i]) + div_cc<EXACT>(un[i], cc, inv_cc));
+                    st_vec<VEC>(A.gk + o - S, gk, n);
+                }
             }
 #pragma unroll
             for (int i = 0; i < VEC; ++i) {
@@ -386,13 +436,13 @@ int label_kernel_grid(long long cells, int num_sms)
     return (int)(blocks < cap ? blocks : cap);
 }
 
-template <int L, bool EXACT>
+template <int L, bool EXACT, bool CARRY>
 static void potts_launch_l(const LabelArgs &a, int grid, cudaStream_t st, int vec)
 {
     if (vec == 2)
-        potts_label_kernel_v<L, EXACT, 2><<<grid, kLabelThreads, 0, st>>>(a);
+        potts_label_kernel_v<L, EXACT, 2, CARRY><<<grid, kLabelThreads, 0, st>>>(a);
     else
-        potts_label_kernel<L, EXACT><<<grid, kLabelThreads, 0, st>>>(a);
+        potts_label_kernel<L, EXACT, CARRY><<<grid, kLabelThreads, 0, st>>>(a);
 }
 
 // voxels per thread: 2 on rows of 64 and more (a short row would leave
@@ -400,44 +450,45 @@ static void potts_launch_l(const LabelArgs &a, int grid, cudaStream_t st, int ve
 // slower: at 80 registers four 256-thread blocks no longer fit on an SM.
 static int potts_vec(int nr) { return nr >= 64 ? 2 : 1; }
 
-template <bool EXACT>
+template <bool EXACT, bool CARRY>
 static void potts_launch(const LabelArgs &a, int grid, cudaStream_t st)
 {
     const int vec = potts_vec(a.nr);
     switch (a.nlab) {
-    case 2: potts_launch_l<2, EXACT>(a, grid, st, vec); break;
-    case 3: potts_launch_l<3, EXACT>(a, grid, st, vec); break;
-    case 4: potts_launch_l<4, EXACT>(a, grid, st, vec); break;
-    case 5: potts_launch_l<5, EXACT>(a, grid, st, vec); break;
-    case 6: potts_launch_l<6, EXACT>(a, grid, st, vec); break;
-    case 8: potts_launch_l<8, EXACT>(a, grid, st, vec); break;
-    default: potts_label_kernel<0, EXACT><<<grid, kLabelThreads, 0, st>>>(a); break;
+    case 2: potts_launch_l<2, EXACT, CARRY>(a, grid, st, vec); break;
+    case 3: potts_launch_l<3, EXACT, CARRY>(a, grid, st, vec); break;
+    case 4: potts_launch_l<4, EXACT, CARRY>(a, grid, st, vec); break;
+    case 5: potts_launch_l<5, EXACT, CARRY>(a, grid, st, vec); break;
+    case 6: potts_launch_l<6, EXACT, CARRY>(a, grid, st, vec); break;
+    case 8: potts_launch_l<8, EXACT, CARRY>(a, grid, st, vec); break;
+    default: potts_label_kernel<0, EXACT, CARRY><<<grid, kLabelThreads, 0, st>>>(a); break;
     }
 }
 
 cudaError_t launch_potts_labels(const LabelArgs &a, int grid, cudaStream_t st)
 {
     if (a.exact)
-        potts_launch<true>(a, grid, st);
+        a.gk ? potts_launch<true, true>(a, grid, st) : potts_launch<true, false>(a, grid, st);
     else
-        potts_launch<false>(a, grid, st);
+        a.gk ? potts_launch<false, true>(a, grid, st) : potts_launch<false, false>(a, grid, st);
     return cudaGetLastError();
+}
+
+template <bool EXACT, bool CARRY>
+static void ishikawa_launch(const LabelArgs &a, int grid, cudaStream_t st)
+{
+    if (potts_vec(a.nr) == 2)  // the same rule: two voxels on rows of 64+
+        ishikawa_label_kernel_v<EXACT, 2, CARRY><<<grid, kLabelThreads, 0, st>>>(a);
+    else
+        ishikawa_label_kernel<EXACT, CARRY><<<grid, kLabelThreads, 0, st>>>(a);
 }
 
 cudaError_t launch_ishikawa_labels(const LabelArgs &a, int grid, cudaStream_t st)
 {
-    const bool two = potts_vec(a.nr) == 2;  // the same rule: two voxels on rows of 64+
-    if (a.exact) {
-        if (two)
-            ishikawa_label_kernel_v<true, 2><<<grid, kLabelThreads, 0, st>>>(a);
-        else
-            ishikawa_label_kernel<true><<<grid, kLabelThreads, 0, st>>>(a);
-    } else {
-        if (two)
-            ishikawa_label_kernel_v<false, 2><<<grid, kLabelThreads, 0, st>>>(a);
-        else
-            ishikawa_label_kernel<false><<<grid, kLabelThreads, 0, st>>>(a);
-    }
+    if (a.exact)
+        a.gk ? ishikawa_launch<true, true>(a, grid, st) : ishikawa_launch<true, false>(a, grid, st);
+    else
+        a.gk ? ishikawa_launch<false, true>(a, grid, st) : ishikawa_launch<false, false>(a, grid, st);
     return cudaGetLastError();
 }
 

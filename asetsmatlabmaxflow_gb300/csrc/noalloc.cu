@@ -8,7 +8,7 @@
 // For them asets_binary_mf3d_noalloc() runs the same fused iteration kernel as
 // asets_binary_mf3d() but takes every input and output as a device pointer and
 // keeps all of its scratch -- padded inputs, the ping-pong flow and
-// ps/pt/u state, the iteration control block and the erriter partials -- in
+// gk/pt/u state, the iteration control block and the erriter partials -- in
 // one file-scope device array of fixed size.  It calls no cudaMalloc,
 // cudaFree or other allocating routine.
 //
@@ -38,7 +38,7 @@ namespace {
 
 constexpr long long kNoallocMaxCells = 262144;  // padded voxels (row pitch x Nx x Nz)
 constexpr size_t kFieldBytes = (size_t)kNoallocMaxCells * sizeof(float);
-// 3 inputs + 2 parities x (3 flow components + ps + pt + u)
+// 3 inputs + 2 parities x (3 flow components + gradient source + pt + u)
 constexpr size_t kNumFields = 3 + 2 * 6;
 constexpr size_t kControlBytes = 256;
 constexpr int kMaxBlocks = 1024;
@@ -196,11 +196,11 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     unsigned char *base = d->scratch;
     auto field = [&](int i) { return reinterpret_cast<float *>(base + (size_t)i * kFieldBytes); };
     float *cs = field(0), *ct = field(1), *al = field(2);
-    float *b[2][3], *ps[2], *pt[2], *uu[2];
+    float *b[2][3], *gk[2], *pt[2], *uu[2];
     for (int par = 0; par < 2; ++par) {
         for (int k = 0; k < 3; ++k)
             b[par][k] = field(3 + par * 6 + k);
-        ps[par] = field(3 + par * 6 + 3);
+        gk[par] = field(3 + par * 6 + 3);
         pt[par] = field(3 + par * 6 + 4);
         uu[par] = field(3 + par * 6 + 5);
     }
@@ -245,7 +245,7 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     ia.ct = ct;
     ia.alpha = al;
     ia.u = uu[0];
-    ia.ps = ps[0];
+    ia.ps = gk[1];  // used to form the source only; the first iteration overwrites it
     ia.pt = pt[0];
     ia.ctl = ctl;
     ia.cells = cells;
@@ -263,15 +263,42 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
         if (bad)
             return na_fail(ASETS_ERR_ALPHA, "alpha(x) must be positive. Exiting...");
     }
-    NA_TRY(launch_init(0, ia, d->num_sms, sm));
-
-    // kernel variant and arguments (the same fused kernel as the other entry points)
+    // kernel variant (the same fused kernels as the other entry points)
     const int exact = (flags & ASETS_FLAG_EXACT) ? 1 : 0;
     int nv = 0;
     const StencilVariant *tab = stencil_variants(3, EPI_BINARY, exact, &nv);
     const StencilVariant *v = nv > 0 ? &tab[0] : nullptr;
     if (!v)
         return na_fail(ASETS_ERR_UNSUPPORTED, "no kernel variant");
+    if (v->cold && maxIt > 0) {
+        int wide = 0;
+        NA_TRY(launch_check_range(ia, d->num_sms, sm));
+        NA_TRY(cudaMemcpyAsync(&wide, &ctl->wide, sizeof wide, cudaMemcpyDeviceToHost, sm));
+        NA_TRY(cudaStreamSynchronize(sm));
+        if (!wide)
+            v = v->cold;
+    }
+    const bool cold = (v->epi == EPI_COLD && maxIt > 0);
+    CarryArgs ca;
+    memset(&ca, 0, sizeof ca);  // zero flows
+    ca.g = GridGeom{Ny, Nx, Nz, pitch, pitch * Nx, cells};
+    ca.flow_labels = 1;
+    ca.exact = exact;
+    ca.cc = cc;
+    ca.inv_cc = 1.0f / cc;
+    ca.ps = gk[1];
+    ca.pt = pt[0];
+    ca.u = uu[0];
+    ca.cs = cs;
+    ca.ct = ct;
+    ca.gk = gk[0];
+    ca.v_out = pt[0];
+    if (cold) {
+        NA_TRY(launch_cold_source(ca, d->num_sms, sm));
+    } else {
+        NA_TRY(launch_init(0, ia, d->num_sms, sm));
+        NA_TRY(launch_source(0, ca, d->num_sms, sm));
+    }
     StencilProblem p;
     memset(&p, 0, sizeof p);
     p.nr = Ny;
@@ -284,10 +311,10 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     for (int par = 0; par < 2; ++par) {
         for (int k = 0; k < 3; ++k)
             p.b[par][k] = b[par][k];
-        p.src[par][0] = ps[par];
+        p.src[par][0] = gk[par];
         p.src[par][1] = pt[par];
         p.src[par][2] = uu[par];
-        p.dst_s[par][0] = ps[par ^ 1];
+        p.dst_s[par][0] = gk[par ^ 1];
         p.dst_s[par][1] = pt[par ^ 1];
         p.dst_s[par][2] = uu[par ^ 1];
     }
@@ -307,8 +334,8 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     if (per_sm < 1)
         return na_fail(ASETS_ERR_UNSUPPORTED, "the iteration kernel does not fit on an SM");
     const long long slots = (long long)d->num_sms * per_sm;
-    A.zchunks = choose_zchunks(p, *v, slots);
-    const int items = problem_items(p, *v, A.zchunks);
+    choose_split3(p, *v, slots, &A);
+    const int items = split3_items(p, *v, A);
     if (items > kMaxItems)
         return na_fail(ASETS_ERR_INVALID_ARG, "problem splits into %d work items; the "
                        "allocation-free entry point handles at most %d", items, kMaxItems);
@@ -360,6 +387,11 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     if (out.error & DEV_ERR_TIMEOUT)
         return na_fail(ASETS_ERR_TIMEOUT, "a device-side wait timed out");
     const int final_par = (maxIt == 0) ? 0 : ((out.last_iter + 1) & 1);
+    if (cold) {
+        ca.v = pt[final_par];
+        ca.u_out = uu[final_par];
+        NA_TRY(launch_cold_state(ca, d->num_sms, sm));
+    }
     NA_TRY(cudaMemcpy2DAsync(u, (size_t)Ny * 4, uu[final_par], pitch * 4, (size_t)Ny * 4, rows,
                              cudaMemcpyDeviceToDevice, sm));
     NA_TRY(cudaStreamSynchronize(sm));

@@ -125,6 +125,16 @@ struct asets_solver {
     float *b[2][3] = {};
     float *ps[2] = {}, *pt[2] = {}, *u[2] = {};
     float *dv = nullptr;
+    // 3D: the carried gradient source (binary: two parities); ps of the
+    // binary model and pt of Potts are formed on request (flows_stale) with
+    // the last run's cc and exactness
+    float *gk[2] = {};
+    bool flows_stale = false;
+    // cold fast binary 3D runs keep pt and u as v in the place of pt; u is
+    // formed from it on request (u_stale).  cold_ok: the inputs allow it
+    bool cold_state = false, u_stale = false, cold_ok = false;
+    float run_cc = 0.f;
+    int run_exact = 0;
     float *warm_u = nullptr, *warm_ps = nullptr, *warm_pt = nullptr;
     bool warm = false;
     float *warm_b[3] = {nullptr, nullptr, nullptr};  // initial spatial flows (padded)
@@ -151,6 +161,7 @@ struct asets_solver {
     cudaEvent_t flag_ev[2] = {nullptr, nullptr};
     // kernel setup cache: this problem as a batch of one
     const StencilVariant *variant = nullptr;
+    const StencilVariant *picked3[2] = {nullptr, nullptr};  // 3D default, fast and EXACT
     int grid = 0;
     ProblemDesc desc;                  // host copy, uploaded at each run
     ProblemDesc *d_desc = nullptr;
@@ -452,7 +463,47 @@ static constexpr long long kTileLabelsMaxPx = 1LL << 17;
 // EXACT sweep runs one iteration per pass)
 static constexpr double kTileBinaryMaxLoad = 1.0, kTileBinaryMaxLoadExact = 8.0;
 
-static const StencilVariant *pick_variant(const asets_solver *s, int exact, int tile_config,
+// What the work split of a problem depends on.
+static StencilProblem item_geometry(const asets_solver *s)
+{
+    StencilProblem sp;
+    memset(&sp, 0, sizeof sp);
+    sp.nr = s->nr;
+    sp.nc = s->nc;
+    sp.ns = s->ns;
+    sp.flow_labels = s->flow_labels;
+    return sp;
+}
+
+// Cost of a plane step of the 3D kernel with tile width TC, in units of the
+// time a column takes: measured at 64^3 to 256^3, the fast forms' steps take
+// (4 + TC) and the EXACT ones' (10 + TC) to within a few percent (binary
+// fast TC = 12, 13, 16 at 256^3: 0.94, 1.00, 1.21 us; EXACT 1.65, 1.77, 2.02).
+static double step_cost3(const StencilVariant &v) { return (v.exact ? 10.0 : 4.0) + v.tc; }
+
+// 3D: the width whose split (choose_split3) takes the least time.  256^3 is
+// split evenly by 14 columns (19 x 4 tiles x 2 chunks = 152 blocks: 141 us
+// per iteration against 150 with 16 or 13), 192^3 and 128^3 by 16 (Potts
+// 192^3 L = 4: 270 us against 298 with 14), 64^3 takes 12 (15.3 us against
+// 16.5 with 16).
+static const StencilVariant *pick_variant3(const asets_solver *s,
+                                           const std::vector<const StencilVariant *> &match)
+{
+    StencilProblem p = item_geometry(s);
+    ProblemDesc d;
+    const StencilVariant *best = nullptr;
+    double best_cost = 0.0;
+    for (const StencilVariant *v : match) {
+        const double c = choose_split3(p, *v, s->ctx->num_sms, &d) * step_cost3(*v);
+        if (!best || c < best_cost) {
+            best = v;
+            best_cost = c;
+        }
+    }
+    return best;
+}
+
+static const StencilVariant *pick_variant(asets_solver *s, int exact, int tile_config,
                                           bool single)
 {
     std::vector<const StencilVariant *> match = solver_candidates(s, exact, single);
@@ -460,6 +511,12 @@ static const StencilVariant *pick_variant(const asets_solver *s, int exact, int 
         return nullptr;
     if (tile_config > 0 && tile_config <= (int)match.size())
         return match[tile_config - 1];
+    if (s->dim == 3) {
+        const StencilVariant *&v = s->picked3[exact ? 1 : 0];
+        if (!v)
+            v = pick_variant3(s, match);
+        return v;
+    }
     // the one-pass multi-label kernels lead the list: three sweeps (in-step
     // update, one label warp, two), then 16 x 16 tiles (one launch per
     // iteration, the whole solve in one).  By default they run where they
@@ -535,12 +592,16 @@ static StencilProblem stencil_problem_of(const asets_solver *s, bool fused)
         for (int k = 0; k < 3; ++k)
             p.b[par][k] = s->b[par][k];
         if (binary) {
-            p.src[par][0] = s->ps[par];
+            float *const *s0 = s->dim == 3 ? s->gk : s->ps;
+            p.src[par][0] = s0[par];
             p.src[par][1] = s->pt[par];
             p.src[par][2] = s->u[par];
-            p.dst_s[par][0] = s->ps[par ^ 1];
+            p.dst_s[par][0] = s0[par ^ 1];
             p.dst_s[par][1] = s->pt[par ^ 1];
             p.dst_s[par][2] = s->u[par ^ 1];
+        } else if (s->dim == 3) {
+            p.src[par][0] = s->gk[0];
+            p.dst_s[par][0] = s->dv;
         } else if (fused) {
             const int q = par ^ 1;
             const bool potts = (s->model == ASETS_POTTS);
@@ -564,6 +625,8 @@ static StencilProblem stencil_problem_of(const asets_solver *s, bool fused)
     }
     if (binary) {
         p.src_labels[0] = p.src_labels[1] = p.src_labels[2] = 1;
+    } else if (s->dim == 3) {
+        p.src_labels[0] = s->flow_labels;
     } else if (s->model == ASETS_POTTS) {
         p.src_labels[0] = 1;
         p.src_labels[1] = p.src_labels[2] = s->nlab;
@@ -593,6 +656,8 @@ static asets_status setup_kernel(asets_solver *s, int exact, int tile_config, bo
     const StencilVariant *v = pick_variant(s, exact, tile_config, single);
     if (!v)
         return fail(ASETS_ERR_UNSUPPORTED, "no kernel variant for this configuration");
+    if (v->cold && !s->warm && !s->warm_flows && s->cold_ok)
+        v = v->cold;
     if (s->variant == v)
         return ASETS_OK;
     if (v->persistent && persistent_slots(s, v) < 1)
@@ -610,8 +675,11 @@ static asets_status setup_kernel(asets_solver *s, int exact, int tile_config, bo
     if (per_sm < 1)
         return fail(ASETS_ERR_UNSUPPORTED, "stencil kernel does not fit on an SM");
     const long long slots = (long long)s->ctx->num_sms * per_sm;
-    A.zchunks = choose_zchunks(p, *v, slots);
-    const int items = problem_items(p, *v, A.zchunks);
+    if (s->dim == 3)
+        choose_split3(p, *v, slots, &A);
+    else
+        A.zchunks = choose_zchunks(p, *v, slots);
+    const int items = s->dim == 3 ? split3_items(p, *v, A) : problem_items(p, *v, A.zchunks);
     A.item_begin = 0;
     A.n_items = items;
     s->grid = (int)std::max<long long>(1, std::min<long long>(items, slots));
@@ -737,17 +805,31 @@ extern "C" ASETS_API asets_status asets_solver_create(asets_context *ctx, asets_
     }
     if (model == ASETS_BINARY) {
         for (int par = 0; par < 2; ++par) {
-            ALLOC(s->ps[par], n);
+            if (dim == 3)
+                ALLOC(s->gk[par], n);
+            if (dim == 2 || par == 0)
+                ALLOC(s->ps[par], n);
             ALLOC(s->pt[par], n);
             ALLOC(s->u[par], n);
         }
+        if (dim == 3)
+            s->ps[1] = s->ps[0];
     } else {
         if (model == ASETS_POTTS)
             ALLOC(s->ps[0], n);
         ALLOC(s->pt[0], n * s->pt_labels);
         ALLOC(s->u[0], n * s->u_labels);
         ALLOC(s->dv, n * s->flow_labels);
-        if (dim == 2 && fused2d_variant((int)model, nLab, 0)) {
+        if (dim == 3) {
+            ALLOC(s->gk[0], n * s->flow_labels);
+            s->pt[1] = s->pt[0];
+            if (model == ASETS_POTTS) {
+                ALLOC(s->ps[1], n);
+                ALLOC(s->u[1], n * s->u_labels);
+            } else {
+                s->u[1] = s->u[0];
+            }
+        } else if (fused2d_variant((int)model, nLab, 0)) {
             // the one-pass kernel writes the new state to a second parity
             if (model == ASETS_POTTS)
                 ALLOC(s->ps[1], n);
@@ -827,6 +909,77 @@ static InitArgs init_args(asets_solver *s)
     return a;
 }
 
+static GridGeom geom_of(const asets_solver *s)
+{
+    GridGeom g;
+    g.nr = s->nr;
+    g.nc = s->nc;
+    g.ns = s->ns;
+    g.pitch = s->pitch;
+    g.plane = s->plane;
+    g.cells = s->cells;
+    return g;
+}
+
+// Arguments of the carried-state passes (carry3d.cu) on the spatial flows of
+// parity `fp` and u/ps/pt of parity `sp`.
+static CarryArgs carry_args(const asets_solver *s, int fp, int sp, float cc, int exact)
+{
+    CarryArgs a;
+    memset(&a, 0, sizeof a);
+    a.g = geom_of(s);
+    a.flow_labels = s->flow_labels;
+    a.exact = exact;
+    a.cc = cc;
+    a.inv_cc = 1.0f / cc;
+    a.bc = s->b[fp][SL_BC];
+    a.br = s->b[fp][SL_BR];
+    a.bs = s->b[fp][SL_BS];
+    a.ps = s->ps[sp];
+    a.pt = s->pt[sp];
+    a.u = s->u[sp];
+    a.cs = s->cs;
+    a.ct = s->ct;
+    a.dv = s->dv;
+    return a;
+}
+
+// Form the final u if the last run has left it unformed (cold binary 3D).
+static asets_status ensure_u(asets_solver *s)
+{
+    if (!s->u_stale)
+        return ASETS_OK;
+    CarryArgs a = carry_args(s, s->flow_parity, s->final_parity, s->run_cc, s->run_exact);
+    a.v = s->pt[s->final_parity];
+    a.u_out = s->u[s->final_parity];
+    CU_TRY(launch_cold_state(a, s->ctx->num_sms, s->ctx->stream));
+    s->u_stale = false;
+    return ASETS_OK;
+}
+
+// 3D: form the final ps (binary; of a cold run pt as well) or pt (Potts) if
+// the last run has left it unformed.  Called before it is read and before
+// the inputs it is formed from are overwritten.
+static asets_status ensure_flows(asets_solver *s)
+{
+    asets_status st = ensure_u(s);
+    if (st != ASETS_OK || !s->flows_stale)
+        return st;
+    const int sms = s->ctx->num_sms, fp = s->final_parity;
+    CarryArgs a = carry_args(s, s->flow_parity, fp ^ 1, s->run_cc, s->run_exact);
+    a.out = s->model == ASETS_BINARY ? s->ps[0] : s->pt[0];
+    if (s->cold_state)
+        a.v = s->pt[fp];
+    CU_TRY(launch_flows((int)s->model, a, sms, s->ctx->stream));
+    if (s->cold_state) {
+        a.pt_out = s->pt[fp];
+        CU_TRY(launch_cold_state(a, sms, s->ctx->stream));
+        s->cold_state = false;
+    }
+    s->flows_stale = false;
+    return ASETS_OK;
+}
+
 extern "C" ASETS_API asets_status asets_solver_set_inputs(asets_solver *s, asets_memory where,
                                                           const float *Cs, const float *Ct,
                                                           const float *alpha)
@@ -837,6 +990,9 @@ extern "C" ASETS_API asets_status asets_solver_set_inputs(asets_solver *s, asets
         return fail(ASETS_ERR_INVALID_ARG, "missing input array");
     std::lock_guard<std::recursive_mutex> lock(s->ctx->mu);
     DeviceGuard guard(s->ctx->device);
+    asets_status fs = ensure_flows(s);
+    if (fs != ASETS_OK)
+        return fs;
     if (s->model == ASETS_BINARY)
         CU_TRY(copy_in(s, s->cs, Cs, 1, where));
     CU_TRY(copy_in(s, s->ct, Ct, s->ct_labels, where));
@@ -848,11 +1004,13 @@ extern "C" ASETS_API asets_status asets_solver_set_inputs(asets_solver *s, asets
     CU_TRY(cudaMemcpyAsync(s->ctl, &zero, sizeof zero, cudaMemcpyHostToDevice, s->ctx->stream));
     InitArgs a = init_args(s);
     CU_TRY(launch_validate_alpha(a, s->ctx->num_sms, s->ctx->stream));
-    int bad = 0;
-    CU_TRY(cudaMemcpyAsync(&bad, &s->ctl->alpha_bad, sizeof(int), cudaMemcpyDeviceToHost,
-                           s->ctx->stream));
+    if (s->model == ASETS_BINARY && s->dim == 3)
+        CU_TRY(launch_check_range(a, s->ctx->num_sms, s->ctx->stream));
+    IterControl checked;
+    CU_TRY(cudaMemcpyAsync(&checked, s->ctl, sizeof checked, cudaMemcpyDeviceToHost, s->ctx->stream));
     CU_TRY(cudaStreamSynchronize(s->ctx->stream));
-    s->alpha_ok = (bad == 0);
+    s->alpha_ok = (checked.alpha_bad == 0);
+    s->cold_ok = (checked.wide == 0);
     s->inputs_set = true;
     return ASETS_OK;
 }
@@ -1003,6 +1161,11 @@ static LabelArgs label_args(asets_solver *s)
     a.u = s->u[0];
     a.pt = s->pt[0];
     a.ps = s->ps[0];
+    if (s->dim == 3) {
+        a.u1 = s->u[1];
+        a.ps1 = s->ps[1];
+        a.gk = s->gk[0];
+    }
     a.dv = s->dv;
     a.ct = s->ct;
     a.ctl = s->ctl;
@@ -1085,9 +1248,23 @@ static asets_status prepare_run(asets_solver *s, int flags, int tile_config, int
         if (s->warm_ps)
             CU_TRY(cudaMemcpyAsync(s->ps[0], s->warm_ps, n * sizeof(float),
                                    cudaMemcpyDeviceToDevice, st));
-    } else {
+    } else if (s->variant->epi != EPI_COLD || maxIt == 0) {
         InitArgs ia = init_args(s);
         CU_TRY(launch_init((int)s->model, ia, s->ctx->num_sms, st));
+    }
+    s->flows_stale = s->u_stale = s->cold_state = false;
+    if (s->dim == 3) {
+        CarryArgs ca = carry_args(s, 0, 0, cc, exact);
+        if (!s->warm_flows)
+            ca.br = nullptr;  // zero flows
+        ca.gk = s->gk[0];
+        ca.v_out = s->pt[0];
+        if (s->variant->epi != EPI_COLD)
+            CU_TRY(launch_source((int)s->model, ca, s->ctx->num_sms, st));
+        else if (maxIt > 0)
+            CU_TRY(launch_cold_source(ca, s->ctx->num_sms, st));
+        s->run_cc = cc;
+        s->run_exact = exact;
     }
     s->last_max_it = maxIt;
     return ASETS_OK;
@@ -1191,9 +1368,13 @@ static asets_status finish_run(asets_solver *s, const IterControl &out, int *itN
                            ? (((out.last_iter >> 1) & 1) ^ 1)
                            : ((out.last_iter + 1) & 1);
     // the two-pass multi-label form keeps pt/u/ps in place (parity 0)
-    const bool pingpong = (s->model == ASETS_BINARY) || (s->variant && s->variant->epi == EPI_FUSED);
+    // (in 3D the arrays kept in place have the same buffer for both parities)
+    const bool pingpong = s->dim == 3 || (s->model == ASETS_BINARY) ||
+                          (s->variant && s->variant->epi == EPI_FUSED);
     s->final_parity = pingpong ? parity : 0;
     s->flow_parity = parity;
+    s->flows_stale = s->dim == 3 && s->model != ASETS_ISHIKAWA && out.last_iter >= 0;
+    s->cold_state = s->u_stale = s->flows_stale && s->variant->epi == EPI_COLD;
     if (itNum)
         *itNum = (maxIt == 0) ? 0 : out.it_num;
     return ASETS_OK;
@@ -1449,6 +1630,9 @@ extern "C" ASETS_API asets_status asets_solver_get_u(asets_solver *s, asets_memo
         return fail(ASETS_ERR_INVALID_ARG, "NULL argument");
     std::lock_guard<std::recursive_mutex> lock(s->ctx->mu);
     DeviceGuard guard(s->ctx->device);
+    asets_status us = ensure_u(s);
+    if (us != ASETS_OK)
+        return us;
     CU_TRY(copy_out(s, u, s->u[s->final_parity], s->u_labels, where));
     CU_TRY(cudaStreamSynchronize(s->ctx->stream));
     return ASETS_OK;
@@ -1481,6 +1665,9 @@ extern "C" ASETS_API asets_status asets_solver_get_flows(asets_solver *s, asets_
         return fail(ASETS_ERR_INVALID_ARG, "NULL solver");
     std::lock_guard<std::recursive_mutex> lock(s->ctx->mu);
     DeviceGuard guard(s->ctx->device);
+    asets_status fs = ensure_flows(s);
+    if (fs != ASETS_OK)
+        return fs;
     if (ps) {
         if (s->model == ASETS_ISHIKAWA)
             return fail(ASETS_ERR_INVALID_ARG, "the Ishikawa model has no source flow");
@@ -1493,18 +1680,6 @@ extern "C" ASETS_API asets_status asets_solver_get_flows(asets_solver *s, asets_
 }
 
 // ---------------------------------------------------------------- multilevel
-
-static GridGeom geom_of(const asets_solver *s)
-{
-    GridGeom g;
-    g.nr = s->nr;
-    g.nc = s->nc;
-    g.ns = s->ns;
-    g.pitch = s->pitch;
-    g.plane = s->plane;
-    g.cells = s->cells;
-    return g;
-}
 
 // Extend the chain of coarse solvers to `levels` levels where the grid
 // allows (every coarse axis keeps at least kMinCoarseCells cells) and
@@ -1527,6 +1702,9 @@ static asets_status ml_prepare(asets_solver *s, int levels, int *built)
             cur->coarse = c;
         }
         asets_solver *c = cur->coarse;
+        asets_status fs = ensure_flows(c);
+        if (fs != ASETS_OK)
+            return fs;
         GridXfer X;
         X.f = geom_of(cur);
         X.c = geom_of(c);
@@ -1538,6 +1716,7 @@ static asets_status ml_prepare(asets_solver *s, int levels, int *built)
         CU_TRY(launch_restrict(X, cur->alpha, c->alpha, cur->alpha_labels, 1.f, sms, stm));
         c->inputs_set = true;
         c->alpha_ok = cur->alpha_ok;
+        c->cold_ok = cur->cold_ok;
         cur = c;
         ++n;
     }
@@ -1550,7 +1729,9 @@ static asets_status ml_prolong(asets_solver *c, asets_solver *f)
 {
     const size_t n = (size_t)f->cells;
     const bool has_ps = (f->model != ASETS_ISHIKAWA);
-    asets_status st;
+    asets_status st = ensure_flows(c);
+    if (st != ASETS_OK)
+        return st;
     if (!f->warm_u) {
         if ((st = dalloc(f, &f->warm_u, n * f->u_labels)) != ASETS_OK)
             return st;
@@ -1706,7 +1887,9 @@ struct asets_batch {
         BatchArgs bargs;
         int grid = 0;
         int tile_config = 0;
-    } groups[4];  // [0] binary 2D, [1] binary 3D, [2] labelled 2D, [3] labelled 3D
+    } groups[5];  // [0] binary 2D, [1] binary 3D, [2] labelled 2D, [3] labelled 3D,
+                  // [4] binary 3D members of a fast batch that cannot take the
+                  // cold start's kernel
     unsigned int *d_done = nullptr;
     IterControl **d_ctls = nullptr;  // every member's control block
     int *d_member_done = nullptr;    // gathered done flags
@@ -1721,8 +1904,11 @@ struct asets_batch {
 };
 
 // done counter, then three queue words per group
-static constexpr int kBatchCounters = 16;
+static constexpr int kBatchGroups = 5, kBatchCounters = 4 + 3 * kBatchGroups;
 
+static constexpr int kWarmGroup = 4;
+
+// The group a member's tile configuration belongs to.
 static int batch_group(const asets_solver *s)
 {
     return (s->dim == 3 ? 1 : 0) + (s->model == ASETS_BINARY ? 0 : 2);
@@ -1740,7 +1926,7 @@ extern "C" ASETS_API asets_status asets_batch_create(asets_context *ctx, asets_b
     CU_TRY(cudaMalloc(&p, kBatchCounters * sizeof(unsigned int)));
     b->allocations.push_back(p);
     b->d_done = static_cast<unsigned int *>(p);
-    for (int g = 0; g < 4; ++g)
+    for (int g = 0; g < kBatchGroups; ++g)
         b->groups[g].d_queue = b->d_done + 4 + 3 * g;
     CU_TRY(cudaEventCreate(&b->ev0));
     CU_TRY(cudaEventCreate(&b->ev1));
@@ -1809,17 +1995,6 @@ static asets_status batch_buffer(asets_batch *b, void **p, size_t bytes)
     return ASETS_OK;
 }
 
-static StencilProblem item_geometry(const asets_solver *s)
-{
-    StencilProblem sp;
-    memset(&sp, 0, sizeof sp);
-    sp.nr = s->nr;
-    sp.nc = s->nc;
-    sp.ns = s->ns;
-    sp.flow_labels = s->flow_labels;
-    return sp;
-}
-
 // Stream-axis chunk counts for the problems of one launch: one common chunk
 // length (planes per item) for all of them, the one with the best
 // (wave fill of `slots` resident blocks) x (useful planes / swept planes,
@@ -1882,6 +2057,7 @@ static asets_status batch_layout(asets_batch *b, asets_batch::Group &g)
         // solve of the member alone uploads as it is.
         ProblemDesc d = s->desc;
         d.zchunks = zc[j];
+        d.units_a = 0;
         const int items = problem_items(item_geometry(s), *g.v, d.zchunks);
         asets_status st = ensure_items(s, items);
         if (st != ASETS_OK)
@@ -1925,7 +2101,7 @@ static asets_status batch_layout(asets_batch *b, asets_batch::Group &g)
 
 static cudaError_t batch_launch_iteration(asets_batch *b)
 {
-    for (int gi = 0; gi < 4; ++gi) {
+    for (int gi = 0; gi < kBatchGroups; ++gi) {
         auto &g = b->groups[gi];
         if (g.live.empty())
             continue;
@@ -1934,7 +2110,7 @@ static cudaError_t batch_launch_iteration(asets_batch *b)
                                          g.v->smem_bytes, b->ctx->stream);
         if (e != cudaSuccess)
             return e;
-        if (gi < 2)
+        if (gi < 2 || gi == kWarmGroup)
             continue;
         // labelled models: each problem's label kernel closes its iteration
         // (it returns at once for a finished problem) and counts it when done
@@ -1964,14 +2140,16 @@ static asets_status batch_prepare(asets_batch *b, int flags, const int tile_conf
         asets_solver *s = b->members[i];
         if (!s->inputs_set)
             return fail(ASETS_ERR_INVALID_ARG, "batch member %zu has no inputs", i);
-        const int gi = batch_group(s);
+        int gi = batch_group(s);
         asets_status st =
             prepare_run(s, flags, tile_config[gi], maxIt, errBound, cc, steps, false);
         if (st != ASETS_OK)
             return st;
+        if (s->variant->cold)
+            gi = kWarmGroup;  // another kernel than the cold members'
         b->groups[gi].idx.push_back((int)i);
         b->groups[gi].v = s->variant;
-        b->groups[gi].tile_config = tile_config[gi];
+        b->groups[gi].tile_config = tile_config[batch_group(s)];
     }
     cudaStream_t st = b->ctx->stream;
     CU_TRY(cudaMemsetAsync(b->d_done, 0, kBatchCounters * sizeof(unsigned int), st));
@@ -2050,9 +2228,9 @@ static asets_status batch_relayout(asets_batch *b, bool *changed)
 static int batch_launches_per_iter(const asets_batch *b)
 {
     int n = 0;
-    for (int gi = 0; gi < 4; ++gi)
+    for (int gi = 0; gi < kBatchGroups; ++gi)
         if (!b->groups[gi].live.empty())
-            n += 1 + (gi >= 2 ? (int)b->groups[gi].live.size() : 0);
+            n += 1 + (gi >= 2 && gi != kWarmGroup ? (int)b->groups[gi].live.size() : 0);
     return n;
 }
 
@@ -2103,6 +2281,28 @@ static asets_status batch_execute(asets_batch *b, int maxIt, int *chunks, int *l
     if (launches)
         *launches = kernels;
     return ASETS_OK;
+}
+
+// Default 3D variant of a batch group (tile_config): the tile width with the
+// least sum of the members' tiles x planes x time per step.
+static int batch_width3(const asets_batch *b, int gi, int exact)
+{
+    int n = 0;
+    const StencilVariant *tab = stencil_variants(3, gi >= 2 ? EPI_DIV : EPI_BINARY, exact, &n);
+    int best = 1;
+    double best_cost = 0.0;
+    for (int i = 0; i < n; ++i) {
+        double cost = 0.0;
+        for (const asets_solver *s : b->members)
+            if (batch_group(s) == gi)
+                cost += (double)problem_items(item_geometry(s), tab[i], 1) * s->ns;
+        cost *= step_cost3(tab[i]);
+        if (i == 0 || cost < best_cost) {
+            best = i + 1;
+            best_cost = cost;
+        }
+    }
+    return best;
 }
 
 // Tile configuration per dimension group, chosen by timing each candidate
@@ -2190,9 +2390,13 @@ extern "C" ASETS_API asets_status asets_batch_run(asets_batch *b, const asets_op
     DeviceGuard guard(b->ctx->device);
     NvtxRange nv("asets_batch_run");
     cudaStream_t st = b->ctx->stream;
-    // one kernel variant per dimension group (default: the first)
+    // one kernel variant per dimension group (default: the first; 3D: the
+    // tile width that sweeps the members in the least time)
     const int tc0 = (opt && opt->tile_config > 0) ? opt->tile_config : 1;
     int tile_config[4] = {tc0, tc0, tc0, tc0};
+    if (!(opt && opt->tile_config > 0))
+        for (int gi = 1; gi < 4; gi += 2)
+            tile_config[gi] = batch_width3(b, gi, (flags & ASETS_FLAG_EXACT) ? 1 : 0);
     if ((flags & ASETS_FLAG_AUTOTUNE) && maxIt > 0) {
         asets_status ts = batch_autotune(b, flags, cc, steps, tile_config);
         if (ts != ASETS_OK)
@@ -2383,6 +2587,7 @@ static asets_status one_shot(asets_context *ctx, const asets_options *opt, asets
         ctx->cached = s;
     }
     s->warm = false;
+    s->flows_stale = s->u_stale = false;  // no one reads the state of the previous call
     asets_status st = asets_solver_set_inputs(s, ASETS_HOST, Cs, Ct, alpha);
     if (st != ASETS_OK)
         return st;

@@ -1,4 +1,4 @@
-// Fused ALM iteration kernel, column-per-thread form: one launch = one
+// Fused 2D ALM iteration kernel, row-per-thread form: one launch = one
 // iteration of the continuous max-flow solver (all labels of a labelled
 // model).
 //
@@ -6,21 +6,19 @@
 // updateBX/BY/BZ and divergence sweeps (maxflow/asetsBinaryMF3D_mex.c:166-180)
 // and, for the binary model, updateDIVPSPTU and the erriter sum (:398-437).
 //
-// Geometry.  Rows r (Matlab y, contiguous), columns c (Matlab x in 3D) and a
-// stream axis s (z in 3D, x in 2D).  Each warp owns 32*CELLS consecutive
-// rows: 32*CELLS - 4 tile rows plus two halo rows on each side.  In 3D warp
-// w is column c0 - 2 + w of a (32*CELLS - 4) x (NW-4) tile; in 2D the NW
-// warps are consecutive (32*CELLS - 4)-row sub-tiles.  Every thread owns
-// CELLS adjacent rows (1 or 2) of one column for the whole sweep along s, so
-// its indices, border flags and carried values stay in registers; row
-// neighbours come from the thread itself or, for its first and last cell,
-// through one warp shuffle, column neighbours through three small shared
-// planes.  With two cells the shared-memory and global accesses are 8-byte
-// pairs, and the per-step index, flag and barrier work is shared by both.  One iteration has a stencil radius of two cells, so
-// step s computes
+// The 2D form (3D: stencil3d_kernel.cuh).  Geometry: rows r (Matlab y,
+// contiguous) and a stream axis s (Matlab x).  Each warp owns 32*CELLS
+// consecutive rows: 32*CELLS - 4 tile rows plus two halo rows on each side;
+// the NW warps of a block are consecutive sub-tiles.  Every thread owns CELLS
+// adjacent rows (1 or 2) for the whole sweep along s, so its indices, border
+// flags and carried values stay in registers; row neighbours come from the
+// thread itself or, for its first and last cell, through one warp shuffle.
+// With two cells the shared-memory and global accesses are 8-byte pairs, and
+// the per-step index, flag and barrier work is shared by both.  One iteration
+// has a stencil radius of two cells, so step s computes
 //   X: gk(s) = div b(s) - ((s0 - s1) + s2/cc)               all threads
 //   Y: gradient step b'(s); projection g2(s-1); b''_s(s-1)   tile + 1
-//   Z: b''_r, b''_c of plane s-1; ps/pt/u (or div) of s-2    tile
+//   Z: b''_r of plane s-1; ps/pt/u (or div) of s-2           tile
 // with two block barriers per step.  Old-state planes come through a ring of
 // 4D TMA tiled loads; a stage holds the halo boxes of its plane and, for the
 // binary model, tile boxes of pt/u/Cs/Ct three planes behind: step t reads
@@ -46,24 +44,18 @@
 
 namespace asets {
 
-template <int DIM, int NW, int CELLS = 1>
+template <int NW, int CELLS = 1>
 struct ColGeom {
-    static_assert(DIM == 2 || DIM == 3, "2D or 3D");
     static_assert(CELLS == 1 || CELLS == 2, "one or two cells per thread");
     static constexpr int NT = 32 * NW;
     static constexpr int TRW = 32 * CELLS - 4;                // tile rows per warp
-    static constexpr int TR = (DIM == 3) ? TRW : TRW * NW;    // tile rows
-    static constexpr int TC = (DIM == 3) ? NW - 4 : 1;        // tile columns
-    static_assert(DIM == 2 || NW >= 5, "3D needs at least one tile column");
+    static constexpr int TR = TRW * NW;                       // tile rows
     static constexpr int LR = TR + 8;                         // halo box rows (origin r0-4)
     static_assert(LR <= 256, "TMA box dimension limit");
-    static constexpr int LC = (DIM == 3) ? TC + 4 : 1;        // halo box columns (origin c0-2)
-    static constexpr int LC_BC = (DIM == 3) ? TC + 5 : 1;     // column-face box (+forward face)
-
     static constexpr int align128(int b) { return (b + 127) & ~127; }
-    static constexpr int halo_floats(int slot) { return slot == SL_BC ? LR * LC_BC : LR * LC; }
-    static constexpr int tile_floats() { return TR * TC; }
-    static constexpr bool has_slot(int slot) { return !(DIM == 2 && slot == SL_BC); }
+    static constexpr int halo_floats(int) { return LR; }
+    static constexpr int tile_floats() { return TR; }
+    static constexpr bool has_slot(int slot) { return slot != SL_BC; }  // no column axis
     template <int EPI>
     static constexpr int stage_bytes()
     {
@@ -86,12 +78,11 @@ struct ColGeom {
             b += NUM_TILE_SLOTS * tile_floats() * 4;
         return b;
     }
-    static constexpr int plane_bytes() { return (DIM == 3) ? align128(NT * CELLS * 4) : 0; }
     template <int NSTAGE, int EPI>
     static constexpr int smem_bytes()
     {
-        // stages | GK | BC | G2 | mbarriers | alignment slack
-        return NSTAGE * stage_bytes<EPI>() + 3 * plane_bytes() + NSTAGE * 8 + 128;
+        // stages | mbarriers | alignment slack
+        return NSTAGE * stage_bytes<EPI>() + NSTAGE * 8 + 128;
     }
 };
 
@@ -237,15 +228,11 @@ __device__ __forceinline__ void finish_item(float erru, const ProblemDesc &P, in
     __syncthreads();
 }
 
-// LATE: the producer issues the refill at the start of Z instead of right
-// after the X barrier.  In 3D its warp is a halo column, which has no
-// epilogue work in Z, so the issue leaves the Y barrier's critical path.
-template <int DIM, int NW, int NSTAGE, int EPI, bool EXACT, int MINB, int UNROLL = 1, int CELLS = 1,
-          bool LATE = false>
+template <int NW, int NSTAGE, int EPI, bool EXACT, int MINB, int UNROLL = 1, int CELLS = 1>
 __global__ void __launch_bounds__(32 * NW, MINB)
     stencil_col_kernel(const __grid_constant__ BatchArgs B)
 {
-    using G = ColGeom<DIM, NW, CELLS>;
+    using G = ColGeom<NW, CELLS>;
     constexpr int NT = G::NT;
     constexpr int C = CELLS;
     static_assert(NSTAGE >= 4, "stage of plane s stays resident until step s ends");
@@ -277,8 +264,7 @@ __global__ void __launch_bounds__(32 * NW, MINB)
         return reinterpret_cast<float *>(smem + off);
     };
     // float offsets of each slot inside a stage (compile-time constants)
-    constexpr int OFF_BC = 0;
-    constexpr int OFF_BR = OFF_BC + (G::has_slot(SL_BC) ? G::align128(G::halo_floats(SL_BC) * 4) / 4 : 0);
+    constexpr int OFF_BR = 0;
     constexpr int OFF_BS = OFF_BR + G::align128(G::halo_floats(SL_BR) * 4) / 4;
     constexpr int OFF_S0 = OFF_BS + G::align128(G::halo_floats(SL_BS) * 4) / 4;
     constexpr int OFF_S1 = OFF_S0 + G::align128(G::halo_floats(SL_S0) * 4) / 4;
@@ -287,15 +273,7 @@ __global__ void __launch_bounds__(32 * NW, MINB)
     constexpr int OFF_T0 = OFF_AL + G::align128(G::halo_floats(SL_ALPHA) * 4) / 4;
     constexpr int TSZ = G::align128(G::tile_floats() * 4) / 4;
     const float *stages = reinterpret_cast<const float *>(smem);
-    float *planes = reinterpret_cast<float *>(smem + NSTAGE * SB);
-    constexpr int PF = G::plane_bytes() / 4;
-    // shared planes: gk, the column faces b'_c (one buffer: the neighbour's
-    // previous face is read in X, before the barrier that precedes this
-    // step's write in Y) and the projection factors g2
-    float *GK = planes;
-    float *BCp = planes + PF;
-    float *G2p = planes + 2 * PF;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + NSTAGE * SB + 3 * G::plane_bytes());
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + NSTAGE * SB);
 
     if (tid == 0) {
         s_abort = 0;
@@ -307,15 +285,11 @@ __global__ void __launch_bounds__(32 * NW, MINB)
 
     // per-thread constants; the thread's cells are rows rho .. rho+C-1 of
     // its warp's 32*C rows (two halo rows on each side)
-    const int rho = (DIM == 3) ? C * lane : G::TRW * w + C * lane;   // first cell's row index
-    const int si = rho + 2 + ((DIM == 3) ? w * G::LR : 0);            // halo box index
-    const int gi = (lane + 32 * w) * C;                               // shared plane index (3D)
-    const int gi_left = (w >= 1) ? gi - 32 * C : gi;                  // column c-1 (clamped)
-    const int gi_right = (w + 1 < NW) ? gi + 32 * C : gi;             // column c+1 (clamped)
+    const int rho = G::TRW * w + C * lane;                            // first cell's row index
+    const int si = rho + 2;                                           // halo box index
     const int lane_row = C * lane;                                    // row within the warp
     const bool tile_row = (lane_row >= 2 && lane_row < 32 * C - 2);
-    const bool tile_col = (DIM == 3) ? (w >= 2 && w < G::TC + 2) : true;
-    const int ti = (DIM == 3) ? (lane_row - 2) + (w - 2) * G::TRW : (rho - 2);
+    const int ti = rho - 2;
     // The thread that issues the TMA loads and waits on their barriers; the
     // other threads block in the following CTA barrier instead of polling.
     const bool producer = (tid == NT - 32);
@@ -350,7 +324,7 @@ __global__ void __launch_bounds__(32 * NW, MINB)
         const int par = it & 1;
         const CUtensorMap *hmaps = P.halo[par];
         const CUtensorMap *tmaps = P.tile[par];
-        const int nr = P.nr, nc = P.nc, ns = P.ns;
+        const int nr = P.nr, ns = P.ns;
         const float cc = P.cc, inv_cc = P.inv_cc, steps = P.steps;
         const int tiles = P.tiles_r * P.tiles_c;
         const int li = item - P.item_begin;
@@ -363,7 +337,6 @@ __global__ void __launch_bounds__(32 * NW, MINB)
         const int s_end = (int)((long long)ns * (chunk + 1) / P.zchunks);
         float erru = 0.0f;
         const int r0 = (tile % P.tiles_r) * G::TR;
-        const int c0 = (DIM == 3) ? (tile / P.tiles_r) * G::TC : 0;
         const int n_steps = s_end - s_begin + 4;
         const int n_loads = n_steps + 1;
         const int p_first = s_begin - 2;
@@ -383,62 +356,48 @@ __global__ void __launch_bounds__(32 * NW, MINB)
             for (int s = 0; s < NUM_SLOTS; ++s) {
                 if (!G::has_slot(s))
                     continue;
-                tma_load_4d(halo_slot(st, s), &hmaps[s], r0 - 4, (DIM == 3) ? c0 - 2 : 0, plane,
-                            lab_coord[s], &bars[st]);
+                tma_load_4d(halo_slot(st, s), &hmaps[s], r0 - 4, 0, plane, lab_coord[s], &bars[st]);
             }
             if constexpr (EPI == EPI_BINARY) {
 #pragma unroll
                 for (int ts = 0; ts < NUM_TILE_SLOTS; ++ts)
-                    tma_load_4d(tile_slot(st, ts), &tmaps[ts], r0, c0, plane - 3, 0, &bars[st]);
+                    tma_load_4d(tile_slot(st, ts), &tmaps[ts], r0, 0, plane - 3, 0, &bars[st]);
             }
         };
         if (producer)
             for (int j = 0; j < NSTAGE && j < n_loads; ++j)
                 issue_load(j);
 
-        // this thread's cells (rows r .. r+C-1 of column c)
+        // this thread's cells (rows r .. r+C-1)
         const int r = r0 - 2 + rho;
-        const int c = (DIM == 3) ? c0 - 2 + w : 0;
-        const bool in_c = (c >= 0 && c < nc);
-        bool inplane[C], is_tile[C], fr_ok[C], fr1_ok[C], fc_ok[C], fc1_ok[C];
-        float fr_f[C], fr1_f[C], fc_f[C], fc1_f[C];
+        bool inplane[C], is_tile[C], fr_ok[C], fr1_ok[C];
+        float fr_f[C], fr1_f[C];
 #pragma unroll
         for (int j = 0; j < C; ++j) {
             const int rj = r + j;
-            const bool in_r = (rj >= 0 && rj < nr);
-            inplane[j] = in_r && in_c;
-            is_tile[j] = tile_row && tile_col && inplane[j];
-            fr_ok[j] = (rj >= 1 && rj < nr && in_c);            // row face rj
-            fr1_ok[j] = (rj + 1 >= 1 && rj + 1 < nr && in_c);   // row face rj+1
-            fc_ok[j] = (in_r && c >= 1 && c < nc);
-            fc1_ok[j] = (in_r && c + 1 >= 1 && c + 1 < nc);
+            inplane[j] = (rj >= 0 && rj < nr);
+            is_tile[j] = tile_row && inplane[j];
+            fr_ok[j] = (rj >= 1 && rj < nr);            // row face rj
+            fr1_ok[j] = (rj + 1 >= 1 && rj + 1 < nr);   // row face rj+1
             fr_f[j] = fr_ok[j] ? 1.f : 0.f;
             fr1_f[j] = fr1_ok[j] ? 1.f : 0.f;
-            fc_f[j] = fc_ok[j] ? 1.f : 0.f;
-            fc1_f[j] = fc1_ok[j] ? 1.f : 0.f;
         }
         // element offsets fit 32 bits: solves are limited to 2^31 - 1 voxel-labels
-        const unsigned int col_off = (unsigned int)(lab_off + (long long)c * P.pitch + r);
+        const unsigned int col_off = (unsigned int)(lab_off + r);
         const unsigned int plane_stride = (unsigned int)P.plane_stride;
-        // halo-box reads si .. si+C (the row face below the last cell), in 3D
-        // the column faces of the next column si+LR .. si+LR+C-1; tile-box
-        // reads ti .. ti+C-1; shared-plane reads gi .. gi+C-1
-        check_index(si + C, G::LR * G::LC, P);
-        if constexpr (DIM == 3)
-            check_index(si + G::LR + C - 1, G::LR * G::LC_BC, P);
+        // halo-box reads si .. si+C (the row face below the last cell);
+        // tile-box reads ti .. ti+C-1
+        check_index(si + C, G::LR, P);
         if (is_tile[0])
             check_index(ti + C - 1, G::tile_floats(), P);
-        if constexpr (DIM == 3)
-            check_index(gi + C - 1, NT * C, P);
         float *__restrict__ d_bs = P.dst_b[par][SL_BS];
         float *__restrict__ d_br = P.dst_b[par][SL_BR];
-        float *__restrict__ d_bc = P.dst_b[par][SL_BC];
         float *__restrict__ d_s0 = P.dst_s[par][0];
         float *__restrict__ d_s1 = P.dst_s[par][1];
         float *__restrict__ d_s2 = P.dst_s[par][2];
 
         float gkprev[C], bsprev[C], g2prev[C], alpha_prev[C];
-        float br_prev[C], bc_prev[C], bss_cur[C], bss_old[C], dvp[C];
+        float br_prev[C], bss_cur[C], bss_old[C], dvp[C];
 #pragma unroll
         for (int j = 0; j < C; ++j) {
             gkprev[j] = 0.f;
@@ -446,7 +405,6 @@ __global__ void __launch_bounds__(32 * NW, MINB)
             g2prev[j] = 1.f;
             alpha_prev[j] = 1.f;
             br_prev[j] = 0.f;
-            bc_prev[j] = 0.f;
             bss_cur[j] = 0.f;
             bss_old[j] = 0.f;
             dvp[j] = 0.f;
@@ -500,7 +458,7 @@ __global__ void __launch_bounds__(32 * NW, MINB)
             // ---- X: gk(s) from the old state
             const float *Sc = stages + st_cur * (SB / 4) + si;   // this column in stage s
             const float *Sn = stages + st_nxt * (SB / 4) + si;   // and in stage s+1
-            float gk[C], by_own[C], bx_own[C], bs_own[C], alpha_cur[C], bc_rt[C];
+            float gk[C], by_own[C], bs_own[C], alpha_cur[C];
             {
                 float d[C], v[C];
                 ld_cells<C>(Sc + OFF_BR, by_own);
@@ -515,19 +473,6 @@ __global__ void __launch_bounds__(32 * NW, MINB)
 #pragma unroll
                     for (int j = 0; j < C; ++j)
                         d[j] = nx[j] - by_own[j];
-                }
-                if constexpr (DIM == 3) {
-                    ld_cells<C>(Sc + OFF_BC, bx_own);
-                    ld_cells<C>(Sc + OFF_BC + G::LR, v);
-#pragma unroll
-                    for (int j = 0; j < C; ++j) {
-                        d[j] = d[j] + v[j];
-                        d[j] = d[j] - bx_own[j];
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < C; ++j)
-                        bx_own[j] = 0.f;
                 }
                 ld_cells<C>(Sc + OFF_BS, bs_own);
                 ld_cells<C>(Sn + OFF_BS, v);
@@ -544,11 +489,6 @@ __global__ void __launch_bounds__(32 * NW, MINB)
                 for (int j = 0; j < C; ++j)
                     gk[j] = d[j] - ((s0[j] - s1[j]) + div_cc<EXACT>(s2[j], cc, inv_cc));
                 ld_cells<C>(Sc + OFF_AL, alpha_cur);
-                if constexpr (DIM == 3) {
-                    st_cells<C>(GK + gi, gk);
-                    // b'_c(s-1) at c+1, written by the previous Y (before Y rewrites it)
-                    ld_cells<C>(BCp + gi_right, bc_rt);
-                }
             }
             if (__syncthreads_or(!wait_ok)) {
                 aborted = true;
@@ -558,30 +498,17 @@ __global__ void __launch_bounds__(32 * NW, MINB)
             }
 
             // refill a slot whose last readers finished before the barrier
-            if (!LATE && producer && t + kLead < n_loads)
+            if (producer && t + kLead < n_loads)
                 issue_load(t + kLead);
 
             // ---- Y: gradient step b'(s), projection g2(s-1), stream faces b''(s-1)
             float gk_up[C];
             rows_up<C>(gk, gk_up);
-            float brn[C], bcn[C], bsn[C], br_dn[C], g2[C];
+            float brn[C], bsn[C], br_dn[C], g2[C];
 #pragma unroll
             for (int j = 0; j < C; ++j)
                 brn[j] = keep_if<EXACT>(steps * (gk[j] - gk_up[j]) + by_own[j], fr_ok[j] && s_in,
                                         fr_f[j]);
-            if constexpr (DIM == 3) {
-                float gk_left[C];
-                ld_cells<C>(GK + gi_left, gk_left);
-#pragma unroll
-                for (int j = 0; j < C; ++j)
-                    bcn[j] = keep_if<EXACT>(steps * (gk[j] - gk_left[j]) + bx_own[j], fc_ok[j] && s_in,
-                                            fc_f[j]);
-                st_cells<C>(BCp + gi, bcn);
-            } else {
-#pragma unroll
-                for (int j = 0; j < C; ++j)
-                    bcn[j] = bc_rt[j] = 0.f;
-            }
 #pragma unroll
             for (int j = 0; j < C; ++j) {
                 bsn[j] = keep_if<EXACT>(steps * (gk[j] - gkprev[j]) + bs_own[j], inplane[j] && sb_in, sb_f);
@@ -590,14 +517,8 @@ __global__ void __launch_bounds__(32 * NW, MINB)
             rows_down<C>(br_prev, br_dn);   // b'_r(s-1) at r+1
 #pragma unroll
             for (int j = 0; j < C; ++j) {
-                if constexpr (DIM == 3)
-                    g2[j] = Proj<EXACT>::gk(bc_rt[j], bc_prev[j], br_dn[j], br_prev[j], bsn[j], bsprev[j],
-                                            alpha_prev[j]);
-                else
-                    g2[j] = Proj<EXACT>::gk(bsn[j], bsprev[j], br_dn[j], br_prev[j], alpha_prev[j]);
+                g2[j] = Proj<EXACT>::gk(bsn[j], bsprev[j], br_dn[j], br_prev[j], alpha_prev[j]);
             }
-            if constexpr (DIM == 3)
-                st_cells<C>(G2p + gi, g2);
             const int sp = s - 1;
             {
                 float bssn[C];
@@ -616,14 +537,12 @@ __global__ void __launch_bounds__(32 * NW, MINB)
                     alpha_prev[j] = alpha_cur[j];
                 }
             }
+
             __syncthreads();
 
-            if (LATE && producer && t + kLead < n_loads)
-                issue_load(t + kLead);
-
-            // ---- Z: row/column faces of plane s-1 and the output of plane s-2
+            // ---- Z: row faces of plane s-1 and the output of plane s-2
             {
-                float g2_up[C], g2_dn[C], brr[C], dn[C], bcc[C];
+                float g2_up[C], g2_dn[C], brr[C], dn[C];
                 rows_up<C>(g2, g2_up);
                 rows_down<C>(g2, g2_dn);
 #pragma unroll
@@ -633,28 +552,11 @@ __global__ void __launch_bounds__(32 * NW, MINB)
                     const float brr1 = keep_if<EXACT>(((g2_dn[j] + g2[j]) * 0.5f) * br_dn[j],
                                                       fr1_ok[j] && sp_in, fr1_f[j]);
                     dn[j] = brr1 - brr[j];
-                    bcc[j] = 0.f;
-                }
-                if constexpr (DIM == 3) {
-                    float g2_l[C], g2_r[C];
-                    ld_cells<C>(G2p + gi_left, g2_l);
-                    ld_cells<C>(G2p + gi_right, g2_r);
-#pragma unroll
-                    for (int j = 0; j < C; ++j) {
-                        bcc[j] = keep_if<EXACT>(((g2[j] + g2_l[j]) * 0.5f) * bc_prev[j], fc_ok[j] && sp_in,
-                                                fc_f[j]);
-                        const float bcc1 = keep_if<EXACT>(((g2_r[j] + g2[j]) * 0.5f) * bc_rt[j],
-                                                          fc1_ok[j] && sp_in, fc1_f[j]);
-                        dn[j] = dn[j] + bcc1;
-                        dn[j] = dn[j] - bcc[j];
-                    }
                 }
                 if (is_tile[0]) {
                     if (sp >= s_begin && sp < s_end) {
                         const unsigned int o = col_off + (unsigned int)sp * plane_stride;
                         st_dst<C>(d_br, o, brr, is_tile, P);
-                        if constexpr (DIM == 3)
-                            st_dst<C>(d_bc, o, bcc, is_tile, P);
                     }
                     const int so = s - 2;
                     if (so >= s_begin && so < s_end) {
@@ -699,12 +601,11 @@ __global__ void __launch_bounds__(32 * NW, MINB)
                 for (int j = 0; j < C; ++j) {
                     dvp[j] = dn[j];
                     br_prev[j] = brn[j];
-                    bc_prev[j] = bcn[j];
                 }
             }
         }
         q0 += n_loads;
-        __syncthreads();  // stage slots and shared planes are reused by the next item
+        __syncthreads();  // stage slots are reused by the next item
         if constexpr (EPI == EPI_BINARY)
             finish_item<NT>(erru, P, li, it, B.done_count, s_red, &s_is_last);
     }

@@ -1,5 +1,6 @@
 // Host-side set-up of the fused iteration kernel: TMA descriptors for the
 // halo and tile boxes of both ping-pong parities, destinations, work split.
+#include <algorithm>
 #include <cstring>
 
 #include "internal.h"
@@ -25,7 +26,7 @@ int build_problem_desc(EncodeTiledFn fn, const StencilVariant &v, const StencilP
                        ProblemDesc *A)
 {
     memset(A, 0, sizeof *A);
-    const bool binary = (v.epi == EPI_BINARY);
+    const bool binary = (v.epi == EPI_BINARY || v.epi == EPI_COLD);
     // label extent of each slot's box
     auto box_labels = [&](int labels) { return v.label_boxes == LB_ALL ? labels : 1; };
     for (int par = 0; par < 2; ++par) {
@@ -36,7 +37,11 @@ int build_problem_desc(EncodeTiledFn fn, const StencilVariant &v, const StencilP
         for (int slot = 0; slot < NUM_SLOTS; ++slot) {
             if (v.dim == 2 && slot == SL_BC)
                 continue;
-            const int cols = (slot == SL_BC) ? v.box_cols_bc : v.box_cols;
+            if (v.dim == 3 && (slot == SL_S1 || slot == SL_S2))
+                continue;  // the carried source stands for all three
+            const int cols = (slot == SL_BC)                 ? v.box_cols_bc
+                             : (slot == SL_S0 && v.dim == 3) ? v.box_cols_s0
+                                                             : v.box_cols;
             int r = encode(fn, &A->halo[par][slot], srcs[slot], p, labels[slot], v.box_rows, cols,
                            box_labels(labels[slot]));
             if (r)
@@ -84,7 +89,8 @@ int build_problem_desc(EncodeTiledFn fn, const StencilVariant &v, const StencilP
     A->nlab_items = p.flow_labels;
     A->tiles_r = (p.nr + v.tr - 1) / v.tr;
     A->tiles_c = (v.dim == 3) ? (p.nc + v.tc - 1) / v.tc : 1;
-    A->zchunks = 1;
+    A->zchunks = A->zchunks_a = 1;
+    A->units_a = 0;
     return 0;
 }
 
@@ -99,6 +105,54 @@ int problem_items(const StencilProblem &p, const StencilVariant &v, int zchunks)
     const long long tiles = (long long)((p.nr + v.tr - 1) / v.tr) *
                             ((v.dim == 3) ? (p.nc + v.tc - 1) / v.tc : 1);
     return (int)(tiles * item_labels(p, v) * zchunks);
+}
+
+// One item costs its planes, the 4 warm-up planes of the sweep and about
+// two steps' time for the ring's first loads and the item's end.
+static constexpr double kItemSteps = 6.0;
+
+double choose_split3(const StencilProblem &p, const StencilVariant &v, long long slots, ProblemDesc *d)
+{
+    const long long units = (long long)((p.nr + v.tr - 1) / v.tr) * ((p.nc + v.tc - 1) / v.tc) *
+                            p.flow_labels;
+    const long long most = std::max(1, std::min(64, p.ns / 4));
+    if (slots < 1)
+        slots = 1;
+    double best = 1e300;
+    int bu = 0, ba = 1, bb = 1;
+    auto steps = [&](long long n, long long k) {
+        return n ? (double)((n * k + slots - 1) / slots) * ((double)((p.ns + k - 1) / k) + kItemSteps) : 0.0;
+    };
+    // first part: as many units in ka chunks as fill whole waves (or none);
+    // the remaining units in kb chunks
+    for (long long ka = 1; ka <= most; ++ka) {
+        const long long waves = units * ka / slots;
+        const long long ua = std::min(units, waves * slots / ka);
+        const double ca = steps(ua, ka);
+        if (ca >= best)
+            continue;
+        for (long long kb = 1; kb <= most; ++kb) {
+            const double c = ca + steps(units - ua, kb);
+            if (c < best - 1e-9) {
+                best = c;
+                bu = (int)ua;
+                ba = (int)ka;
+                bb = (int)kb;
+            }
+            if (ua == units)
+                break;
+        }
+    }
+    d->units_a = bu;
+    d->zchunks_a = ba;
+    d->zchunks = bb;
+    return best;
+}
+
+int split3_items(const StencilProblem &p, const StencilVariant &v, const ProblemDesc &d)
+{
+    const int units = ((p.nr + v.tr - 1) / v.tr) * ((p.nc + v.tc - 1) / v.tc) * p.flow_labels;
+    return d.units_a * d.zchunks_a + (units - d.units_a) * d.zchunks;
 }
 
 int choose_zchunks(const StencilProblem &p, const StencilVariant &v, long long slots)

@@ -3,6 +3,7 @@
 
 #include "internal.h"
 #include "stencil2_kernel.cuh"
+#include "stencil3d_kernel.cuh"
 #include "stencil2d_t2.cuh"
 #include "stencil2d_labels.cuh"
 #include "stencil2d_tile.cuh"
@@ -10,26 +11,50 @@
 
 namespace asets {
 
-template <int DIM, int NW, int NSTAGE, int EPI, bool EXACT, int MINB = (DIM == 3 ? 2 : 4),
-          int UNROLL = 1, int CELLS = 1, bool LATE = false>
+template <int NW, int NSTAGE, int EPI, bool EXACT, int MINB = 4, int UNROLL = 1, int CELLS = 1>
 StencilVariant make_variant()
 {
-    using G = ColGeom<DIM, NW, CELLS>;
+    using G = ColGeom<NW, CELLS>;
     StencilVariant v;
-    v.dim = DIM;
+    v.dim = 2;
+    v.epi = EPI;
+    v.exact = EXACT ? 1 : 0;
+    v.tr = G::TR;
+    v.tc = 1;
+    v.nt = G::NT;
+    v.nstage = NSTAGE;
+    v.smem_bytes = G::template smem_bytes<NSTAGE, EPI>();
+    v.box_rows = G::LR;
+    v.box_cols = 1;
+    v.box_cols_bc = 1;
+    v.tile_box_rows = G::TR;
+    v.temporal = 1;
+    v.fn = reinterpret_cast<const void *>(&stencil_col_kernel<NW, NSTAGE, EPI, EXACT, MINB, UNROLL, CELLS>);
+    return v;
+}
+
+// The 3D kernels with the carried gradient source (stencil3d_kernel.cuh).
+template <int TC, int CELLS, int NSTAGE, int EPI, bool EXACT>
+StencilVariant make_variant3()
+{
+    using G = Geom3<TC, CELLS, EPI>;
+    StencilVariant v;
+    v.dim = 3;
     v.epi = EPI;
     v.exact = EXACT ? 1 : 0;
     v.tr = G::TR;
     v.tc = G::TC;
     v.nt = G::NT;
     v.nstage = NSTAGE;
-    v.smem_bytes = G::template smem_bytes<NSTAGE, EPI>();
+    v.smem_bytes = G::smem_bytes(NSTAGE);
     v.box_rows = G::LR;
-    v.box_cols = G::LC;
-    v.box_cols_bc = G::LC_BC;
+    v.box_cols = G::COLS;
+    v.box_cols_bc = G::COLS_BC;
+    v.box_cols_s0 = G::COLS_G;
     v.tile_box_rows = G::TR;
     v.temporal = 1;
-    v.fn = reinterpret_cast<const void *>(&stencil_col_kernel<DIM, NW, NSTAGE, EPI, EXACT, MINB, UNROLL, CELLS, LATE>);
+    static_assert(G::smem_bytes(NSTAGE) <= 227 * 1024, "shared memory of a block");
+    v.fn = reinterpret_cast<const void *>(&stencil3d_kernel<TC, CELLS, NSTAGE, EPI, EXACT>);
     return v;
 }
 
