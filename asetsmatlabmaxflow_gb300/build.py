@@ -52,6 +52,7 @@ CU_SOURCES = (
     "carry3d.cu",
     "binary3d_fast.cu",
     "binary3d_exact.cu",
+    "binary3d_twin.cu",
     "binary2d_fast.cu",
     "binary2d_exact.cu",
     "flow3d_fast.cu",

@@ -51,24 +51,6 @@ __global__ void __launch_bounds__(kCarryThreads) source_kernel(const CarryArgs A
     }
 }
 
-// The cold binary start: u = (Cs - Ct >= 0), ps = pt = min(Cs, Ct)
-// (init_kernels.cu) with zero flows, as v and gk
-__global__ void __launch_bounds__(kCarryThreads) cold_source_kernel(const CarryArgs A)
-{
-    const int lane = threadIdx.x & 31;
-    const long long rows = (long long)A.g.nc * A.g.ns;
-    const long long step = (long long)gridDim.x * (kCarryThreads / 32);
-    for (long long q = blockIdx.x * (long long)(kCarryThreads / 32) + (threadIdx.x >> 5); q < rows;
-         q += step)
-        for (int r = lane; r < A.g.nr; r += 32) {
-            const long long o = q * A.g.pitch + r;
-            const float cs = A.cs[o], ct = A.ct[o], m = min_ref(cs, ct);
-            float u = (cs - ct >= 0.0f) ? 1.0f : 0.0f;
-            A.v_out[o] = cold_v(m, ct, u);
-            A.gk[o] = 0.0f - u * A.inv_cc;
-        }
-}
-
 // u or pt of the cold start's state v
 __global__ void __launch_bounds__(kCarryThreads) cold_state_kernel(const CarryArgs A)
 {
@@ -136,12 +118,6 @@ cudaError_t launch_source(int model, const CarryArgs &a, int num_sms, cudaStream
     SRC(1)
     SRC(2)
 #undef SRC
-    return cudaGetLastError();
-}
-
-cudaError_t launch_cold_source(const CarryArgs &a, int num_sms, cudaStream_t st)
-{
-    cold_source_kernel<<<carry_grid(a, num_sms), kCarryThreads, 0, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -349,11 +349,10 @@ __device__ __forceinline__ float cold_v(float pt, float ct, float &u)
     return sat ? u * kColdScale : pt;
 }
 
-// Warp + block sum of a per-thread float into one double (lane order fixed).
+// Warp + block sum of a per-thread value into one double (lane order fixed).
 template <int NT>
-__device__ __forceinline__ double block_sum_double(float v, double *scratch)
+__device__ __forceinline__ double block_sum_double(double d, double *scratch)
 {
-    double d = (double)v;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
         d += __shfl_xor_sync(0xffffffffu, d, o);

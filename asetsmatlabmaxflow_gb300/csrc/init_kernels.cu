@@ -17,18 +17,13 @@ namespace asets {
 
 constexpr int kInitThreads = 256;
 
-__global__ void init_binary_kernel(InitArgs A)
+__device__ __forceinline__ void init_binary(const InitArgs &A, long long g)
 {
-    for (long long g = blockIdx.x * (long long)kInitThreads + threadIdx.x; g < A.cells;
-         g += (long long)gridDim.x * kInitThreads) {
-        if ((int)(g % A.pitch) >= A.nr)
-            continue;
-        const float cs = A.cs[g], ct = A.ct[g];
-        A.u[g] = (cs - ct >= 0.0f) ? 1.0f : 0.0f;
-        const float m = min_ref(cs, ct);
-        A.ps[g] = m;
-        A.pt[g] = m;
-    }
+    const float cs = A.cs[g], ct = A.ct[g];
+    A.u[g] = (cs - ct >= 0.0f) ? 1.0f : 0.0f;
+    const float m = min_ref(cs, ct);
+    A.ps[g] = m;
+    A.pt[g] = m;
 }
 
 __device__ __forceinline__ void argmin_labels(const float *ct, long long g, long long S, int L,
@@ -45,40 +40,85 @@ __device__ __forceinline__ void argmin_labels(const float *ct, long long g, long
     }
 }
 
-__global__ void init_potts_kernel(InitArgs A)
+__device__ __forceinline__ void init_potts(const InitArgs &A, long long g)
 {
     const long long S = A.label_stride;
+    float mv;
+    int mi;
+    argmin_labels(A.ct, g, S, A.nlab, mv, mi);
+    A.ps[g] = mv;
+    for (int l = 0; l < A.nlab; ++l) {
+        A.pt[g + l * S] = mv;
+        A.u[g + l * S] = (l == mi) ? 1.0f : 0.0f;
+    }
+}
+
+__device__ __forceinline__ void init_ishikawa(const InitArgs &A, long long g)
+{
+    const long long S = A.label_stride;
+    float mv;
+    int mi;
+    argmin_labels(A.ct, g, S, A.nlab, mv, mi);
+    for (int l = 0; l < A.nlab - 1; ++l) {
+        A.pt[g + l * S] = mv;
+        A.u[g + l * S] = (l >= mi) ? 0.0f : 1.0f;
+    }
+    A.pt[g + (A.nlab - 1) * S] = 0.0f;
+}
+
+// MODEL 0-2: the model's state; kPrepareCold: the binary state as v (cold_v)
+// with its gradient source; kPrepareNone: nothing
+template <int MODEL>
+__device__ __forceinline__ void init_cells(const InitArgs &A, float *gk, float *v, float inv_cc)
+{
+    if (MODEL == kPrepareNone)
+        return;
     for (long long g = blockIdx.x * (long long)kInitThreads + threadIdx.x; g < A.cells;
          g += (long long)gridDim.x * kInitThreads) {
-        if ((int)(g % A.pitch) >= A.nr)
+        if ((int)((unsigned int)g % (unsigned int)A.pitch) >= A.nr)  // cells are below 2^32
             continue;
-        float mv;
-        int mi;
-        argmin_labels(A.ct, g, S, A.nlab, mv, mi);
-        A.ps[g] = mv;
-        for (int l = 0; l < A.nlab; ++l) {
-            A.pt[g + l * S] = mv;
-            A.u[g + l * S] = (l == mi) ? 1.0f : 0.0f;
+        if (MODEL == 0) {
+            init_binary(A, g);
+        } else if (MODEL == 1) {
+            init_potts(A, g);
+        } else if (MODEL == 2) {
+            init_ishikawa(A, g);
+        } else {
+            const float cs = A.cs[g], ct = A.ct[g];
+            float u = (cs - ct >= 0.0f) ? 1.0f : 0.0f;
+            v[g] = cold_v(min_ref(cs, ct), ct, u);
+            gk[g] = 0.0f - u * inv_cc;  // zero flows, ps = pt
         }
     }
 }
 
-__global__ void init_ishikawa_kernel(InitArgs A)
+template <int MODEL>
+__global__ void init_kernel(const InitArgs A, float *gk, float *v, float inv_cc)
 {
-    const long long S = A.label_stride;
-    for (long long g = blockIdx.x * (long long)kInitThreads + threadIdx.x; g < A.cells;
-         g += (long long)gridDim.x * kInitThreads) {
-        if ((int)(g % A.pitch) >= A.nr)
-            continue;
-        float mv;
-        int mi;
-        argmin_labels(A.ct, g, S, A.nlab, mv, mi);
-        for (int l = 0; l < A.nlab - 1; ++l) {
-            A.pt[g + l * S] = mv;
-            A.u[g + l * S] = (l >= mi) ? 0.0f : 1.0f;
-        }
-        A.pt[g + (A.nlab - 1) * S] = 0.0f;
+    init_cells<MODEL>(A, gk, v, inv_cc);
+}
+
+template <int MODEL>
+__global__ void __launch_bounds__(kInitThreads) prepare_kernel(const __grid_constant__ PrepareArgs A)
+{
+    const long long t0 = blockIdx.x * (long long)kInitThreads + threadIdx.x;
+    const long long step = (long long)gridDim.x * kInitThreads;
+    if (blockIdx.x == 0) {
+        const int *src = reinterpret_cast<const int *>(&A.desc);
+        for (int i = threadIdx.x; i < (int)(sizeof(ProblemDesc) / 4); i += kInitThreads)
+            reinterpret_cast<int *>(A.d_desc)[i] = src[i];
+        if (threadIdx.x == 0)
+            *A.d_ctl = A.ctl;
+        if (threadIdx.x < 4)
+            A.queue[threadIdx.x] = 0;
     }
+    for (long long i = t0; i < A.n_cvg; i += step)
+        A.cvg[i] = 0.0f;
+    for (int k = 0; k < 3; ++k)
+        if (A.zero[k])
+            for (long long i = t0; i < A.zero_floats / 4; i += step)
+                reinterpret_cast<float4 *>(A.zero[k])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    init_cells<MODEL>(A.init, A.gk, A.v, A.desc.inv_cc);
 }
 
 // projStep's check, `if (alpha <= 0) error` (asetsBinaryMF3D_mex.c:317-319),
@@ -89,8 +129,8 @@ __global__ void validate_alpha_kernel(InitArgs A)
     const long long total = A.cells * A.alpha_labels;
     for (long long i = blockIdx.x * (long long)kInitThreads + threadIdx.x; i < total;
          i += (long long)gridDim.x * kInitThreads) {
-        const long long g = i % A.cells;
-        if ((int)(g % A.pitch) >= A.nr)
+        // label slices are whole padded volumes; elements are below 2^32
+        if ((int)((unsigned int)i % (unsigned int)A.pitch) >= A.nr)
             continue;
         if (A.alpha[i] <= 0.0f)
             bad = 1;
@@ -128,9 +168,32 @@ cudaError_t launch_init(int model, const InitArgs &a, int num_sms, cudaStream_t 
 {
     const int grid = grid_for(a.cells, num_sms);
     switch (model) {
-    case 0: init_binary_kernel<<<grid, kInitThreads, 0, st>>>(a); break;
-    case 1: init_potts_kernel<<<grid, kInitThreads, 0, st>>>(a); break;
-    case 2: init_ishikawa_kernel<<<grid, kInitThreads, 0, st>>>(a); break;
+    case 0: init_kernel<0><<<grid, kInitThreads, 0, st>>>(a, nullptr, nullptr, 0.f); break;
+    case 1: init_kernel<1><<<grid, kInitThreads, 0, st>>>(a, nullptr, nullptr, 0.f); break;
+    case 2: init_kernel<2><<<grid, kInitThreads, 0, st>>>(a, nullptr, nullptr, 0.f); break;
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_cold_init(const InitArgs &a, float *gk, float *v, float inv_cc, int num_sms,
+                             cudaStream_t st)
+{
+    init_kernel<kPrepareCold><<<grid_for(a.cells, num_sms), kInitThreads, 0, st>>>(a, gk, v, inv_cc);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_prepare(const PrepareArgs &a, int num_sms, cudaStream_t st)
+{
+    static_assert(sizeof(PrepareArgs) <= 4096, "kernel parameter space");
+    static_assert(sizeof(ProblemDesc) % 4 == 0, "copied by words");
+    const int grid = grid_for(a.init.cells, num_sms);
+    switch (a.model) {
+    case 0: prepare_kernel<0><<<grid, kInitThreads, 0, st>>>(a); break;
+    case 1: prepare_kernel<1><<<grid, kInitThreads, 0, st>>>(a); break;
+    case 2: prepare_kernel<2><<<grid, kInitThreads, 0, st>>>(a); break;
+    case kPrepareCold: prepare_kernel<kPrepareCold><<<grid, kInitThreads, 0, st>>>(a); break;
+    case kPrepareNone: prepare_kernel<kPrepareNone><<<grid, kInitThreads, 0, st>>>(a); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

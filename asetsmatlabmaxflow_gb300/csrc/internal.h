@@ -71,6 +71,17 @@ int choose_zchunks(const StencilProblem &p, const StencilVariant &v, long long s
 // Work split of a 3D problem into d->units_a, zchunks_a and zchunks for
 // `slots` resident blocks; returns its length in plane steps.
 double choose_split3(const StencilProblem &p, const StencilVariant &v, long long slots, ProblemDesc *d);
+// Cost of a plane step of the 3D kernel with tile width TC, in units of the
+// time a column takes: measured at 64^3 to 256^3, the fast forms' steps take
+// (4 + TC) and the EXACT ones' (10 + TC) to within a few percent (binary
+// fast TC = 12, 13, 16 at 256^3: 0.94, 1.00, 1.21 us; EXACT 1.65, 1.77, 2.02).
+double step_cost3(const StencilVariant &v);
+// The variant whose split takes the least time.  Fast 256^3 is split evenly
+// by 14 columns (19 x 4 tiles x 2 chunks = 152 blocks: 141 us per iteration
+// against 150 with 16 or 13), 192^3 and 128^3 by 16 (Potts 192^3 L = 4: 270 us
+// against 280 with 14), 64^3 takes 12 (15.4 us against 16.6 with 16).
+const StencilVariant *pick_split3(const StencilProblem &p, const StencilVariant *const *v, int n,
+                                  int num_sms);
 // Items of a 3D problem with the split of d.
 int split3_items(const StencilProblem &p, const StencilVariant &v, const ProblemDesc &d);
 // Items of one problem with the given chunk count.
@@ -79,6 +90,7 @@ int problem_items(const StencilProblem &p, const StencilVariant &v, int zchunks)
 // Variant tables, one per translation unit.
 const StencilVariant *binary3d_fast_variants(int *count);
 const StencilVariant *binary3d_exact_variants(int *count);
+const StencilVariant *binary3d_twin_variants(int *count);
 const StencilVariant *binary2d_fast_variants(int *count);
 const StencilVariant *binary2d_exact_variants(int *count);
 const StencilVariant *flow3d_fast_variants(int *count);
@@ -154,6 +166,27 @@ struct InitArgs {
     int alpha_labels;        // alpha slices to validate
 };
 
+// Everything a run starts from, in one launch.
+enum { kPrepareCold = 3, kPrepareNone = -1 };  // beside the models 0-2
+struct PrepareArgs {
+    ProblemDesc desc;        // to *d_desc
+    IterControl ctl;         // to *d_ctl
+    ProblemDesc *d_desc;
+    IterControl *d_ctl;
+    unsigned int *queue;     // four words, zeroed
+    float *cvg;              // n_cvg floats, zeroed
+    float *zero[3];          // zero_floats floats each, zeroed (null: none)
+    long long zero_floats;   // a multiple of 4
+    int n_cvg;
+    int model;               // initial state: a model, kPrepareCold or kPrepareNone
+    InitArgs init;
+    float *gk, *v;           // kPrepareCold: the first gradient source and state (cold_v)
+};
+cudaError_t launch_prepare(const PrepareArgs &a, int num_sms, cudaStream_t st);
+
+// The cold binary start's v and gk (as launch_prepare with kPrepareCold).
+cudaError_t launch_cold_init(const InitArgs &a, float *gk, float *v, float inv_cc, int num_sms,
+                             cudaStream_t st);
 cudaError_t launch_init(int model, const InitArgs &a, int num_sms, cudaStream_t st);
 // Sets a.ctl->wide if an input of a binary problem is not finite or is
 // beyond the range of the cold start's state.
@@ -194,12 +227,10 @@ struct CarryArgs {
     const float *ps, *pt, *u;
     const float *cs, *ct, *dv;
     const float *v;                  // cold binary start: v after the last iteration
-    float *gk;                       // launch_source, launch_cold_source
+    float *gk;                       // launch_source
     float *out;                      // launch_flows: binary ps, Potts pt
-    float *v_out, *u_out, *pt_out;   // launch_cold_source; launch_cold_state
+    float *u_out, *pt_out;           // launch_cold_state
 };
-// Initial v and gk of the cold binary start, from Cs and Ct.
-cudaError_t launch_cold_source(const CarryArgs &a, int num_sms, cudaStream_t st);
 // u (u_out) or pt (pt_out) of the state v.
 cudaError_t launch_cold_state(const CarryArgs &a, int num_sms, cudaStream_t st);
 cudaError_t launch_source(int model, const CarryArgs &a, int num_sms, cudaStream_t st);

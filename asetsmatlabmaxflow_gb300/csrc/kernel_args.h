@@ -29,7 +29,8 @@ struct IterControl {
     int alpha_bad;      // set by the validation pass
     int rollback;       // two-iteration pass: the solve ended at its first iteration
     int wide;           // set by the range check (binary 3D)
-    int pad[3];
+    int pad;
+    double vol;         // EPI_TWIN: cvg = (float)(erru / vol)
 };
 
 // Stage slots: which field each TMA box holds.
@@ -48,6 +49,7 @@ enum Epilogue : int {
     EPI_BINARY = 0,  // binary model: ps/pt/u update + erriter
     EPI_DIV = 1,     // multi-label models: write the new flow and its divergence
     EPI_COLD = 3,    // binary 3D from the cold start: pt and u in one array (dst_s: gk, v)
+    EPI_TWIN = 4,    // binary 3D, the Matlab twin's expressions (dst_s: gk, pt, u)
     EPI_FUSED = 2,   // multi-label 2D, one pass: flows of all labels and the label update
 };
 
@@ -85,7 +87,8 @@ struct ProblemDesc {
     int lab_mul[NUM_SLOTS];
     int lab_add[NUM_SLOTS];
     float cc, inv_cc, steps;
-    float inv_cc_l;                        // EPI_FUSED Potts: 1/(cc*L), cc*L rounded to float
+    float inv_cc_l;                        // EPI_FUSED Potts: 1/(cc*L), cc*L rounded to float;
+                                           // EPI_TWIN: 1/cc formed in double
 };
 
 // A launch over one or more problems of the same kind (dimension, model).

@@ -255,14 +255,6 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     ia.nlab = 1;
     ia.alpha_labels = 1;
     const int flags = opt ? opt->flags : 0;
-    if (maxIt >= 1 && !(flags & ASETS_FLAG_NO_ALPHA_CHECK)) {
-        NA_TRY(launch_validate_alpha(ia, d->num_sms, sm));
-        int bad = 0;
-        NA_TRY(cudaMemcpyAsync(&bad, &ctl->alpha_bad, sizeof bad, cudaMemcpyDeviceToHost, sm));
-        NA_TRY(cudaStreamSynchronize(sm));
-        if (bad)
-            return na_fail(ASETS_ERR_ALPHA, "alpha(x) must be positive. Exiting...");
-    }
     // kernel variant (the same fused kernels as the other entry points)
     const int exact = (flags & ASETS_FLAG_EXACT) ? 1 : 0;
     int nv = 0;
@@ -270,12 +262,21 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     const StencilVariant *v = nv > 0 ? &tab[0] : nullptr;
     if (!v)
         return na_fail(ASETS_ERR_UNSUPPORTED, "no kernel variant");
-    if (v->cold && maxIt > 0) {
-        int wide = 0;
-        NA_TRY(launch_check_range(ia, d->num_sms, sm));
-        NA_TRY(cudaMemcpyAsync(&wide, &ctl->wide, sizeof wide, cudaMemcpyDeviceToHost, sm));
-        NA_TRY(cudaStreamSynchronize(sm));
-        if (!wide)
+    if (maxIt >= 1) {
+        const bool check_alpha = !(flags & ASETS_FLAG_NO_ALPHA_CHECK);
+        IterControl checked;
+        memset(&checked, 0, sizeof checked);
+        if (check_alpha)
+            NA_TRY(launch_validate_alpha(ia, d->num_sms, sm));
+        if (v->cold)
+            NA_TRY(launch_check_range(ia, d->num_sms, sm));
+        if (check_alpha || v->cold) {
+            NA_TRY(cudaMemcpyAsync(&checked, ctl, sizeof checked, cudaMemcpyDeviceToHost, sm));
+            NA_TRY(cudaStreamSynchronize(sm));
+        }
+        if (checked.alpha_bad)
+            return na_fail(ASETS_ERR_ALPHA, "alpha(x) must be positive. Exiting...");
+        if (v->cold && !checked.wide)
             v = v->cold;
     }
     const bool cold = (v->epi == EPI_COLD && maxIt > 0);
@@ -292,9 +293,8 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     ca.cs = cs;
     ca.ct = ct;
     ca.gk = gk[0];
-    ca.v_out = pt[0];
     if (cold) {
-        NA_TRY(launch_cold_source(ca, d->num_sms, sm));
+        NA_TRY(launch_cold_init(ia, gk[0], pt[0], ca.inv_cc, d->num_sms, sm));
     } else {
         NA_TRY(launch_init(0, ia, d->num_sms, sm));
         NA_TRY(launch_source(0, ca, d->num_sms, sm));

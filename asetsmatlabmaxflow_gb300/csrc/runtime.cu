@@ -135,6 +135,8 @@ struct asets_solver {
     bool cold_state = false, u_stale = false, cold_ok = false;
     float run_cc = 0.f;
     int run_exact = 0;
+    float *stage = nullptr;  // unpadded copy of a host array on its way in or out
+    size_t stage_cap = 0;
     float *warm_u = nullptr, *warm_ps = nullptr, *warm_pt = nullptr;
     bool warm = false;
     float *warm_b[3] = {nullptr, nullptr, nullptr};  // initial spatial flows (padded)
@@ -366,6 +368,7 @@ extern "C" ASETS_API void asets_solver_destroy(asets_solver *s)
     s->graph.reset();
     for (void *p : s->allocations)
         cudaFree(p);
+    cudaFree(s->stage);
     if (s->ev0)
         cudaEventDestroy(s->ev0);
     if (s->ev1)
@@ -475,34 +478,6 @@ static StencilProblem item_geometry(const asets_solver *s)
     return sp;
 }
 
-// Cost of a plane step of the 3D kernel with tile width TC, in units of the
-// time a column takes: measured at 64^3 to 256^3, the fast forms' steps take
-// (4 + TC) and the EXACT ones' (10 + TC) to within a few percent (binary
-// fast TC = 12, 13, 16 at 256^3: 0.94, 1.00, 1.21 us; EXACT 1.65, 1.77, 2.02).
-static double step_cost3(const StencilVariant &v) { return (v.exact ? 10.0 : 4.0) + v.tc; }
-
-// 3D: the width whose split (choose_split3) takes the least time.  256^3 is
-// split evenly by 14 columns (19 x 4 tiles x 2 chunks = 152 blocks: 141 us
-// per iteration against 150 with 16 or 13), 192^3 and 128^3 by 16 (Potts
-// 192^3 L = 4: 270 us against 298 with 14), 64^3 takes 12 (15.3 us against
-// 16.5 with 16).
-static const StencilVariant *pick_variant3(const asets_solver *s,
-                                           const std::vector<const StencilVariant *> &match)
-{
-    StencilProblem p = item_geometry(s);
-    ProblemDesc d;
-    const StencilVariant *best = nullptr;
-    double best_cost = 0.0;
-    for (const StencilVariant *v : match) {
-        const double c = choose_split3(p, *v, s->ctx->num_sms, &d) * step_cost3(*v);
-        if (!best || c < best_cost) {
-            best = v;
-            best_cost = c;
-        }
-    }
-    return best;
-}
-
 static const StencilVariant *pick_variant(asets_solver *s, int exact, int tile_config,
                                           bool single)
 {
@@ -514,7 +489,7 @@ static const StencilVariant *pick_variant(asets_solver *s, int exact, int tile_c
     if (s->dim == 3) {
         const StencilVariant *&v = s->picked3[exact ? 1 : 0];
         if (!v)
-            v = pick_variant3(s, match);
+            v = pick_split3(item_geometry(s), match.data(), (int)match.size(), s->ctx->num_sms);
         return v;
     }
     // the one-pass multi-label kernels lead the list: three sweeps (in-step
@@ -866,27 +841,68 @@ cleanup:
 }
 
 // Copy a Matlab-layout array (rows of nr floats) into / out of the padded
-// layout (rows of pitch floats).
+// layout (rows of pitch floats).  Between pageable host memory and the
+// device a pitched copy goes row by row (17.7 MB in rows of 640 B: 999 us in,
+// 184 out, against 111 and 102 as one run), so host arrays cross as one run
+// and are padded on the device; small ones go out as they are (a megabyte
+// costs 16 us pitched, 19 in two steps).
+static constexpr size_t kPitchedOutMost = 4u << 20;
+
+static cudaError_t stage_for(asets_solver *s, size_t floats)
+{
+    if (floats <= s->stage_cap)
+        return cudaSuccess;
+    void *p = nullptr;
+    cudaError_t e = cudaMalloc(&p, floats * sizeof(float));
+    if (e != cudaSuccess)
+        return e;
+    // a grown buffer replaces the old one, which is still in use by queued copies
+    if (s->stage) {
+        e = cudaStreamSynchronize(s->ctx->stream);
+        cudaFree(s->stage);
+    }
+    s->stage = static_cast<float *>(p);
+    s->stage_cap = floats;
+    return e;
+}
+
 static cudaError_t copy_in(asets_solver *s, float *dst, const float *src, int labels,
                            asets_memory where)
 {
-    const size_t rows = (size_t)s->nc * s->ns * labels;
-    return cudaMemcpy2DAsync(dst, s->pitch * sizeof(float), src, s->nr * sizeof(float),
-                             s->nr * sizeof(float), rows,
-                             where == ASETS_DEVICE ? cudaMemcpyDeviceToDevice
-                                                   : cudaMemcpyHostToDevice,
-                             s->ctx->stream);
+    const size_t rows = (size_t)s->nc * s->ns * labels, w = s->nr * sizeof(float);
+    cudaStream_t st = s->ctx->stream;
+    if (where != ASETS_DEVICE) {
+        if (s->pitch == s->nr)
+            return cudaMemcpyAsync(dst, src, w * rows, cudaMemcpyHostToDevice, st);
+        cudaError_t e = stage_for(s, (size_t)s->nr * rows);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(s->stage, src, w * rows, cudaMemcpyHostToDevice, st);
+        if (e != cudaSuccess)
+            return e;
+        src = s->stage;
+    }
+    return cudaMemcpy2DAsync(dst, s->pitch * sizeof(float), src, w, w, rows, cudaMemcpyDeviceToDevice, st);
 }
 
 static cudaError_t copy_out(asets_solver *s, float *dst, const float *src, int labels,
                             asets_memory where)
 {
-    const size_t rows = (size_t)s->nc * s->ns * labels;
-    return cudaMemcpy2DAsync(dst, s->nr * sizeof(float), src, s->pitch * sizeof(float),
-                             s->nr * sizeof(float), rows,
-                             where == ASETS_DEVICE ? cudaMemcpyDeviceToDevice
-                                                   : cudaMemcpyDeviceToHost,
-                             s->ctx->stream);
+    const size_t rows = (size_t)s->nc * s->ns * labels, w = s->nr * sizeof(float);
+    cudaStream_t st = s->ctx->stream;
+    if (where == ASETS_DEVICE)
+        return cudaMemcpy2DAsync(dst, w, src, s->pitch * sizeof(float), w, rows, cudaMemcpyDeviceToDevice,
+                                 st);
+    if (s->pitch == s->nr)
+        return cudaMemcpyAsync(dst, src, w * rows, cudaMemcpyDeviceToHost, st);
+    if (w * rows <= kPitchedOutMost)
+        return cudaMemcpy2DAsync(dst, w, src, s->pitch * sizeof(float), w, rows, cudaMemcpyDeviceToHost, st);
+    cudaError_t e = stage_for(s, (size_t)s->nr * rows);
+    if (e == cudaSuccess)
+        e = cudaMemcpy2DAsync(s->stage, w, src, s->pitch * sizeof(float), w, rows,
+                              cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(dst, s->stage, w * rows, cudaMemcpyDeviceToHost, st);
+    return e;
 }
 
 static InitArgs init_args(asets_solver *s)
@@ -999,9 +1015,7 @@ extern "C" ASETS_API asets_status asets_solver_set_inputs(asets_solver *s, asets
     CU_TRY(copy_in(s, s->alpha, alpha, s->alpha_labels, where));
     // alpha(x) > 0 is checked once per input set; run() reports it when it
     // iterates, as projStep does on the first iteration.
-    IterControl zero;
-    memset(&zero, 0, sizeof zero);
-    CU_TRY(cudaMemcpyAsync(s->ctl, &zero, sizeof zero, cudaMemcpyHostToDevice, s->ctx->stream));
+    CU_TRY(cudaMemsetAsync(s->ctl, 0, sizeof(IterControl), s->ctx->stream));
     InitArgs a = init_args(s);
     CU_TRY(launch_validate_alpha(a, s->ctx->num_sms, s->ctx->stream));
     if (s->model == ASETS_BINARY && s->dim == 3)
@@ -1215,20 +1229,24 @@ static asets_status prepare_run(asets_solver *s, int flags, int tile_config, int
     // `1/(cc*nLab)` of updatePSU: cc*nLab rounded to float, then divided
     A.inv_cc_l = 1.0f / (cc * (float)s->nlab);
     A.steps = steps;
-    CU_TRY(cudaMemcpyAsync(s->d_desc, &A, sizeof A, cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaMemsetAsync(s->d_queue, 0, 4 * sizeof(unsigned int), st));
-
-    IterControl c;
-    memset(&c, 0, sizeof c);
+    // one launch sets the descriptor, the control block, the queue, cvg, zero
+    // flows and the model's initial state (the eight copies, sets and launches
+    // it replaces took longer to issue than the solve of a small image)
+    PrepareArgs pa;
+    memset(&pa, 0, sizeof pa);
+    pa.desc = A;
+    pa.d_desc = s->d_desc;
+    pa.queue = s->d_queue;
+    IterControl &c = pa.ctl;
     c.done = (maxIt == 0) ? 1 : 0;
     c.last_iter = -1;
     c.max_it = maxIt;
     c.err_bound = errBound;
     c.break_lt = (s->model == ASETS_ISHIKAWA && s->dim == 2) ? 1 : 0;
     c.denom = (float)(int)((long long)s->ny * s->nx * s->nz * s->u_labels);  // (float)(Nx*Ny*Nz[*L])
-    CU_TRY(cudaMemcpyAsync(s->ctl, &c, sizeof c, cudaMemcpyHostToDevice, st));
-    if (maxIt > 0)
-        CU_TRY(cudaMemsetAsync(s->cvg, 0, sizeof(float) * maxIt, st));
+    pa.d_ctl = s->ctl;
+    pa.cvg = s->cvg;
+    pa.n_cvg = maxIt;
 
     const size_t n = (size_t)s->cells;
     for (int k = 0; k < 3; ++k) {
@@ -1238,9 +1256,14 @@ static asets_status prepare_run(asets_solver *s, int flags, int tile_config, int
             CU_TRY(cudaMemcpyAsync(s->b[0][k], s->warm_b[k], n * s->flow_labels * sizeof(float),
                                    cudaMemcpyDeviceToDevice, st));
         else
-            CU_TRY(cudaMemsetAsync(s->b[0][k], 0, n * s->flow_labels * sizeof(float), st));
+            pa.zero[k] = s->b[0][k];
     }
+    pa.zero_floats = (long long)n * s->flow_labels;
+    const bool cold = s->variant->epi == EPI_COLD && maxIt > 0;
+    pa.init = init_args(s);
+    pa.model = cold ? kPrepareCold : (int)s->model;
     if (s->warm) {
+        pa.model = kPrepareNone;
         CU_TRY(cudaMemcpyAsync(s->u[0], s->warm_u, n * s->u_labels * sizeof(float),
                                cudaMemcpyDeviceToDevice, st));
         CU_TRY(cudaMemcpyAsync(s->pt[0], s->warm_pt, n * s->pt_labels * sizeof(float),
@@ -1248,21 +1271,20 @@ static asets_status prepare_run(asets_solver *s, int flags, int tile_config, int
         if (s->warm_ps)
             CU_TRY(cudaMemcpyAsync(s->ps[0], s->warm_ps, n * sizeof(float),
                                    cudaMemcpyDeviceToDevice, st));
-    } else if (s->variant->epi != EPI_COLD || maxIt == 0) {
-        InitArgs ia = init_args(s);
-        CU_TRY(launch_init((int)s->model, ia, s->ctx->num_sms, st));
     }
+    if (cold) {
+        pa.gk = s->gk[0];
+        pa.v = s->pt[0];
+    }
+    CU_TRY(launch_prepare(pa, s->ctx->num_sms, st));
     s->flows_stale = s->u_stale = s->cold_state = false;
     if (s->dim == 3) {
         CarryArgs ca = carry_args(s, 0, 0, cc, exact);
         if (!s->warm_flows)
             ca.br = nullptr;  // zero flows
         ca.gk = s->gk[0];
-        ca.v_out = s->pt[0];
         if (s->variant->epi != EPI_COLD)
             CU_TRY(launch_source((int)s->model, ca, s->ctx->num_sms, st));
-        else if (maxIt > 0)
-            CU_TRY(launch_cold_source(ca, s->ctx->num_sms, st));
         s->run_cc = cc;
         s->run_exact = exact;
     }

@@ -177,8 +177,9 @@ __device__ __forceinline__ void rows_down(const float (&v)[CELLS], float (&dn)[C
     dn[CELLS - 1] = __shfl_down_sync(0xffffffffu, v[0], 1);
 }
 
-template <int NT>
-__device__ __forceinline__ void finish_item(float erru, const ProblemDesc &P, int li, int it,
+// TWIN: the Matlab twins' mean (formed in double, then rounded)
+template <int NT, bool TWIN = false>
+__device__ __forceinline__ void finish_item(double erru, const ProblemDesc &P, int li, int it,
                                             unsigned int *done_count, double *s_red,
                                             int *s_is_last)
 {
@@ -204,7 +205,7 @@ __device__ __forceinline__ void finish_item(float erru, const ProblemDesc &P, in
         if (threadIdx.x == 0) {
             // cvg[i] = total_err / (float)N, total_err a float
             // (maxflow/asetsBinaryMF3D_mex.c:183)
-            const float c = __fdiv_rn((float)acc, ctl->denom);
+            const float c = TWIN ? (float)(acc / ctl->vol) : __fdiv_rn((float)acc, ctl->denom);
             P.cvg[it] = c;
             ctl->last_iter = it;
             const bool conv = ctl->break_lt ? (c < ctl->err_bound) : (c <= ctl->err_bound);

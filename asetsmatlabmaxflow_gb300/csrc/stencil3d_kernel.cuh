@@ -42,6 +42,9 @@
 // (EPI_BINARY), as do EXACT, for the reference's own roundings, and inputs
 // that are not finite or beyond 2^60.
 //
+// EPI_TWIN: the binary 3D Matlab twin in single precision (mtwin.cu), whose
+// expressions differ in order; its erriter is summed to double precision.
+//
 // Bound: HBM.  Binary 52 B per voxel and iteration (gk, three flows, v in and
 // out; alpha, Cs, Ct in), 64 B with pt and u apart; labelled models 36 B per
 // label.
@@ -77,7 +80,7 @@ struct Geom3 {
     static constexpr int COLS_G = TC + 4;          // gk: columns -2 .. TC+1
     static constexpr int COLS_BC = TC + 3;         // column faces: -1 .. TC+1
     static constexpr int COLS = TC + 2;            // the others: -1 .. TC
-    static constexpr int NTILE = (EPI == EPI_BINARY) ? 4 : (EPI == EPI_COLD ? 3 : 0);
+    static constexpr int NTILE = (EPI == EPI_BINARY || EPI == EPI_TWIN) ? 4 : (EPI == EPI_COLD ? 3 : 0);
     static constexpr int align128(int b) { return (b + 127) & ~127; }
     // float offsets of the boxes in a stage
     static constexpr int OFF_G = 0;
@@ -147,13 +150,54 @@ __device__ __forceinline__ float face_step(float b, float d, float steps, bool o
         return steps_ok * d + b;
 }
 
+// Projection factor in the Matlab twins' order and precision (mtwin.cu):
+// lower and upper faces along columns, rows, slices; 1/1 is exactly 1, so no
+// division below alpha, and no root where a sum of squares with a margin over
+// all roundings is.
+__device__ __forceinline__ float proj_twin(float a, float b, float d, float e, float p, float q,
+                                           float al)
+{
+    float m = __fmul_rn(a, a);
+    m = __fmaf_rn(b, b, m);
+    m = __fmaf_rn(d, d, m);
+    m = __fmaf_rn(e, e, m);
+    m = __fmaf_rn(p, p, m);
+    m = __fmaf_rn(q, q, m);
+    if (al > 0x1p-40f && m * (0.5f * (1.0f + 0x1p-18f)) < al * al)
+        return 1.0f;
+    float s = __fadd_rn(__fmul_rn(a, a), __fmul_rn(b, b));
+    s = __fadd_rn(s, __fmul_rn(d, d));
+    s = __fadd_rn(s, __fmul_rn(e, e));
+    s = __fadd_rn(s, __fmul_rn(p, p));
+    s = __fadd_rn(s, __fmul_rn(q, q));
+    const float g = __fsqrt_rn(__fmul_rn(s, 0.5f));
+    return (g <= al) ? 1.0f : __fdiv_rn(1.0f, __fdiv_rn(g, al));
+}
+
+// Matlab's min(a, b); a NaN a is kept.
+__device__ __forceinline__ float min_twin(float a, float b) { return (a <= b || a != a) ? a : b; }
+
+// A sum of floats as an unevaluated pair (TwoSum, Knuth): about 48 bits, at
+// float speed (the FP64 pipe would take as long as the rest of the step).
+struct FloatPair {
+    float hi = 0.f, lo = 0.f;
+    __device__ __forceinline__ void add(float x)
+    {
+        const float s = __fadd_rn(hi, x), bv = __fsub_rn(s, hi);
+        lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bv)), __fsub_rn(x, bv)));
+        hi = s;
+    }
+};
+
 template <int TC, int CELLS, int NSTAGE, int EPI, bool EXACT>
 __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
     stencil3d_kernel(const __grid_constant__ BatchArgs B)
 {
     using G = Geom3<TC, CELLS, EPI>;
     constexpr int NT = G::NT, C = CELLS, LR = G::LR, TR = G::TR;
-    constexpr bool BIN = (EPI == EPI_BINARY || EPI == EPI_COLD);
+    constexpr bool BIN = (EPI == EPI_BINARY || EPI == EPI_COLD || EPI == EPI_TWIN);
+    constexpr bool TWIN = (EPI == EPI_TWIN);
+    static_assert(!TWIN || EXACT, "the twins' float operations are IEEE ones");
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ int s_abort;
@@ -241,6 +285,7 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
         const int s_begin = (int)((long long)ns * chunk / chunks);
         const int s_end = (int)((long long)ns * (chunk + 1) / chunks);
         float erru = 0.0f;
+        FloatPair errp;  // the twins sum erriter in double
         const int r0 = (tile % P.tiles_r) * TR;
         const int c0 = (tile / P.tiles_r) * TC;
         const int n_steps = s_end - s_begin + 4;
@@ -405,8 +450,12 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
                 if (j > 0 && !main_w)
                     break;
                 const float dn = (j + 1 < C && main_w) ? br_prev[j + 1 < C ? j + 1 : j] : brd_prev;
-                g2[j] = proj_half<EXACT>(bcr_prev[j], bc_prev[j], dn, br_prev[j], bs[j], bsprev[j],
-                                        alpha_prev[j]);
+                if constexpr (TWIN)
+                    g2[j] = proj_twin(bc_prev[j], bcr_prev[j], br_prev[j], dn, bsprev[j], bs[j],
+                                      alpha_prev[j]);
+                else
+                    g2[j] = proj_half<EXACT>(bcr_prev[j], bc_prev[j], dn, br_prev[j], bs[j], bsprev[j],
+                                             alpha_prev[j]);
             }
             if (main_w)
                 st_cells<C>(G2, g2);
@@ -472,7 +521,7 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
                 }
 #pragma unroll
                 for (int j = 0; j < C; ++j) {
-                    dn[j] = (j + 1 < C ? brr[j + 1 < C ? j + 1 : j] : brr_dn) - brr[j];
+                    const float brr1 = j + 1 < C ? brr[j + 1 < C ? j + 1 : j] : brr_dn;
                     bcc[j] = face_mean<EXACT>(g2[j], g2l[j]) * bc_prev[j];
                     float bcc1 = face_mean<EXACT>(g2r[j], g2[j]) * bcr_prev[j];
                     if (EXACT) {
@@ -481,8 +530,11 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
                         if (!(fc1_ok && in_r[j] && sp_in))
                             bcc1 = 0.f;
                     }
-                    dn[j] = dn[j] + bcc1;
-                    dn[j] = dn[j] - bcc[j];
+                    // the reference adds rows, then columns; the twins the other way
+                    if constexpr (TWIN)
+                        dn[j] = ((bcc1 - bcc[j]) + brr1) - brr[j];
+                    else
+                        dn[j] = ((brr1 - brr[j]) + bcc1) - bcc[j];
                 }
                 if (is_tile) {
                     if (sp >= s_begin && sp < s_end) {
@@ -516,6 +568,24 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
                             }
                             st_rows<C>(d_s0, o, g_o, is_tile, P);
                             st_rows<C>(d_s1, o, v_o, is_tile, P);
+                        } else if constexpr (TWIN) {
+                            float g_o[C], pt_o[C], u_o[C];
+                            const float one_over_cc = P.inv_cc_l;
+#pragma unroll
+                            for (int j = 0; j < C; ++j) {
+                                const float u = tv[TS_S2][j], uc = div_cc<true>(u, cc, inv_cc);
+                                const float ps_n = min_twin(((dv[j] + tv[TS_S1][j]) - uc) + one_over_cc,
+                                                            tv[TS_CS][j]);
+                                pt_o[j] = min_twin((-dv[j] + ps_n) + uc, tv[TS_CT][j]);
+                                const float e = cc * ((dv[j] + pt_o[j]) - ps_n);
+                                if (j == 0 || in_r[j])
+                                    errp.add(fabsf(e));
+                                u_o[j] = u - e;
+                                g_o[j] = dv[j] - ((ps_n - pt_o[j]) + div_cc<true>(u_o[j], cc, inv_cc));
+                            }
+                            st_rows<C>(d_s0, o, g_o, is_tile, P);
+                            st_rows<C>(d_s1, o, pt_o, is_tile, P);
+                            st_rows<C>(d_s2, o, u_o, is_tile, P);
                         } else if constexpr (EPI == EPI_BINARY) {
                             float g_o[C], pt_o[C], u_o[C];
 #pragma unroll
@@ -556,7 +626,8 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
         }
         __syncthreads();  // stage slots and factor planes are reused by the next item
         if constexpr (BIN)
-            finish_item<NT>(erru, P, li, it, B.done_count, s_red, &s_is_last);
+            finish_item<NT, TWIN>(TWIN ? (double)errp.hi + (double)errp.lo : (double)erru, P, li, it,
+                                  B.done_count, s_red, &s_is_last);
     }
 
     // the last block to leave re-arms the queue for the next launch

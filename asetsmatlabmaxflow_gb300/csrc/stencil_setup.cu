@@ -26,7 +26,7 @@ int build_problem_desc(EncodeTiledFn fn, const StencilVariant &v, const StencilP
                        ProblemDesc *A)
 {
     memset(A, 0, sizeof *A);
-    const bool binary = (v.epi == EPI_BINARY || v.epi == EPI_COLD);
+    const bool binary = (v.epi == EPI_BINARY || v.epi == EPI_COLD || v.epi == EPI_TWIN);
     // label extent of each slot's box
     auto box_labels = [&](int labels) { return v.label_boxes == LB_ALL ? labels : 1; };
     for (int par = 0; par < 2; ++par) {
@@ -146,6 +146,24 @@ double choose_split3(const StencilProblem &p, const StencilVariant &v, long long
     d->units_a = bu;
     d->zchunks_a = ba;
     d->zchunks = bb;
+    return best;
+}
+
+double step_cost3(const StencilVariant &v) { return (v.exact ? 10.0 : 4.0) + v.tc; }
+
+const StencilVariant *pick_split3(const StencilProblem &p, const StencilVariant *const *v, int n,
+                                  int num_sms)
+{
+    const StencilVariant *best = nullptr;
+    double best_cost = 0.0;
+    for (int i = 0; i < n; ++i) {
+        ProblemDesc d;
+        const double c = choose_split3(p, *v[i], num_sms, &d) * step_cost3(*v[i]);
+        if (!best || c < best_cost) {
+            best = v[i];
+            best_cost = c;
+        }
+    }
     return best;
 }
 
