@@ -12,12 +12,15 @@
 //   contrast alpha    alpha = a + b*exp(-c*|grad I'|^p), central differences
 //                     inside, one-sided at the border (Matlab's gradient;
 //                     smoothManualSegmentations2D.m:82-91)
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "asets.h"
+#include "device_common.cuh"
 #include "internal.h"
 
 using namespace asets;
@@ -65,7 +68,8 @@ __device__ __forceinline__ bool aligned16(const void *p)
     return (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
 }
 
-// mm[0] = key(min), mm[1] = key(max); NaNs are skipped (as Matlab's min/max).
+// mm[0] = ~key(min), mm[1] = key(max), both from zero; NaNs are skipped (as
+// Matlab's min/max).
 __global__ void minmax_kernel(const float *x, long long n, unsigned int *mm)
 {
     unsigned int lo = 0xFFFFFFFFu, hi = 0u;
@@ -111,25 +115,35 @@ __global__ void minmax_kernel(const float *x, long long n, unsigned int *mm)
             lo = min(lo, s_lo[w]);
             hi = max(hi, s_hi[w]);
         }
-        atomicMin(&mm[0], lo);
+        atomicMax(&mm[0], ~lo);
         atomicMax(&mm[1], hi);
     }
 }
 
 // (I - min) / (max - min), as Matlab's single arithmetic; the range is read
-// once per thread (mm == nullptr: the identity)
+// once per thread (mm == nullptr: the identity).  The quotient is IEEE's:
+// for an ordinary range by the corrected product with its reciprocal (div_by),
+// three operations instead of a division's dozen.
 struct Norm {
-    float lo = 0.f, den = 1.f;
+    float lo = 0.f, den = 1.f, rd = 0.f;  // rd = 0: divide
     bool on = false;
     __device__ explicit Norm(const unsigned int *mm)
     {
         if (mm) {
-            lo = key_float(mm[0]);
+            lo = key_float(~mm[0]);
             den = __fsub_rn(key_float(mm[1]), lo);
+            if (den >= 0x1p-60f && den <= 0x1p60f)
+                rd = __fdiv_rn(1.0f, den);
             on = true;
         }
     }
-    __device__ float operator()(float v) const { return on ? __fdiv_rn(__fsub_rn(v, lo), den) : v; }
+    __device__ float operator()(float v) const
+    {
+        if (!on)
+            return v;
+        const float x = __fsub_rn(v, lo);
+        return rd != 0.f ? div_by(x, den, rd) : __fdiv_rn(x, den);
+    }
 };
 
 __global__ void l1_kernel(const float *img, long long n, Labels m, int L,
@@ -190,29 +204,79 @@ __device__ __forceinline__ float scaled255(float v, const Norm &nrm)
 }
 
 // histc(x, 0:255): bin k holds k <= x < k+1, the last bin also x == 255.
-__global__ void hist_kernel(const float *img, const int *scrib, long long n, int L,
-                            const unsigned int *mm, unsigned int *hist)
+// Scribbles and image are read 16 bytes at a time, several in flight (the
+// image everywhere: loads that wait for a scribble cost more than the lines
+// they save).  256 x 231 x 256, one voxel in twenty scribbled: 36 us (the image
+// only where scribbled: 52; one element at a time: 91).
+__global__ void __launch_bounds__(kThreads) hist_kernel(const float *img, const int *scrib, long long n,
+                                                        int L, const unsigned int *mm, unsigned int *hist)
 {
-    __shared__ unsigned int h[kMaxLabels * kBins];
+    extern __shared__ unsigned int h[];  // L * kBins: as many blocks on an SM as threads allow
     const Norm nrm(mm);
     for (int i = threadIdx.x; i < L * kBins; i += kThreads)
         h[i] = 0;
     __syncthreads();
-    for (long long i = blockIdx.x * (long long)kThreads + threadIdx.x; i < n;
-         i += (long long)gridDim.x * kThreads) {
-        const int lab = scrib[i];
+    auto take = [&](int lab, float v) {
         if (lab < 1 || lab > L)
-            continue;
-        const float x = scaled255(img[i], nrm);
+            return;
+        const float x = scaled255(v, nrm);
         if (!(x >= 0.f && x <= 255.f))
-            continue;
+            return;
         const int b = min((int)floorf(x), kBins - 1);
         atomicAdd(&h[(lab - 1) * kBins + b], 1u);
+    };
+    const long long t0 = blockIdx.x * (long long)kThreads + threadIdx.x;
+    const long long stride = (long long)gridDim.x * kThreads;
+    long long head = 0;
+    if (aligned16(scrib) && aligned16(img)) {
+        const long long n4 = n >> 2;
+        const int4 *s4 = reinterpret_cast<const int4 *>(scrib);
+        const float4 *x4 = reinterpret_cast<const float4 *>(img);
+        constexpr int kAhead = 4;
+        for (long long i = t0; i < n4; i += kAhead * stride) {
+            int4 v[kAhead];
+            float4 x[kAhead];
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                const bool ok = i + j * stride < n4;
+                v[j] = ok ? __ldcs(s4 + i + j * stride) : make_int4(0, 0, 0, 0);
+                x[j] = ok ? __ldg(x4 + i + j * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                take(v[j].x, x[j].x);
+                take(v[j].y, x[j].y);
+                take(v[j].z, x[j].z);
+                take(v[j].w, x[j].w);
+            }
+        }
+        head = n4 << 2;
     }
+    for (long long i = head + t0; i < n; i += stride)
+        take(scrib[i], img[i]);
     __syncthreads();
     for (int i = threadIdx.x; i < L * kBins; i += kThreads)
         if (h[i])
             atomicAdd(&hist[i], h[i]);
+}
+
+// Per-bin cost of label blockIdx.x in double, as the reference's
+// binCounts./sum and -log10(P + epsilon), rounded to float (NaN if no scribble).
+__global__ void __launch_bounds__(kBins) cost_table_kernel(const unsigned int *hist, double eps, float *table)
+{
+    __shared__ unsigned long long s_sum[kBins / 32];
+    const int i = blockIdx.x * kBins + threadIdx.x;
+    const unsigned int h = hist[i];
+    unsigned long long t = h;
+    for (int o = 16; o > 0; o >>= 1)
+        t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0)
+        s_sum[threadIdx.x >> 5] = t;
+    __syncthreads();
+    unsigned long long total = 0;
+    for (int w = 0; w < kBins / 32; ++w)
+        total += s_sum[w];
+    table[i] = (float)(-log10((double)h / (double)total + eps));
 }
 
 // Ct_l = cost_l[uint16(I'*255)]: Matlab's uint16() rounds half away from zero.
@@ -249,111 +313,119 @@ __global__ void lookup_kernel(const float *img, long long n, int L, const unsign
 }
 
 // alpha = a + b*exp(-c*|grad I'|^p) (p = 1 or 2), replicated over L slices.
-// A block owns a 32 (rows) x 8 (columns) tile of kAZ planes and walks them
-// in order: each thread keeps its column's normalised values of the planes
-// z-1, z, z+1 in registers, the tile's plane z and its one-cell halo pass
-// through shared memory, so every voxel is read and normalised once (halo
-// cells once more).  The raw values are loaded four planes ahead (register
-// queues).  At 256^3 the kernel is issue-bound (about 6.5 warp instructions
-// per voxel: the IEEE division of the normalisation, expf, the three
-// one-sided/central differences), not HBM-bound.
-constexpr int kAY = 32, kAX = 8, kAZ = 32;
+// Matlab's gradient: (f(k+1) - f(k-1))/2 inside, one-sided at the ends, 0 on an
+// axis of length 1.  The differences are taken of the image itself and scaled
+// by 1/(max - min) after: closer to the exact gradient than differences of
+// rounded quotients, and no division per voxel.
+//
+// A thread owns VEC (4 or 1) adjacent rows of one column and walks some planes,
+// with the planes z-1, z, z+1 in registers; the rows beside come from the
+// neighbouring lanes, the columns beside from L1 and L2.  16-byte accesses
+// (VEC = 4) where rows are whole multiples of them.  256 x 231 x 256: 52
+// us for one label, 67 for four, which the stores bound (a 32 x 8 tile in
+// shared memory, every voxel normalised: 138 and 152).
+constexpr int kAWarps = 8, kAZ = 16;  // columns and planes of a block
 
-// Matlab gradient along one axis: (f(k+1) - f(k-1))/2 inside, one-sided at
-// the ends, 0 on an axis of length 1
-__device__ __forceinline__ float mgrad(int k, int nk, float lo, float mid, float hi)
+template <int VEC>
+struct Rows {
+    float v[VEC];
+};
+
+template <int VEC>
+__device__ __forceinline__ Rows<VEC> ld_rows(const float *p, bool ok)
 {
-    if (nk < 2)
-        return 0.f;
-    if (k == 0)
-        return __fsub_rn(hi, mid);
-    if (k == nk - 1)
-        return __fsub_rn(mid, lo);
-    return __fmul_rn(__fsub_rn(hi, lo), 0.5f);
+    Rows<VEC> r;
+    if constexpr (VEC == 4) {
+        const float4 t = ok ? __ldg(reinterpret_cast<const float4 *>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        r.v[0] = t.x;
+        r.v[1] = t.y;
+        r.v[2] = t.z;
+        r.v[3] = t.w;
+    } else {
+        r.v[0] = ok ? __ldg(p) : 0.f;
+    }
+    return r;
 }
 
-__global__ void __launch_bounds__(kAY * kAX)
-    alpha_kernel(const float *img, int ny, int nx, int nz, const unsigned int *mm, float a,
-                 float b, float c, int squared, int L, float *alpha)
+// sqrt(x) for x >= 0: the hardware reciprocal root with one Newton correction
+// of x*rsqrt(x) (zero, subnormal and non-finite values take the IEEE root)
+__device__ __forceinline__ float root(float x)
 {
-    __shared__ float pl[kAX + 2][kAY + 2];
-    const int ty = threadIdx.x, tx = threadIdx.y;
-    const int y = blockIdx.x * kAY + ty, x = blockIdx.y * kAX + tx;
-    const int z0 = blockIdx.z * kAZ, z1 = min(nz, z0 + kAZ);
-    const bool in = (y < ny && x < nx);
+    if (!(x >= 0x1p-100f && x <= 0x1p100f))
+        return __fsqrt_rn(x);
+    const float r = rsqrtf(x), s = __fmul_rn(x, r);
+    return __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, r), s);
+}
+
+template <int VEC>
+__global__ void __launch_bounds__(32 * kAWarps)
+    alpha_kernel(const float *img, int ny, int nx, int nz, const unsigned int *mm, float a, float b, float c,
+                 int squared, int L, int az, float *alpha)
+{
+    const int lane = threadIdx.x & 31;
+    const int y = (blockIdx.x * 32 + lane) * VEC, x = blockIdx.y * kAWarps + (threadIdx.x >> 5);
+    if (x >= nx)
+        return;  // a whole warp
+    const int z0 = blockIdx.z * az, z1 = min(nz, z0 + az);
+    const bool in = y < ny;
     const long long plane = (long long)ny * nx, n = plane * nz;
-    const long long col = (long long)x * ny + y;
-    const Norm nrm(mm);
-    // halo roles: the first/last row of the tile reads the row outside it,
-    // the first/last column the column outside it (inside the volume only)
-    const int yy = (ty == 0) ? y - 1 : (ty == kAY - 1 ? y + 1 : -1);
-    const int xx = (tx == 0) ? x - 1 : (tx == kAX - 1 ? x + 1 : -1);
-    const bool yh = in && yy >= 0 && yy < ny;
-    const bool xh = in && xx >= 0 && xx < nx;
-    const long long ycol = (long long)x * ny + yy, xcol = (long long)xx * ny + y;
-    auto ld = [&](bool ok, int z, long long off) {
-        return ok ? __ldg(img + (long long)z * plane + off) : 0.f;
-    };
-    float v = 0.f, vm = 0.f;
-    if (in) {
-        v = nrm(img[(long long)z0 * plane + col]);
-        vm = z0 > 0 ? nrm(img[(long long)(z0 - 1) * plane + col]) : v;
+    const float *p = img + (long long)x * ny + y;
+    // 1/(max - min); a range that is not finite gives what the quotients would
+    float den = 1.f, rd = 1.f;
+    if (mm) {
+        const float lo = key_float(~mm[0]);
+        den = __fsub_rn(key_float(mm[1]), lo);
+        rd = fabsf(lo) < INFINITY ? __fdiv_rn(1.f, den) : NAN;
     }
-    // raw centre values of the planes z+1 .. z+4, halo values of z .. z+3
-    float c1 = ld(in && z0 + 1 < nz, z0 + 1, col), c2 = ld(in && z0 + 2 < nz, z0 + 2, col);
-    float c3 = ld(in && z0 + 3 < nz, z0 + 3, col), c4 = ld(in && z0 + 4 < nz, z0 + 4, col);
-    float y0 = ld(yh, z0, ycol), y1 = ld(yh && z0 + 1 < z1, z0 + 1, ycol);
-    float y2 = ld(yh && z0 + 2 < z1, z0 + 2, ycol), y3 = ld(yh && z0 + 3 < z1, z0 + 3, ycol);
-    float x0 = ld(xh, z0, xcol), x1 = ld(xh && z0 + 1 < z1, z0 + 1, xcol);
-    float x2 = ld(xh && z0 + 2 < z1, z0 + 2, xcol), x3 = ld(xh && z0 + 3 < z1, z0 + 3, xcol);
-    // unrolled by the queue depth, so that the queues rotate by renaming
-    // rather than by moves (a move of a pending load waits for it)
-#pragma unroll 4
+    const bool plain = !mm || !(den < 0x1p-100f);  // else 1/den may overflow: divide
+    auto unit = [&](float d) { return plain ? __fmul_rn(d, rd) : __fdiv_rn(d, den); };
+    const bool x_lo = x > 0, x_up = x + 1 < nx;
+    const float sx = (x_lo && x_up) ? 0.5f : 1.f;
+    // the rows beyond the warp's 32*VEC
+    const bool edge_lo = lane == 0 && in && y > 0, edge_up = lane == 31 && y + VEC < ny;
+    const long long z_off = (long long)z0 * plane;
+    Rows<VEC> cur = ld_rows<VEC>(p + z_off, in), lo = z0 > 0 ? ld_rows<VEC>(p + z_off - plane, in) : cur;
     for (int z = z0; z < z1; ++z) {
-        const float vp = (in && z + 1 < nz) ? nrm(c1) : v;
-        const float hyv = yh ? nrm(y0) : v, hxv = xh ? nrm(x0) : v;
-        c1 = c2;
-        c2 = c3;
-        c3 = c4;
-        c4 = ld(in && z + 5 < nz, z + 5, col);
-        y0 = y1;
-        y1 = y2;
-        y2 = y3;
-        y3 = ld(yh && z + 4 < z1, z + 4, ycol);
-        x0 = x1;
-        x1 = x2;
-        x2 = x3;
-        x3 = ld(xh && z + 4 < z1, z + 4, xcol);
-        __syncthreads();  // the previous plane's readers are done
-        pl[tx + 1][ty + 1] = v;
-        // a halo slot is read only by the thread that writes it
-        if (in) {
-            if (ty == 0)
-                pl[tx + 1][0] = hyv;
-            if (ty == kAY - 1)
-                pl[tx + 1][kAY + 1] = hyv;
-            if (tx == 0)
-                pl[0][ty + 1] = hxv;
-            if (tx == kAX - 1)
-                pl[kAX + 1][ty + 1] = hxv;
-        }
-        __syncthreads();
-        if (in) {
-            const float gy = mgrad(y, ny, pl[tx + 1][ty], v, pl[tx + 1][ty + 2]);
-            const float gx = mgrad(x, nx, pl[tx][ty + 1], v, pl[tx + 2][ty + 1]);
-            float g2 = __fadd_rn(__fmul_rn(gx, gx), __fmul_rn(gy, gy));
+        const float *q = p + (long long)z * plane;
+        const Rows<VEC> up = z + 1 < nz ? ld_rows<VEC>(q + plane, in) : cur;
+        const Rows<VEC> xl = x_lo ? ld_rows<VEC>(q - ny, in) : cur;
+        const Rows<VEC> xu = x_up ? ld_rows<VEC>(q + ny, in) : cur;
+        float yl = __shfl_up_sync(0xffffffffu, cur.v[VEC - 1], 1);
+        float yu = __shfl_down_sync(0xffffffffu, cur.v[0], 1);
+        if (edge_lo)
+            yl = __ldg(q - 1);
+        if (edge_up)
+            yu = __ldg(q + VEC);
+        const float sz = (z > 0 && z + 1 < nz) ? 0.5f : 1.f;
+        float al[VEC];
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            const int yy = y + j;
+            const bool y_lo = yy > 0, y_up = yy + 1 < ny;
+            const float vl = y_lo ? (j ? cur.v[j - 1] : yl) : cur.v[j];
+            const float vu = y_up ? (j + 1 < VEC ? cur.v[j + 1 < VEC ? j + 1 : j] : yu) : cur.v[j];
+            // an axis of length 1 adds nothing, whatever the value there
+            const float gy = ny < 2 ? 0.f : unit(__fmul_rn(__fsub_rn(vu, vl), (y_lo && y_up) ? 0.5f : 1.f));
+            const float gx = nx < 2 ? 0.f : unit(__fmul_rn(__fsub_rn(xu.v[j], xl.v[j]), sx));
+            float g2 = __fmaf_rn(gx, gx, __fmul_rn(gy, gy));
             if (nz > 1) {
-                const float gz = mgrad(z, nz, vm, v, vp);
-                g2 = __fadd_rn(g2, __fmul_rn(gz, gz));
+                const float gz = unit(__fmul_rn(__fsub_rn(up.v[j], lo.v[j]), sz));
+                g2 = __fmaf_rn(gz, gz, g2);
             }
-            const float t = squared ? g2 : __fsqrt_rn(g2);
-            const float al = __fadd_rn(a, __fmul_rn(b, expf(__fmul_rn(-c, t))));
-            const long long i = (long long)z * plane + col;
-            for (int l = 0; l < L; ++l)
-                __stcs(alpha + l * n + i, al);
+            const float t = squared ? g2 : root(g2);
+            al[j] = __fadd_rn(a, __fmul_rn(b, expf(__fmul_rn(-c, t))));
         }
-        vm = v;
-        v = vp;
+        if (in) {
+            float *o = alpha + (long long)z * plane + (long long)x * ny + y;
+            for (int l = 0; l < L; ++l) {
+                if constexpr (VEC == 4)
+                    __stcs(reinterpret_cast<float4 *>(o + l * n), make_float4(al[0], al[1], al[2], al[3]));
+                else
+                    __stcs(o + l * n, al[0]);
+            }
+        }
+        lo = cur;
+        cur = up;
     }
 }
 
@@ -435,19 +507,16 @@ cudaError_t finish(Scratch &s, View<T> &v)
     return cudaSuccess;
 }
 
-cudaError_t run_minmax(Scratch &s, const float *x, long long n, int sms, unsigned int **mm)
+// Scratch words of a call, set to zero: the range (two words) first.
+cudaError_t zeroed(Scratch &s, size_t words, unsigned int **p)
 {
-    cudaError_t e = s.get(mm, 2 * sizeof(unsigned int));
-    if (e != cudaSuccess)
-        return e;
-    // key(min) starts at 0xFFFFFFFF, key(max) at 0 (device-side sets, no
-    // staging of a pageable host word)
-    e = cudaMemsetAsync(*mm, 0xFF, sizeof(unsigned int), s.st);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(*mm + 1, 0, sizeof(unsigned int), s.st);
-    if (e != cudaSuccess)
-        return e;
-    minmax_kernel<<<grid_for(n, sms), kThreads, 0, s.st>>>(x, n, *mm);
+    cudaError_t e = s.get(p, words * sizeof(unsigned int));
+    return e == cudaSuccess ? cudaMemsetAsync(*p, 0, words * sizeof(unsigned int), s.st) : e;
+}
+
+cudaError_t run_minmax(Scratch &s, const float *x, long long n, int sms, unsigned int *mm)
+{
+    minmax_kernel<<<grid_for(n, sms), kThreads, 0, s.st>>>(x, n, mm);
     return cudaGetLastError();
 }
 
@@ -478,8 +547,10 @@ extern "C" ASETS_API asets_status asets_cost_l1(asets_context *ctx, asets_memory
     CT_TRY(in_view(s, where, img, (size_t)n, vi));
     CT_TRY(out_view(s, where, Ct, (size_t)n * L, vo));
     unsigned int *mm = nullptr;
-    if (normalize)
-        CT_TRY(run_minmax(s, vi.d, n, context_num_sms(ctx), &mm));
+    if (normalize) {
+        CT_TRY(zeroed(s, 2, &mm));
+        CT_TRY(run_minmax(s, vi.d, n, context_num_sms(ctx), mm));
+    }
     Labels m{};
     for (int l = 0; l < L; ++l)
         m.v[l] = models[l];
@@ -529,37 +600,23 @@ extern "C" ASETS_API asets_status asets_cost_histogram_ll(asets_context *ctx, as
     CT_TRY(in_view(s, where, img, (size_t)n, vi));
     CT_TRY(in_view(s, where, scribbles, (size_t)n, vs));
     CT_TRY(out_view(s, where, Ct, (size_t)n * L, vo));
-    unsigned int *mm = nullptr, *hist = nullptr;
-    float *table = nullptr;
-    CT_TRY(run_minmax(s, vi.d, n, sms, &mm));
-    CT_TRY(s.get(&hist, (size_t)L * kBins * sizeof(unsigned int)));
-    CT_TRY(cudaMemsetAsync(hist, 0, (size_t)L * kBins * sizeof(unsigned int), s.st));
-    hist_kernel<<<grid_for(n, sms), kThreads, 0, s.st>>>(vi.d, vs.d, n, L, mm, hist);
+    // the range, the counts and (written whole) the table
+    const size_t bins = (size_t)L * kBins;
+    unsigned int *mm = nullptr;
+    CT_TRY(zeroed(s, 2 + 2 * bins, &mm));
+    unsigned int *hist = mm + 2;
+    float *table = reinterpret_cast<float *>(hist + bins);
+    CT_TRY(run_minmax(s, vi.d, n, sms, mm));
+    hist_kernel<<<grid_for(n, sms), kThreads, bins * sizeof(unsigned int), s.st>>>(vi.d, vs.d, n, L, mm, hist);
     CT_TRY(cudaGetLastError());
-    // per-bin cost on the host in double, as the reference's binCounts./sum
-    // and -log10(P + epsilon)
-    std::vector<unsigned int> h((size_t)L * kBins);
-    CT_TRY(cudaMemcpyAsync(h.data(), hist, h.size() * sizeof(unsigned int), cudaMemcpyDeviceToHost,
-                           s.st));
-    CT_TRY(cudaStreamSynchronize(s.st));
-    std::vector<float> tab((size_t)L * kBins);
-    for (int l = 0; l < L; ++l) {
-        double total = 0.0;
-        for (int k = 0; k < kBins; ++k)
-            total += (double)h[(size_t)l * kBins + k];
-        for (int k = 0; k < kBins; ++k) {
-            const double p = (double)h[(size_t)l * kBins + k] / total;  // NaN if no scribble
-            tab[(size_t)l * kBins + k] = (float)(-std::log10(p + eps));
-        }
-    }
-    if (hist_out)
-        memcpy(hist_out, h.data(), h.size() * sizeof(unsigned int));
-    CT_TRY(s.get(&table, tab.size() * sizeof(float)));
-    CT_TRY(cudaMemcpyAsync(table, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice,
-                           s.st));
+    cost_table_kernel<<<L, kBins, 0, s.st>>>(hist, eps, table);
+    CT_TRY(cudaGetLastError());
     lookup_kernel<<<grid_for(n, sms), kThreads, 0, s.st>>>(vi.d, n, L, mm, table, vo.d);
     CT_TRY(cudaGetLastError());
     CT_TRY(finish(s, vo));
+    if (hist_out)
+        CT_TRY(cudaMemcpyAsync(hist_out, hist, bins * sizeof(unsigned int),
+                               cudaMemcpyDeviceToHost, s.st));
     CT_TRY(cudaStreamSynchronize(s.st));
     return ASETS_OK;
 }
@@ -570,7 +627,7 @@ extern "C" ASETS_API asets_status asets_alpha_contrast(asets_context *ctx, asets
                                                        int squared, int L, float *alpha)
 {
     if (!ctx || !img || !alpha || Ny < 1 || Nx < 1 || Nz < 1 || L < 1 ||
-        (Nx + kAX - 1) / kAX > 65535 || (Nz + kAZ - 1) / kAZ > 65535) {
+        (Nx - 1) / kAWarps > 65534 || (Nz - 1) / 32 > 65534) {
         set_last_error("asets_alpha_contrast: bad arguments");
         return ASETS_ERR_INVALID_ARG;
     }
@@ -582,11 +639,21 @@ extern "C" ASETS_API asets_status asets_alpha_contrast(asets_context *ctx, asets
     CT_TRY(in_view(s, where, img, (size_t)n, vi));
     CT_TRY(out_view(s, where, alpha, (size_t)n * L, vo));
     unsigned int *mm = nullptr;
-    if (normalize)
-        CT_TRY(run_minmax(s, vi.d, n, sms, &mm));
-    const dim3 agrid((Ny + kAY - 1) / kAY, (Nx + kAX - 1) / kAX, (Nz + kAZ - 1) / kAZ);
-    alpha_kernel<<<agrid, dim3(kAY, kAX), 0, s.st>>>(vi.d, Ny, Nx, Nz, mm, a, b, c, squared, L,
-                                                      vo.d);
+    if (normalize) {
+        CT_TRY(zeroed(s, 2, &mm));
+        CT_TRY(run_minmax(s, vi.d, n, sms, mm));
+    }
+    const int az = std::max(kAZ, (Nz + 65534) / 65535);  // planes per block: the grid's z extent
+    auto launch = [&](auto vec) {
+        constexpr int V = decltype(vec)::value;
+        const dim3 grid((Ny + 32 * V - 1) / (32 * V), (Nx + kAWarps - 1) / kAWarps, (Nz + az - 1) / az);
+        alpha_kernel<V><<<grid, 32 * kAWarps, 0, s.st>>>(vi.d, Ny, Nx, Nz, mm, a, b, c, squared, L, az, vo.d);
+    };
+    const bool vec4 = (Ny & 3) == 0 && ((reinterpret_cast<uintptr_t>(vi.d) | reinterpret_cast<uintptr_t>(vo.d)) & 15) == 0;
+    if (vec4)
+        launch(std::integral_constant<int, 4>{});
+    else
+        launch(std::integral_constant<int, 1>{});
     CT_TRY(cudaGetLastError());
     CT_TRY(finish(s, vo));
     CT_TRY(cudaStreamSynchronize(s.st));
