@@ -3,12 +3,21 @@
 //
 // Activations are channels-last, 16 channels of BF16 per voxel
 // ([z][x][y][16]).  A convolution is an implicit GEMM: an output tile is 128
-// consecutive voxels along y at one (x, z) (M = 128), each of the 27 taps is
-// one MMA with K = 16 input channels and N = 16 output channels, and the
-// accumulator (128 x 16 FP32) lives in TMEM.  One 5D TMA load per tile stages
-// the 3 x 3 neighbouring rows, y-1 .. y+128, zero-filled outside the volume
-// (the convolution's zero padding), as [row][channel half][voxel][8 channels]:
-// the no-swizzle K-major layout in which a tap's A operand is a plain offset.
+// voxels of one z (M = 128), each of the 27 taps is one MMA with K = 16 input
+// channels and N = 16 output channels, and the accumulator (128 x 16 FP32)
+// lives in TMEM.  One 5D TMA load per tile stages the tile's rows and their
+// neighbours, zero-filled outside the volume (the convolution's zero padding),
+// as [row][channel half][voxel][8 channels]: the no-swizzle K-major layout in
+// which a tap's A operand is a plain offset.
+//
+// The operand's sixteen groups of eight voxels lie at a fixed distance: a
+// tile is eight voxels along y at 16 x, whose neighbourhood is 3 x 18 rows of
+// ten voxels (4.2 loaded for each of the tile; 128 along y at one x: 9, and
+// three quarters of a tile empty at 32^3).  A layer is bound by its fixed part
+// when the volume is small and by the MMAs when it is large (27 at 28 ns a
+// tile): 8.3 us at 32^3 and 12 us at 128 x 32 x 32, where a tile of 128 along y
+// at one x, loaded in runs of 128 bytes, took 24 and 22.  Two blocks an SM
+// overlap one's start and end with the other's work.
 //
 // The same kernel computes the data gradient: with `flip` the taps are
 // mirrored and the weight matrix transposed.  The weight gradient is a
@@ -27,16 +36,12 @@ namespace asets {
 constexpr int kConvThreads = 192;            // warp 0: TMA, warp 1: MMA, warps 2-5: epilogue
 constexpr int kConvStages = 4;               // TMA ring depth
 constexpr int kConvAcc = 8;                  // TMEM accumulators (16 FP32 columns each)
-constexpr int kConvRows = 9;                 // (dz, dx) neighbour rows
-// Staged voxels per row: channels-last input y-1 .. y+128 (130, loaded in
-// 16-byte runs); half-planar input y-8 .. y+135 (144 = 18 groups of 8
-// voxels, loaded in 128-byte runs from rows padded to a multiple of 8).
-constexpr int kConvVoxCL = 130, kConvVoxHP = 144;
-constexpr int kConvStageStride = (kConvRows * 2 * kConvVoxHP * 16 + 127) / 128 * 128;  // 41,472
+constexpr int kConvHalfBytes = 10 * 16, kConvRowBytes = 2 * kConvHalfBytes;
+constexpr int kConvStageStride = (3 * 18 * kConvRowBytes + 127) / 128 * 128;  // 17,280
 constexpr int kConvTapBytes = 2 * 16 * 16;              // B operand of one tap
 constexpr int kConvWBytes = 27 * kConvTapBytes;         // 13,824 B
-// + 32 KB: operand descriptors can only address inside the allocation
-constexpr int kConvSmem = kConvStages * kConvStageStride + kConvWBytes + 128 + 32768;
+constexpr int kConvSmem = kConvStages * kConvStageStride + kConvWBytes + 128;
+static_assert(2 * (kConvSmem + 1024) <= 227 * 1024, "two blocks an SM");
 
 struct ConvTcArgs {
     CUtensorMap act;           // 5D view (8 ch, y, half, x, z) of the BF16 input
@@ -46,12 +51,12 @@ struct ConvTcArgs {
     const float *addend;       // [v][16] FP32 or null: added before ReLU and mask
     void *out;                 // [v][16] BF16 or FP32
     int *err;
-    int ny, nx, nz, ytiles;
+    int ny, nx, nz;
+    int ytiles, xtiles;        // tiles of 8 x 16 voxels
     int relu, out_fp32, flip;
     int hp_in, hp_out;         // half-planar BF16 input (and mask) / output
     int ypad;                  // half-planar row length (ny rounded up to 8)
-    int half_bytes, row_bytes, stage_bytes;  // staged layout: [row][half][voxel][8]
-    int vox_base;              // staged voxel of y - 1 is vox_base - 1 (1 or 8)
+    int stage_bytes, plane_bytes;  // of the staged [z][x][half][voxel][8], of one z of it
 };
 
 // Warp-specialised: warp 0 (one lane) keeps a ring of kConvStages tile
@@ -64,7 +69,7 @@ struct ConvTcArgs {
 // of MMAs.  Every wait is bounded; a timeout raises the shared abort flag,
 // every role leaves its loop, the producer waits (bounded) for its copies
 // in flight and the MMA lane for its last commit before TMEM is freed.
-__global__ void __launch_bounds__(kConvThreads, 1) conv3_tc_kernel(const __grid_constant__ ConvTcArgs A)
+__global__ void __launch_bounds__(kConvThreads, 2) conv3_tc_kernel(const __grid_constant__ ConvTcArgs A)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint64_t full_bar[kConvStages], empty_bar[kConvStages];
@@ -91,12 +96,36 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3_tc_kernel(const __grid_
     if (warp == 1)
         tmem_alloc(&s_tmem, kConvAcc * 16);
 
-    // B operands: tap t as [k half][n][8 k] (core matrices of 8 n x 8 k)
-    for (int i = tid; i < 27 * 16 * 16; i += kConvThreads) {
-        const int t = i / 256, k = (i / 16) % 16, n = i % 16;
-        const __nv_bfloat16 v = A.flip ? A.w[(26 - t) * 256 + n * 16 + k] : A.w[t * 256 + k * 16 + n];
-        const int off = t * kConvTapBytes + (k / 8) * 256 + n * 16 + (k % 8) * 2;
-        *reinterpret_cast<__nv_bfloat16 *>(wsm + off) = v;
+    const int ntiles = A.ytiles * A.xtiles * A.nz;
+    const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    auto issue = [&](int j) {
+        const int st = j % kConvStages, tile = blockIdx.x + j * gridDim.x;
+        const int yt = tile % A.ytiles, rest = tile / A.ytiles;
+        const int y = yt * 8, x = rest % A.xtiles * 16, z = rest / A.xtiles;
+        mbar_arrive_expect_tx(&full_bar[st], A.stage_bytes);
+        tma_load_5d(smem + st * kConvStageStride, &A.act, A.hp_in ? 2 * (y - 1) : 0, A.hp_in ? 0 : y - 1, 0,
+                    x - 1, z - 1, &full_bar[st]);
+    };
+    int issued = 0;
+    if (tid == 0)  // the first tiles load while the other warps lay out the weights
+        for (; issued < kConvStages && issued < mine; ++issued)
+            issue(issued);
+
+    // B operands: tap t as [k half][n][8 k] (core matrices of 8 n x 8 k).  A
+    // thread's eight loads are independent: one round trip each for the five
+    // or six groups, where one load per iteration took 36 (a third of a
+    // layer's time at 32^3).
+#pragma unroll 3
+    for (int i = tid - 32; warp > 0 && i < 27 * 32; i += kConvThreads - 32) {
+        const int t = i / 32, half = (i / 16) & 1, n = i % 16;
+        __align__(16) __nv_bfloat16 v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int k = half * 8 + e;
+            v[e] = A.flip ? A.w[(26 - t) * 256 + n * 16 + k] : A.w[t * 256 + k * 16 + n];
+        }
+        *reinterpret_cast<uint4 *>(wsm + t * kConvTapBytes + half * 256 + n * 16) =
+            *reinterpret_cast<const uint4 *>(v);
     }
     fence_proxy_async_smem();
     tc_fence_before_sync();
@@ -104,29 +133,14 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3_tc_kernel(const __grid_
     tc_fence_after_sync();
     const uint32_t tmem = s_tmem;
 
-    const int ntiles = A.ytiles * A.nx * A.nz;
-    const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-
     if (warp == 0) {
         // ---- producer
-        int issued = 0;
         if (lane == 0) {
-            for (int j = 0; j < mine; ++j) {
-                const int st = j % kConvStages;
-                if (j >= kConvStages &&
-                    !mbar_wait_bounded(&empty_bar[st], ((j / kConvStages) - 1) & 1, &s_abort))
+            for (; issued < mine; ++issued) {
+                const int st = issued % kConvStages;
+                if (!mbar_wait_bounded(&empty_bar[st], ((issued / kConvStages) - 1) & 1, &s_abort))
                     break;
-                const int tile = blockIdx.x + j * gridDim.x;
-                const int yt = tile % A.ytiles, rest = tile / A.ytiles;
-                const int x = rest % A.nx, z = rest / A.nx;
-                mbar_arrive_expect_tx(&full_bar[st], A.stage_bytes);
-                if (A.hp_in)  // 18 groups of 8 voxels from y - 8
-                    tma_load_5d(smem + st * kConvStageStride, &A.act, 0, yt * 16 - 1, 0, x - 1,
-                                z - 1, &full_bar[st]);
-                else
-                    tma_load_5d(smem + st * kConvStageStride, &A.act, 0, yt * 128 - 1, 0, x - 1,
-                                z - 1, &full_bar[st]);
-                ++issued;
+                issue(issued);
             }
             if (s_abort) {
                 // drain the copies in flight of this CTA (bounded)
@@ -150,12 +164,11 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3_tc_kernel(const __grid_
                     !mbar_wait_bounded(&acce_bar[slot], ((j / kConvAcc) - 1) & 1, &s_abort))
                     break;
                 tc_fence_after_sync();
-                const uint32_t a0 =
-                    smem_addr(smem + st * kConvStageStride) + (A.vox_base - 1) * 16;
+                const uint32_t a0 = smem_addr(smem + st * kConvStageStride);
                 for (int t = 0; t < 27; ++t) {
                     const int dz = t / 9, dx = (t / 3) % 3, dy = t % 3;
-                    const uint32_t a = a0 + (dz * 3 + dx) * A.row_bytes + dy * 16;
-                    const uint64_t ad = umma_smem_desc(a, A.half_bytes, 128);
+                    const uint32_t a = a0 + dz * A.plane_bytes + dx * kConvRowBytes + dy * 16;
+                    const uint64_t ad = umma_smem_desc(a, kConvHalfBytes, kConvRowBytes);
                     const uint64_t bd = umma_smem_desc(b0 + t * kConvTapBytes, 256, 128);
                     umma_bf16(tmem + slot * 16, ad, bd, idesc, t > 0 ? 1u : 0u);
                 }
@@ -191,9 +204,9 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3_tc_kernel(const __grid_
                              : "memory");
             const int tile = blockIdx.x + j * gridDim.x;
             const int yt = tile % A.ytiles, rest = tile / A.ytiles;
-            const int x = rest % A.nx, z = rest / A.nx;
-            const int y = yt * 128 + 32 * q + lane;
-            if (y < A.ny) {
+            const int m = 32 * q + lane, z = rest / A.xtiles;
+            const int x = rest % A.xtiles * 16 + (m >> 3), y = yt * 8 + (m & 7);
+            if (y < A.ny && x < A.nx) {
                 const long long v = ((long long)z * A.nx + x) * A.ny + y;
                 float o[16];
 #pragma unroll
@@ -268,29 +281,32 @@ cudaError_t launch_conv3_tc(EncodeTiledFn encode, const ConvLaunch &c, int num_s
     ConvTcArgs A;
     memset(&A, 0, sizeof A);
     // The BF16 input as (8 ch, y, half, x, z) for channels-last
-    // [z][x][y][16]; half-planar [z][x][half][ypad][8] as (64 = 8 voxels x 8
-    // ch, ypad/8 groups, half, x, z), whose 128-byte inner box is one burst.
-    const int ypad = (c.ny + 7) / 8 * 8;
+    // [z][x][y][16]; half-planar [z][x][half][ypad][8] as (ypad voxels of two
+    // 8-byte elements, 1, half, x, z), so that a box row is one run of memory.
+    // No more rows than a narrow volume has: what stays in the stage from
+    // another tile meets only outputs past the volume.
+    const int ypad = (c.ny + 7) / 8 * 8, xrows = c.nx < 16 ? c.nx + 2 : 18;
     cuuint64_t dims[5], strides[4];
     cuuint32_t box[5];
     if (c.hp_in) {
-        const cuuint64_t d[5] = {64, (cuuint64_t)ypad / 8, 2, (cuuint64_t)c.nx, (cuuint64_t)c.nz};
-        const cuuint64_t s[4] = {128, (cuuint64_t)16 * ypad, (cuuint64_t)32 * ypad,
+        const cuuint64_t d[5] = {(cuuint64_t)ypad * 2, 1, 2, (cuuint64_t)c.nx, (cuuint64_t)c.nz};
+        const cuuint64_t s[4] = {(cuuint64_t)16 * ypad, (cuuint64_t)16 * ypad, (cuuint64_t)32 * ypad,
                                  (cuuint64_t)32 * ypad * c.nx};
-        const cuuint32_t b[5] = {64, kConvVoxHP / 8, 2, 3, 3};
+        const cuuint32_t b[5] = {20, 1, 2, (cuuint32_t)xrows, 3};
         memcpy(dims, d, sizeof d);
         memcpy(strides, s, sizeof s);
         memcpy(box, b, sizeof b);
     } else {
         const cuuint64_t d[5] = {8, (cuuint64_t)c.ny, 2, (cuuint64_t)c.nx, (cuuint64_t)c.nz};
         const cuuint64_t s[4] = {32, 16, (cuuint64_t)32 * c.ny, (cuuint64_t)32 * c.ny * c.nx};
-        const cuuint32_t b[5] = {8, kConvVoxCL, 2, 3, 3};
+        const cuuint32_t b[5] = {8, 10, 2, (cuuint32_t)xrows, 3};
         memcpy(dims, d, sizeof d);
         memcpy(strides, s, sizeof s);
         memcpy(box, b, sizeof b);
     }
     cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    CUresult r = encode(&A.act, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void *>(c.x), dims,
+    CUresult r = encode(&A.act, c.hp_in ? CU_TENSOR_MAP_DATA_TYPE_INT64 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5,
+                        const_cast<void *>(c.x), dims,
                         strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -305,24 +321,22 @@ cudaError_t launch_conv3_tc(EncodeTiledFn encode, const ConvLaunch &c, int num_s
     A.ny = c.ny;
     A.nx = c.nx;
     A.nz = c.nz;
-    A.ytiles = (c.ny + 127) / 128;
+    A.ytiles = ypad / 8;
+    A.xtiles = (c.nx + 15) / 16;
     A.relu = c.relu;
     A.out_fp32 = c.out_fp32;
     A.flip = c.flip;
     A.hp_in = c.hp_in;
     A.hp_out = c.hp_out;
     A.ypad = ypad;
-    const int vox = c.hp_in ? kConvVoxHP : kConvVoxCL;
-    A.half_bytes = vox * 16;
-    A.row_bytes = 2 * vox * 16;
-    A.stage_bytes = kConvRows * A.row_bytes;
-    A.vox_base = c.hp_in ? 8 : 1;
+    A.plane_bytes = xrows * kConvRowBytes;
+    A.stage_bytes = 3 * A.plane_bytes;
     cudaError_t e = cudaFuncSetAttribute(conv3_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kConvSmem);
     if (e != cudaSuccess)
         return e;
-    const int tiles = A.ytiles * c.nx * c.nz;
-    const int grid = tiles < num_sms ? tiles : num_sms;
+    const int tiles = A.ytiles * A.xtiles * c.nz;
+    const int grid = tiles < 2 * num_sms ? tiles : 2 * num_sms;
     conv3_tc_kernel<<<grid, kConvThreads, kConvSmem, st>>>(A);
     return cudaGetLastError();
 }

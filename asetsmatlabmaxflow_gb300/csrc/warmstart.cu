@@ -135,29 +135,6 @@ struct NetIO {
     float *u, *ps, *pt, *bx, *by, *bz;  // Matlab layout, label slowest
 };
 
-__global__ void pack_target_kernel(NetIO io, float *t, long long n, int L)
-{
-    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < n;
-         g += (long long)gridDim.x * blockDim.x) {
-        const float ia = 1.f / io.alpha[g];
-        for (int c = 0; c < kOut; ++c) {
-            float f = 0.f;
-            if (c < L)
-                f = io.u[c * n + g];
-            else if (c == L)
-                f = io.ps[g];
-            else if (c <= 2 * L)
-                f = io.pt[(c - L - 1) * n + g];
-            else if (c <= 5 * L) {
-                const int k = c - 2 * L - 1, axis = k / L, l = k % L;
-                const float *b = axis == 0 ? io.bx : (axis == 1 ? io.by : io.bz);
-                f = b[l * n + g] * ia;
-            }
-            t[out_index(c, g, n)] = f;
-        }
-    }
-}
-
 __global__ void unpack_output_kernel(const float *out, NetIO io, long long n, int L)
 {
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < n;
@@ -179,36 +156,72 @@ __global__ void unpack_output_kernel(const float *out, NetIO io, long long n, in
     }
 }
 
-// Mean squared error over the 5L+1 used output channels; writes the
-// gradient w.r.t. the output (BF16, per 16-channel block half-planar like
-// the activations: [2][z][x][half][ypad][8]) and accumulates the loss.
-__global__ void loss_kernel(const float *out, const float *tgt, __nv_bfloat16 *g, long long n,
-                            int used, float scale, float *loss, int ny)
+// Mean squared error over the 5L+1 used output channels against the solver
+// state; writes the gradient w.r.t. the output (BF16, per 16-channel block
+// half-planar like the activations: [2][z][x][half][ypad][8]) and accumulates
+// the loss.  blockIdx.y is an eight-channel part; a thread has one voxel of
+// it: coalesced reads of every target array, one 16-byte store.  32^3, L = 6:
+// 5.5 us (targets packed first, one channel per thread: 42).
+constexpr int kLossThreads = 256;
+__global__ void __launch_bounds__(kLossThreads) loss_kernel(const float *out, const NetIO io,
+                                                            __nv_bfloat16 *g, long long n, int L, float scale,
+                                                            float *loss, int ny)
 {
+    __shared__ float s_acc[kLossThreads / 32];
+    __shared__ const float *s_src[8];  // targets: u, ps, pt, then the flow over alpha
+    const int part = blockIdx.y, blk = part >> 1, half = part & 1, used = 5 * L + 1;
+    const long long yp = (ny + 7) / 8 * 8, pn = yp * (n / ny);  // padded voxels of one 16-channel block
+    if (threadIdx.x < 8) {
+        const int c = part * 8 + threadIdx.x, k = c - 2 * L - 1, axis = k / L;
+        s_src[threadIdx.x] = c < L     ? io.u + c * n
+                             : c == L  ? io.ps
+                             : k < 0   ? io.pt + (c - L - 1) * n
+                             : axis < 3 ? (axis == 0 ? io.bx : axis == 1 ? io.by : io.bz) + (k - axis * L) * n
+                                       : nullptr;
+    }
+    __syncthreads();
     float acc = 0.f;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 2 * n * 16;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)((i / (n * 16)) * 16 + (i & 15));
-        float d = 0.f;
-        if (c < used) {
-            d = out[i] - tgt[i];
-            acc += d * d;
+    for (long long v = blockIdx.x * (long long)kLossThreads + threadIdx.x; v < n;
+         v += (long long)gridDim.x * kLossThreads) {
+        const float4 *o4 = reinterpret_cast<const float4 *>(out + (blk * n + v) * 16 + half * 8);
+        const float4 a = __ldg(o4), b = __ldg(o4 + 1);
+        const float o[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        const float ia = 1.f / io.alpha[v];
+        float f[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            f[j] = part * 8 + j < used ? __ldg(s_src[j] + v) : 0.f;
+        __align__(16) __nv_bfloat16 gv[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int c = part * 8 + j;
+            float d = 0.f;
+            if (c < used) {
+                d = o[j] - (c <= 2 * L ? f[j] : f[j] * ia);
+                acc += d * d;
+            }
+            gv[j] = __float2bfloat16_rn(2.f * d * scale);
         }
-        const long long blk = i / (n * 16), v = (i / 16) % n, cc = i & 15;
-        const long long zx = v / ny, y = v % ny, yp = (ny + 7) / 8 * 8;
-        const long long pn = yp * (n / ny);  // padded voxels of one 16-channel block
-        g[blk * pn * 16 + (zx * 2 + cc / 8) * yp * 8 + y * 8 + (cc & 7)] =
-            __float2bfloat16_rn(2.f * d * scale);
+        const long long zx = n <= 0x7fffffff ? (long long)((unsigned)v / (unsigned)ny) : v / ny;
+        const long long y = v - zx * ny;
+        *reinterpret_cast<uint4 *>(g + blk * pn * 16 + (zx * 2 + half) * yp * 8 + y * 8) =
+            *reinterpret_cast<const uint4 *>(gv);
     }
     for (int o = 16; o > 0; o >>= 1)
         acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0)
+        s_acc[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kLossThreads / 32; ++w)
+            acc += s_acc[w];
         atomicAdd(loss, acc * scale);
+    }
 }
 
-// Adam on the FP32 master parameters; clears the gradients.
-__global__ void adam_kernel(float *p, float *m, float *v, float *grad, int n, float lr, float b1,
-                            float b2, float eps, float c1, float c2)
+// Adam on the FP32 master parameters and their BF16 copies; clears the gradients.
+__global__ void adam_kernel(float *p, float *m, float *v, float *grad, __nv_bfloat16 *w16, int n, float lr,
+                            float b1, float b2, float eps, float c1, float c2)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float gi = grad[i];
@@ -216,8 +229,12 @@ __global__ void adam_kernel(float *p, float *m, float *v, float *grad, int n, fl
         const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
         m[i] = mi;
         v[i] = vi;
-        p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        p[i] = pi;
         grad[i] = 0.f;
+        const int b = i / (kW + 16), j = i % (kW + 16);
+        if (j < kW)
+            w16[b * kW + j] = __float2bfloat16_rn(pi);
     }
 }
 
@@ -245,14 +262,14 @@ struct asets_wsnet {
     int L = 6;
     float *params = nullptr, *grads = nullptr, *m = nullptr, *v = nullptr;
     __nv_bfloat16 *w16 = nullptr;
-    float *loss = nullptr;
-    int *err = nullptr;
+    float *loss = nullptr;            // the pass's loss
+    int *err = nullptr;               // its error flag, in the word after
     long long vox_cap = 0, pvox_cap = 0;
     int shape[3] = {0, 0, 0};         // volume the half-planar padding was cleared for
     __nv_bfloat16 *x0 = nullptr, *act[3] = {nullptr, nullptr, nullptr};
-    __nv_bfloat16 *gbuf[2] = {nullptr, nullptr};  // [v][16] gradients of hidden layers
+    __nv_bfloat16 *gbuf[3] = {nullptr, nullptr, nullptr};  // [v][16] gradients of hidden layers
     __nv_bfloat16 *gout = nullptr;                // [2][v][16] gradient of the output
-    float *out = nullptr, *tgt = nullptr;         // [2][v][16]
+    float *out = nullptr;                         // [2][v][16]
     float *part = nullptr;                        // [v][16] first half of a summed dgrad
     float *wg_partial = nullptr;                  // [SMs][28][16][16] weight-gradient partials
     int step = 0;
@@ -283,8 +300,7 @@ static asets_status ws_reserve(asets_wsnet *n, int Ny, int Nx, int Nz)
     }
     void **bufs[] = {(void **)&n->x0,      (void **)&n->act[0], (void **)&n->act[1],
                      (void **)&n->act[2],  (void **)&n->gbuf[0], (void **)&n->gbuf[1],
-                     (void **)&n->gout,    (void **)&n->out,    (void **)&n->tgt,
-                     (void **)&n->part};
+                     (void **)&n->gbuf[2], (void **)&n->gout,    (void **)&n->out,    (void **)&n->part};
     for (void **b : bufs)
         if (*b) {
             cudaFreeAsync(*b, st);
@@ -293,10 +309,10 @@ static asets_status ws_reserve(asets_wsnet *n, int Ny, int Nx, int Nz)
     n->vox_cap = 0;
     n->pvox_cap = 0;
     const size_t b16 = (size_t)pvox * 16 * sizeof(__nv_bfloat16), f32 = (size_t)vox * 16 * 4;
-    const size_t sizes[] = {b16, b16, b16, b16, b16, b16, 2 * b16, 2 * f32, 2 * f32, f32};
+    const size_t sizes[] = {b16, b16, b16, b16, b16, b16, b16, 2 * b16, 2 * f32, f32};
     for (int i = 0; i < 10; ++i) {
         WS_TRY(cudaMallocAsync(bufs[i], sizes[i], st));
-        if (i < 7)
+        if (i < 8)
             WS_TRY(cudaMemsetAsync(*bufs[i], 0, sizes[i], st));
     }
     n->vox_cap = vox;
@@ -329,12 +345,12 @@ extern "C" ASETS_API asets_status asets_wsnet_create(asets_context *ctx, int nLa
         if (cudaMallocAsync((void **)b, kParams * 4, st) != cudaSuccess)
             return fail_free(ws_fail(ASETS_ERR_OUT_OF_MEMORY, "warm-start net: out of memory"));
     if (cudaMallocAsync((void **)&n->w16, kBlocks * kW * 2, st) != cudaSuccess ||
-        cudaMallocAsync((void **)&n->loss, 4, st) != cudaSuccess ||
-        cudaMallocAsync((void **)&n->err, 4, st) != cudaSuccess ||
+        cudaMallocAsync((void **)&n->loss, 8, st) != cudaSuccess ||
         cudaMallocAsync((void **)&n->wg_partial,
                         (size_t)context_num_sms(ctx) * kWgtTaps * 256 * sizeof(float), st) !=
             cudaSuccess)
         return fail_free(ws_fail(ASETS_ERR_OUT_OF_MEMORY, "warm-start net: out of memory"));
+    n->err = reinterpret_cast<int *>(n->loss + 1);
     // He-normal initial weights from a seeded generator (Box-Muller on a
     // 64-bit LCG), zero biases; weights of unused channels stay zero.
     std::vector<float> h(kParams, 0.f);
@@ -377,8 +393,8 @@ extern "C" ASETS_API void asets_wsnet_destroy(asets_wsnet *n)
         return;
     cudaStream_t st = context_stream(n->ctx);
     void *ps[] = {n->params, n->grads,   n->m,       n->v,    n->w16,  n->loss,
-                  n->err,    n->x0,      n->act[0],  n->act[1], n->act[2], n->gbuf[0],
-                  n->gbuf[1], n->gout,   n->out,     n->tgt,  n->part, n->wg_partial};
+                  n->x0,      n->act[0],  n->act[1], n->act[2], n->gbuf[0],
+                  n->gbuf[1], n->gbuf[2], n->gout,   n->out,     n->part, n->wg_partial};
     for (void *p : ps)
         if (p)
             cudaFreeAsync(p, st);
@@ -437,7 +453,7 @@ static asets_status ws_forward(asets_wsnet *n, int Ny, int Nx, int Nz, const flo
     EncodeTiledFn enc = context_encoder(n->ctx);
     pack_input_kernel<<<blocks_for(vox, 256, sms), 256, 0, st>>>(ct, alpha, n->x0, vox, n->L, Ny);
     WS_TRY(cudaGetLastError());
-    WS_TRY(cudaMemsetAsync(n->err, 0, 4, st));
+    WS_TRY(cudaMemsetAsync(n->loss, 0, 8, st));  // and err
     const void *in = n->x0;
     for (int b = 0; b < kBlocks; ++b) {
         void *y = b < 3 ? static_cast<void *>(n->act[b])
@@ -453,13 +469,19 @@ static asets_status ws_forward(asets_wsnet *n, int Ny, int Nx, int Nz, const flo
     return ASETS_OK;
 }
 
-static asets_status ws_check(asets_wsnet *n)
+// Waits for the pass; its loss and its error flag arrive in one copy.
+static asets_status ws_check(asets_wsnet *n, float *loss_out = nullptr)
 {
-    int herr = 0;
-    WS_TRY(cudaMemcpyAsync(&herr, n->err, 4, cudaMemcpyDeviceToHost, context_stream(n->ctx)));
+    struct {
+        float loss;
+        int err;
+    } h{};
+    WS_TRY(cudaMemcpyAsync(&h, n->loss, 8, cudaMemcpyDeviceToHost, context_stream(n->ctx)));
     WS_TRY(cudaStreamSynchronize(context_stream(n->ctx)));
-    if (herr)
+    if (h.err)
         return ws_fail(ASETS_ERR_TIMEOUT, "a device-side wait timed out in the warm-start net");
+    if (loss_out)
+        *loss_out = h.loss;
     return ASETS_OK;
 }
 
@@ -497,54 +519,42 @@ static asets_status ws_backward(asets_wsnet *n, int Ny, int Nx, int Nz, const fl
     cudaStream_t st = context_stream(n->ctx);
     const int sms = context_num_sms(n->ctx);
     EncodeTiledFn enc = context_encoder(n->ctx);
-    pack_target_kernel<<<blocks_for(vox, 256, sms), 256, 0, st>>>(target, n->tgt, vox, n->L);
-    WS_TRY(cudaMemsetAsync(n->loss, 0, 4, st));
     const int used = 5 * n->L + 1;
     const float scale = 1.0f / (float)((double)vox * used);
-    loss_kernel<<<blocks_for(vox * 32, 256, sms), 256, 0, st>>>(n->out, n->tgt, n->gout, vox, used,
-                                                                scale, n->loss, Ny);
+    loss_kernel<<<dim3(blocks_for(vox, kLossThreads, sms), 4), kLossThreads, 0, st>>>(
+        n->out, target, n->gout, vox, n->L, scale, n->loss, Ny);
     WS_TRY(cudaGetLastError());
-    // output blocks 3 and 4: weight gradients, then the data gradient
-    // flip(g3, W3) + flip(g4, W4), masked by the ReLU of act[2]
-    for (int b = 3; b < kBlocks; ++b) {
-        float *gw = n->grads + (size_t)b * (kW + 16);
-        WS_TRY(launch_wgrad_tc(enc, n->act[2], n->gout + (size_t)(b - 3) * pvox * 16, gw, gw + kW,
-                               Ny, Nx, Nz, n->wg_partial, sms, n->err, st, 1));
-    }
+    // the data gradients: of output blocks 3 and 4, flip(g3, W3) + flip(g4, W4),
+    // then of hidden layers 2 and 1, each masked by the ReLU of its input
     {
         ConvLaunch c = conv_of(n, 3, n->gout, n->part, Ny, Nx, Nz);
         c.flip = 1;
         c.out_fp32 = 1;
         WS_TRY(launch_conv3_tc(enc, c, sms, st, n->err));
-        ConvLaunch d = conv_of(n, 4, n->gout + (size_t)pvox * 16, n->gbuf[0], Ny, Nx, Nz);
+        ConvLaunch d = conv_of(n, 4, n->gout + (size_t)pvox * 16, n->gbuf[2], Ny, Nx, Nz);
         d.flip = 1;
         d.addend = n->part;
         d.mask = n->act[2];
         WS_TRY(launch_conv3_tc(enc, d, sms, st, n->err));
     }
-    // hidden layers 2, 1, 0: input activation and the gradient w.r.t. the output
-    const __nv_bfloat16 *ins[3] = {n->x0, n->act[0], n->act[1]};
-    int cur = 0;
-    for (int l = 2; l >= 0; --l) {
-        float *gw = n->grads + (size_t)l * (kW + 16);
-        WS_TRY(launch_wgrad_tc(enc, ins[l], n->gbuf[cur], gw, gw + kW, Ny, Nx, Nz, n->wg_partial,
-                               sms, n->err, st, 1));
-        if (l == 0)
-            break;
-        ConvLaunch c = conv_of(n, l, n->gbuf[cur], n->gbuf[cur ^ 1], Ny, Nx, Nz);
-        c.mask = ins[l];  // ReLU of the layer below: its output is this layer's input
+    for (int l = 2; l >= 1; --l) {
+        ConvLaunch c = conv_of(n, l, n->gbuf[l], n->gbuf[l - 1], Ny, Nx, Nz);
+        c.mask = n->act[l - 1];  // the layer below: its output is this layer's input
         c.flip = 1;
         WS_TRY(launch_conv3_tc(enc, c, sms, st, n->err));
-        cur ^= 1;
     }
-    s = ws_check(n);
-    if (s != ASETS_OK)
-        return s;
-    if (loss_out) {
-        WS_TRY(cudaMemcpyAsync(loss_out, n->loss, 4, cudaMemcpyDeviceToHost, st));
-        WS_TRY(cudaStreamSynchronize(st));
+    // the weight gradients: each layer's input and the gradient of its output
+    const __nv_bfloat16 *ins[kBlocks] = {n->x0, n->act[0], n->act[1], n->act[2], n->act[2]};
+    const __nv_bfloat16 *gr[kBlocks] = {n->gbuf[0], n->gbuf[1], n->gbuf[2], n->gout,
+                                        n->gout + (size_t)pvox * 16};
+    WgradOut out{};
+    for (int b = 0; b < kBlocks; ++b) {
+        out.dw[b] = n->grads + (size_t)b * (kW + 16);
+        out.db[b] = out.dw[b] + kW;
     }
-    return ASETS_OK;
+    static_assert(kBlocks <= kWgtLayers, "one launch");
+    WS_TRY(launch_wgrad_layers(enc, kBlocks, ins, gr, out, Ny, Nx, Nz, n->wg_partial, sms, n->err, st, 1));
+    return ws_check(n, loss_out);
 }
 
 static bool target_ok(const float *Ct, const float *alpha, const float *u, const float *ps,
@@ -596,9 +606,8 @@ extern "C" ASETS_API asets_status asets_wsnet_train_step(asets_wsnet *n, int Ny,
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, (float)n->step), c2 = 1.f - powf(b2, (float)n->step);
     cudaStream_t st = context_stream(n->ctx);
-    adam_kernel<<<64, 256, 0, st>>>(n->params, n->m, n->v, n->grads, kParams, lr, b1, b2, 1e-8f,
-                                    c1, c2);
-    to_bf16_kernel<<<64, 256, 0, st>>>(n->params, n->w16);
+    adam_kernel<<<(kParams + 255) / 256, 256, 0, st>>>(n->params, n->m, n->v, n->grads, n->w16, kParams,
+                                                       lr, b1, b2, 1e-8f, c1, c2);
     WS_TRY(cudaGetLastError());
     return ASETS_OK;
 }
