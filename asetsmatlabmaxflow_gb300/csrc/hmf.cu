@@ -12,7 +12,7 @@
 //      memory when they fit, k1_staged);
 //   K2 gradient step of the spatial flows, K3 flow magnitude and projection
 //   factor, K4 flow rescale, K5 divergence (the rest of UpdateSpatialFlows);
-//   in 2D without direction fields one tiled kernel runs K2-K5.
+//   without direction fields in one kernel (2D) or two (3D).
 // Costs (CalculateCostsFullFlow) are summed on the device in double.
 //
 // The DAG solver (maxflow/asetsDAGMF2D.m / 3D, nodes may have several
@@ -34,9 +34,12 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "asets.h"
+#include "device_common.cuh"
+#include "div_const.cuh"
 #include "internal.h"
 
 using namespace asets;
@@ -62,13 +65,17 @@ struct HArgs {
     int dim, d1, d2, d3, m;
     int paren;  // gradient step p + (g1 - g0) (asetsHMF2D.m) instead of (p + g1) - g0
     long long n, f1, f2, f3;  // cells and face counts per node
+    long long ns;             // cells from a node to the next (whole 16-byte vectors)
     T cc, steps, inv_cc;      // inv_cc: 1/cc formed in double (the root's 1/cc .* ones)
+    DivConst<T> by_cc;        // x/cc without a division where that is exact
     const NodeDev<T> *nodes;
     const int *children;
     const T *wchild;    // DAG: weight of each child edge
     const int *order;   // DAG: the top-down node list
     T *pn;              // DAG: pushed-down flow of multi-parent nodes
     T *pt, *u, *div, *g, *p1, *p2, *p3;
+    T *q1, *q2, *q3;    // without direction fields: a second copy of the flows
+    T *f;               // and the projection factors (2D: the last pass's only)
     int nedges;         // DAG: child edges (entries of children)
     T *e1, *e2, *e3;  // exempt flow per face (nodes with direction fields)
     double *cost;  // [m][2]: sum u*Ct (leaves), sum u*div (non-root)
@@ -148,10 +155,10 @@ __global__ void k1_pointwise(const HArgs<T> A)
         // reads its parent's pt before the parent is updated
         for (int i = A.m - 1; i >= 0; --i) {
             const NodeDev<T> nd = A.nodes[i];
-            const long long o = (long long)i * A.n + c;
+            const long long o = (long long)i * A.ns + c;
             T acc;
             if (nd.parent >= 0)
-                acc = add(sub(A.pt[(long long)nd.parent * A.n + c], A.div[o]), dvd(A.u[o], A.cc));
+                acc = add(sub(A.pt[(long long)nd.parent * A.ns + c], A.div[o]), dvd(A.u[o], A.cc));
             else
                 acc = A.inv_cc;
             if (nd.nchild == 0) {
@@ -160,15 +167,15 @@ __global__ void k1_pointwise(const HArgs<T> A)
                 continue;
             }
             for (int j = 0; j < nd.nchild; ++j) {
-                const long long oc = (long long)A.children[nd.child_begin + j] * A.n + c;
+                const long long oc = (long long)A.children[nd.child_begin + j] * A.ns + c;
                 acc = sub(add(add(acc, A.pt[oc]), A.div[oc]), dvd(A.u[oc], A.cc));
             }
             A.pt[o] = dvd(acc, (T)(nd.parent >= 0 ? 1 + nd.nchild : nd.nchild));
         }
         // labels, then the flow-gradient input g of every non-root node
         for (int i = 1; i < A.m; ++i) {
-            const long long o = (long long)i * A.n + c;
-            const T ptp = A.pt[(long long)A.nodes[i].parent * A.n + c];
+            const long long o = (long long)i * A.ns + c;
+            const T ptp = A.pt[(long long)A.nodes[i].parent * A.ns + c];
             const T dv = A.div[o], pt = A.pt[o];
             const T u = add(A.u[o], mul(A.cc, sub(sub(ptp, dv), pt)));
             A.u[o] = u;
@@ -177,81 +184,113 @@ __global__ void k1_pointwise(const HArgs<T> A)
     }
 }
 
-// k1_pointwise with the pixel's values of every node staged in shared
-// memory (one column per thread): the pixel's loads are issued together
-// and the children-first chain of sink flows runs on shared memory instead
-// of reading back through L2 what the thread has just stored.  A leaf's old
-// sink flow is never read (its parent reads it after the leaf's update), so
-// its slot holds Ct until then.  The node table is staged once per block.
-// Same operations in the same order as k1_pointwise.
-struct K1Stage {
-    // the node table: parent, first child and child count per node and the
-    // children list (4m ints), then the nodes' Ct pointers; then the three
-    // per-thread columns (sink flow, divergence, label) of every node
-    __host__ __device__ static constexpr int ptr_off(int m) { return 16 * m; }
-    __host__ __device__ static constexpr int table_bytes(int m) { return 16 * m + (8 * m + 15) / 16 * 16; }
-    __host__ __device__ static constexpr int bytes(int m, int elem) { return table_bytes(m) + 3 * m * kThreads * elem; }
+// The same for trees whose pixels fit in shared memory.  A thread has 16 bytes
+// of pixels (four in single precision, two in double) and a column of them per
+// node for the sink flow, the divergence and the label, which asynchronous
+// copies fill at once; the children-first chain then runs on shared memory.
+// The tree comes with the launch's parameters.  A leaf's old sink flow is never
+// read (its parent reads it after the leaf's update), so its slot holds Ct
+// until then, and only the last iteration stores it.  Same operations in the
+// same order as k1_pointwise.  768 x 640, seven nodes: 15 us (one pixel a
+// thread, loads through registers, tree staged in each block: 27); what is left
+// is the 34 arrays' traffic.
+constexpr int kK1Threads = 128;
+constexpr int kK1Nodes = 18;  // columns of 110 KB: two blocks an SM
+struct K1Tree {
+    int parent[kK1Nodes], first[kK1Nodes], nchild[kK1Nodes], kids[kK1Nodes];
+    const void *ct[kK1Nodes];
 };
+constexpr int k1_bytes(int m) { return 3 * m * kK1Threads * 16; }
+static_assert(2 * (k1_bytes(kK1Nodes) + 1024) <= 227 * 1024, "two blocks an SM");
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all()
+{
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
 
 template <class T>
-__global__ void __launch_bounds__(kThreads) k1_staged(const HArgs<T> A)
+__global__ void __launch_bounds__(kK1Threads) k1_staged(const HArgs<T> A, const __grid_constant__ K1Tree R, int last)
 {
+    constexpr int N = 16 / sizeof(T);
+    struct alignas(16) V {
+        T v[N];
+    };
     extern __shared__ __align__(16) unsigned char k1sm[];
     const int m = A.m, tid = threadIdx.x;
-    int *npar = reinterpret_cast<int *>(k1sm);
-    int *nfirst = npar + m, *ncount = nfirst + m, *kids = ncount + m;
-    const T **cts = reinterpret_cast<const T **>(k1sm + K1Stage::ptr_off(m));
-    T *PT = reinterpret_cast<T *>(k1sm + K1Stage::table_bytes(m));
-    T *DV = PT + m * kThreads, *U = DV + m * kThreads;
-    for (int i = tid; i < m; i += kThreads) {
-        const NodeDev<T> &nd = A.nodes[i];
-        npar[i] = nd.parent;
-        nfirst[i] = nd.child_begin;
-        ncount[i] = nd.nchild;
-        cts[i] = nd.ct;
+    const long long c = ((long long)blockIdx.x * kK1Threads + tid) * N;
+    if (c >= A.ns)
+        return;
+    V *PT = reinterpret_cast<V *>(k1sm) + tid;
+    V *DV = PT + m * kK1Threads, *U = DV + m * kK1Threads;
+    for (int i = 0; i < m; ++i) {
+        const long long o = (long long)i * A.ns + c;
+        cp_async16(PT + i * kK1Threads, R.nchild[i] == 0 ? static_cast<const T *>(R.ct[i]) + c : A.pt + o);
+        if (i > 0) {
+            cp_async16(DV + i * kK1Threads, A.div + o);
+            cp_async16(U + i * kK1Threads, A.u + o);
+        }
     }
-    for (int j = tid; j < m - 1; j += kThreads)
-        kids[j] = A.children[j];
-    __syncthreads();
-    H_LOOP(A.n)
-    {
-        const long long c = t;
-        for (int i = 0; i < m; ++i) {
-            const long long o = (long long)i * A.n + c;
-            PT[i * kThreads + tid] = ncount[i] == 0 ? cts[i][c] : A.pt[o];
-            if (i > 0) {
-                DV[i * kThreads + tid] = A.div[o];
-                U[i * kThreads + tid] = A.u[o];
-            }
+    cp_async_wait_all();
+    for (int i = m - 1; i >= 0; --i) {
+        const int par = R.parent[i], nc = R.nchild[i];
+        V acc;
+        if (par >= 0) {
+            const V pp = PT[par * kK1Threads], dv = DV[i * kK1Threads], u = U[i * kK1Threads];
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                acc.v[k] = add(sub(pp.v[k], dv.v[k]), A.by_cc(u.v[k], A.cc));
+        } else {
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                acc.v[k] = A.inv_cc;
         }
-        for (int i = m - 1; i >= 0; --i) {
-            const int par = npar[i];
-            T acc = par >= 0 ? add(sub(PT[par * kThreads + tid], DV[i * kThreads + tid]),
-                                   dvd(U[i * kThreads + tid], A.cc))
-                             : A.inv_cc;
-            const int nc = ncount[i];
-            if (nc == 0) {
-                const T ct = PT[i * kThreads + tid];
-                PT[i * kThreads + tid] = (ct <= acc || ct != ct) ? ct : acc;
-                continue;
-            }
+        if (nc == 0) {
+            const V ct = PT[i * kK1Threads];
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                acc.v[k] = (ct.v[k] <= acc.v[k] || ct.v[k] != ct.v[k]) ? ct.v[k] : acc.v[k];
+        } else {
             for (int j = 0; j < nc; ++j) {
-                const int ch = kids[nfirst[i] + j];
-                acc = sub(add(add(acc, PT[ch * kThreads + tid]), DV[ch * kThreads + tid]),
-                          dvd(U[ch * kThreads + tid], A.cc));
+                const int ch = R.kids[R.first[i] + j];
+                const V pc = PT[ch * kK1Threads], dv = DV[ch * kK1Threads], u = U[ch * kK1Threads];
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    acc.v[k] = sub(add(add(acc.v[k], pc.v[k]), dv.v[k]), A.by_cc(u.v[k], A.cc));
             }
-            PT[i * kThreads + tid] = dvd(acc, (T)(par >= 0 ? 1 + nc : nc));
+            const int parts = par >= 0 ? 1 + nc : nc;
+            if ((parts & (parts - 1)) == 0) {  // a power of two: the product rounds alike
+                const T r = (T)1 / (T)parts;
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    acc.v[k] = mul(acc.v[k], r);
+            } else {
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    acc.v[k] = dvd(acc.v[k], (T)parts);
+            }
         }
-        A.pt[c] = PT[tid];
-        for (int i = 1; i < m; ++i) {
-            const long long o = (long long)i * A.n + c;
-            const T ptp = PT[npar[i] * kThreads + tid];
-            const T dv = DV[i * kThreads + tid], pt = PT[i * kThreads + tid];
-            const T u = add(U[i * kThreads + tid], mul(A.cc, sub(sub(ptp, dv), pt)));
-            A.pt[o] = pt;
-            A.u[o] = u;
-            A.g[o] = mul(A.steps, sub(sub(add(dv, pt), ptp), dvd(u, A.cc)));
+        PT[i * kK1Threads] = acc;
+    }
+    for (int i = 0; i < m; ++i) {
+        const long long o = (long long)i * A.ns + c;
+        const V pt = PT[i * kK1Threads];
+        if (last || R.nchild[i] > 0)
+            *reinterpret_cast<V *>(A.pt + o) = pt;
+        if (i == 0)
+            continue;
+        const V pp = PT[R.parent[i] * kK1Threads], dv = DV[i * kK1Threads];
+        V u = U[i * kK1Threads], g;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            u.v[k] = add(u.v[k], mul(A.cc, sub(sub(pp.v[k], dv.v[k]), pt.v[k])));
+            g.v[k] = mul(A.steps, sub(sub(add(dv.v[k], pt.v[k]), pp.v[k]), A.by_cc(u.v[k], A.cc)));
         }
+        *reinterpret_cast<V *>(A.u + o) = u;
+        *reinterpret_cast<V *>(A.g + o) = g;
     }
 }
 
@@ -262,7 +301,7 @@ __global__ void k2_gradient(const HArgs<T> A)
     {
         const int i = 1 + node_of(t, A.n);
         const Pix<T> p(A, t - (long long)(i - 1) * A.n);
-        const T *g = A.g + (long long)i * A.n;
+        const T *g = A.g + (long long)i * A.ns;
         const T gc = g[p.c];
         // 2D: p + (g(k+1) - g(k)); 3D: (p + g(k+1)) - g(k)
         auto step = [&](T pv, T gn) { return A.paren ? add(pv, sub(gn, gc)) : sub(add(pv, gn), gc); };
@@ -279,6 +318,23 @@ __global__ void k2_gradient(const HArgs<T> A)
             *f = step(*f, g[p.c + (long long)A.d1 * A.d2]);
         }
     }
+}
+
+// The projection factor min(1, al / sqrt(s)).  s < lim = RN(al^2): the next
+// number below that is below al^2, so RN(sqrt(s)) <= al and the root and the
+// division are left out (no number is below lim where al is not positive).
+template <class T>
+__device__ __forceinline__ T surely_inside(T al)
+{
+    return al > (T)0 ? mul(al, al) : (T)-1;
+}
+template <class T>
+__device__ __forceinline__ T factor(T s, T al, T lim)
+{
+    if (s < lim)
+        return (T)1;
+    const T mag = sqr(s);
+    return (mag <= al) ? (T)1 : dvd(al, mag);
 }
 
 template <class T>
@@ -319,10 +375,9 @@ __global__ void k3_projection(const HArgs<T> A)
                 s = add(s, mul(v, v));
             }
         }
-        const T mag = sqr(s);
         const NodeDev<T> &nd = A.nodes[i];
         const T al = nd.alpha ? nd.alpha[p.c] : nd.alpha_s;
-        A.g[(long long)i * A.n + p.c] = (mag <= al) ? (T)1 : dvd(al, mag);
+        A.g[(long long)i * A.ns + p.c] = factor(s, al, surely_inside<T>(al));
     }
 }
 
@@ -333,7 +388,7 @@ __global__ void k4_rescale(const HArgs<T> A)
     {
         const int i = 1 + node_of(t, A.n);
         const Pix<T> p(A, t - (long long)(i - 1) * A.n);
-        const T *g = A.g + (long long)i * A.n;
+        const T *g = A.g + (long long)i * A.ns;
         const T gc = g[p.c];
         const bool ex = A.nodes[i].l[0] != nullptr;
         // p = 0.5 p (g(k+1) + g(k)), or e + that with direction fields
@@ -376,7 +431,7 @@ __global__ void k5_divergence(const HArgs<T> A)
             if (p.z >= 1)
                 d = sub(d, f3[i3(A, p.y, p.x, p.z - 1)]);
         }
-        A.div[(long long)i * A.n + p.c] = d;
+        A.div[(long long)i * A.ns + p.c] = d;
     }
 }
 
@@ -460,7 +515,7 @@ __global__ void k_exempt_a(const HArgs<T> A)
                 a = add(a, pos_part(v < (T)0, v, l[2][p.c]));
             }
         }
-        A.g[(long long)i * A.n + p.c] = a;
+        A.g[(long long)i * A.ns + p.c] = a;
     }
 }
 
@@ -477,7 +532,7 @@ __global__ void k_exempt_e(const HArgs<T> A)
         if (!l[0])
             continue;
         const Pix<T> p(A, t - (long long)(i - 1) * A.n);
-        const T *a = A.g + (long long)i * A.n;
+        const T *a = A.g + (long long)i * A.ns;
         auto face = [&](T *f, T *e, const T *lk, long long step) {
             const T v = *f;
             const T llo = lk[p.c], lhi = lk[p.c + step];
@@ -510,7 +565,7 @@ __global__ void k_pseudo_point(const HArgs<T> A)
         const long long c = t;
         T *g = A.g + c;
         T *u = A.u + c;
-        const long long n = A.n;
+        const long long n = A.ns;
         for (int i = 0; i < A.m; ++i) {
             const NodeDev<T> &nd = A.nodes[i];
             g[i * n] = nd.nchild == 0 ? add(A.div[i * n + c], nd.ct[c]) : (T)0;
@@ -567,10 +622,10 @@ __global__ void k_pseudo_final(const HArgs<T> A)
             const NodeDev<T> &nd = A.nodes[i];
             if (nd.nchild == 0)
                 continue;
-            T s = u[(long long)A.children[nd.child_begin] * A.n];
+            T s = u[(long long)A.children[nd.child_begin] * A.ns];
             for (int j = 1; j < nd.nchild; ++j)
-                s = add(s, u[(long long)A.children[nd.child_begin + j] * A.n]);
-            u[(long long)i * A.n] = s;
+                s = add(s, u[(long long)A.children[nd.child_begin + j] * A.ns]);
+            u[(long long)i * A.ns] = s;
         }
     }
 }
@@ -585,7 +640,7 @@ __global__ void k_costs(const HArgs<T> A)
     const int i = blockIdx.y;
     const bool leaf = A.nodes[i].nchild == 0, below_root = A.nodes[i].parent >= 0;
     const T *ct = A.nodes[i].ct;
-    const T *u = A.u + (long long)i * A.n, *dv = A.div + (long long)i * A.n;
+    const T *u = A.u + (long long)i * A.ns, *dv = A.div + (long long)i * A.ns;
     double dc = 0.0, rc = 0.0;
     for (long long c = blockIdx.x * (long long)kThreads + threadIdx.x; c < A.n;
          c += (long long)gridDim.x * kThreads) {
@@ -620,7 +675,7 @@ __global__ void k_costs(const HArgs<T> A)
 template <class T>
 __device__ __forceinline__ T dag_in(const HArgs<T> &A, const NodeDev<T> &nd, int i, long long c)
 {
-    return nd.nparent > 1 ? A.pn[(long long)i * A.n + c] : A.pt[(long long)nd.parent * A.n + c];
+    return nd.nparent > 1 ? A.pn[(long long)i * A.ns + c] : A.pt[(long long)nd.parent * A.ns + c];
 }
 
 // InitializeFullFlow: pt = Ct (leaves) or max(0, pt of the first child);
@@ -633,12 +688,12 @@ __global__ void k_dag_init(const HArgs<T> A)
         for (int j = A.m - 1; j >= 0; --j) {
             const int i = A.order[j];
             const NodeDev<T> nd = A.nodes[i];
-            const long long o = (long long)i * A.n + t;
+            const long long o = (long long)i * A.ns + t;
             T pt;
             if (nd.nchild == 0) {
                 pt = nd.ct[t];
             } else {
-                const T x = A.pt[(long long)A.children[nd.child_begin] * A.n + t];
+                const T x = A.pt[(long long)A.children[nd.child_begin] * A.ns + t];
                 const T z = (T)0;
                 pt = (z >= x) ? z : x;
             }
@@ -657,7 +712,7 @@ __global__ void k_dag_g(const HArgs<T> A)
     {
         const int i = 1 + node_of(t, A.n);
         const long long c = t - (long long)(i - 1) * A.n;
-        const long long o = (long long)i * A.n + c;
+        const long long o = (long long)i * A.ns + c;
         const T in = dag_in(A, A.nodes[i], i, c);
         A.g[o] = mul(A.steps, sub(sub(add(A.div[o], A.pt[o]), in), dvd(A.u[o], A.cc)));
     }
@@ -672,16 +727,16 @@ __global__ void k_dag_point(const HArgs<T> A)
         const long long c = t;
         for (int i = 0; i < A.m; ++i)
             if (A.nodes[i].nparent > 1)
-                A.pn[(long long)i * A.n + c] = (T)0;
+                A.pn[(long long)i * A.ns + c] = (T)0;
         for (int j = 0; j < A.m; ++j) {
             const int i = A.order[j];
             const NodeDev<T> nd = A.nodes[i];
-            const long long o = (long long)i * A.n + c;
+            const long long o = (long long)i * A.ns + c;
             const T pt = A.pt[o];
             for (int k = 0; k < nd.nchild; ++k) {
                 const int ch = A.children[nd.child_begin + k];
                 if (A.nodes[ch].nparent > 1) {
-                    T *pn = A.pn + (long long)ch * A.n + c;
+                    T *pn = A.pn + (long long)ch * A.ns + c;
                     *pn = add(*pn, mul(A.wchild[nd.child_begin + k], pt));
                 }
             }
@@ -693,7 +748,7 @@ __global__ void k_dag_point(const HArgs<T> A)
         for (int j = A.m - 1; j >= 0; --j) {
             const int i = A.order[j];
             const NodeDev<T> nd = A.nodes[i];
-            const long long o = (long long)i * A.n + c;
+            const long long o = (long long)i * A.ns + c;
             if (nd.nchild == 0) {
                 const T x = add(sub(dag_in(A, nd, i, c), A.div[o]), dvd(A.u[o], A.cc));
                 const T ct = nd.ct[c];
@@ -704,7 +759,7 @@ __global__ void k_dag_point(const HArgs<T> A)
             T g = A.g[o];
             for (int k = 0; k < nd.nchild; ++k) {
                 const int ch = A.children[nd.child_begin + k];
-                const long long oc = (long long)ch * A.n + c;
+                const long long oc = (long long)ch * A.ns + c;
                 const T uc = dvd(A.u[oc], A.cc);
                 if (A.nodes[ch].nparent > 1) {
                     const T w = A.wchild[nd.child_begin + k];
@@ -722,7 +777,7 @@ __global__ void k_dag_point(const HArgs<T> A)
             const NodeDev<T> nd = A.nodes[i];
             if (nd.nparent == 0)
                 continue;
-            const long long o = (long long)i * A.n + c;
+            const long long o = (long long)i * A.ns + c;
             A.u[o] = add(A.u[o], mul(A.cc, sub(sub(dag_in(A, nd, i, c), A.div[o]), A.pt[o])));
         }
     }
@@ -786,7 +841,7 @@ __global__ void __launch_bounds__(kThreads) k_dag_point_staged(const HArgs<T> A)
     {
         const long long c = t;
         for (int i = 0; i < m; ++i) {
-            const long long o = (long long)i * A.n + c;
+            const long long o = (long long)i * A.ns + c;
             col(PT, i) = cnt[i] == 0 ? cts[i][c] : A.pt[o];
             col(DV, i) = A.div[o];
             col(U, i) = A.u[o];
@@ -839,7 +894,7 @@ __global__ void __launch_bounds__(kThreads) k_dag_point_staged(const HArgs<T> A)
             col(U, i) = add(col(U, i), mul(A.cc, sub(sub(in_of(i), col(DV, i)), col(PT, i))));
         }
         for (int i = 0; i < m; ++i) {
-            const long long o = (long long)i * A.n + c;
+            const long long o = (long long)i * A.ns + c;
             A.pt[o] = col(PT, i);
             if (npar[i] > 0)
                 A.u[o] = col(U, i);
@@ -852,141 +907,241 @@ __global__ void __launch_bounds__(kThreads) k_dag_point_staged(const HArgs<T> A)
 }
 
 // The four spatial passes (k2 .. k5) fused for 2D solves without direction
-// fields: one block per (node, R x S tile of cells) computes, in shared
-// memory over the tile and a two-cell halo, the gradient step of the faces
-// (k2), the projection factor (k3), the rescale (k4) and the divergence
-// (k5), with each pass's expression and validity tests, and stores the
-// tile's faces, divergence and factor (g) as the passes leave them.  The
-// halo's faces are recomputed by the neighbouring tiles' blocks; one read
-// and one write of each array instead of four passes over them.  The frame
-// is R + 4 = 32 rows high: lane q of every warp owns frame row q (y0 - 2 +
-// q) in every phase, and warp w the frame columns w, w + 8, ..., so a
-// thread's row tests are made once and a warp's loads and stores are one
-// 128-byte run of a column.
-template <class T, int R, int S>
-struct SpatialTile {
-    static constexpr int FR = R + 4;   // frame cells y0-2 .. y0+R+1
-    static constexpr int FC = S + 4;   // frame cells x0-2 .. x0+S+1
-    static constexpr int F = FR * FC;
-    static_assert(FR == 32, "one frame row per lane");
-    static constexpr int smem_bytes() { return 5 * F * (int)sizeof(T); }
-};
+// fields.  A warp has 32 rows of one node, its lane a row (28 the warp's own,
+// two of its neighbours' above and below), and walks along x with the last two
+// columns in registers: per column the gradient step of its faces (k2), the
+// projection factor (k3), and, of the column before, the rescale (k4) and the
+// divergence (k5), rows exchanged by shuffles, each with its pass's expression
+// and validity tests.  The next four columns are in flight while four are
+// worked on.  The flows of a pass are written to a second copy: a neighbour
+// warp may still have to read this pass's.  Cells whose squared flow is surely
+// within alpha^2 have factor 1 without the square root and the division.  The
+// factor is stored (to A.f) on the last pass only: nothing else reads it.
+// 768 x 640, six nodes: 20 us (28 x 32 tiles in shared memory, four phases
+// with barriers between them, factors stored each time: 26).
+constexpr int kSweepThreads = 128, kSweepRows = 28;
 
-template <class T, int R, int S>
-__global__ void __launch_bounds__(kThreads) k_spatial_tile2d(const HArgs<T> A, int tiles_y)
+template <class T>
+__global__ void __launch_bounds__(kSweepThreads) k_spatial_sweep2d(const HArgs<T> A, int last, int strips,
+                                                                   int total, int S)
 {
-    using Q = SpatialTile<T, R, S>;
-    constexpr int FR = Q::FR, FC = Q::FC, F = Q::F, NW = kThreads / 32;
-    extern __shared__ __align__(16) unsigned char hsm[];
-    T *G = reinterpret_cast<T *>(hsm);   // g, at cells
-    T *P1 = G + F;                        // face (y, y+1) at cell y
-    T *P2 = P1 + F;                       // face (x, x+1) at cell x
-    T *FS = P2 + F;                       // projection factor
-    T *AL = FS + F;
-    const int i = 1 + (int)blockIdx.y;    // non-root node
-    const int y0 = ((int)blockIdx.x % tiles_y) * R, x0 = ((int)blockIdx.x / tiles_y) * S;
+    constexpr int Q = 4;
+    const int w = (int)(blockIdx.x * (kSweepThreads / 32) + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
+    if (w >= total)
+        return;
+    const int i = 1 + (int)blockIdx.y;  // non-root node
     const int d1 = A.d1, d2 = A.d2;
-    const NodeDev<T> nd = A.nodes[i];
-    const T *g = A.g + (long long)i * A.n;
-    T *p1 = A.p1 + (long long)i * A.f1;
-    T *p2 = A.p2 + (long long)i * A.f2;
-    const int q = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int y = y0 - 2 + q;
-    const bool y_in = (y >= 0 && y < d1), y_up = (y + 1 < d1), y_dn = (y >= 1);
-    for (int c = w; c < FC; c += NW) {
-        const int x = x0 - 2 + c, f = c * FR + q;
-        const bool in = y_in && x >= 0 && x < d2;
-        const unsigned int cell = (unsigned int)x * (unsigned int)d1 + (unsigned int)y;
-        G[f] = in ? g[cell] : (T)0;
-        P1[f] = (in && y_up) ? p1[(unsigned int)x * (unsigned int)(d1 - 1) + (unsigned int)y] : (T)0;
-        P2[f] = (in && x + 1 < d2) ? p2[cell] : (T)0;
-        AL[f] = in ? (nd.alpha ? nd.alpha[cell] : nd.alpha_s) : (T)0;
-    }
-    __syncthreads();
+    const int x0 = w / strips * S, x1 = min(x0 + S, d2);
+    const int y = w % strips * kSweepRows - 2 + lane;
+    const bool in = y >= 0 && y < d1, up = in && y + 1 < d1;
+    const bool own = in && lane >= 2 && lane < 2 + kSweepRows;
+    const T *gp = A.g + (long long)i * A.ns + y;
+    const T *p1p = A.p1 + (long long)i * A.f1 + y, *p2p = A.p2 + (long long)i * A.f2 + y;
+    T *q1p = A.q1 + (long long)i * A.f1 + y, *q2p = A.q2 + (long long)i * A.f2 + y;
+    T *dp = A.div + (long long)i * A.ns + y;
+    T *fp = last ? A.f + (long long)i * A.ns + y : nullptr;
+    const T *alp = A.nodes[i].alpha ? A.nodes[i].alpha + y : nullptr;
+    T al = A.nodes[i].alpha_s, lim = surely_inside<T>(al);
+
+    auto ld_g = [&](int x) { return in && x >= 0 && x < d2 ? gp[x * d1] : (T)0; };
+    auto ld_1 = [&](int x) { return up && x >= 0 && x < d2 ? p1p[x * (d1 - 1)] : (T)0; };
+    auto ld_2 = [&](int x) { return in && x >= 0 && x + 1 < d2 ? p2p[x * d1] : (T)0; };
     // k2: 2D p + (g(k+1) - g(k)) (asetsHMF2D.m), else (p + g(k+1)) - g(k)
     auto step = [&](T pv, T gn, T gc) { return A.paren ? add(pv, sub(gn, gc)) : sub(add(pv, gn), gc); };
-    if (q <= R + 2 && y_in && y_up) {                            // p1: y0-2 .. y0+R, x0-1 .. x0+S
-        for (int c = 1 + w; c <= S + 2; c += NW) {
-            const int x = x0 - 2 + c, f = c * FR + q;
-            if (x >= 0 && x < d2)
-                P1[f] = step(P1[f], G[f + 1], G[f]);
+
+    // state at column x: g(x), and of x - 1 the stepped faces, the factor and
+    // of x - 2 the new face to x - 1
+    T gc = ld_g(x0 - 1);
+    T P1m = (T)0, Fm = (T)1, R2m = (T)0;
+    T P2m = x0 >= 2 ? step(ld_2(x0 - 2), gc, ld_g(x0 - 2)) : (T)0;
+    if (!in)
+        P2m = (T)0;
+    T gn[Q], p1n[Q], p2n[Q], aln[Q];
+    // columns x .. x + Q - 1 all with both their neighbours, rows as well
+    const bool rows_in = y - lane >= 1 && y - lane + 32 < d1;
+    auto inner = [&](int x) { return rows_in && x >= 1 && x + Q < d2; };
+    auto fetch = [&](int x) {
+        if (inner(x)) {
+#pragma unroll
+            for (int k = 0; k < Q; ++k) {
+                const int o = (x + k) * d1;
+                gn[k] = gp[o + d1];
+                p1n[k] = p1p[o - (x + k)];
+                p2n[k] = p2p[o];
+                if (alp)
+                    aln[k] = alp[o];
+            }
+            return;
+        }
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+            gn[k] = ld_g(x + k + 1);
+            p1n[k] = ld_1(x + k);
+            p2n[k] = ld_2(x + k);
+            if (alp)
+                aln[k] = in && x + k >= 0 && x + k < d2 ? alp[(x + k) * d1] : (T)0;
+        }
+    };
+    auto column = [&](auto edge, int x, T gr, T p1, T p2, T av) {
+        constexpr bool EDGE = decltype(edge)::value;
+        // stepped faces of column x; 0 where there is none
+        T P1 = step(p1, __shfl_down_sync(0xffffffffu, gc, 1), gc);
+        T P2 = step(p2, gr, gc);
+        if (EDGE && (!up || x < 0 || x >= d2))
+            P1 = (T)0;
+        if (EDGE && (!in || x < 0 || x + 1 >= d2))
+            P2 = (T)0;
+        const T P1d = __shfl_up_sync(0xffffffffu, P1, 1);
+        // the cell's faces' squares in the .m files' order (a missing face's
+        // zero changes nothing)
+        T sq = mul(P1, P1);
+        sq = add(sq, mul(P1d, P1d));
+        sq = add(sq, mul(P2, P2));
+        sq = add(sq, mul(P2m, P2m));
+        if (alp) {
+            al = av;
+            lim = surely_inside<T>(al);
+        }
+        const T F = factor(sq, al, lim);
+        // column x - 1: the rescale, its divergence
+        T R2 = mul(mul((T)0.5, P2m), add(F, Fm));
+        const T Fu = __shfl_down_sync(0xffffffffu, Fm, 1);
+        T R1 = mul(mul((T)0.5, P1m), add(Fu, Fm));
+        if (EDGE && !up)
+            R1 = (T)0;
+        const T R1d = __shfl_up_sync(0xffffffffu, R1, 1);
+        if (x > x0 && own) {
+            T d = R1;
+            if (!EDGE || y >= 1)
+                d = sub(d, R1d);
+            if (!EDGE || x < d2)
+                d = add(d, R2);
+            if (!EDGE || x >= 2)
+                d = sub(d, R2m);
+            const int o = (x - 1) * d1;
+            if (!EDGE || up)
+                q1p[o - (x - 1)] = R1;
+            if (!EDGE || x < d2)
+                q2p[o] = R2;
+            dp[o] = d;
+            if (last)
+                fp[o] = Fm;
+        }
+        gc = gr;
+        P1m = P1;
+        P2m = P2;
+        Fm = F;
+        R2m = R2;
+    };
+    fetch(x0 - 1);
+    for (int xb = x0 - 1; xb <= x1; xb += Q) {
+        T g4[Q], a4[Q], b4[Q], al4[Q];
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+            g4[k] = gn[k];
+            a4[k] = p1n[k];
+            b4[k] = p2n[k];
+            al4[k] = aln[k];
+        }
+        if (xb + Q <= x1)
+            fetch(xb + Q);
+        // from x = 2 on a column's two to the left are there too
+        if (xb >= 2 && xb + Q - 1 <= x1 && inner(xb)) {
+#pragma unroll
+            for (int k = 0; k < Q; ++k)
+                column(std::false_type{}, xb + k, g4[k], a4[k], b4[k], al4[k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < Q; ++k)
+                if (xb + k <= x1)
+                    column(std::true_type{}, xb + k, g4[k], a4[k], b4[k], al4[k]);
         }
     }
-    if (q >= 1 && q <= R + 2 && y_in) {                          // p2: y0-1 .. y0+R, x0-2 .. x0+S
-        for (int c = w; c <= S + 2; c += NW) {
-            const int x = x0 - 2 + c, f = c * FR + q;
-            if (x >= 0 && x + 1 < d2)
-                P2[f] = step(P2[f], G[f + FR], G[f]);
-        }
+}
+
+// 3D without direction fields: k2 with k3, and k4 with k5.  A cell forms its own
+// stepped faces and the three of the cells before it again (their inputs come
+// from L1), so a pass writes what it does not read and two passes do for four;
+// the stepped flows are the second copy.  The factors stay beside g, which the
+// cells around still read.  Same expressions in the same order as the passes.
+// Single precision only: an iteration of 80 x 80 x 64 voxels and seven nodes
+// takes 65 us against 115 with the four passes; in double precision, bound by
+// its operations, the faces formed twice cost more (60 x 50 x 40: 155 against
+// 142).
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_step_factor3d(const HArgs<T> A)
+{
+    const int i = 1 + (int)blockIdx.y;
+    const long long c = blockIdx.x * (long long)kThreads + threadIdx.x;
+    if (c >= A.n)
+        return;
+    const Pix<T> p(A, c);
+    const T *g = A.g + (long long)i * A.ns + c;
+    const int sx = A.d1, sz = A.d1 * A.d2;
+    const T gc = g[0];
+    // (p + g(k+1)) - g(k), asetsHMF3D.m
+    auto step = [&](T pv, T lo, T hi) { return A.paren ? add(pv, sub(hi, lo)) : sub(add(pv, hi), lo); };
+    T s = (T)0;
+    auto face = [&](const T *f, T lo, T hi, T *out) {
+        const T v = step(*f, lo, hi);
+        if (out)
+            *out = v;
+        s = add(s, mul(v, v));
+    };
+    const long long o1 = (long long)i * A.f1 + i1(A, p.y, p.x, p.z), o2 = (long long)i * A.f2 + i2(A, p.y, p.x, p.z),
+                    o3 = (long long)i * A.f3 + i3(A, p.y, p.x, p.z);
+    if (p.y + 1 < A.d1)
+        face(A.p1 + o1, gc, g[1], A.q1 + o1);
+    if (p.y >= 1)
+        face(A.p1 + o1 - 1, g[-1], gc, nullptr);
+    if (p.x + 1 < A.d2)
+        face(A.p2 + o2, gc, g[sx], A.q2 + o2);
+    if (p.x >= 1)
+        face(A.p2 + o2 - sx, g[-sx], gc, nullptr);
+    if (p.z + 1 < A.d3)
+        face(A.p3 + o3, gc, g[sz], A.q3 + o3);
+    if (p.z >= 1)
+        face(A.p3 + o3 - sz, g[-sz], gc, nullptr);
+    const NodeDev<T> &nd = A.nodes[i];
+    const T al = nd.alpha ? nd.alpha[c] : nd.alpha_s;
+    A.f[(long long)i * A.ns + c] = factor(s, al, surely_inside<T>(al));
+}
+
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_rescale_div3d(const HArgs<T> A)
+{
+    const int i = 1 + (int)blockIdx.y;
+    const long long c = blockIdx.x * (long long)kThreads + threadIdx.x;
+    if (c >= A.n)
+        return;
+    const Pix<T> p(A, c);
+    const T *f = A.f + (long long)i * A.ns + c;
+    const int sx = A.d1, sz = A.d1 * A.d2;
+    const T fc = f[0];
+    // p = 0.5 p (f(k+1) + f(k))
+    auto scale = [&](T v, T lo, T hi) { return mul(mul((T)0.5, v), add(hi, lo)); };
+    const long long o1 = (long long)i * A.f1 + i1(A, p.y, p.x, p.z), o2 = (long long)i * A.f2 + i2(A, p.y, p.x, p.z),
+                    o3 = (long long)i * A.f3 + i3(A, p.y, p.x, p.z);
+    T d = (T)0;
+    if (p.y + 1 < A.d1)
+        A.p1[o1] = d = scale(A.q1[o1], fc, f[1]);
+    if (p.y >= 1)
+        d = sub(d, scale(A.q1[o1 - 1], f[-1], fc));
+    if (p.x + 1 < A.d2) {
+        const T v = scale(A.q2[o2], fc, f[sx]);
+        A.p2[o2] = v;
+        d = add(d, v);
     }
-    __syncthreads();
-    // k3: the cell's faces' squares in the .m files' order, the factor
-    if (q >= 1 && q <= R + 2 && y_in) {                          // y0-1 .. y0+R, x0-1 .. x0+S
-        for (int c = 1 + w; c <= S + 2; c += NW) {
-            const int x = x0 - 2 + c, f = c * FR + q;
-            if (x < 0 || x >= d2)
-                continue;
-            T sq = (T)0;
-            if (y_up)
-                sq = add(sq, mul(P1[f], P1[f]));
-            if (y_dn)
-                sq = add(sq, mul(P1[f - 1], P1[f - 1]));
-            if (x + 1 < d2)
-                sq = add(sq, mul(P2[f], P2[f]));
-            if (x >= 1)
-                sq = add(sq, mul(P2[f - FR], P2[f - FR]));
-            const T mag = sqr(sq);
-            const T al = AL[f];
-            FS[f] = (mag <= al) ? (T)1 : dvd(al, mag);
-        }
+    if (p.x >= 1)
+        d = sub(d, scale(A.q2[o2 - sx], f[-sx], fc));
+    if (p.z + 1 < A.d3) {
+        const T v = scale(A.q3[o3], fc, f[sz]);
+        A.p3[o3] = v;
+        d = add(d, v);
     }
-    __syncthreads();
-    // k4: p = 0.5 p (f(k+1) + f(k)); the tile's own faces are stored
-    if (q >= 1 && q <= R + 1 && y >= 0 && y_up) {                // p1: y0-1 .. y0+R-1, tile columns
-        for (int c = 2 + w; c <= S + 1; c += NW) {
-            const int x = x0 - 2 + c, f = c * FR + q;
-            if (x >= d2)
-                break;
-            const T r = mul(mul((T)0.5, P1[f]), add(FS[f + 1], FS[f]));
-            P1[f] = r;
-            if (q >= 2)
-                p1[(unsigned int)x * (unsigned int)(d1 - 1) + (unsigned int)y] = r;
-        }
-    }
-    if (q >= 2 && q <= R + 1 && y < d1) {                        // p2: tile rows, x0-1 .. x0+S-1
-        for (int c = 1 + w; c <= S + 1; c += NW) {
-            const int x = x0 - 2 + c, f = c * FR + q;
-            if (x + 1 >= d2)
-                break;
-            if (x < 0)
-                continue;
-            const T r = mul(mul((T)0.5, P2[f]), add(FS[f + FR], FS[f]));
-            P2[f] = r;
-            if (c >= 2)
-                p2[(unsigned int)x * (unsigned int)d1 + (unsigned int)y] = r;
-        }
-    }
-    __syncthreads();
-    // k5: the tile's divergence; g keeps the factor, as k3 leaves it
-    T *divp = A.div + (long long)i * A.n;
-    T *gw = A.g + (long long)i * A.n;
-    if (q >= 2 && q <= R + 1 && y < d1) {
-        for (int c = 2 + w; c <= S + 1; c += NW) {
-            const int x = x0 - 2 + c, f = c * FR + q;
-            if (x >= d2)
-                break;
-            T d = y_up ? P1[f] : (T)0;
-            if (y_dn)
-                d = sub(d, P1[f - 1]);
-            if (x + 1 < d2)
-                d = add(d, P2[f]);
-            if (x >= 1)
-                d = sub(d, P2[f - FR]);
-            const unsigned int cell = (unsigned int)x * (unsigned int)d1 + (unsigned int)y;
-            divp[cell] = d;
-            gw[cell] = FS[f];
-        }
-    }
+    if (p.z >= 1)
+        d = sub(d, scale(A.q3[o3 - sz], f[-sz], fc));
+    A.div[(long long)i * A.ns + c] = d;
 }
 
 int h_grid(long long n, int sms)
@@ -999,16 +1154,32 @@ int h_grid(long long n, int sms)
 // gradient step on g, the geodesic exemption (nodes with direction fields),
 // flow magnitude and projection factor, rescale, divergence
 template <class T>
-void spatial_passes(const HArgs<T> &A, int gn, cudaStream_t st, bool dirs)
+void spatial_passes(HArgs<T> &A, int gn, int sms, cudaStream_t st, bool dirs, bool last)
 {
-    if (A.dim == 2 && !dirs && A.m > 1) {
-        // 28 x 32 tiles: a 32-row frame (one row per lane), within the
-        // default 48 KB of dynamic shared memory in double as well
-        constexpr int R = 28, S = 32;
-        using Q = SpatialTile<T, R, S>;
-        static_assert(Q::smem_bytes() <= 48 * 1024, "frame above the default shared memory");
-        const int ty = (A.d1 + R - 1) / R, tx = (A.d2 + S - 1) / S;
-        k_spatial_tile2d<T, R, S><<<dim3(ty * tx, A.m - 1), kThreads, Q::smem_bytes(), st>>>(A, ty);
+    if (A.q1 && A.dim == 3 && A.m > 1) {
+        const dim3 grid((unsigned int)((A.n + kThreads - 1) / kThreads), A.m - 1);
+        k_step_factor3d<T><<<grid, kThreads, 0, st>>>(A);
+        k_rescale_div3d<T><<<grid, kThreads, 0, st>>>(A);
+        if (last)
+            std::swap(A.g, A.f);
+        return;
+    }
+    if (A.q1 && A.m > 1) {
+        // columns a warp: six warps for each of an SM's four schedulers if the
+        // image has them, no fewer than six columns (three more are read on
+        // either side), in whole groups of four steps
+        const int strips = (A.d1 + kSweepRows - 1) / kSweepRows;
+        const long long rows = (long long)strips * (A.m - 1);
+        long long chunks = (sms * 24LL + rows - 1) / rows;
+        chunks = std::max(1LL, std::min(chunks, (long long)(A.d2 + 5) / 6));
+        const int S = ((int)((A.d2 + chunks - 1) / chunks) + 2 + 3) / 4 * 4 - 2;
+        const int total = strips * ((A.d2 + S - 1) / S), per = kSweepThreads / 32;
+        k_spatial_sweep2d<T><<<dim3((total + per - 1) / per, A.m - 1), kSweepThreads, 0, st>>>(
+            A, last ? 1 : 0, strips, total, S);
+        std::swap(A.p1, A.q1);
+        std::swap(A.p2, A.q2);
+        if (last)
+            std::swap(A.g, A.f);
         return;
     }
     k2_gradient<T><<<gn, kThreads, 0, st>>>(A);
@@ -1052,6 +1223,30 @@ bool setup_dirs(Get &get, cudaStream_t st, int dim, int m, void *const *const ld
     return true;
 }
 
+// The second copy of the flows, and the factors; the root has no flows and no
+// factor.
+template <class T, class Get>
+bool setup_copies(Get &get, cudaStream_t st, HArgs<T> &A, bool dirs, cudaError_t &e)
+{
+    if (dirs || (A.dim == 3 && sizeof(T) == 8))
+        return true;
+    void *vp = nullptr;
+    if (!get(&vp, sizeof(T) * (A.f1 + A.f2 + A.f3 + A.ns) * A.m))
+        return false;
+    A.f = static_cast<T *>(vp);
+    A.q1 = A.f + A.ns * A.m;
+    A.q2 = A.q1 + A.f1 * A.m;
+    A.q3 = A.q2 + A.f2 * A.m;
+    struct {
+        T *p;
+        long long count;
+    } const root[] = {{A.f, A.ns}, {A.q1, A.f1}, {A.q2, A.f2}, {A.q3, A.f3}};
+    for (const auto &r : root)
+        if (e == cudaSuccess && r.count > 0)
+            e = cudaMemsetAsync(r.p, 0, sizeof(T) * r.count, st);
+    return true;
+}
+
 // the normalised direction fields back into the caller's arrays
 template <class T>
 cudaError_t download_dirs(cudaStream_t st, int dim, int m, long long n, void *const *const ld[3],
@@ -1076,6 +1271,7 @@ asets_status run_hmf(asets_context *ctx, int algo, int dim, int d1, int d2, int 
     cudaStream_t st = context_stream(ctx);
     const int sms = context_num_sms(ctx);
     const long long n = (long long)d1 * d2 * d3;
+    const long long ns = (n + 3) / 4 * 4;
     const long long f1 = (long long)(d1 - 1) * d2 * d3, f2 = (long long)d1 * (d2 - 1) * d3,
                     f3 = dim == 3 ? (long long)d1 * d2 * (d3 - 1) : 0;
     // tree tables (children of each node in index order)
@@ -1114,19 +1310,21 @@ asets_status run_hmf(asets_context *ctx, int algo, int dim, int d1, int d2, int 
     A.cc = (T)cc;
     A.steps = (T)steps;
     A.inv_cc = (T)(1.0 / cc);
+    A.by_cc.set(A.cc);
+    A.ns = ns;
     // asetsHMF2D.m parenthesises the full-flow gradient step, not the pseudo-flow one
     A.paren = (dim == 2 && !pseudo) ? 1 : 0;
     std::vector<NodeDev<T>> nodes(m);
     void *vp = nullptr;
     cudaError_t e = cudaSuccess;
-    bool ok = get(&vp, sizeof(T) * n * m * 4);
+    bool ok = get(&vp, sizeof(T) * ns * m * 4);
     if (ok) {
         T *base = static_cast<T *>(vp);
         A.pt = base;
-        A.u = base + n * m;
-        A.div = base + 2 * n * m;
-        A.g = base + 3 * n * m;
-        e = cudaMemsetAsync(vp, 0, sizeof(T) * n * m * 4, st);
+        A.u = base + ns * m;
+        A.div = base + 2 * ns * m;
+        A.g = base + 3 * ns * m;
+        e = cudaMemsetAsync(vp, 0, sizeof(T) * ns * m * 4, st);
     }
     const long long fsum = (f1 + f2 + f3) * m;
     ok = ok && get(&vp, sizeof(T) * fsum);
@@ -1153,7 +1351,7 @@ asets_status run_hmf(asets_context *ctx, int algo, int dim, int d1, int d2, int 
         nd.alpha = nullptr;
         nd.nnorm = 1;
         if (nchild[i] == 0 && e == cudaSuccess) {
-            ok = get(&vp, sizeof(T) * n);
+            ok = get(&vp, sizeof(T) * ns);
             if (ok) {
                 e = cudaMemcpyAsync(vp, Ct[i], sizeof(T) * n, cudaMemcpyHostToDevice, st);
                 nd.ct = static_cast<const T *>(vp);
@@ -1168,10 +1366,11 @@ asets_status run_hmf(asets_context *ctx, int algo, int dim, int d1, int d2, int 
         }
         // pseudo-flow starts from the leaves' labels
         if (ok && pseudo && nchild[i] == 0 && e == cudaSuccess)
-            e = cudaMemcpyAsync(A.u + (long long)i * n, u_out[i], sizeof(T) * n, cudaMemcpyHostToDevice, st);
+            e = cudaMemcpyAsync(A.u + (long long)i * ns, u_out[i], sizeof(T) * n, cudaMemcpyHostToDevice, st);
     }
     bool dirs = false;
     ok = ok && setup_dirs<T>(get, st, dim, m, ld, nodes, A, e, dirs);
+    ok = ok && setup_copies<T>(get, st, A, dirs, e);
     ok = ok && get(&vp, sizeof(NodeDev<T>) * m);
     if (ok && e == cudaSuccess) {
         e = cudaMemcpyAsync(vp, nodes.data(), sizeof(NodeDev<T>) * m, cudaMemcpyHostToDevice, st);
@@ -1187,19 +1386,28 @@ asets_status run_hmf(asets_context *ctx, int algo, int dim, int d1, int d2, int 
         set_last_error("asets_hmf_full_flow: out of device memory");
     } else if (e == cudaSuccess) {
         const int gp = h_grid(n, sms), gn = h_grid(n * (m - 1), sms);
-        // the staged per-pixel pass for trees whose columns fit the default
-        // 48 KB of shared memory (15 nodes in float, 7 in double)
-        const int k1_smem = K1Stage::bytes(m, (int)sizeof(T));
+        const bool k1_tree = m <= kK1Nodes && !pseudo;
+        K1Tree tree{};
+        for (int i = 0; k1_tree && i < m; ++i) {
+            tree.parent[i] = nodes[i].parent;
+            tree.first[i] = begin[i];
+            tree.nchild[i] = nchild[i];
+            tree.kids[i] = i < m - 1 ? kids[i] : 0;
+            tree.ct[i] = nodes[i].ct;
+        }
+        if (k1_tree)
+            e = cudaFuncSetAttribute(k1_staged<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, k1_bytes(kK1Nodes));
         if (dirs)
             k_norm_dirs<T><<<h_grid(n * m, sms), kThreads, 0, st>>>(A);
         for (int it = 0; it < its && e == cudaSuccess; ++it) {
             if (pseudo)
                 k_pseudo_point<T><<<gp, kThreads, 0, st>>>(A);
-            else if (k1_smem <= 48 * 1024)
-                k1_staged<T><<<gp, kThreads, k1_smem, st>>>(A);
+            else if (k1_tree)
+                k1_staged<T><<<(int)((ns * sizeof(T) / 16 + kK1Threads - 1) / kK1Threads), kK1Threads, k1_bytes(m),
+                               st>>>(A, tree, it + 1 == its);
             else
                 k1_pointwise<T><<<gp, kThreads, 0, st>>>(A);
-            spatial_passes(A, gn, st, dirs);
+            spatial_passes(A, gn, sms, st, dirs, it + 1 == its);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) {
@@ -1217,13 +1425,13 @@ asets_status run_hmf(asets_context *ctx, int algo, int dim, int d1, int d2, int 
         for (int i = 0; i < m && e == cudaSuccess; ++i) {
             const size_t nb = sizeof(T) * n;
             if (u_out && u_out[i])
-                e = cudaMemcpyAsync(u_out[i], A.u + (long long)i * n, nb, cudaMemcpyDeviceToHost, st);
+                e = cudaMemcpyAsync(u_out[i], A.u + (long long)i * ns, nb, cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess && pt_out && pt_out[i] && !pseudo)
-                e = cudaMemcpyAsync(pt_out[i], A.pt + (long long)i * n, nb, cudaMemcpyDeviceToHost, st);
+                e = cudaMemcpyAsync(pt_out[i], A.pt + (long long)i * ns, nb, cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess && div_out && div_out[i])
-                e = cudaMemcpyAsync(div_out[i], A.div + (long long)i * n, nb, cudaMemcpyDeviceToHost, st);
+                e = cudaMemcpyAsync(div_out[i], A.div + (long long)i * ns, nb, cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess && g_out && g_out[i])
-                e = cudaMemcpyAsync(g_out[i], A.g + (long long)i * n, nb, cudaMemcpyDeviceToHost, st);
+                e = cudaMemcpyAsync(g_out[i], A.g + (long long)i * ns, nb, cudaMemcpyDeviceToHost, st);
             const T *fp[3] = {A.p1 + f1 * i, A.p2 + f2 * i, A.p3 + f3 * i};
             const long long fn[3] = {f1, f2, f3};
             for (int k = 0; k < dim && e == cudaSuccess; ++k)
@@ -1274,6 +1482,7 @@ asets_status run_dag(asets_context *ctx, int dim, int d1, int d2, int d3, int m,
     cudaStream_t st = context_stream(ctx);
     const int sms = context_num_sms(ctx);
     const long long n = (long long)d1 * d2 * d3;
+    const long long ns = (n + 3) / 4 * 4;
     const long long f1 = (long long)(d1 - 1) * d2 * d3, f2 = (long long)d1 * (d2 - 1) * d3,
                     f3 = dim == 3 ? (long long)d1 * d2 * (d3 - 1) : 0;
     std::vector<void *> bufs;
@@ -1297,6 +1506,8 @@ asets_status run_dag(asets_context *ctx, int dim, int d1, int d2, int d3, int m,
     A.cc = (T)cc;
     A.steps = (T)steps;
     A.inv_cc = (T)(1.0 / cc);
+    A.by_cc.set(A.cc);
+    A.ns = ns;
     A.paren = 0;  // both DAG files: (p + g(k+1)) - g(k)
     A.nedges = (int)kids.size();
     // child weights 1/(parents of the child); per node the sum of their squares
@@ -1331,15 +1542,15 @@ asets_status run_dag(asets_context *ctx, int dim, int d1, int d2, int d3, int m,
     }
     cudaError_t e = cudaSuccess;
     void *vp = nullptr;
-    bool ok = get(&vp, sizeof(T) * n * m * 5);
+    bool ok = get(&vp, sizeof(T) * ns * m * 5);
     if (ok) {
         T *base = static_cast<T *>(vp);
         A.pt = base;
-        A.u = base + n * m;
-        A.div = base + 2 * n * m;
-        A.g = base + 3 * n * m;
-        A.pn = base + 4 * n * m;
-        e = cudaMemsetAsync(vp, 0, sizeof(T) * n * m * 5, st);
+        A.u = base + ns * m;
+        A.div = base + 2 * ns * m;
+        A.g = base + 3 * ns * m;
+        A.pn = base + 4 * ns * m;
+        e = cudaMemsetAsync(vp, 0, sizeof(T) * ns * m * 5, st);
     }
     const long long fsum = (f1 + f2 + f3) * m;
     ok = ok && get(&vp, sizeof(T) * fsum);
@@ -1352,7 +1563,7 @@ asets_status run_dag(asets_context *ctx, int dim, int d1, int d2, int d3, int m,
     }
     for (int i = 0; ok && i < m && e == cudaSuccess; ++i) {
         if (nchild[i] == 0) {
-            ok = get(&vp, sizeof(T) * n);
+            ok = get(&vp, sizeof(T) * ns);
             if (ok) {
                 e = cudaMemcpyAsync(vp, Ct[i], sizeof(T) * n, cudaMemcpyHostToDevice, st);
                 nodes[i].ct = static_cast<const T *>(vp);
@@ -1368,6 +1579,7 @@ asets_status run_dag(asets_context *ctx, int dim, int d1, int d2, int d3, int m,
     }
     bool dirs = false;
     ok = ok && setup_dirs<T>(get, st, dim, m, ld, nodes, A, e, dirs);
+    ok = ok && setup_copies<T>(get, st, A, dirs, e);
     struct Up {
         const void *src;
         size_t bytes;
@@ -1397,7 +1609,7 @@ asets_status run_dag(asets_context *ctx, int dim, int d1, int d2, int d3, int m,
             k_norm_dirs<T><<<h_grid(n * m, sms), kThreads, 0, st>>>(A);
         for (int it = 0; it < its && e == cudaSuccess; ++it) {
             k_dag_g<T><<<gn, kThreads, 0, st>>>(A);
-            spatial_passes(A, gn, st, dirs);
+            spatial_passes(A, gn, sms, st, dirs, it + 1 == its);
             if (dag_smem <= 48 * 1024)
                 k_dag_point_staged<T><<<gp, kThreads, dag_smem, st>>>(A);
             else
@@ -1410,7 +1622,7 @@ asets_status run_dag(asets_context *ctx, int dim, int d1, int d2, int d3, int m,
         for (int i = 0; i < m && e == cudaSuccess; ++i) {
             for (int k = 0; k < 5 && e == cudaSuccess; ++k)
                 if (outs[k] && outs[k][i])
-                    e = cudaMemcpyAsync(outs[k][i], srcs[k] + (long long)i * n, sizeof(T) * n,
+                    e = cudaMemcpyAsync(outs[k][i], srcs[k] + (long long)i * ns, sizeof(T) * n,
                                         cudaMemcpyDeviceToHost, st);
             const T *fp[3] = {A.p1 + f1 * i, A.p2 + f2 * i, A.p3 + f3 * i};
             const long long fn[3] = {f1, f2, f3};

@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "asets.h"
+#include "div_const.cuh"
 #include "internal.h"
 
 using namespace asets;
@@ -52,8 +53,7 @@ struct MTArgs {
     int rows, cols, slices, nlab, nflow;
     long long n, f1, f2, f3;  // cells and faces per flow label
     T cc, steps, half, one_over_cc, one_over_ccl, beta;
-    T rcc, rcc_lo;        // double: 1/cc rounded, and the rest of 1/cc
-    unsigned int div_span;  // exponents that div_cc corrects (0: none)
+    DivConst<T> by_cc;
     T inv_nlab;           // 1/nlab where nlab is a power of two, else 0
     const T *cs, *ct, *alpha;
     T *u, *ucc, *ud, *pt, *ps, *divp, *gk, *p1, *p2, *p3, *q1, *q2, *q3;
@@ -97,25 +97,6 @@ __device__ __forceinline__ bool is_one(double x)
     return __double2hiint(x) == 0x3ff00000 && __double2loint(x) == 0;
 }
 
-// x/cc rounded to nearest from 1/cc = rcc + rcc_lo (rcc rounded to nearest).
-// q = x*rcc + x*rcc_lo is within an ulp of the quotient (half an ulp of its
-// own rounding, 2^-50 of one for the terms), so Markstein's correction
-// (Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000", 1990) with the exact residual x - q*cc rounds it correctly.
-// Zero keeps its sign; exponents where a term could leave the normal range
-// (and non-finite x) take the division.
-__device__ __forceinline__ double div_cc(double x, double cc, double rcc, double rcc_lo,
-                                         unsigned int span)
-{
-    const int e = __double2hiint(x) & 0x7ff00000;
-    if ((unsigned int)(e - 0x10000000) < span) {
-        double q = __fma_rn(x, rcc, __dmul_rn(x, rcc_lo));
-        const double r = __fma_rn(-q, cc, x);
-        return __fma_rn(r, rcc, q);
-    }
-    return x == 0.0 ? __dmul_rn(x, rcc) : __ddiv_rn(x, cc);
-}
-
 // u/cc of element o: kept beside u in double precision, divided here in single
 template <class T>
 __device__ __forceinline__ T u_cc(const MTArgs<T> &A, long long o, T u)
@@ -140,7 +121,7 @@ __device__ __forceinline__ T set_u(const MTArgs<T> &A, long long o, T v)
 {
     A.u[o] = v;
     if constexpr (sizeof(T) == 8) {
-        const T q = div_cc(v, A.cc, A.rcc, A.rcc_lo, A.div_span);
+        const T q = A.by_cc(v, A.cc);
         A.ucc[o] = q;
         return q;
     } else {
@@ -911,16 +892,7 @@ asets_status mt_run(asets_context *ctx, int rows, int cols, int slices, int nlab
     A.one_over_cc = (T)(1.0 / cc);
     A.one_over_ccl = (T)(1.0 / (cc * A.nlab));
     A.beta = (T)beta;
-    A.rcc = (T)1 / A.cc;
-    // 1/cc - rcc to about twice the precision: the residual 1 - rcc*cc is exact
-    A.rcc_lo = (T)(std::fma(-(double)A.rcc, (double)A.cc, 1.0) / (double)A.cc);
-    // 2^-767 <= |x| < 2^769 for an ordinary cc; the correction's proof leaves
-    // out a divisor whose significand is all ones
-    int cc_exp = 0;
-    const double cc_frac = std::fabs(std::frexp((double)A.cc, &cc_exp));
-    A.div_span = (std::isnormal((double)A.cc) && std::abs(cc_exp) < 200 && cc_frac < 1.0 - 0x1p-53)
-                     ? 0x60000000u
-                     : 0u;
+    A.by_cc.set(A.cc);
     A.inv_nlab = (A.nlab & (A.nlab - 1)) == 0 ? (T)1 / (T)A.nlab : (T)0;
     const int nct = A.nlab, nu = (M == MT_ISHIKAWA) ? nlab - 1 : A.nlab;
     const int npt = A.nlab;
