@@ -15,7 +15,7 @@ __device__ __forceinline__ void finish_iteration(float erru, IterControl *ctl, d
                                                  float *cvg, int it, double *s_red,
                                                  int *s_is_last, unsigned int *done_count)
 {
-    const double part = block_sum_double<NT>(erru, s_red);
+    const double part = block_sum<NT>(erru, s_red);
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = part;
         __threadfence();
@@ -25,9 +25,7 @@ __device__ __forceinline__ void finish_iteration(float erru, IterControl *ctl, d
     __syncthreads();
     if (*s_is_last && threadIdx.x < 32) {
         __threadfence();
-        double acc = 0.0;
-        for (int b = threadIdx.x; b < (int)gridDim.x; b += 32)
-            acc += __ldcg(partials + b);
+        double acc = lane_partials(partials, (int)gridDim.x);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
             acc += __shfl_xor_sync(0xffffffffu, acc, o);

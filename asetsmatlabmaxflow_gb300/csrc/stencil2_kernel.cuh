@@ -178,14 +178,14 @@ __device__ __forceinline__ void rows_down(const float (&v)[CELLS], float (&dn)[C
 }
 
 // TWIN: the Matlab twins' mean (formed in double, then rounded)
-template <int NT, bool TWIN = false>
-__device__ __forceinline__ void finish_item(double erru, const ProblemDesc &P, int li, int it,
+template <int NT, bool TWIN = false, class Sum>
+__device__ __forceinline__ void finish_item(Sum erru, const ProblemDesc &P, int li, int it,
                                             unsigned int *done_count, double *s_red,
                                             int *s_is_last)
 {
-    // erriter of this item in double, then the last item of the problem's
+    // erriter of this item (a float or a pair of floats), then the last item of the problem's
     // iteration sums the item partials in item order (deterministic)
-    const double part = block_sum_double<NT>(erru, s_red);
+    const double part = block_sum<NT>(erru, s_red);
     IterControl *ctl = P.ctl;
     if (threadIdx.x == 0) {
         P.item_partials[li] = part;
@@ -196,9 +196,7 @@ __device__ __forceinline__ void finish_item(double erru, const ProblemDesc &P, i
     __syncthreads();
     if (*s_is_last && threadIdx.x < 32) {
         __threadfence();
-        double acc = 0.0;
-        for (int b = threadIdx.x; b < P.n_items; b += 32)
-            acc += __ldcg(P.item_partials + b);
+        double acc = lane_partials(P.item_partials, P.n_items);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
             acc += __shfl_xor_sync(0xffffffffu, acc, o);

@@ -60,9 +60,9 @@ __device__ __forceinline__ void finish_item_t2(float erru_a, float erru_b, const
                                                int li, int it, unsigned int *done_count,
                                                double *s_red, int *s_is_last)
 {
-    const double pa = block_sum_double<NT>(erru_a, s_red);
+    const double pa = block_sum<NT>(erru_a, s_red);
     __syncthreads();
-    const double pb = block_sum_double<NT>(erru_b, s_red);
+    const double pb = block_sum<NT>(erru_b, s_red);
     IterControl *ctl = P.ctl;
     if (threadIdx.x == 0) {
         P.item_partials[2 * li] = pa;
@@ -74,11 +74,8 @@ __device__ __forceinline__ void finish_item_t2(float erru_a, float erru_b, const
     __syncthreads();
     if (*s_is_last && threadIdx.x < 32) {
         __threadfence();
-        double acc_a = 0.0, acc_b = 0.0;
-        for (int b = threadIdx.x; b < P.n_items; b += 32) {
-            acc_a += __ldcg(P.item_partials + 2 * b);
-            acc_b += __ldcg(P.item_partials + 2 * b + 1);
-        }
+        double acc_a = lane_partials(P.item_partials, P.n_items, 2);
+        double acc_b = lane_partials(P.item_partials + 1, P.n_items, 2);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             acc_a += __shfl_xor_sync(0xffffffffu, acc_a, o);

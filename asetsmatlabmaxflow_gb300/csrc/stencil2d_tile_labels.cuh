@@ -78,6 +78,87 @@ __device__ __forceinline__ void cp_async_wait_all()
     asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
+// Starts the copies of tile li's old state into the frames.  `keep`: the
+// frames already hold the tile's own cells, alpha and Ct from the iteration
+// before, and only the cells around the tile are copied, whose place in the
+// frame is a chunk's first or last row group or one of the five outer columns.
+// Warp 0 takes no part: it decides meanwhile whether the solve goes on.  The
+// others take a frame each, a lane the same chunks of every frame, so that a
+// chunk's place is found once.
+template <int MODEL, int NT>
+__device__ __forceinline__ void ltile_load(const ProblemDesc &P, int par, int li, float *sm, bool keep)
+{
+    using G = LTileGeom<MODEL>;
+    constexpr int R = G::R, S = G::S, FR = G::FR, FC = G::FC, F = G::F;
+    constexpr int Q = FR / 4;                    // chunks of a frame column
+    constexpr int OUTER = (FC - S) * Q + S * 2;  // of them around the tile
+    constexpr int W = NT / 32 - 1;
+    const int w = (int)(threadIdx.x >> 5) - 1, lane = threadIdx.x & 31;
+    if (w < 0)
+        return;
+    const int FL = P.nlab_items, L = (MODEL == 1) ? FL : FL + 1;
+    const int nr = P.nr, ns = P.ns;
+    const int r0 = (li % P.tiles_r) * R, s0 = (li / P.tiles_r) * S;
+    const unsigned int pitch = (unsigned int)P.plane_stride, lst = (unsigned int)P.label_stride;
+    // old state: the other parity
+    const float *src_br = P.dst_b[par ^ 1][SL_BR], *src_bs = P.dst_b[par ^ 1][SL_BS];
+    const float *src_u = P.dst_s[par ^ 1][2];
+    const float *src_pt = (MODEL == 1) ? P.dst_s[par ^ 1][1] : P.dst_s[par ^ 1][0];
+    const float *src_ps = P.dst_s[par ^ 1][0];                  // Potts
+    // the chunk of column c, rows r .. r+3 of the image: 0 .. 16 bytes of it inside
+    auto inside = [&](int r, int s) { return s >= 0 && s < ns && r >= 0 && r < nr ? min(16, (nr - r) * 4) : 0; };
+    const int nframe = 4 * FL + L + (MODEL == 1 ? 1 : 0);
+    const int per = keep ? OUTER : FC * Q;
+    for (int i0 = lane; i0 < per; i0 += 64) {
+        unsigned int off[2];
+        int dst[2], bytes[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int i = i0 + 32 * k;
+            int c = i / Q, j = i - c * Q;
+            if (keep) {
+                const int o = (i - S * 2) / Q;
+                c = i < S * 2 ? 2 + (i >> 1) : (o < 2 ? o : o + S);
+                j = i < S * 2 ? (i & 1) * (Q - 1) : i - S * 2 - o * Q;
+            }
+            const int r = r0 - 4 + 4 * j, s = s0 - 2 + c;
+            bytes[k] = i < per ? inside(r, s) : -1;
+            off[k] = bytes[k] > 0 ? (unsigned int)s * pitch + (unsigned int)r : 0u;
+            dst[k] = c * FR + 4 * j;
+        }
+        for (int f = w; f < (keep ? nframe - FL : nframe); f += W) {
+            const int fr = keep && f >= 3 * FL ? f + FL : f;  // without alpha
+            const float *src;
+            if (fr < FL) src = src_br + (unsigned int)fr * lst;
+            else if (fr < 2 * FL) src = src_bs + (unsigned int)(fr - FL) * lst;
+            else if (fr < 3 * FL) src = src_u + (unsigned int)(fr - 2 * FL) * lst;
+            else if (fr < 4 * FL) src = P.alpha + (unsigned int)(fr - 3 * FL) * lst;
+            else if (fr < 4 * FL + L) src = src_pt + (unsigned int)(fr - 4 * FL) * lst;
+            else src = src_ps;
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                if (bytes[k] >= 0)
+                    cp_async16(sm + fr * F + dst[k], src + off[k], bytes[k]);
+        }
+    }
+    if (!keep) {
+        // Ct on the tile: a lane has chunks of 4 rows, 64 to a label
+        static_assert(S * (R / 4) == 64, "two chunks a lane");
+        float *CT = sm + (nframe + 4 * G::GROUPS) * F + FL * R * S;
+        for (int l = w; l < L; l += W)
+#pragma unroll
+            for (int i = lane; i < 64; i += 32) {
+                const int c = i / (R / 4), j = i % (R / 4), r = r0 + 4 * j, s = s0 + c;
+                const int bytes = inside(r, s);
+                cp_async16(CT + l * R * S + c * R + 4 * j,
+                           P.ct + (bytes ? (unsigned int)l * lst + (unsigned int)s * pitch + r : 0u), bytes);
+            }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// One iteration of tile li whose loads are in flight; leaves the tile's new
+// state in the frames as well as in the other parity.
 template <int MODEL, int NT, bool EXACT>
 __device__ __forceinline__ float ltile_iteration(const ProblemDesc &P, int par, int li, float *sm)
 {
@@ -97,54 +178,13 @@ __device__ __forceinline__ float ltile_iteration(const ProblemDesc &P, int par, 
     float *PSf = PTf + L * F;                                   // Potts only
     float *Wk = PSf + (MODEL == 1 ? F : 0);                     // per group: GK, BR1, BS1, G2
     float *DV = Wk + 4 * G::GROUPS * F, *CT = DV + FL * R * S;
-    // old state (the other parity), and the new
-    const float *src_br = P.dst_b[par ^ 1][SL_BR], *src_bs = P.dst_b[par ^ 1][SL_BS];
-    const float *src_u = P.dst_s[par ^ 1][2];
-    const float *src_pt = (MODEL == 1) ? P.dst_s[par ^ 1][1] : P.dst_s[par ^ 1][0];
-    const float *src_ps = P.dst_s[par ^ 1][0];                  // Potts
     float *d_br = P.dst_b[par][SL_BR], *d_bs = P.dst_b[par][SL_BS];
     float *d_u = P.dst_s[par][2];
     float *d_pt = (MODEL == 1) ? P.dst_s[par][1] : P.dst_s[par][0];
     float *d_ps = P.dst_s[par][0];                              // Potts
 
-    // ---- all loads in flight at once: frame chunk (column c, rows
-    // r0-4+4j .. +3) of each frame array, Ct on the tile
-    {
-        const int nframe = 4 * FL + L + (MODEL == 1 ? 1 : 0);
-        const int chunks = FC * (FR / 4);
-        for (int i = tid; i < nframe * chunks; i += NT) {
-            const int fr = i / chunks, rem = i - fr * chunks;
-            const int c = rem / (FR / 4), j = rem - c * (FR / 4);
-            const int r = r0 - 4 + 4 * j, s = s0 - 2 + c;
-            const float *src;
-            int lab;
-            if (fr < FL) { src = src_br; lab = fr; }
-            else if (fr < 2 * FL) { src = src_bs; lab = fr - FL; }
-            else if (fr < 3 * FL) { src = src_u; lab = fr - 2 * FL; }
-            else if (fr < 4 * FL) { src = P.alpha; lab = fr - 3 * FL; }
-            else if (fr < 4 * FL + L) { src = src_pt; lab = fr - 4 * FL; }
-            else { src = src_ps; lab = 0; }
-            int bytes = 0;
-            if (s >= 0 && s < ns && r >= 0 && r < nr)
-                bytes = min(16, (nr - r) * 4);
-            const float *g = bytes ? src + (unsigned int)lab * lst + (unsigned int)s * pitch + r : src;
-            cp_async16(sm + fr * F + c * FR + 4 * j, g, bytes);
-        }
-        // Ct of the tile: L labels x S columns x R/4 chunks
-        for (int i = tid; i < L * S * (R / 4); i += NT) {
-            const int l = i / (S * (R / 4)), rem = i - l * (S * (R / 4));
-            const int c = rem / (R / 4), j = rem - c * (R / 4);
-            const int r = r0 + 4 * j, s = s0 + c;
-            int bytes = 0;
-            if (s < ns && r < nr)
-                bytes = min(16, (nr - r) * 4);
-            const float *g =
-                bytes ? P.ct + (unsigned int)l * lst + (unsigned int)s * pitch + r : P.ct;
-            cp_async16(CT + l * R * S + c * R + 4 * j, g, bytes);
-        }
-        cp_async_wait_all();
-        __syncthreads();
-    }
+    cp_async_wait_all();
+    __syncthreads();
 
     // ---- per flow label: gk, b', g2, b'' (stored), the divergence on the
     // tile; group gi takes labels gi, gi + GROUPS, ... with its own work
@@ -243,17 +283,17 @@ __device__ __forceinline__ float ltile_iteration(const ProblemDesc &P, int par, 
                 const float ctv = CT[l * R * S + i];
                 float p = (ps + uc) - dv;
                 p = (p < ctv) ? p : ctv;
-                d_pt[(unsigned int)l * lst + g] = p;
+                d_pt[(unsigned int)l * lst + g] = PTf[l * F + f] = p;
                 const float ft = dv + p;
                 DV[l * R * S + i] = ft;   // ft_l for the multipliers
                 fsum += (ft - uc);
             }
             const float ps_n = (EXACT ? __fdiv_rn(fsum, (float)L) : fsum * (1.0f / (float)L)) +
                                P.inv_cc_l;
-            d_ps[g] = ps_n;
+            d_ps[g] = PSf[f] = ps_n;
             for (int l = 0; l < L; ++l) {
                 const float e = cc * (DV[l * R * S + i] - ps_n);
-                d_u[(unsigned int)l * lst + g] = Uf[l * F + f] - e;
+                d_u[(unsigned int)l * lst + g] = Uf[l * F + f] = Uf[l * F + f] - e;
                 erru += abs_ref(e);
             }
         } else {
@@ -277,11 +317,11 @@ __device__ __forceinline__ float ltile_iteration(const ProblemDesc &P, int par, 
                     fpt = ((-dv_below) + pt_below) + ucc_below;
                 }
                 const float pt_new = min_ref(fpt, CT[l * R * S + i]);
-                d_pt[(unsigned int)l * lst + g] = pt_new;
+                d_pt[(unsigned int)l * lst + g] = PTf[l * F + f] = pt_new;
                 if (l >= 1) {
                     // multiplier of layer l-1 with the new pts
                     const float e = cc * ((dv_below + pt_new) - pt_below);
-                    d_u[(unsigned int)(l - 1) * lst + g] = u_below - e;
+                    d_u[(unsigned int)(l - 1) * lst + g] = Uf[(l - 1) * F + f] = u_below - e;
                     erru += abs_ref(e);
                 }
                 pt_below = pt_new;
@@ -326,6 +366,7 @@ __global__ void __launch_bounds__(NT, 2) stencil2d_tile_labels_kernel(const __gr
             continue;  // the problem has converged
         const ProblemDesc &P = B.probs[B.item_problem[item]];
         const int li = item - P.item_begin;
+        ltile_load<MODEL, NT>(P, it & 1, li, fsm, false);
         const float erru = ltile_iteration<MODEL, NT, EXACT>(P, it & 1, li, fsm);
         finish_item<NT>(erru, P, li, it, B.done_count, s_red, &s_is_last);
     }
@@ -348,9 +389,11 @@ __global__ void __launch_bounds__(NT, 2)
     __shared__ double s_red[NT / 32];
     __shared__ int s_stop;
     const ProblemDesc &P = B.probs[0];
-    tile_solve_loop<NT>(P, B.queue, s_red, &s_stop, [&](int it, int tile) {
-        return ltile_iteration<MODEL, NT, EXACT>(P, it & 1, tile, fsm);
-    });
+    tile_solve_loop<NT>(
+        P, B.queue, s_red, &s_stop,
+        [&](int it, int tile, bool keep) { ltile_load<MODEL, NT>(P, it & 1, tile, fsm, keep); },
+        [&](int it, int tile) { return ltile_iteration<MODEL, NT, EXACT>(P, it & 1, tile, fsm); });
+    cp_async_wait_all();
 }
 
 }  // namespace asets

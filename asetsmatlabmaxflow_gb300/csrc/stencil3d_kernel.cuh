@@ -177,18 +177,6 @@ __device__ __forceinline__ float proj_twin(float a, float b, float d, float e, f
 // Matlab's min(a, b); a NaN a is kept.
 __device__ __forceinline__ float min_twin(float a, float b) { return (a <= b || a != a) ? a : b; }
 
-// A sum of floats as an unevaluated pair (TwoSum, Knuth): about 48 bits, at
-// float speed (the FP64 pipe would take as long as the rest of the step).
-struct FloatPair {
-    float hi = 0.f, lo = 0.f;
-    __device__ __forceinline__ void add(float x)
-    {
-        const float s = __fadd_rn(hi, x), bv = __fsub_rn(s, hi);
-        lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bv)), __fsub_rn(x, bv)));
-        hi = s;
-    }
-};
-
 template <int TC, int CELLS, int NSTAGE, int EPI, bool EXACT>
 __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
     stencil3d_kernel(const __grid_constant__ BatchArgs B)
@@ -625,9 +613,10 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
             o_sp += plane_stride;
         }
         __syncthreads();  // stage slots and factor planes are reused by the next item
-        if constexpr (BIN)
-            finish_item<NT, TWIN>(TWIN ? (double)errp.hi + (double)errp.lo : (double)erru, P, li, it,
-                                  B.done_count, s_red, &s_is_last);
+        if constexpr (TWIN)
+            finish_item<NT, true>(errp, P, li, it, B.done_count, s_red, &s_is_last);
+        else if constexpr (BIN)
+            finish_item<NT>(erru, P, li, it, B.done_count, s_red, &s_is_last);
     }
 
     // the last block to leave re-arms the queue for the next launch
