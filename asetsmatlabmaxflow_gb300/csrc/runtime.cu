@@ -458,8 +458,61 @@ static double persistent_load(const asets_solver *s, const StencilVariant *v)
     return (double)tiles / (double)slots;
 }
 
-// Largest multi-label 2D image (pixels) the whole-solve tile kernel takes by default.
-static constexpr long long kTileLabelsMaxPx = 1LL << 17;
+// Default forms of a single multi-label 2D solve.  An image whose 16 x 16 tiles
+// are at most two per resident block runs as one whole-solve launch, and with
+// few flow labels fl also some more: r tiles a block (rounded up) with r*(fl + 2)
+// up to 16 in fast mode below 300,000 pixels, up to 21 in EXACT, whose sweeps
+// are slower.  Measured (us per iteration, tiles | best other form or default):
+// fast Potts 512^2 L = 2 (16) 20.0 | 21.5, 440^2 L = 3 (15) 19.4 | 21.2, L = 4
+// (18) 22.8 | 21.7; EXACT 512^2 L = 3 (20) 26.9 | 28.7, 440^2 L = 5 (21) 33.0 |
+// 36.3, L = 6 (24) 36.8 | 34.7.
+static constexpr double kTileLabelsLoad = 2.0, kTileLabelsWork = 16.0, kTileLabelsWorkExact = 21.0;
+static constexpr long long kFusedMinPx = 300000, kFusedMinPxExact = 1LL << 17;
+// Then one of the one-pass sweeps (0 in-step update, 1 one label warp, 2 two)
+// or the two-pass form (-1), by pixels: each from its line on, the last one
+// that is reached.  A sweep's time depends on how many warps its flow and
+// label updates make and what they wait for, so the lines are those of
+// measurements at 131,000 to 7.8 million pixels (as 362^2, 640 x 600, 800 x
+// 820, 1024^2, 1450 x 1300, 2048^2, 3000 x 2600) for each label count; the
+// choice wins 5 to 25 % at most sizes, e.g. fast Potts 800 x 820 L = 4 33.9 |
+// 37.6 two-pass, Ishikawa 1024^2 L = 6 49.9 | 65.3, Potts 2048^2 L = 7 235 | 350
+// (one label warp 498).
+struct FusedLine {
+    long long from;
+    int form;
+};
+static constexpr FusedLine kFusedForms[2][2][8][3] = {
+    {{// fast Potts, 1 .. 8 flow labels
+      {{0, 0}}, {{0, 0}, {450000, -1}, {2000000, 1}}, {{0, 2}}, {{0, 0}, {1200000, 1}},
+      {{0, 0}, {4000000, 2}}, {{0, 0}, {4000000, 2}}, {{0, 0}, {1500000, 2}}, {{0, 2}}},
+     {// fast Ishikawa
+      {{0, 0}}, {{0, 0}, {600000, -1}, {2000000, 1}}, {{0, 0}, {2000000, 2}}, {{0, 0}, {2000000, 1}},
+      {{0, 0}, {5000000, 2}}, {{0, 0}, {4000000, 2}}, {{0, 0}}, {{0, 0}, {5000000, 2}}}},
+    {{// EXACT Potts
+      {{0, -1}, {2200000, 0}}, {{0, -1}}, {{0, -1}, {1500000, 0}}, {{0, 1}},
+      {{0, 2}, {350000, 1}, {1200000, 0}}, {{0, -1}, {250000, 1}}, {{0, 2}, {700000, 1}}, {{0, 2}}},
+     {// EXACT Ishikawa
+      {{0, 1}, {900000, -1}, {1500000, 0}}, {{0, 1}}, {{0, 2}, {900000, 0}}, {{0, 1}},
+      {{0, 2}, {500000, 0}}, {{0, 2}}, {{0, 2}, {4000000, 0}}, {{0, 2}}}}};
+
+// Below two million pixels only images at most four times as wide as tall (the
+// sweep runs along the width: 181 x 2000 fast Potts L = 6 43.0 | 38.7 two-pass,
+// 333 x 1100 L = 4 28.7 | 30.4) and, with fewer than six flow labels, at most
+// twice as tall as wide (1383 x 555 Ishikawa L = 3 31.5 | 29.0; 3000 x 130 Potts
+// L = 6 31.8 | 33.0).
+static int fused_form(bool ishikawa, int flow_labels, int exact, int nr, int ns)
+{
+    const long long px = (long long)nr * ns;
+    if (px < (exact ? kFusedMinPxExact : kFusedMinPx) || flow_labels > 8)
+        return -1;
+    if (px < 2000000 && (ns > 4LL * nr || (flow_labels < 6 && nr > 2LL * ns)))
+        return -1;
+    const FusedLine *line = kFusedForms[exact ? 1 : 0][ishikawa ? 1 : 0][flow_labels - 1];
+    int form = line[0].form;
+    for (int k = 1; k < 3 && line[k].from > 0 && px >= line[k].from; ++k)
+        form = line[k].form;
+    return form;
+}
 // Most 32 x 32 tiles per resident block the binary whole-solve kernel takes
 // by default: fast, every tile resident at once (beyond that the
 // two-iteration sweep wins); EXACT, up to eight (about 1600^2 pixels: the
@@ -494,25 +547,20 @@ static const StencilVariant *pick_variant(asets_solver *s, int exact, int tile_c
     }
     // the one-pass multi-label kernels lead the list: three sweeps (in-step
     // update, one label warp, two), then 16 x 16 tiles (one launch per
-    // iteration, the whole solve in one).  By default they run where they
-    // measured faster than the two-pass form on a GB300: the whole-solve
-    // tiles on images of up to 2^17 pixels (two tiles per block at most);
-    // the sweeps on two
-    // million pixels and more (two label warps for up to three flow labels,
-    // one above), and half a million with six flow labels or more (in-step)
+    // iteration, the whole solve in one)
     int n_fused = 0;
     while (n_fused < (int)match.size() && match[n_fused]->epi == EPI_FUSED)
         ++n_fused;
     if (n_fused == 5) {
         const long long px = (long long)s->nr * s->ns;
         const int fl = s->flow_labels;
-        const double load = persistent_load(s, match[4]);
-        if (px <= kTileLabelsMaxPx && load > 0.0 && load <= 2.0)
+        const double load = persistent_load(s, match[4]), work = std::ceil(load) * (fl + 2);
+        if (load > 0.0 && (load <= kTileLabelsLoad ||
+                           (exact ? work <= kTileLabelsWorkExact : work <= kTileLabelsWork && px < kFusedMinPx)))
             return match[4];
-        if (px >= 2000000)
-            return match[fl <= 3 ? 2 : 1];
-        if (px >= 500000 && fl >= 6)
-            return match[0];
+        const int form = fused_form(s->model == ASETS_ISHIKAWA, fl, exact, s->nr, s->ns);
+        if (form >= 0)
+            return match[form];
     }
     match.erase(match.begin(), match.begin() + n_fused);
     // small binary 2D images: the whole solve in one cooperative launch when

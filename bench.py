@@ -6,7 +6,7 @@ iterations per step (the throughput run of the binary 3D workload).
 One JSON line on rank 0.  `value` is whole-job Gvoxel-iter/s with inputs
 resident in HBM; `e2e` the same through the C ABI one-shot call
 (asets_binary_mf3d) from pinned host buffers, host<->device copies included.
-`roofline` relates the fused iteration kernel's algorithmic bytes (60 B per
+`roofline` relates the fused iteration kernel's algorithmic bytes (52 B per
 voxel-iteration: 6 state arrays read+written, 3 inputs read) to the measured
 HBM copy bandwidth.  `--impl reference` times the CPU restatement of the
 reference C solver (bit-identical to it) on all host cores, one independent
@@ -35,7 +35,8 @@ UNIT = "Gvoxel-iter/s"
 SHAPE = (256, 256, 256)
 ITERS = 200
 CC, STEPS = 0.35, 0.11
-BYTES_PER_VOXEL_ITER = 60  # 6 state arrays x (read + write) x 4 B + 3 inputs x 4 B
+# a cold start: gk, three flows, pt and u in one word, read + written; alpha, Cs, Ct read
+BYTES_PER_VOXEL_ITER = 52
 WORKLOAD = "binary3d_256^3_200it"
 
 
@@ -853,7 +854,7 @@ def main():
                     "h2d_bytes_per_step": 3 * nvox * 4, "d2h_bytes_per_step": nvox * 4 + ITERS * 4},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
-                         "peak_kind": peak_kind, "kernel": "stencil_col_kernel<3, 16 warps, 2 rows per thread (60x12 tile), 5 stages, refill in Z, binary, fast>",
+                         "peak_kind": peak_kind, "kernel": "stencil3d_kernel<14 columns, 2 rows per thread (64x14 tile), 3 stages, cold start, fast>",
                          "bytes_per_voxel_iter": BYTES_PER_VOXEL_ITER,
                          "launch_ms": per_launch_ms},
             "time_to_errbound": {"err_bound": 1e-4, "iterations": conv_it, "ms": conv_ms,
