@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "asets.h"
+#include "device_common.cuh"
 #include "internal.h"
 
 using namespace asets;
@@ -273,11 +274,15 @@ __global__ void pass_f(const SSArgs A)
         s_last = (atomicAdd(&A.ctl->ticket, 1u) == gridDim.x - 1);
     }
     __syncthreads();
-    if (s_last && threadIdx.x == 0) {
-        __threadfence();
-        double tot = 0.0;
-        for (unsigned int b = 0; b < gridDim.x; ++b)
-            tot += __ldcg(A.partials + b);
+    if (!s_last || threadIdx.x >= 32)
+        return;
+    // one warp, eight loads in flight (one thread, one after another: 53 us of the
+    // 304 of an iteration of 512 x 512, L = 4)
+    __threadfence();
+    double tot = lane_partials(A.partials, (int)gridDim.x);
+    for (int o = 16; o > 0; o >>= 1)
+        tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    if (threadIdx.x == 0) {
         const double e = tot / A.ctl->vol;
         A.erriter[it] = e;
         if (e < A.ctl->beta) {
