@@ -564,13 +564,15 @@ static const StencilVariant *pick_variant(asets_solver *s, int exact, int tile_c
     }
     match.erase(match.begin(), match.begin() + n_fused);
     // small binary 2D images: the whole solve in one cooperative launch when
-    // every tile can be resident (16 x 16 tiles up to 2^17 pixels, else
-    // 32 x 32; EXACT also with up to eight 32 x 32 tiles per block),
-    // measured faster than the sweeps there
+    // every tile can be resident (16 x 16 tiles up to three an SM, in EXACT
+    // mode 3.3, else 32 x 32; EXACT also with up to eight 32 x 32 tiles per
+    // block), measured faster than the sweeps there.  16 x 16 | 32 x 32, us per
+    // iteration: 320^2 (2.6 an SM) 6.6 | 7.0, 340^2 (3.2) 7.4 | 7.1, 362^2 (3.5)
+    // 8.4 | 7.1; EXACT 340^2 8.1 | 8.8, 362^2 9.2 | 8.8
     if (single && s->dim == 2 && s->model == ASETS_BINARY) {
-        const long long px = (long long)s->nr * s->ns;
+        const long long tiles16 = (long long)((s->nr + 15) / 16) * ((s->ns + 15) / 16);
         for (int want : {16, 32}) {
-            if (want == 16 && px > (1LL << 17))
+            if (want == 16 && tiles16 > (exact ? 3.3 : 3.0) * s->ctx->num_sms)
                 continue;
             for (auto *v : match)
                 if (v->persistent && v->s_tile == want) {
