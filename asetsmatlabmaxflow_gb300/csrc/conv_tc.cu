@@ -34,7 +34,7 @@
 namespace asets {
 
 constexpr int kConvThreads = 192;            // warp 0: TMA, warp 1: MMA, warps 2-5: epilogue
-constexpr int kConvStages = 4;               // TMA ring depth
+constexpr int kConvStagesLog2 = 2, kConvStages = 1 << kConvStagesLog2;  // deepest TMA ring
 constexpr int kConvAcc = 8;                  // TMEM accumulators (16 FP32 columns each)
 constexpr int kConvHalfBytes = 10 * 16, kConvRowBytes = 2 * kConvHalfBytes;
 constexpr int kConvStageStride = (3 * 18 * kConvRowBytes + 127) / 128 * 128;  // 17,280
@@ -56,9 +56,17 @@ struct ConvTcArgs {
     int relu, out_fp32, flip;
     int hp_in, hp_out;         // half-planar BF16 input (and mask) / output
     int ypad;                  // half-planar row length (ny rounded up to 8)
+    int stages_log2;           // TMA ring depth of this launch
     int stage_bytes, plane_bytes;  // of the staged [z][x][half][voxel][8], of one z of it
 };
 
+// Chained launches (ConvLaunch::chained) start while the layer before still
+// runs, as far as its blocks leave room, and do what does not depend on it --
+// barriers, tensor memory, the weights' layout -- before they wait for it.
+// A launch takes no more stages than its blocks have tiles, so that blocks of
+// both layers fit on an SM.  A training pass at 32^3: 172 -> 143 us, 137 with the
+// weight gradients' launch chained too.
+//
 // Warp-specialised: warp 0 (one lane) keeps a ring of kConvStages tile
 // stages loading, warp 1 (one lane) issues each tile's 27 MMAs into one of
 // kConvAcc TMEM accumulators as soon as its stage and accumulator are free
@@ -78,12 +86,14 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3_tc_kernel(const __grid_
     __shared__ int s_abort;
     unsigned char *smem = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
-    unsigned char *wsm = smem + kConvStages * kConvStageStride;
+    const int stages = 1 << A.stages_log2, smask = stages - 1;
+    unsigned char *wsm = smem + stages * kConvStageStride;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+    grid_launch_dependents();
     if (tid == 0) {
         s_abort = 0;
-        for (int i = 0; i < kConvStages; ++i) {
+        for (int i = 0; i < stages; ++i) {
             mbar_init(&full_bar[i], 1);
             mbar_init(&empty_bar[i], 1);
         }
@@ -99,7 +109,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3_tc_kernel(const __grid_
     const int ntiles = A.ytiles * A.xtiles * A.nz;
     const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     auto issue = [&](int j) {
-        const int st = j % kConvStages, tile = blockIdx.x + j * gridDim.x;
+        const int st = j & smask, tile = blockIdx.x + j * gridDim.x;
         const int yt = tile % A.ytiles, rest = tile / A.ytiles;
         const int y = yt * 8, x = rest % A.xtiles * 16, z = rest / A.xtiles;
         mbar_arrive_expect_tx(&full_bar[st], A.stage_bytes);
@@ -107,9 +117,11 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3_tc_kernel(const __grid_
                     x - 1, z - 1, &full_bar[st]);
     };
     int issued = 0;
-    if (tid == 0)  // the first tiles load while the other warps lay out the weights
-        for (; issued < kConvStages && issued < mine; ++issued)
+    if (tid == 0) {  // the first tiles load while the other warps lay out the weights
+        grid_dependency_wait();
+        for (; issued < stages && issued < mine; ++issued)
             issue(issued);
+    }
 
     // B operands: tap t as [k half][n][8 k] (core matrices of 8 n x 8 k).  A
     // thread's eight loads are independent: one round trip each for the five
@@ -129,6 +141,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3_tc_kernel(const __grid_
     }
     fence_proxy_async_smem();
     tc_fence_before_sync();
+    grid_dependency_wait();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = s_tmem;
@@ -137,16 +150,16 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3_tc_kernel(const __grid_
         // ---- producer
         if (lane == 0) {
             for (; issued < mine; ++issued) {
-                const int st = issued % kConvStages;
-                if (!mbar_wait_bounded(&empty_bar[st], ((issued / kConvStages) - 1) & 1, &s_abort))
+                const int st = issued & smask;
+                if (!mbar_wait_bounded(&empty_bar[st], ((issued >> A.stages_log2) - 1) & 1, &s_abort))
                     break;
                 issue(issued);
             }
             if (s_abort) {
                 // drain the copies in flight of this CTA (bounded)
                 volatile int drain_flag = 0;
-                for (int j = issued > kConvStages ? issued - kConvStages : 0; j < issued; ++j)
-                    mbar_wait_bounded(&full_bar[j % kConvStages], (j / kConvStages) & 1,
+                for (int j = issued > stages ? issued - stages : 0; j < issued; ++j)
+                    mbar_wait_bounded(&full_bar[j & smask], (j >> A.stages_log2) & 1,
                                       (int *)&drain_flag);
             }
         }
@@ -157,8 +170,8 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3_tc_kernel(const __grid_
             const uint32_t b0 = smem_addr(wsm);
             int done = 0;
             for (int j = 0; j < mine; ++j) {
-                const int st = j % kConvStages, slot = j % kConvAcc;
-                if (!mbar_wait_bounded(&full_bar[st], (j / kConvStages) & 1, &s_abort))
+                const int st = j & smask, slot = j % kConvAcc;
+                if (!mbar_wait_bounded(&full_bar[st], (j >> A.stages_log2) & 1, &s_abort))
                     break;
                 if (j >= kConvAcc &&
                     !mbar_wait_bounded(&acce_bar[slot], ((j / kConvAcc) - 1) & 1, &s_abort))
@@ -337,8 +350,19 @@ cudaError_t launch_conv3_tc(EncodeTiledFn encode, const ConvLaunch &c, int num_s
         return e;
     const int tiles = A.ytiles * A.xtiles * c.nz;
     const int grid = tiles < 2 * num_sms ? tiles : 2 * num_sms;
-    conv3_tc_kernel<<<grid, kConvThreads, kConvSmem, st>>>(A);
-    return cudaGetLastError();
+    while (A.stages_log2 < kConvStagesLog2 && (grid << A.stages_log2) < tiles)
+        ++A.stages_log2;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kConvThreads);
+    cfg.dynamicSmemBytes = (kConvStageStride << A.stages_log2) + kConvWBytes + 128;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = c.chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, conv3_tc_kernel, A);
 }
 
 }  // namespace asets

@@ -256,6 +256,9 @@ struct ConvLaunch {
     // and `mask` follow hp_in, a BF16 `y` hp_out; FP32 arrays are always
     // channels-last.
     int hp_in = 0, hp_out = 0;
+    // nothing that is still running in the stream writes w: the launch may begin
+    // before the one before has finished (programmatic dependent launch)
+    int chained = 0;
 };
 cudaError_t launch_conv3_tc(EncodeTiledFn encode, const ConvLaunch &c, int num_sms,
                             cudaStream_t st, int *d_err);

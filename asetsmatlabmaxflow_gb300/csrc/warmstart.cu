@@ -437,6 +437,7 @@ static ConvLaunch conv_of(asets_wsnet *n, int b, const void *x, void *y, int Ny,
     c.nz = Nz;
     c.hp_in = 1;   // the net's BF16 activations are half-planar
     c.hp_out = 1;
+    c.chained = 1;  // the weights' last writer finished before the pass's first kernel
     return c;
 }
 
@@ -553,7 +554,7 @@ static asets_status ws_backward(asets_wsnet *n, int Ny, int Nx, int Nz, const fl
         out.db[b] = out.dw[b] + kW;
     }
     static_assert(kBlocks <= kWgtLayers, "one launch");
-    WS_TRY(launch_wgrad_layers(enc, kBlocks, ins, gr, out, Ny, Nx, Nz, n->wg_partial, sms, n->err, st, 1));
+    WS_TRY(launch_wgrad_layers(enc, kBlocks, ins, gr, out, Ny, Nx, Nz, n->wg_partial, sms, n->err, st, 1, 1));
     return ws_check(n, loss_out);
 }
 

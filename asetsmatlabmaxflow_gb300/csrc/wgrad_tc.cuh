@@ -114,9 +114,11 @@ __global__ void __launch_bounds__(kWgtThreads, 1)
             ++z;
         }
     };
-    if (tid == 0)
+    if (tid == 0) {
+        grid_dependency_wait();  // a chained launch: as in conv_tc.cu
         while (issued < stages && issued < mine)
             issue();
+    }
     // the block of ones (bias gradient), BF16 1.0
     for (int i = tid; i < kWgtOnesBytes / 2; i += kWgtThreads)
         reinterpret_cast<unsigned short *>(smem)[i] = 0x3F80u;
@@ -124,6 +126,7 @@ __global__ void __launch_bounds__(kWgtThreads, 1)
         tmem_alloc(&s_tmem, kWgtTmem);
     fence_proxy_async_smem();
     tc_fence_before_sync();
+    grid_dependency_wait();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = s_tmem;
@@ -269,7 +272,8 @@ __global__ void __launch_bounds__(kWgtRedOut * kWgtRedSplit)
 // of channels-last ([z][x][y][16]).
 inline cudaError_t launch_wgrad_layers(EncodeTiledFn encode, int layers, const __nv_bfloat16 *const *act,
                                        const __nv_bfloat16 *const *grad, const WgradOut &out, int ny, int nx,
-                                       int nz, float *partial, int num_sms, int *d_err, cudaStream_t st, int hp)
+                                       int nz, float *partial, int num_sms, int *d_err, cudaStream_t st, int hp,
+                                       int chained = 0)
 {
     if (layers < 1 || layers > kWgtLayers || num_sms < layers)
         return cudaErrorInvalidValue;
@@ -325,8 +329,17 @@ inline cudaError_t launch_wgrad_layers(EncodeTiledFn encode, int layers, const _
     cudaError_t e = cudaFuncSetAttribute(wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgtSmem);
     if (e != cudaSuccess)
         return e;
-    wgrad_tc_kernel<<<A.ctas * layers, kWgtThreads, kWgtSmem, st>>>(A);
-    if ((e = cudaGetLastError()) != cudaSuccess)
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(A.ctas * layers);
+    cfg.blockDim = dim3(kWgtThreads);
+    cfg.dynamicSmemBytes = kWgtSmem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    if ((e = cudaLaunchKernelEx(&cfg, wgrad_tc_kernel, A)) != cudaSuccess)
         return e;
     wgrad_tc_reduce_kernel<<<dim3((27 * 256 + 16 + kWgtRedOut - 1) / kWgtRedOut, layers),
                              kWgtRedOut * kWgtRedSplit, 0, st>>>(partial, A.ctas, out);
