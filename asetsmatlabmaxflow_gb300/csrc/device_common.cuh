@@ -349,6 +349,18 @@ __device__ __forceinline__ float cold_v(float pt, float ct, float &u)
     return sat ? u * kColdScale : pt;
 }
 
+// Programmatic dependent launch: lets the next launch of the stream begin
+// (those made so) / waits until the launches before have finished and their
+// writes are visible (returns at once where there are none).
+__device__ __forceinline__ void grid_launch_dependents()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_dependency_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // A sum of floats as an unevaluated pair (TwoSum, Knuth): about 48 bits, at
 // float speed.
 struct FloatPair {

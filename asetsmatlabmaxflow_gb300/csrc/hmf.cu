@@ -220,10 +220,12 @@ __global__ void __launch_bounds__(kK1Threads) k1_staged(const HArgs<T> A, const 
         T v[N];
     };
     extern __shared__ __align__(16) unsigned char k1sm[];
+    grid_launch_dependents();
     const int m = A.m, tid = threadIdx.x;
     const long long c = ((long long)blockIdx.x * kK1Threads + tid) * N;
     if (c >= A.ns)
         return;
+    grid_dependency_wait();
     V *PT = reinterpret_cast<V *>(k1sm) + tid;
     V *DV = PT + m * kK1Threads, *U = DV + m * kK1Threads;
     for (int i = 0; i < m; ++i) {
@@ -926,6 +928,7 @@ __global__ void __launch_bounds__(kSweepThreads) k_spatial_sweep2d(const HArgs<T
                                                                    int total, int S)
 {
     constexpr int Q = 4;
+    grid_launch_dependents();
     const int w = (int)(blockIdx.x * (kSweepThreads / 32) + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
     if (w >= total)
         return;
@@ -943,6 +946,7 @@ __global__ void __launch_bounds__(kSweepThreads) k_spatial_sweep2d(const HArgs<T
     const T *alp = A.nodes[i].alpha ? A.nodes[i].alpha + y : nullptr;
     T al = A.nodes[i].alpha_s, lim = surely_inside<T>(al);
 
+    grid_dependency_wait();
     auto ld_g = [&](int x) { return in && x >= 0 && x < d2 ? gp[x * d1] : (T)0; };
     auto ld_1 = [&](int x) { return up && x >= 0 && x < d2 ? p1p[x * (d1 - 1)] : (T)0; };
     auto ld_2 = [&](int x) { return in && x >= 0 && x + 1 < d2 ? p2p[x * d1] : (T)0; };
@@ -1071,10 +1075,12 @@ __global__ void __launch_bounds__(kSweepThreads) k_spatial_sweep2d(const HArgs<T
 template <class T>
 __global__ void __launch_bounds__(kThreads) k_step_factor3d(const HArgs<T> A)
 {
+    grid_launch_dependents();
     const int i = 1 + (int)blockIdx.y;
     const long long c = blockIdx.x * (long long)kThreads + threadIdx.x;
     if (c >= A.n)
         return;
+    grid_dependency_wait();
     const Pix<T> p(A, c);
     const T *g = A.g + (long long)i * A.ns + c;
     const int sx = A.d1, sz = A.d1 * A.d2;
@@ -1110,10 +1116,12 @@ __global__ void __launch_bounds__(kThreads) k_step_factor3d(const HArgs<T> A)
 template <class T>
 __global__ void __launch_bounds__(kThreads) k_rescale_div3d(const HArgs<T> A)
 {
+    grid_launch_dependents();
     const int i = 1 + (int)blockIdx.y;
     const long long c = blockIdx.x * (long long)kThreads + threadIdx.x;
     if (c >= A.n)
         return;
+    grid_dependency_wait();
     const Pix<T> p(A, c);
     const T *f = A.f + (long long)i * A.ns + c;
     const int sx = A.d1, sz = A.d1 * A.d2;
@@ -1151,6 +1159,26 @@ int h_grid(long long n, int sms)
     return (int)(b < 1 ? 1 : (b < cap ? b : cap));
 }
 
+// The kernels of an iteration follow one another as programmatic dependent
+// launches: a kernel's blocks start as the one before runs out of blocks and wait
+// for it there (768 x 640 34.7 -> 31.4 us an iteration, 128 x 96 12.2 -> 8.9, 37 x
+// 30 x 20 18 -> 13).
+template <class... P, class... Q>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t st, Q... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // gradient step on g, the geodesic exemption (nodes with direction fields),
 // flow magnitude and projection factor, rescale, divergence
 template <class T>
@@ -1158,8 +1186,8 @@ void spatial_passes(HArgs<T> &A, int gn, int sms, cudaStream_t st, bool dirs, bo
 {
     if (A.q1 && A.dim == 3 && A.m > 1) {
         const dim3 grid((unsigned int)((A.n + kThreads - 1) / kThreads), A.m - 1);
-        k_step_factor3d<T><<<grid, kThreads, 0, st>>>(A);
-        k_rescale_div3d<T><<<grid, kThreads, 0, st>>>(A);
+        launch_chained(k_step_factor3d<T>, grid, kThreads, 0, st, A);
+        launch_chained(k_rescale_div3d<T>, grid, kThreads, 0, st, A);
         if (last)
             std::swap(A.g, A.f);
         return;
@@ -1174,8 +1202,8 @@ void spatial_passes(HArgs<T> &A, int gn, int sms, cudaStream_t st, bool dirs, bo
         chunks = std::max(1LL, std::min(chunks, (long long)(A.d2 + 5) / 6));
         const int S = ((int)((A.d2 + chunks - 1) / chunks) + 2 + 3) / 4 * 4 - 2;
         const int total = strips * ((A.d2 + S - 1) / S), per = kSweepThreads / 32;
-        k_spatial_sweep2d<T><<<dim3((total + per - 1) / per, A.m - 1), kSweepThreads, 0, st>>>(
-            A, last ? 1 : 0, strips, total, S);
+        launch_chained(k_spatial_sweep2d<T>, dim3((total + per - 1) / per, A.m - 1), kSweepThreads, 0, st, A,
+                       last ? 1 : 0, strips, total, S);
         std::swap(A.p1, A.q1);
         std::swap(A.p2, A.q2);
         if (last)
@@ -1403,8 +1431,8 @@ asets_status run_hmf(asets_context *ctx, int algo, int dim, int d1, int d2, int 
             if (pseudo)
                 k_pseudo_point<T><<<gp, kThreads, 0, st>>>(A);
             else if (k1_tree)
-                k1_staged<T><<<(int)((ns * sizeof(T) / 16 + kK1Threads - 1) / kK1Threads), kK1Threads, k1_bytes(m),
-                               st>>>(A, tree, it + 1 == its);
+                launch_chained(k1_staged<T>, dim3((unsigned int)((ns * sizeof(T) / 16 + kK1Threads - 1) / kK1Threads)),
+                               kK1Threads, k1_bytes(m), st, A, tree, it + 1 == its ? 1 : 0);
             else
                 k1_pointwise<T><<<gp, kThreads, 0, st>>>(A);
             spatial_passes(A, gn, sms, st, dirs, it + 1 == its);

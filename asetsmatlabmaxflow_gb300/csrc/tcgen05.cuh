@@ -35,18 +35,6 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16_f32(int M, int N)
            | ((uint32_t)(M >> 4) << 24);      // M / 16
 }
 
-// Programmatic dependent launch: lets the next launch of the stream begin
-// (those made so) / waits until the launches before have finished and their
-// writes are visible (returns at once where there are none).
-__device__ __forceinline__ void grid_launch_dependents()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void grid_dependency_wait()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 __device__ __forceinline__ void tmem_alloc(uint32_t *smem_result, uint32_t ncols)
 {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
