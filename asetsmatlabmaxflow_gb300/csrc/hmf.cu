@@ -1159,26 +1159,8 @@ int h_grid(long long n, int sms)
     return (int)(b < 1 ? 1 : (b < cap ? b : cap));
 }
 
-// The kernels of an iteration follow one another as programmatic dependent
-// launches: a kernel's blocks start as the one before runs out of blocks and wait
-// for it there (768 x 640 34.7 -> 31.4 us an iteration, 128 x 96 12.2 -> 8.9, 37 x
-// 30 x 20 18 -> 13).
-template <class... P, class... Q>
-cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t st, Q... args)
-{
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
+// The kernels of an iteration are chained launches (768 x 640 34.7 -> 31.4 us an
+// iteration, 128 x 96 12.2 -> 8.9, 37 x 30 x 20 18 -> 13).
 // gradient step on g, the geodesic exemption (nodes with direction fields),
 // flow magnitude and projection factor, rescale, divergence
 template <class T>

@@ -241,6 +241,28 @@ cudaError_t launch_restrict(const GridXfer &X, const float *src, float *dst, int
 cudaError_t launch_prolong(const GridXfer &X, const float *src, float *dst, int labels,
                            float scale, int axis, int num_sms, cudaStream_t st);
 
+// Programmatic dependent launch: the kernel's blocks start as the launch before
+// in the stream runs out of blocks.  Only for kernels that wait for it
+// (grid_dependency_wait) before they touch global memory, and that have a block
+// for each piece of work: of a persistent grid, blocks that start early go where
+// room is left, two to one SM and none to another (a 2D sweep of 20 us an
+// iteration took 23).
+template <class... P, class... Q>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t st, Q... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 struct ConvLaunch {
     const void *x;       // BF16 [z][x][y][16]
     const void *w;       // BF16 [27][16 in][16 out], tap = (dz*3 + dx)*3 + dy

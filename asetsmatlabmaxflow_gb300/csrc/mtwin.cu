@@ -21,9 +21,10 @@
 // once where u is written.
 //
 // Bound: single precision by load latency and L2, double by the FP64 pipe.
-// Potts 2D 512 x 480 L = 4 in double: 85 us per iteration; before (four passes, sqrt and
-// division on every cell, one thread summing the blocks' errors) 185 us.
-// Potts 2D 1024^2 L = 4 in single: 102 us, before 196.
+// Potts 2D 512 x 480 L = 4 in double: 79 us per iteration, 85 with the two launches
+// one after another instead of chained; before (four passes, sqrt and division on
+// every cell, one thread summing the blocks' errors) 185 us.  Potts 2D 1024^2 L = 4
+// in single: 98 us, before 196; binary 512^2 25 (29 not chained).
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -31,6 +32,7 @@
 #include <vector>
 
 #include "asets.h"
+#include "device_common.cuh"
 #include "div_const.cuh"
 #include "internal.h"
 
@@ -349,6 +351,8 @@ __global__ void __launch_bounds__(kThreads) mt_step_gk(const MTArgs<T> A)
     __shared__ T s3[QUEUE && D == 3 ? 2 : 1][QUEUE && D == 3 ? kThreads : 1];
     __shared__ unsigned char s_q[kThreads];
     __shared__ int s_n;
+    grid_launch_dependents();
+    grid_dependency_wait();
     if (finished(A))
         return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -726,6 +730,8 @@ __global__ void __launch_bounds__(kThreads, 4) mt_cell(const MTArgs<T> A)
 {
     __shared__ double s_red[kThreads / 32];
     __shared__ int s_last;
+    grid_launch_dependents();
+    grid_dependency_wait();
     if (finished(A))
         return;
     const int it = *(volatile int *)&A.ctl->iter;
@@ -855,15 +861,15 @@ void launch_cell(const MTArgs<T> &A, int grid, cudaStream_t st)
 {
     if constexpr (M == MT_POTTS) {
         switch (A.nlab) {
-        case 2: mt_cell<T, M, D, 2><<<grid, kThreads, 0, st>>>(A); return;
-        case 3: mt_cell<T, M, D, 3><<<grid, kThreads, 0, st>>>(A); return;
-        case 4: mt_cell<T, M, D, 4><<<grid, kThreads, 0, st>>>(A); return;
-        case 5: mt_cell<T, M, D, 5><<<grid, kThreads, 0, st>>>(A); return;
-        case 6: mt_cell<T, M, D, 6><<<grid, kThreads, 0, st>>>(A); return;
+        case 2: launch_chained(mt_cell<T, M, D, 2>, dim3(grid), kThreads, 0, st, A); return;
+        case 3: launch_chained(mt_cell<T, M, D, 3>, dim3(grid), kThreads, 0, st, A); return;
+        case 4: launch_chained(mt_cell<T, M, D, 4>, dim3(grid), kThreads, 0, st, A); return;
+        case 5: launch_chained(mt_cell<T, M, D, 5>, dim3(grid), kThreads, 0, st, A); return;
+        case 6: launch_chained(mt_cell<T, M, D, 6>, dim3(grid), kThreads, 0, st, A); return;
         default: break;
         }
     }
-    mt_cell<T, M, D, 0><<<grid, kThreads, 0, st>>>(A);
+    launch_chained(mt_cell<T, M, D, 0>, dim3(grid), kThreads, 0, st, A);
 }
 
 template <class T, int M, int D>
@@ -965,7 +971,7 @@ asets_status mt_run(asets_context *ctx, int rows, int cols, int slices, int nlab
         int h_done = 0;
         for (int done_it = 0; e == cudaSuccess && done_it < iterNum; done_it += kChunk) {
             for (int i = 0; i < kChunk && done_it + i < iterNum; ++i) {
-                mt_step_gk<T, M, D><<<(unsigned int)(tiles * A.nflow), kThreads, 0, st>>>(A);
+                launch_chained(mt_step_gk<T, M, D>, dim3((unsigned int)(tiles * A.nflow)), kThreads, 0, st, A);
                 launch_cell<T, M, D>(A, gcell, st);
             }
             e = cudaGetLastError();
