@@ -311,13 +311,13 @@ static_assert(kTY * kTX == kThreads, "one thread per cell of the tile");
 template <class T>
 struct Tile {
     int y0, x0, pl;
-    __device__ explicit Tile(const MTArgs<T> &A)
+    __device__ explicit Tile(const MTArgs<T> &A, int tx = kTX)
     {
         const unsigned int nty = (unsigned int)(A.rows + kTY - 1) / kTY;
-        const unsigned int ntx = (unsigned int)(A.cols + kTX - 1) / kTX;
+        const unsigned int ntx = (unsigned int)(A.cols + tx - 1) / tx;
         const unsigned int q = blockIdx.x / nty;
         y0 = (int)(blockIdx.x % nty) * kTY;
-        x0 = (int)(q % ntx) * kTX;
+        x0 = (int)(q % ntx) * tx;
         pl = (int)(q / ntx);
     }
 };
@@ -517,10 +517,11 @@ __device__ __forceinline__ T rescaled_divergence(const MTArgs<T> &A, int k, cons
 // and of the row and column past it is rescaled once, into shared memory, and
 // the faces with a factor below 1 by full warps together.  Called by every
 // thread of the block.
-template <class T, int D>
+template <class T, int D, int TX>
 struct FaceTile {
-    static constexpr int kFaces = (kTX + 1) * kTY + kTX * (kTY + 1) + (D == 3 ? 2 * kThreads : 0);
-    static constexpr int kRow = (kTX + 1) * kTY, kSlice = kRow + kTX * (kTY + 1);
+    static constexpr int NT = 32 * TX;
+    static constexpr int kFaces = (TX + 1) * kTY + TX * (kTY + 1) + (D == 3 ? 2 * NT : 0);
+    static constexpr int kRow = (TX + 1) * kTY, kSlice = kRow + TX * (kTY + 1);
     T f[kFaces];               // column faces [x][y], row faces [x][y], slice faces (lower, upper)
     T g[kFaces][2];            // factors of the faces in the queue
     unsigned short q[kFaces];  // their places in f
@@ -562,8 +563,8 @@ struct FaceTile {
         row(1, my2, y, x);
         at[2] = at[3] = at[4] = -1;
         if (w == 0)
-            col(2, kTX * kTY + lane, y, x + kTX);
-        else if (w == 1 && lane < kTX)
+            col(2, TX * kTY + lane, y, x + TX);
+        else if (w == 1 && lane < TX)
             row(2, kRow + lane * (kTY + 1) + kTY, y - lane + kTY, x - w + lane);
         if (D == 3) {
             const T *q3 = A.q3 + (long long)k * A.f3;
@@ -572,7 +573,7 @@ struct FaceTile {
             const T gc = in ? g0[0] : (T)1;
             put(3, kSlice + (int)threadIdx.x, lo, lo ? q3[j3(A, y, x, z)] : (T)0, gc,
                 lo ? g0[-plane] : (T)1);
-            put(4, kSlice + kThreads + (int)threadIdx.x, up, up ? q3[j3(A, y, x, z + 1)] : (T)0,
+            put(4, kSlice + NT + (int)threadIdx.x, up, up ? q3[j3(A, y, x, z + 1)] : (T)0,
                 up ? g0[plane] : (T)1, gc);
         }
         int slot = take_slots(&n, want);
@@ -586,7 +587,7 @@ struct FaceTile {
             }
         __syncthreads();
         const int m = n;
-        for (int i = threadIdx.x; i < m; i += kThreads)
+        for (int i = threadIdx.x; i < m; i += NT)
             f[q[i]] = mul(mul(A.half, add(g[i][0], g[i][1])), f[q[i]]);
         __syncthreads();
         const T a = f[my1], b = f[my1 + kTY], d = f[my2], e = f[my2 + 1];
@@ -598,7 +599,7 @@ struct FaceTile {
         dv = add(dv, e);
         dv = sub(dv, d);
         if (D == 3) {
-            const T p = f[kSlice + threadIdx.x], pu = f[kSlice + kThreads + threadIdx.x];
+            const T p = f[kSlice + threadIdx.x], pu = f[kSlice + NT + threadIdx.x];
             if (in && z >= 1)
                 A.p3[(long long)k * A.f3 + j3(A, y, x, z)] = p;
             dv = add(dv, pu);
@@ -725,10 +726,11 @@ __device__ __forceinline__ double ishikawa_update(const MTArgs<T> &A, long long 
 // Per cell: divp of every flow label with the rescale of the stepped flows,
 // the cell update; the last block records erriter and the break.  Single
 // precision strides over the cells; in double a block has a tile (FaceTile).
-template <class T, int M, int D, int LFIX>
-__global__ void __launch_bounds__(kThreads, 4) mt_cell(const MTArgs<T> A)
+template <class T, int M, int D, int LFIX, int TX>
+__global__ void __launch_bounds__(32 * TX, 32 / TX) mt_cell(const MTArgs<T> A)
 {
-    __shared__ double s_red[kThreads / 32];
+    constexpr int NT = 32 * TX;
+    __shared__ double s_red[NT / 32];
     __shared__ int s_last;
     grid_launch_dependents();
     grid_dependency_wait();
@@ -751,8 +753,8 @@ __global__ void __launch_bounds__(kThreads, 4) mt_cell(const MTArgs<T> A)
         }
     };
     if constexpr (sizeof(T) == 8) {
-        __shared__ FaceTile<T, D> faces;
-        const Tile<T> tile(A);
+        __shared__ FaceTile<T, D, TX> faces;
+        const Tile<T> tile(A, TX);
         const int y = tile.y0 + (threadIdx.x & 31), x = tile.x0 + (threadIdx.x >> 5), z = tile.pl;
         const bool in = y < A.rows && x < A.cols;
         update(((long long)z * A.cols + x) * A.rows + y, in,
@@ -771,7 +773,7 @@ __global__ void __launch_bounds__(kThreads, 4) mt_cell(const MTArgs<T> A)
     __syncthreads();
     if (threadIdx.x == 0) {
         double b = 0.0;
-        for (int w = 0; w < kThreads / 32; ++w)
+        for (int w = 0; w < NT / 32; ++w)
             b += s_red[w];
         A.partials[blockIdx.x] = b;
         __threadfence();
@@ -784,7 +786,7 @@ __global__ void __launch_bounds__(kThreads, 4) mt_cell(const MTArgs<T> A)
     // (one thread alone would take longer than the pass at 10^6 cells)
     __threadfence();
     double tot = 0.0;
-    for (unsigned int b = threadIdx.x; b < gridDim.x; b += kThreads)
+    for (unsigned int b = threadIdx.x; b < gridDim.x; b += NT)
         tot += __ldcg(A.partials + b);
     for (int o = 16; o > 0; o >>= 1)
         tot += __shfl_xor_sync(0xffffffffu, tot, o);
@@ -794,7 +796,7 @@ __global__ void __launch_bounds__(kThreads, 4) mt_cell(const MTArgs<T> A)
     __syncthreads();
     if (threadIdx.x == 0) {
         tot = 0.0;
-        for (int w = 0; w < kThreads / 32; ++w)
+        for (int w = 0; w < NT / 32; ++w)
             tot += s_red[w];
         const T e = (T)(tot / A.ctl->vol);
         A.erriter[it] = e;
@@ -856,20 +858,21 @@ int mt_grid(long long n, int sms)
     return (int)(b < 1 ? 1 : (b < cap ? b : cap));
 }
 
-template <class T, int M, int D>
+template <class T, int M, int D, int TX>
 void launch_cell(const MTArgs<T> &A, int grid, cudaStream_t st)
 {
+    auto launch = [&](auto kernel) { launch_chained(kernel, dim3(grid), 32 * TX, 0, st, A); };
     if constexpr (M == MT_POTTS) {
         switch (A.nlab) {
-        case 2: launch_chained(mt_cell<T, M, D, 2>, dim3(grid), kThreads, 0, st, A); return;
-        case 3: launch_chained(mt_cell<T, M, D, 3>, dim3(grid), kThreads, 0, st, A); return;
-        case 4: launch_chained(mt_cell<T, M, D, 4>, dim3(grid), kThreads, 0, st, A); return;
-        case 5: launch_chained(mt_cell<T, M, D, 5>, dim3(grid), kThreads, 0, st, A); return;
-        case 6: launch_chained(mt_cell<T, M, D, 6>, dim3(grid), kThreads, 0, st, A); return;
+        case 2: launch(mt_cell<T, M, D, 2, TX>); return;
+        case 3: launch(mt_cell<T, M, D, 3, TX>); return;
+        case 4: launch(mt_cell<T, M, D, 4, TX>); return;
+        case 5: launch(mt_cell<T, M, D, 5, TX>); return;
+        case 6: launch(mt_cell<T, M, D, 6, TX>); return;
         default: break;
         }
     }
-    launch_chained(mt_cell<T, M, D, 0>, dim3(grid), kThreads, 0, st, A);
+    launch(mt_cell<T, M, D, 0, TX>);
 }
 
 template <class T, int M, int D>
@@ -915,7 +918,14 @@ asets_status mt_run(asets_context *ctx, int rows, int cols, int slices, int nlab
     asets_status status = ASETS_OK;
     const int grid = mt_grid(n * A.nflow, sms);
     const long long tiles = (long long)((rows + kTY - 1) / kTY) * ((cols + kTX - 1) / kTX) * slices;
-    const int gcell = sizeof(T) == 8 ? (int)tiles : mt_grid(n, sms), ginit = mt_grid(n, sms);
+    // the cell update's tiles in double: half as wide where there are fewer than
+    // SMs, since a tile's time is its FP64 operations on one SM (us an iteration,
+    // 8 | 4 columns: 27 x 28 x 21 Potts L = 3, 84 tiles, 41.6 | 31.1; 181 x 64 L =
+    // 5, 48 tiles, 31.1 | 27.9; at 264 tiles one block an SM is busy either way)
+    const bool half_tiles = sizeof(T) == 8 && tiles < sms;
+    const long long cell_tiles =
+        half_tiles ? (long long)((rows + kTY - 1) / kTY) * ((cols + kTX / 2 - 1) / (kTX / 2)) * slices : tiles;
+    const int gcell = sizeof(T) == 8 ? (int)cell_tiles : mt_grid(n, sms), ginit = mt_grid(n, sms);
     bool ok = get(&ct, n * nct) && get(&al, n * A.nflow) && get(&A.u, n * nu) &&
               get(&A.ud, n * A.nflow) &&
               get(&A.q1, A.f1 * A.nflow) && get(&A.q2, A.f2 * A.nflow) && get(&A.q3, A.f3 * A.nflow) &&
@@ -972,7 +982,13 @@ asets_status mt_run(asets_context *ctx, int rows, int cols, int slices, int nlab
         for (int done_it = 0; e == cudaSuccess && done_it < iterNum; done_it += kChunk) {
             for (int i = 0; i < kChunk && done_it + i < iterNum; ++i) {
                 launch_chained(mt_step_gk<T, M, D>, dim3((unsigned int)(tiles * A.nflow)), kThreads, 0, st, A);
-                launch_cell<T, M, D>(A, gcell, st);
+                if constexpr (sizeof(T) == 8) {
+                    if (half_tiles) {
+                        launch_cell<T, M, D, kTX / 2>(A, gcell, st);
+                        continue;
+                    }
+                }
+                launch_cell<T, M, D, kTX>(A, gcell, st);
             }
             e = cudaGetLastError();
             if (e == cudaSuccess)

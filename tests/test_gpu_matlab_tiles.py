@@ -72,3 +72,11 @@ def test_capacity_extremes(lo, hi, dtype):
     """Every cell at capacity, none, and capacities around zero."""
     _check(*_run("potts", (35, 18), 3, dtype, 5, lo=lo, hi=hi), dtype)
     _check(*_run("binary", (35, 18, 5), 1, dtype, 6, lo=lo, hi=hi), dtype)
+
+
+# 8 or 4 columns a tile by the tiles there are per SM (152): 150 and 154 tiles of
+# 8, 148 and 160 slices' tiles, cut in rows and columns
+@pytest.mark.parametrize("shape", [(64, 600), (64, 615), (33, 9, 37), (33, 13, 40)])
+@pytest.mark.parametrize("model,L", [("binary", 1), ("potts", 3), ("potts", 7), ("ishikawa", 4)])
+def test_tile_width_in_double(model, L, shape):
+    _check(*_run(model, shape, L, np.float64, 7, its=8), np.float64)
