@@ -311,12 +311,12 @@ static_assert(kTY * kTX == kThreads, "one thread per cell of the tile");
 template <class T>
 struct Tile {
     int y0, x0, pl;
-    __device__ explicit Tile(const MTArgs<T> &A, int tx = kTX)
+    __device__ explicit Tile(const MTArgs<T> &A, int tx = kTX, int ty = kTY)
     {
-        const unsigned int nty = (unsigned int)(A.rows + kTY - 1) / kTY;
+        const unsigned int nty = (unsigned int)(A.rows + ty - 1) / ty;
         const unsigned int ntx = (unsigned int)(A.cols + tx - 1) / tx;
         const unsigned int q = blockIdx.x / nty;
-        y0 = (int)(blockIdx.x % nty) * kTY;
+        y0 = (int)(blockIdx.x % nty) * ty;
         x0 = (int)(q % ntx) * tx;
         pl = (int)(q / ntx);
     }
@@ -517,11 +517,12 @@ __device__ __forceinline__ T rescaled_divergence(const MTArgs<T> &A, int k, cons
 // and of the row and column past it is rescaled once, into shared memory, and
 // the faces with a factor below 1 by full warps together.  Called by every
 // thread of the block.
-template <class T, int D, int TX>
+template <class T, int D, int TX, int TY>
 struct FaceTile {
-    static constexpr int NT = 32 * TX;
-    static constexpr int kFaces = (TX + 1) * kTY + TX * (kTY + 1) + (D == 3 ? 2 * NT : 0);
-    static constexpr int kRow = (TX + 1) * kTY, kSlice = kRow + TX * (kTY + 1);
+    static constexpr int NT = TX * TY;
+    static_assert(TY >= TX && NT % 32 == 0, "the row past the tile is its second column's");
+    static constexpr int kFaces = (TX + 1) * TY + TX * (TY + 1) + (D == 3 ? 2 * NT : 0);
+    static constexpr int kRow = (TX + 1) * TY, kSlice = kRow + TX * (TY + 1);
     T f[kFaces];               // column faces [x][y], row faces [x][y], slice faces (lower, upper)
     T g[kFaces][2];            // factors of the faces in the queue
     unsigned short q[kFaces];  // their places in f
@@ -530,11 +531,11 @@ struct FaceTile {
     // `in`: the thread's cell (y, x, z) is in the volume
     __device__ T divergence(const MTArgs<T> &A, int k, int y, int x, int z, bool in)
     {
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        const int lane = threadIdx.x % TY, w = threadIdx.x / TY;  // row and column in the tile
         const long long plane = (long long)A.rows * A.cols;
         const T *gk = A.gk + (long long)k * A.n + z * plane;
         const T *q1 = A.q1 + (long long)k * A.f1, *q2 = A.q2 + (long long)k * A.f2;
-        const int my1 = w * kTY + lane, my2 = kRow + w * (kTY + 1) + lane;
+        const int my1 = w * TY + lane, my2 = kRow + w * (TY + 1) + lane;
         // up to five faces a thread: (place, factors), not yet in the queue
         int want = 0, at[5];
         T gu[5], gl[5];
@@ -563,9 +564,9 @@ struct FaceTile {
         row(1, my2, y, x);
         at[2] = at[3] = at[4] = -1;
         if (w == 0)
-            col(2, TX * kTY + lane, y, x + TX);
+            col(2, TX * TY + lane, y, x + TX);
         else if (w == 1 && lane < TX)
-            row(2, kRow + lane * (kTY + 1) + kTY, y - lane + kTY, x - w + lane);
+            row(2, kRow + lane * (TY + 1) + TY, y - lane + TY, x - w + lane);
         if (D == 3) {
             const T *q3 = A.q3 + (long long)k * A.f3;
             const T *g0 = gk + (long long)x * A.rows + y;
@@ -590,7 +591,7 @@ struct FaceTile {
         for (int i = threadIdx.x; i < m; i += NT)
             f[q[i]] = mul(mul(A.half, add(g[i][0], g[i][1])), f[q[i]]);
         __syncthreads();
-        const T a = f[my1], b = f[my1 + kTY], d = f[my2], e = f[my2 + 1];
+        const T a = f[my1], b = f[my1 + TY], d = f[my2], e = f[my2 + 1];
         if (in && x >= 1)
             A.p1[(long long)k * A.f1 + j1(A, y, x, z)] = a;
         if (in && y >= 1)
@@ -726,10 +727,10 @@ __device__ __forceinline__ double ishikawa_update(const MTArgs<T> &A, long long 
 // Per cell: divp of every flow label with the rescale of the stepped flows,
 // the cell update; the last block records erriter and the break.  Single
 // precision strides over the cells; in double a block has a tile (FaceTile).
-template <class T, int M, int D, int LFIX, int TX>
-__global__ void __launch_bounds__(32 * TX, 32 / TX) mt_cell(const MTArgs<T> A)
+template <class T, int M, int D, int LFIX, int TX, int TY>
+__global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mt_cell(const MTArgs<T> A)
 {
-    constexpr int NT = 32 * TX;
+    constexpr int NT = TX * TY;
     __shared__ double s_red[NT / 32];
     __shared__ int s_last;
     grid_launch_dependents();
@@ -753,9 +754,9 @@ __global__ void __launch_bounds__(32 * TX, 32 / TX) mt_cell(const MTArgs<T> A)
         }
     };
     if constexpr (sizeof(T) == 8) {
-        __shared__ FaceTile<T, D, TX> faces;
-        const Tile<T> tile(A, TX);
-        const int y = tile.y0 + (threadIdx.x & 31), x = tile.x0 + (threadIdx.x >> 5), z = tile.pl;
+        __shared__ FaceTile<T, D, TX, TY> faces;
+        const Tile<T> tile(A, TX, TY);
+        const int y = tile.y0 + threadIdx.x % TY, x = tile.x0 + threadIdx.x / TY, z = tile.pl;
         const bool in = y < A.rows && x < A.cols;
         update(((long long)z * A.cols + x) * A.rows + y, in,
                [&](int k) { return faces.divergence(A, k, y, x, z, in); });
@@ -858,21 +859,21 @@ int mt_grid(long long n, int sms)
     return (int)(b < 1 ? 1 : (b < cap ? b : cap));
 }
 
-template <class T, int M, int D, int TX>
+template <class T, int M, int D, int TX, int TY>
 void launch_cell(const MTArgs<T> &A, int grid, cudaStream_t st)
 {
-    auto launch = [&](auto kernel) { launch_chained(kernel, dim3(grid), 32 * TX, 0, st, A); };
+    auto launch = [&](auto kernel) { launch_chained(kernel, dim3(grid), TX * TY, 0, st, A); };
     if constexpr (M == MT_POTTS) {
         switch (A.nlab) {
-        case 2: launch(mt_cell<T, M, D, 2, TX>); return;
-        case 3: launch(mt_cell<T, M, D, 3, TX>); return;
-        case 4: launch(mt_cell<T, M, D, 4, TX>); return;
-        case 5: launch(mt_cell<T, M, D, 5, TX>); return;
-        case 6: launch(mt_cell<T, M, D, 6, TX>); return;
+        case 2: launch(mt_cell<T, M, D, 2, TX, TY>); return;
+        case 3: launch(mt_cell<T, M, D, 3, TX, TY>); return;
+        case 4: launch(mt_cell<T, M, D, 4, TX, TY>); return;
+        case 5: launch(mt_cell<T, M, D, 5, TX, TY>); return;
+        case 6: launch(mt_cell<T, M, D, 6, TX, TY>); return;
         default: break;
         }
     }
-    launch(mt_cell<T, M, D, 0, TX>);
+    launch(mt_cell<T, M, D, 0, TX, TY>);
 }
 
 template <class T, int M, int D>
@@ -918,13 +919,19 @@ asets_status mt_run(asets_context *ctx, int rows, int cols, int slices, int nlab
     asets_status status = ASETS_OK;
     const int grid = mt_grid(n * A.nflow, sms);
     const long long tiles = (long long)((rows + kTY - 1) / kTY) * ((cols + kTX - 1) / kTX) * slices;
-    // the cell update's tiles in double: half as wide where there are fewer than
-    // SMs, since a tile's time is its FP64 operations on one SM (us an iteration,
-    // 8 | 4 columns: 27 x 28 x 21 Potts L = 3, 84 tiles, 41.6 | 31.1; 181 x 64 L =
-    // 5, 48 tiles, 31.1 | 27.9; at 264 tiles one block an SM is busy either way)
-    const bool half_tiles = sizeof(T) == 8 && tiles < sms;
-    const long long cell_tiles =
-        half_tiles ? (long long)((rows + kTY - 1) / kTY) * ((cols + kTX / 2 - 1) / (kTX / 2)) * slices : tiles;
+    // The cell update's tiles in double, 32 x 8; a tile's time is its chain of
+    // labels and its FP64 operations on one SM, so that small volumes take half
+    // ones: with less than a tile an SM 32 x 4 (us an iteration, 8 | 4 columns: 27 x
+    // 28 x 21 Potts L = 3, 84 tiles, 41.6 | 31.1; 181 x 64 L = 5, 48 tiles, 31.1 |
+    // 27.9), with less than four 16 x 8 where these leave a fifth fewer lanes
+    // past the last row (35 x 30 x 19 L = 3: 47.8 | 38.8).
+    const auto tiles_of = [&](int ty, int tx) {
+        return (long long)((rows + ty - 1) / ty) * ((cols + tx - 1) / tx) * slices;
+    };
+    const int rows32 = (rows + 31) / 32 * 32, rows16 = (rows + 15) / 16 * 16;
+    const bool short_tiles = sizeof(T) == 8 && tiles < 4 * sms && 5 * rows16 <= 4 * rows32;
+    const bool half_tiles = sizeof(T) == 8 && tiles < sms && !short_tiles;
+    const long long cell_tiles = short_tiles ? tiles_of(16, kTX) : half_tiles ? tiles_of(kTY, kTX / 2) : tiles;
     const int gcell = sizeof(T) == 8 ? (int)cell_tiles : mt_grid(n, sms), ginit = mt_grid(n, sms);
     bool ok = get(&ct, n * nct) && get(&al, n * A.nflow) && get(&A.u, n * nu) &&
               get(&A.ud, n * A.nflow) &&
@@ -983,12 +990,15 @@ asets_status mt_run(asets_context *ctx, int rows, int cols, int slices, int nlab
             for (int i = 0; i < kChunk && done_it + i < iterNum; ++i) {
                 launch_chained(mt_step_gk<T, M, D>, dim3((unsigned int)(tiles * A.nflow)), kThreads, 0, st, A);
                 if constexpr (sizeof(T) == 8) {
-                    if (half_tiles) {
-                        launch_cell<T, M, D, kTX / 2>(A, gcell, st);
+                    if (short_tiles || half_tiles) {
+                        if (short_tiles)
+                            launch_cell<T, M, D, kTX, 16>(A, gcell, st);
+                        else
+                            launch_cell<T, M, D, kTX / 2, kTY>(A, gcell, st);
                         continue;
                     }
                 }
-                launch_cell<T, M, D, kTX>(A, gcell, st);
+                launch_cell<T, M, D, kTX, kTY>(A, gcell, st);
             }
             e = cudaGetLastError();
             if (e == cudaSuccess)

@@ -74,9 +74,9 @@ def test_capacity_extremes(lo, hi, dtype):
     _check(*_run("binary", (35, 18, 5), 1, dtype, 6, lo=lo, hi=hi), dtype)
 
 
-# 8 or 4 columns a tile by the tiles there are per SM (152): 150 and 154 tiles of
-# 8, 148 and 160 slices' tiles, cut in rows and columns
-@pytest.mark.parametrize("shape", [(64, 600), (64, 615), (33, 9, 37), (33, 13, 40)])
+# 32 x 8, 32 x 4 or 16 x 8 tiles by the tiles there are per SM (152) and the rows
+# past the last: either side of one tile an SM and of four, cut in rows and columns
+@pytest.mark.parametrize("shape", [(64, 600), (64, 615), (33, 9, 37), (33, 13, 40), (41, 1217), (41, 1209), (29, 30, 20)])
 @pytest.mark.parametrize("model,L", [("binary", 1), ("potts", 3), ("potts", 7), ("ishikawa", 4)])
 def test_tile_width_in_double(model, L, shape):
     _check(*_run(model, shape, L, np.float64, 7, its=8), np.float64)
