@@ -102,9 +102,36 @@ __device__ __forceinline__ void tma_load_4d(void *smem_dst, const CUtensorMap *m
         : "memory");
 }
 
-__device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map)
+// Tensor maps in global memory are read through a proxy of their own, which
+// neither an earlier copy nor an earlier kernel's stores to the same place
+// reach by themselves: the writer releases them, and the thread that issues
+// the loads acquires each map it uses before the first.  A launch that finds
+// other maps at the address of the one before (another variant's) would else
+// be free to load through the old ones.
+__device__ __forceinline__ void tensormap_release()
 {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+    asm volatile("fence.proxy.tensormap::generic.release.sys;" ::: "memory");
+}
+__device__ __forceinline__ void tensormap_acquire(const CUtensorMap *map)
+{
+    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(
+        reinterpret_cast<uint64_t>(map)));
+}
+// The maps of parity par whose bits are set (HALO: Slot, TILE: TileSlot), one
+// a lane of the producer's warp.  Called between the two barriers that hand out
+// an item, before any of its values is held: further down, the fence cost
+// registers (100 iterations of Ishikawa 1024^2 L = 8 took 7.6 ms, 6.7 here;
+// binary 256^3 16.0, 14.8).
+constexpr unsigned int kHaloMaps2D =
+    1u << SL_BR | 1u << SL_BS | 1u << SL_S0 | 1u << SL_S1 | 1u << SL_S2 | 1u << SL_ALPHA;
+constexpr unsigned int kTileMapsBinary = 1u << TS_S1 | 1u << TS_S2 | 1u << TS_CS | 1u << TS_CT;
+template <unsigned int HALO, unsigned int TILE>
+__device__ __forceinline__ void tensormaps_acquire(const ProblemDesc &P, int par)
+{
+    const unsigned int lane = threadIdx.x & 31;
+    if ((HALO | TILE << NUM_SLOTS) >> lane & 1u)
+        tensormap_acquire(lane < NUM_SLOTS ? &P.halo[par][lane] : &P.tile[par][lane - NUM_SLOTS]);
+    __syncwarp();
 }
 
 // ---------------------------------------------------------------- arithmetic

@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(kInitThreads) prepare_kernel(const __grid_cons
         const int *src = reinterpret_cast<const int *>(&A.desc);
         for (int i = threadIdx.x; i < (int)(sizeof(ProblemDesc) / 4); i += kInitThreads)
             reinterpret_cast<int *>(A.d_desc)[i] = src[i];
+        tensormap_release();
         if (threadIdx.x == 0)
             *A.d_ctl = A.ctl;
         if (threadIdx.x < 4)

@@ -60,9 +60,9 @@ enum Epilogue : int {
 // new ps needs no old ps).
 enum TileSlot : int { TS_S1 = 0, TS_S2 = 1, TS_CS = 2, TS_CT = 3, NUM_TILE_SLOTS = 4 };
 
-// One problem of a launch, in device memory (TMA descriptors need 64-byte
-// alignment, which the CUtensorMap members give the struct).
-struct ProblemDesc {
+// One problem of a launch, in device memory.  Each TMA descriptor is one
+// 128-byte unit of the fence that orders its use (tensormap_acquire).
+struct alignas(128) ProblemDesc {
     CUtensorMap halo[2][NUM_SLOTS];        // [source parity][slot]
     CUtensorMap tile[2][NUM_TILE_SLOTS];   // binary; EPI_FUSED: [.][TS_CT] = Ct, all labels,
                                            // halo rows (the same map for both parities)

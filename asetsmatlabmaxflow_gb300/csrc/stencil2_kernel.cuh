@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(32 * NW, MINB)
     const int ti = rho - 2;
     // The thread that issues the TMA loads and waits on their barriers; the
     // other threads block in the following CTA barrier instead of polling.
-    const bool producer = (tid == NT - 32);
+    const bool producer = (tid == NT - 32), producer_warp = (tid >= NT - 32);
 
     unsigned int q0 = 0;
     bool aborted = false;
@@ -313,6 +313,8 @@ __global__ void __launch_bounds__(32 * NW, MINB)
         __syncthreads();
         const int item = s_item;
         const int it = s_iter;
+        if (producer_warp && it >= 0)
+            tensormaps_acquire<kHaloMaps2D, EPI == EPI_BINARY ? kTileMapsBinary : 0u>(B.probs[B.item_problem[item]], it & 1);
         __syncthreads();  // s_item/s_iter are rewritten by the next fetch
         if (item >= B.total_items)
             break;

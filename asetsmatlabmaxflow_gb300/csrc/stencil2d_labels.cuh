@@ -279,7 +279,7 @@ __device__ __forceinline__ float ishikawa_layer(int l, float dv_l, float ucc_l, 
 // Claim the next item of the launch: thread 0 reads its problem's iteration
 // once for the block.  Returns false when the launch has no items left.
 __device__ __forceinline__ bool lab2_next_item(const BatchArgs &B, int *s_item, int *s_iter,
-                                               int &item, int &it)
+                                               int &item, int &it, bool producer_warp)
 {
     if (threadIdx.x == 0) {
         const int itm = (int)atomicAdd(&B.queue[0], 1u);
@@ -294,6 +294,8 @@ __device__ __forceinline__ bool lab2_next_item(const BatchArgs &B, int *s_item, 
     __syncthreads();
     item = *s_item;
     it = *s_iter;
+    if (producer_warp && it >= 0)
+        tensormaps_acquire<kHaloMaps2D, 1u << TS_CT>(B.probs[B.item_problem[item]], it & 1);
     __syncthreads();  // s_item/s_iter are rewritten by the next fetch
     return item < B.total_items;
 }
@@ -361,7 +363,7 @@ __global__ void __launch_bounds__(32 * Lab2WarpsGeom<MODEL, L, LW>::NW, MINB)
     __syncthreads();
 
     const int lane_row = C * lane;                  // a flow thread's rows within the 64
-    const bool producer = (tid == FL * 32);         // lane 0 of the first label warp
+    const bool producer_warp = (k == FL), producer = producer_warp && lane == 0;  // the first label warp
     // a label-warp thread's rows within the 64: two (one label warp) or one
     const int lab_row = (LW == 1) ? lane_row : (k - FL) * 32 + lane;
     // hand-over entry (value v, label l) of buffer b at row `row`
@@ -370,7 +372,7 @@ __global__ void __launch_bounds__(32 * Lab2WarpsGeom<MODEL, L, LW>::NW, MINB)
     unsigned int q0 = 0;
     bool aborted = false;
     int item, it;
-    while (!aborted && lab2_next_item(B, &s_item, &s_iter, item, it)) {
+    while (!aborted && lab2_next_item(B, &s_item, &s_iter, item, it, producer_warp)) {
         if (it < 0)
             continue;  // the problem has converged
         const ProblemDesc &P = B.probs[B.item_problem[item]];
@@ -630,12 +632,12 @@ __global__ void __launch_bounds__(32 * Lab2Geom<MODEL, L>::FL, MINB)
     __syncthreads();
 
     const int lane_row = C * lane;                  // the thread's rows within the 64
-    const bool producer = (tid == NT - 32);
+    const bool producer = (tid == NT - 32), producer_warp = (tid >= NT - 32);
 
     unsigned int q0 = 0;
     bool aborted = false;
     int item, it;
-    while (!aborted && lab2_next_item(B, &s_item, &s_iter, item, it)) {
+    while (!aborted && lab2_next_item(B, &s_item, &s_iter, item, it, producer_warp)) {
         if (it < 0)
             continue;  // the problem has converged
         const ProblemDesc &P = B.probs[B.item_problem[item]];

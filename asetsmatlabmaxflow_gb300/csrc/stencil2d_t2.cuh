@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(32 * NW, MINB)
     const int rho = G::TRW * w + C * lane;
     const int lane_row = C * lane;
     const bool rows_b = (lane_row >= 4 && lane_row < 60);   // B's output rows
-    const bool producer = (tid == NT - 32);
+    const bool producer = (tid == NT - 32), producer_warp = (tid >= NT - 32);
 
     unsigned int q0 = 0;
     bool aborted = false;
@@ -176,6 +176,8 @@ __global__ void __launch_bounds__(32 * NW, MINB)
         __syncthreads();
         const int item = s_item;
         const int it = s_iter;
+        if (producer_warp && it >= 0)
+            tensormaps_acquire<kHaloMaps2D, kTileMapsBinary>(B.probs[B.item_problem[item]], (it >> 1) & 1);
         __syncthreads();
         if (item >= B.total_items)
             break;

@@ -224,8 +224,11 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
     const bool tile_col = main_w && w >= 1 && w <= TC;
     const int ti = row + col * TR;                             // index in the tile boxes
     // the thread that issues the TMA loads: its warp has no work in Z
-    const bool producer = (tid == NT - 32);
+    const bool producer = (tid == NT - 32), producer_warp = (tid >= NT - 32);
 
+    constexpr unsigned int kHaloMaps = kHaloMaps2D & ~(1u << SL_S1 | 1u << SL_S2) | 1u << SL_BC;
+    constexpr unsigned int kTileMaps =
+        !BIN ? 0u : EPI == EPI_COLD ? kTileMapsBinary & ~(1u << TS_S2) : kTileMapsBinary;
     int st = 0;        // ring slot of the next stage to read
     uint32_t ph = 0;   // and its mbarrier phase
     bool aborted = false;
@@ -246,6 +249,8 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
         __syncthreads();
         const int item = s_item;
         const int it = s_iter;
+        if (producer_warp && it >= 0)
+            tensormaps_acquire<kHaloMaps, kTileMaps>(B.probs[B.item_problem[item]], it & 1);
         __syncthreads();  // s_item/s_iter are rewritten by the next fetch
         if (item >= B.total_items)
             break;

@@ -42,3 +42,28 @@ def test_dependents_start_after_the_tensor_memory_is_held(name, kernel):
         # by the allocating warp itself, or after a barrier of the block
         between = body[alloc:m.start()]
         assert "}" not in between or "__syncthreads()" in between
+
+
+@pytest.mark.parametrize("name", ["stencil2_kernel.cuh", "stencil2d_t2.cuh", "stencil2d_labels.cuh",
+                                  "stencil3d_kernel.cuh"])
+def test_tensor_maps_are_acquired_before_the_first_load(name):
+    text = _code(name)
+    found = 0
+    for kernel, body in _kernels(name):
+        if "issue_load" not in body:
+            continue
+        found += 1
+        head = body[:body.index("issue_load")]
+        if "lab2_next_item(" in head:
+            head = _body(text, text.index("bool lab2_next_item("))
+        at = re.search(r"if \(producer_warp && it >= 0\)\s*tensormaps_acquire<", head)
+        assert at, kernel
+        # a barrier between the warp's fences and the producer's loads
+        assert "__syncthreads()" in head[at.end():], kernel
+    assert found
+
+
+def test_tensor_maps_written_by_a_kernel_are_released():
+    text = _code("init_kernels.cu")
+    body = _body(text, text.index("prepare_kernel(const"))
+    assert body.index("tensormap_release()") > body.index("A.d_desc)[i]")
