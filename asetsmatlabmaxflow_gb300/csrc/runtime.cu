@@ -95,6 +95,8 @@ struct asets_context {
     asets_solver *cached = nullptr;  // solver reused by the one-shot calls
     int *pinned_flags = nullptr;     // host-visible done flags of in-flight chunks
     cudaMemPool_t pool = nullptr;    // scratch of the cost-term calls (keeps small blocks mapped)
+    size_t stage_most = 32u << 20;   // device bytes a solver keeps to pad host arrays on their way
+                                     // (ASETS_STAGE_BYTES; 0: none, they cross row by row)
 };
 
 struct ChunkGraph {
@@ -135,7 +137,7 @@ struct asets_solver {
     bool cold_state = false, u_stale = false, cold_ok = false;
     float run_cc = 0.f;
     int run_exact = 0;
-    float *stage = nullptr;  // unpadded copy of a host array on its way in or out
+    float *stage = nullptr;  // unpadded rows of a host array on their way in or out
     size_t stage_cap = 0;
     float *warm_u = nullptr, *warm_ps = nullptr, *warm_pt = nullptr;
     bool warm = false;
@@ -260,6 +262,8 @@ extern "C" ASETS_API asets_status asets_context_create(int device, asets_context
     std::unique_ptr<asets_context> ctx(new asets_context);
     ctx->device = device;
     ctx->num_sms = prop.multiProcessorCount;
+    if (const char *env = getenv("ASETS_STAGE_BYTES"))
+        ctx->stage_most = (size_t)strtoull(env, nullptr, 10);
     asets_status s = get_encoder(ctx.get());
     if (s != ASETS_OK)
         return s;
@@ -893,65 +897,75 @@ cleanup:
 // Copy a Matlab-layout array (rows of nr floats) into / out of the padded
 // layout (rows of pitch floats).  Between pageable host memory and the
 // device a pitched copy goes row by row (17.7 MB in rows of 640 B: 999 us in,
-// 184 out, against 111 and 102 as one run), so host arrays cross as one run
-// and are padded on the device; small ones go out as they are (a megabyte
-// costs 16 us pitched, 19 in two steps).
+// 184 out, against 111 and 102 as one run), so host arrays cross as runs of up
+// to the context's stage_most bytes and are padded on the device; small ones
+// go out as they are (a megabyte costs 16 us pitched, 19 in two steps).
 static constexpr size_t kPitchedOutMost = 4u << 20;
 
-static cudaError_t stage_for(asets_solver *s, size_t floats)
+// Rows of an array of `rows` that the solver's staging buffer takes at once; 0
+// where there is none to be had, and the array crosses pitched.
+static size_t stage_rows(asets_solver *s, size_t rows)
 {
-    if (floats <= s->stage_cap)
-        return cudaSuccess;
-    void *p = nullptr;
-    cudaError_t e = cudaMalloc(&p, floats * sizeof(float));
-    if (e != cudaSuccess)
-        return e;
-    // a grown buffer replaces the old one, which is still in use by queued copies
-    if (s->stage) {
-        e = cudaStreamSynchronize(s->ctx->stream);
-        cudaFree(s->stage);
+    rows = std::min(rows, s->ctx->stage_most / (s->nr * sizeof(float)));
+    if (rows * s->nr > s->stage_cap) {
+        // the old buffer may still be in use by queued copies
+        if (s->stage) {
+            cudaStreamSynchronize(s->ctx->stream);
+            cudaFree(s->stage);
+        }
+        void *p = nullptr;
+        const bool ok = cudaMalloc(&p, rows * s->nr * sizeof(float)) == cudaSuccess;
+        if (!ok)
+            cudaGetLastError();
+        s->stage = static_cast<float *>(p);
+        s->stage_cap = ok ? rows * s->nr : 0;
+        if (!ok)
+            return 0;
     }
-    s->stage = static_cast<float *>(p);
-    s->stage_cap = floats;
-    return e;
+    return rows;
 }
 
 static cudaError_t copy_in(asets_solver *s, float *dst, const float *src, int labels,
                            asets_memory where)
 {
-    const size_t rows = (size_t)s->nc * s->ns * labels, w = s->nr * sizeof(float);
+    const size_t rows = (size_t)s->nc * s->ns * labels, w = s->nr * sizeof(float), dw = s->pitch * sizeof(float);
     cudaStream_t st = s->ctx->stream;
-    if (where != ASETS_DEVICE) {
-        if (s->pitch == s->nr)
-            return cudaMemcpyAsync(dst, src, w * rows, cudaMemcpyHostToDevice, st);
-        cudaError_t e = stage_for(s, (size_t)s->nr * rows);
+    if (where == ASETS_DEVICE)
+        return cudaMemcpy2DAsync(dst, dw, src, w, w, rows, cudaMemcpyDeviceToDevice, st);
+    if (s->pitch == s->nr)
+        return cudaMemcpyAsync(dst, src, w * rows, cudaMemcpyHostToDevice, st);
+    const size_t step = stage_rows(s, rows);
+    if (step == 0)
+        return cudaMemcpy2DAsync(dst, dw, src, w, w, rows, cudaMemcpyHostToDevice, st);
+    cudaError_t e = cudaSuccess;
+    for (size_t r = 0; r < rows && e == cudaSuccess; r += step) {
+        const size_t n = std::min(step, rows - r);
+        e = cudaMemcpyAsync(s->stage, src + r * s->nr, w * n, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(s->stage, src, w * rows, cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess)
-            return e;
-        src = s->stage;
+            e = cudaMemcpy2DAsync(dst + r * s->pitch, dw, s->stage, w, w, n, cudaMemcpyDeviceToDevice, st);
     }
-    return cudaMemcpy2DAsync(dst, s->pitch * sizeof(float), src, w, w, rows, cudaMemcpyDeviceToDevice, st);
+    return e;
 }
 
 static cudaError_t copy_out(asets_solver *s, float *dst, const float *src, int labels,
                             asets_memory where)
 {
-    const size_t rows = (size_t)s->nc * s->ns * labels, w = s->nr * sizeof(float);
+    const size_t rows = (size_t)s->nc * s->ns * labels, w = s->nr * sizeof(float), sw = s->pitch * sizeof(float);
     cudaStream_t st = s->ctx->stream;
     if (where == ASETS_DEVICE)
-        return cudaMemcpy2DAsync(dst, w, src, s->pitch * sizeof(float), w, rows, cudaMemcpyDeviceToDevice,
-                                 st);
+        return cudaMemcpy2DAsync(dst, w, src, sw, w, rows, cudaMemcpyDeviceToDevice, st);
     if (s->pitch == s->nr)
         return cudaMemcpyAsync(dst, src, w * rows, cudaMemcpyDeviceToHost, st);
-    if (w * rows <= kPitchedOutMost)
-        return cudaMemcpy2DAsync(dst, w, src, s->pitch * sizeof(float), w, rows, cudaMemcpyDeviceToHost, st);
-    cudaError_t e = stage_for(s, (size_t)s->nr * rows);
-    if (e == cudaSuccess)
-        e = cudaMemcpy2DAsync(s->stage, w, src, s->pitch * sizeof(float), w, rows,
-                              cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dst, s->stage, w * rows, cudaMemcpyDeviceToHost, st);
+    const size_t step = w * rows <= kPitchedOutMost ? 0 : stage_rows(s, rows);
+    if (step == 0)
+        return cudaMemcpy2DAsync(dst, w, src, sw, w, rows, cudaMemcpyDeviceToHost, st);
+    cudaError_t e = cudaSuccess;
+    for (size_t r = 0; r < rows && e == cudaSuccess; r += step) {
+        const size_t n = std::min(step, rows - r);
+        e = cudaMemcpy2DAsync(s->stage, w, src + r * s->pitch, sw, w, n, cudaMemcpyDeviceToDevice, st);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(dst + r * s->nr, s->stage, w * n, cudaMemcpyDeviceToHost, st);
+    }
     return e;
 }
 
