@@ -86,7 +86,7 @@ template <> __device__ __forceinline__ double sqr(double a) { return __dsqrt_rn(
 // exactly without them is.
 
 // x truncated towards zero to a float, from its bits (magnitude only; below
-// 2^-126 gives 0, beyond the float range infinity)
+// 2^-126 gives 0, beyond the float range and for NaN infinity)
 __device__ __forceinline__ float mag_f32(double x)
 {
     const int hi = __double2hiint(x) & 0x7fffffff;
@@ -267,9 +267,9 @@ __device__ __forceinline__ bool surely_inside(T a, T b, T d, T e, T p, T q, T al
         m = __fmaf_rn(f(q), f(q), m);
     }
     const float fa = f(al);
-    bool pos;
+    bool pos;  // above zero and not NaN, which mag_f32 takes for infinity
     if constexpr (sizeof(T) == 8)
-        pos = __double2hiint(al) > 0;
+        pos = (unsigned long long)__double_as_longlong(al) - 1 < 0x7ff0000000000000ull;
     else
         pos = al > 0.0f;
     return pos && fa > 0x1p-40f && m * (0.5f * (1.0f + 0x1p-18f)) < fa * fa;
