@@ -14,7 +14,7 @@
 // ci; the last row's taps are the M of two more, one a half, whose groups lie
 // one voxel apart (three shifts used, the others discarded).  N = 16 co, K =
 // 16 voxels.  A sixth MMA with M a constant block of ones gives the bias
-// gradient.  6 x 16 FP32 columns of TMEM.  What bounds it is the operands'
+// gradient.  6 x 16 FP32 columns of TMEM, five times.  What bounds it is the operands'
 // way out of shared memory: 28 MMAs with the gradient as M (16 rows of 128
 // used) took 0.78 us per 16 voxels, four of N = 144 0.47, these six 0.18.
 //
@@ -50,7 +50,12 @@ constexpr int kWgtOnesBytes = 16 * 256;                    // [16 M groups][16 v
 // the largest rows; shorter rows leave room for up to eight.
 constexpr int kWgtSmem = kWgtOnesBytes + 4 * (kWgtActMax + kWgtGradMax) + 256 + 128;
 static_assert(kWgtGradMax % 128 == 0, "stage alignment");
-constexpr int kWgtTmem = 128;                              // columns: 6 x 16 used
+// Accumulators: a CTA's rows go round sets of six, which are added up at the
+// end.  With one set, the 30 CTAs a layer of five has would sum five times as
+// many voxels in one single-precision chain as 152 CTAs do.
+constexpr int kWgtSets = 5, kWgtSetCols = 6 * 16;
+constexpr int kWgtTmem = 512;                              // columns: 480 used
+static_assert(kWgtSets * kWgtSetCols <= kWgtTmem, "tensor memory of a CTA");
 constexpr int kWgtLayers = 5;
 
 struct WgradTcArgs {
@@ -151,7 +156,7 @@ __global__ void __launch_bounds__(kWgtThreads, 1)
         // ---- MMA issue
         const uint32_t ones = smem_addr(smem);
         int st = 0, y_left = A.ny - first % A.ytiles * A.span;
-        uint32_t ph = 0;
+        uint32_t ph = 0, d = tmem;  // this row's accumulators
         bool ok = true;
         int j = 0;
         for (; j < mine; ++j) {
@@ -165,16 +170,17 @@ __global__ void __launch_bounds__(kWgtThreads, 1)
             for (int ks = 0; ks < ksteps; ++ks) {  // 16 voxels per MMA
                 // B: co x voxels, core matrices 8 voxels x 8 co; K step 128 B, N step: half
                 const uint64_t bd = umma_smem_desc(g0 + ks * 256, 128, A.grad_half);
-                const uint32_t acc = (j > 0 || ks > 0) ? 1u : 0u;
+                const uint32_t acc = (j >= kWgtSets || ks > 0) ? 1u : 0u;
                 const uint32_t a = a0 + ks * 256;
                 for (int dy = 0; dy < 3; ++dy)  // M step: a channel half, the rows following one another
-                    umma_bf16(tmem + dy * 16, umma_smem_desc(a + dy * 16, 128, A.act_half), bd, idesc, acc);
+                    umma_bf16(d + dy * 16, umma_smem_desc(a + dy * 16, 128, A.act_half), bd, idesc, acc);
                 for (int h = 0; h < 2; ++h)     // row 8; M step: a voxel
-                    umma_bf16(tmem + (3 + h) * 16, umma_smem_desc(a + (16 + h) * A.act_half, 128, 16), bd,
+                    umma_bf16(d + (3 + h) * 16, umma_smem_desc(a + (16 + h) * A.act_half, 128, 16), bd,
                               idesc, acc);
-                umma_bf16(tmem + 5 * 16, umma_smem_desc(ones, 128, 256), bd, idesc, acc);
+                umma_bf16(d + 5 * 16, umma_smem_desc(ones, 128, 256), bd, idesc, acc);
             }
             umma_commit(&mma_bar[st]);
+            d = d == tmem + (kWgtSets - 1) * kWgtSetCols ? tmem : d + kWgtSetCols;
             if (++st == stages) {
                 st = 0;
                 ph ^= 1;
@@ -207,17 +213,28 @@ __global__ void __launch_bounds__(kWgtThreads, 1)
                 p[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
         };
         float v[16];
+        const int sets = mine < kWgtSets ? mine : kWgtSets;
+        auto load = [&](uint32_t addr) {
+            tmem_load16(addr, v);
+            for (int i = 1; i < sets; ++i) {
+                float w[16];
+                tmem_load16(addr + i * kWgtSetCols, w);
+#pragma unroll
+                for (int k = 0; k < 16; ++k)
+                    v[k] += w[k];
+            }
+        };
         for (int dy = 0; dy < 3; ++dy) {
-            tmem_load16(tmem + ((uint32_t)(32 * warp) << 16) + dy * 16, v);
+            load(tmem + ((uint32_t)(32 * warp) << 16) + dy * 16);
             store(m / 16 * 3 + dy, m % 16, v);
         }
         if (warp == 0) {
             for (int h = 0; h < 2; ++h) {  // row 8: lane = 8 * (shift dy) + ci % 8
-                tmem_load16(tmem + (3 + h) * 16, v);
+                load(tmem + (3 + h) * 16);
                 if (lane < 24)
                     store(24 + lane / 8, h * 8 + lane % 8, v);
             }
-            tmem_load16(tmem + 5 * 16, v);
+            load(tmem + 5 * 16);
             if (lane == 0)
                 store(27, 0, v);  // the bias
         }
