@@ -347,16 +347,6 @@ __device__ __forceinline__ Rows<VEC> ld_rows(const float *p, bool ok)
     return r;
 }
 
-// sqrt(x) for x >= 0: the hardware reciprocal root with one Newton correction
-// of x*rsqrt(x) (zero, subnormal and non-finite values take the IEEE root)
-__device__ __forceinline__ float root(float x)
-{
-    if (!(x >= 0x1p-100f && x <= 0x1p100f))
-        return __fsqrt_rn(x);
-    const float r = rsqrtf(x), s = __fmul_rn(x, r);
-    return __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, r), s);
-}
-
 template <int VEC>
 __global__ void __launch_bounds__(32 * kAWarps)
     alpha_kernel(const float *img, int ny, int nx, int nz, const unsigned int *mm, float a, float b, float c,
@@ -412,7 +402,7 @@ __global__ void __launch_bounds__(32 * kAWarps)
                 const float gz = unit(__fmul_rn(__fsub_rn(up.v[j], lo.v[j]), sz));
                 g2 = __fmaf_rn(gz, gz, g2);
             }
-            const float t = squared ? g2 : root(g2);
+            const float t = squared ? g2 : __fsqrt_rn(g2);
             al[j] = __fadd_rn(a, __fmul_rn(b, expf(__fmul_rn(-c, t))));
         }
         if (in) {
