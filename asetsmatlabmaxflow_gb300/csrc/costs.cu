@@ -132,7 +132,8 @@ struct Norm {
         if (mm) {
             lo = key_float(~mm[0]);
             den = __fsub_rn(key_float(mm[1]), lo);
-            if (den >= 0x1p-60f && den <= 0x1p60f)
+            // quotients of at least 2^-100 / 2^20, all in the normal range
+            if (den >= 0x1p-20f && den <= 0x1p20f)
                 rd = __fdiv_rn(1.0f, den);
             on = true;
         }
@@ -360,15 +361,20 @@ __global__ void __launch_bounds__(32 * kAWarps)
     const bool in = y < ny;
     const long long plane = (long long)ny * nx, n = plane * nz;
     const float *p = img + (long long)x * ny + y;
-    // 1/(max - min); a range that is not finite gives what the quotients would
-    float den = 1.f, rd = 1.f;
+    // 1/(max - min); a range whose reciprocal is not an ordinary number (and
+    // one that is not finite, or zero) takes the quotients themselves
+    float low = 0.f, den = 1.f, rd = 1.f;
     if (mm) {
-        const float lo = key_float(~mm[0]);
-        den = __fsub_rn(key_float(mm[1]), lo);
-        rd = fabsf(lo) < INFINITY ? __fdiv_rn(1.f, den) : NAN;
+        low = key_float(~mm[0]);
+        den = __fsub_rn(key_float(mm[1]), low);
+        rd = __fdiv_rn(1.f, den);
     }
-    const bool plain = !mm || !(den < 0x1p-100f);  // else 1/den may overflow: divide
-    auto unit = [&](float d) { return plain ? __fmul_rn(d, rd) : __fdiv_rn(d, den); };
+    const bool plain = !mm || (fabsf(low) < INFINITY && den >= 0x1p-100f && den <= 0x1p100f);
+    auto unit = [&](float hi, float lo, float half) {
+        if (plain)
+            return __fmul_rn(__fmul_rn(__fsub_rn(hi, lo), half), rd);
+        return __fmul_rn(__fsub_rn(__fdiv_rn(__fsub_rn(hi, low), den), __fdiv_rn(__fsub_rn(lo, low), den)), half);
+    };
     const bool x_lo = x > 0, x_up = x + 1 < nx;
     const float sx = (x_lo && x_up) ? 0.5f : 1.f;
     // the rows beyond the warp's 32*VEC
@@ -395,11 +401,11 @@ __global__ void __launch_bounds__(32 * kAWarps)
             const float vl = y_lo ? (j ? cur.v[j - 1] : yl) : cur.v[j];
             const float vu = y_up ? (j + 1 < VEC ? cur.v[j + 1 < VEC ? j + 1 : j] : yu) : cur.v[j];
             // an axis of length 1 adds nothing, whatever the value there
-            const float gy = ny < 2 ? 0.f : unit(__fmul_rn(__fsub_rn(vu, vl), (y_lo && y_up) ? 0.5f : 1.f));
-            const float gx = nx < 2 ? 0.f : unit(__fmul_rn(__fsub_rn(xu.v[j], xl.v[j]), sx));
+            const float gy = ny < 2 ? 0.f : unit(vu, vl, (y_lo && y_up) ? 0.5f : 1.f);
+            const float gx = nx < 2 ? 0.f : unit(xu.v[j], xl.v[j], sx);
             float g2 = __fmaf_rn(gx, gx, __fmul_rn(gy, gy));
             if (nz > 1) {
-                const float gz = unit(__fmul_rn(__fsub_rn(up.v[j], lo.v[j]), sz));
+                const float gz = unit(up.v[j], lo.v[j], sz);
                 g2 = __fmaf_rn(gz, gz, g2);
             }
             const float t = squared ? g2 : __fsqrt_rn(g2);
