@@ -358,10 +358,11 @@ __device__ __forceinline__ float min_sel(float a, float b)
 // The cold binary start's state (stencil3d_kernel.cuh): from the reference's
 // initial state on, a cell has u > 0 only where pt = Ct, so one float v holds
 // both: pt itself where u = 0, else u scaled by 2^112, told apart by the
-// magnitude (inputs are below kColdInputLimit, u below 2^14).  Both keep all
-// their bits; a u below 2^-32 counts as 0.
-constexpr float kColdScale = 0x1p112f, kColdUnscale = 0x1p-112f, kColdSplit = 0x1p80f;
-constexpr float kColdInputLimit = 0x1p60f;
+// magnitude.  Both keep all their bits.  Costs and capacities are below 2^34
+// (kColdInputLimit), so that pt, at least Cs less a divergence of at most 8.5
+// capacities, stays below 2^44 in magnitude, and u, at most 1 and a few roundings
+// of such values times cc <= 1, below 2^14; only a u below 2^-68 counts as 0.
+constexpr float kColdScale = 0x1p112f, kColdUnscale = 0x1p-112f, kColdSplit = 0x1p44f;
 
 __device__ __forceinline__ float cold_u(float v)
 {
@@ -371,7 +372,7 @@ __device__ __forceinline__ float cold_pt(float v, float ct) { return fabsf(v) >=
 // v of a new pt and u; sets u to the value that v holds
 __device__ __forceinline__ float cold_v(float pt, float ct, float &u)
 {
-    const bool sat = (pt == ct) && (u >= 0x1p-32f);
+    const bool sat = (pt == ct) && (u >= kColdSplit * kColdUnscale);
     u = sat ? fminf(u, 0x1p14f) : 0.0f;
     return sat ? u * kColdScale : pt;
 }

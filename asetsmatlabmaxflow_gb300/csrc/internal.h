@@ -188,8 +188,12 @@ cudaError_t launch_prepare(const PrepareArgs &a, int num_sms, cudaStream_t st);
 cudaError_t launch_cold_init(const InitArgs &a, float *gk, float *v, float inv_cc, int num_sms,
                              cudaStream_t st);
 cudaError_t launch_init(int model, const InitArgs &a, int num_sms, cudaStream_t st);
-// Sets a.ctl->wide if an input of a binary problem is not finite or is
-// beyond the range of the cold start's state.
+// The cold start's state (device_common.cuh) holds pt and u in one float for
+// costs and capacities below the limit and 0 < cc <= 1.
+constexpr float kColdInputLimit = 0x1p34f;
+inline bool cold_cc(float cc) { return cc > 0.0f && cc <= 1.0f; }
+// Sets a.ctl->wide if an input of a binary problem is not finite or is not
+// below kColdInputLimit.
 cudaError_t launch_check_range(const InitArgs &a, int num_sms, cudaStream_t st);
 cudaError_t launch_validate_alpha(const InitArgs &a, int num_sms, cudaStream_t st);
 cudaError_t launch_wait_selftest(int *d_err, cudaStream_t st);

@@ -276,7 +276,7 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
         }
         if (checked.alpha_bad)
             return na_fail(ASETS_ERR_ALPHA, "alpha(x) must be positive. Exiting...");
-        if (v->cold && !checked.wide)
+        if (v->cold && !checked.wide && cold_cc(cc))
             v = v->cold;
     }
     const bool cold = (v->epi == EPI_COLD && maxIt > 0);

@@ -680,12 +680,12 @@ static StencilProblem stencil_problem_of(const asets_solver *s, bool fused)
 }
 
 // Build the kernel arguments (TMA maps for both parities, destinations).
-static asets_status setup_kernel(asets_solver *s, int exact, int tile_config, bool single)
+static asets_status setup_kernel(asets_solver *s, int exact, int tile_config, bool single, float cc)
 {
     const StencilVariant *v = pick_variant(s, exact, tile_config, single);
     if (!v)
         return fail(ASETS_ERR_UNSUPPORTED, "no kernel variant for this configuration");
-    if (v->cold && !s->warm && !s->warm_flows && s->cold_ok)
+    if (v->cold && !s->warm && !s->warm_flows && s->cold_ok && cold_cc(cc))
         v = v->cold;
     if (s->variant == v)
         return ASETS_OK;
@@ -1274,7 +1274,7 @@ static asets_status prepare_run(asets_solver *s, int flags, int tile_config, int
                                                ? "alpha(x,l) must be positive. Exiting..."
                                                : "alpha(x) must be positive. Exiting...");
     const int exact = (flags & ASETS_FLAG_EXACT) ? 1 : 0;
-    asets_status ss = setup_kernel(s, exact, tile_config, single);
+    asets_status ss = setup_kernel(s, exact, tile_config, single, cc);
     if (ss != ASETS_OK)
         return ss;
     if (maxIt + 1 > s->cvg_cap) {

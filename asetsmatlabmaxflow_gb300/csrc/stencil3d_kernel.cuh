@@ -40,7 +40,7 @@
 // the rounding noise that the subtraction leaves in u where pt < Ct is a zero.
 // A start from given pt and u need not satisfy that and keeps both
 // (EPI_BINARY), as do EXACT, for the reference's own roundings, and inputs
-// that are not finite or beyond 2^60.
+// out of the joint state's range (kColdInputLimit, cold_cc).
 //
 // EPI_TWIN: the binary 3D Matlab twin in single precision (mtwin.cu), whose
 // expressions differ in order; its erriter is summed to double precision.
