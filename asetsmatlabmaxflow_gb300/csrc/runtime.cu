@@ -836,21 +836,29 @@ extern "C" ASETS_API asets_status asets_solver_create(asets_context *ctx, asets_
         for (int par = 0; par < 2; ++par) {
             if (dim == 3)
                 ALLOC(s->gk[par], n);
-            if (dim == 2 || par == 0)
+            else
                 ALLOC(s->ps[par], n);
             ALLOC(s->pt[par], n);
             ALLOC(s->u[par], n);
         }
+        // ps is there before the first iteration, which writes this gradient
+        // source, and after the last, when nothing reads it any more
         if (dim == 3)
-            s->ps[1] = s->ps[0];
+            s->ps[0] = s->ps[1] = s->gk[1];
     } else {
         if (model == ASETS_POTTS)
             ALLOC(s->ps[0], n);
-        ALLOC(s->pt[0], n * s->pt_labels);
+        if (dim == 3)
+            ALLOC(s->gk[0], n * s->flow_labels);
+        // Potts in 3D: as ps of the binary model, pt is the source's until the
+        // source is formed (in place) and again after the last iteration
+        if (dim == 3 && model == ASETS_POTTS)
+            s->pt[0] = s->gk[0];
+        else
+            ALLOC(s->pt[0], n * s->pt_labels);
         ALLOC(s->u[0], n * s->u_labels);
         ALLOC(s->dv, n * s->flow_labels);
         if (dim == 3) {
-            ALLOC(s->gk[0], n * s->flow_labels);
             s->pt[1] = s->pt[0];
             if (model == ASETS_POTTS) {
                 ALLOC(s->ps[1], n);
@@ -1347,7 +1355,7 @@ static asets_status prepare_run(asets_solver *s, int flags, int tile_config, int
         if (!s->warm_flows)
             ca.br = nullptr;  // zero flows
         ca.gk = s->gk[0];
-        if (s->variant->epi != EPI_COLD)
+        if (s->variant->epi != EPI_COLD && maxIt > 0)  // Potts' pt stays where no iteration follows
             CU_TRY(launch_source((int)s->model, ca, s->ctx->num_sms, st));
         s->run_cc = cc;
         s->run_exact = exact;
