@@ -1234,15 +1234,18 @@ bool setup_dirs(Get &get, cudaStream_t st, int dim, int m, void *const *const ld
 }
 
 // The second copy of the flows, and the factors; the root has no flows and no
-// factor.
+// factor.  Without them the four passes run, in place: where they are not used,
+// and where they cannot be had.
 template <class T, class Get>
-bool setup_copies(Get &get, cudaStream_t st, HArgs<T> &A, bool dirs, cudaError_t &e)
+void setup_copies(Get &get, cudaStream_t st, HArgs<T> &A, bool dirs, cudaError_t &e)
 {
     if (dirs || (A.dim == 3 && sizeof(T) == 8))
-        return true;
+        return;
     void *vp = nullptr;
-    if (!get(&vp, sizeof(T) * (A.f1 + A.f2 + A.f3 + A.ns) * A.m))
-        return false;
+    if (!get(&vp, sizeof(T) * (A.f1 + A.f2 + A.f3 + A.ns) * A.m)) {
+        cudaGetLastError();
+        return;
+    }
     A.f = static_cast<T *>(vp);
     A.q1 = A.f + A.ns * A.m;
     A.q2 = A.q1 + A.f1 * A.m;
@@ -1254,7 +1257,6 @@ bool setup_copies(Get &get, cudaStream_t st, HArgs<T> &A, bool dirs, cudaError_t
     for (const auto &r : root)
         if (e == cudaSuccess && r.count > 0)
             e = cudaMemsetAsync(r.p, 0, sizeof(T) * r.count, st);
-    return true;
 }
 
 // the normalised direction fields back into the caller's arrays
@@ -1380,7 +1382,6 @@ asets_status run_hmf(asets_context *ctx, int algo, int dim, int d1, int d2, int 
     }
     bool dirs = false;
     ok = ok && setup_dirs<T>(get, st, dim, m, ld, nodes, A, e, dirs);
-    ok = ok && setup_copies<T>(get, st, A, dirs, e);
     ok = ok && get(&vp, sizeof(NodeDev<T>) * m);
     if (ok && e == cudaSuccess) {
         e = cudaMemcpyAsync(vp, nodes.data(), sizeof(NodeDev<T>) * m, cudaMemcpyHostToDevice, st);
@@ -1391,6 +1392,8 @@ asets_status run_hmf(asets_context *ctx, int algo, int dim, int d1, int d2, int 
         e = cudaMemcpyAsync(vp, kids.data(), sizeof(int) * kids.size(), cudaMemcpyHostToDevice, st);
         A.children = static_cast<const int *>(vp);
     }
+    if (ok)
+        setup_copies<T>(get, st, A, dirs, e);  // last: the rest has to fit
     if (!ok) {
         status = ASETS_ERR_OUT_OF_MEMORY;
         set_last_error("asets_hmf_full_flow: out of device memory");
@@ -1589,7 +1592,6 @@ asets_status run_dag(asets_context *ctx, int dim, int d1, int d2, int d3, int m,
     }
     bool dirs = false;
     ok = ok && setup_dirs<T>(get, st, dim, m, ld, nodes, A, e, dirs);
-    ok = ok && setup_copies<T>(get, st, A, dirs, e);
     struct Up {
         const void *src;
         size_t bytes;
@@ -1605,6 +1607,8 @@ asets_status run_dag(asets_context *ctx, int dim, int d1, int d2, int d3, int m,
             *u.dst = vp;
         }
     }
+    if (ok)
+        setup_copies<T>(get, st, A, dirs, e);  // last: the rest has to fit
     asets_status status = ASETS_OK;
     if (!ok) {
         status = ASETS_ERR_OUT_OF_MEMORY;
