@@ -1235,11 +1235,12 @@ bool setup_dirs(Get &get, cudaStream_t st, int dim, int m, void *const *const ld
 
 // The second copy of the flows, and the factors; the root has no flows and no
 // factor.  Without them the four passes run, in place: where they are not used,
-// and where they cannot be had.
+// where they cannot be had, and in 3D for more nodes than a grid's second
+// dimension has blocks.
 template <class T, class Get>
 void setup_copies(Get &get, cudaStream_t st, HArgs<T> &A, bool dirs, cudaError_t &e)
 {
-    if (dirs || (A.dim == 3 && sizeof(T) == 8))
+    if (dirs || (A.dim == 3 && (sizeof(T) == 8 || A.m > 65536)))
         return;
     void *vp = nullptr;
     if (!get(&vp, sizeof(T) * (A.f1 + A.f2 + A.f3 + A.ns) * A.m)) {
