@@ -197,34 +197,18 @@ __device__ __forceinline__ bool finished(const MTArgs<T> &A)
     for (long long t = blockIdx.x * (long long)kThreads + threadIdx.x; t < (total);    \
          t += (long long)gridDim.x * kThreads)
 
-// ud of flow label k at cell g: divp - ((A - B) + u/cc)
-template <class T, int M>
-__device__ __forceinline__ T ud(const MTArgs<T> &A, int k, long long g)
-{
-    const long long o = (long long)k * A.n + g;
-    T a, b;
-    if (M == MT_BINARY) {
-        a = A.ps[g];
-        b = A.pt[g];
-    } else if (M == MT_POTTS) {
-        a = A.ps[g];
-        b = A.pt[o];
-    } else {
-        a = A.pt[o];
-        b = A.pt[o + A.n];
-    }
-    return sub(A.divp[o], add(sub(a, b), u_cc(A, o)));
-}
-
-// ud of every flow label and cell of the initial state; the cell pass forms
-// it for the next iteration
+// ud = divp - ((A - B) + u/cc) of every flow label and cell of the initial
+// state, whose flows are zero (and binary ps the same as pt); the cell pass
+// forms it for the next iteration
 template <class T, int M>
 __global__ void mt_ud(const MTArgs<T> A)
 {
     MT_LOOP(A.n * A.nflow)
     {
-        const int k = label_of(t, A.n);
-        A.ud[t] = ud<T, M>(A, k, t - (long long)k * A.n);
+        const long long g = t - (long long)label_of(t, A.n) * A.n;
+        const T b = M == MT_ISHIKAWA ? A.pt[t + A.n] : A.pt[t];
+        const T a = M == MT_POTTS ? A.ps[g] : A.pt[t];
+        A.ud[t] = sub((T)0, add(sub(a, b), u_cc(A, t)));
     }
 }
 
@@ -824,9 +808,7 @@ __global__ void mt_init(const MTArgs<T> A)
         if (M == MT_BINARY) {
             const T cs = A.cs[g], ct = A.ct[g];
             set_u(A, g, (sub(cs, ct) >= (T)0) ? (T)1 : (T)0);
-            const T ps = mn(cs, ct);
-            A.ps[g] = ps;
-            A.pt[g] = ps;
+            A.pt[g] = mn(cs, ct);
             continue;
         }
         // [m, I] = min(Ct, [], labels): the first minimum
@@ -858,6 +840,9 @@ int mt_grid(long long n, int sms)
     const long long cap = (long long)sms * 8;
     return (int)(b < 1 ? 1 : (b < cap ? b : cap));
 }
+
+// Label counts with a Potts update of their own, which needs no divp
+constexpr bool potts_kernel_labels(int nlab) { return nlab >= 2 && nlab <= 6; }
 
 template <class T, int M, int D, int TX, int TY>
 void launch_cell(const MTArgs<T> &A, int grid, cudaStream_t st)
@@ -936,8 +921,8 @@ asets_status mt_run(asets_context *ctx, int rows, int cols, int slices, int nlab
     bool ok = get(&ct, n * nct) && get(&al, n * A.nflow) && get(&A.u, n * nu) &&
               get(&A.ud, n * A.nflow) &&
               get(&A.q1, A.f1 * A.nflow) && get(&A.q2, A.f2 * A.nflow) && get(&A.q3, A.f3 * A.nflow) &&
-              (sizeof(T) != 8 || get(&A.ucc, n * nu)) && get(&A.pt, n * npt) && get(&A.ps, n) &&
-              get(&A.divp, n * A.nflow) &&
+              (sizeof(T) != 8 || get(&A.ucc, n * nu)) && get(&A.pt, n * npt) &&
+              (M != MT_POTTS || (get(&A.ps, n) && (potts_kernel_labels(nlab) || get(&A.divp, n * nlab)))) &&
               get(&A.gk, n * A.nflow) && get(&A.p1, A.f1 * A.nflow) && get(&A.p2, A.f2 * A.nflow) &&
               get(&A.p3, A.f3 * A.nflow) && get(&A.erriter, iterNum) &&
               (M != MT_BINARY || get(&cs, n));
@@ -969,11 +954,10 @@ asets_status mt_run(asets_context *ctx, int rows, int cols, int slices, int nlab
             e = cudaMemcpyAsync(A.ctl, &c0, sizeof c0, cudaMemcpyHostToDevice, st);
         // the flows and the second face buffer start at zero; their border
         // faces are never written and stay zero (the zero-flux border)
-        T *zero[] = {A.divp, A.p1, A.p2, A.p3, A.erriter, A.q1, A.q2, A.q3};
-        const long long fq = A.nflow;
-        const long long zn[] = {n * A.nflow, A.f1 * A.nflow, A.f2 * A.nflow, A.f3 * A.nflow,
-                                (long long)iterNum, A.f1 * fq, A.f2 * fq, A.f3 * fq};
-        for (int i = 0; i < 8 && e == cudaSuccess; ++i)
+        T *zero[] = {A.p1, A.p2, A.p3, A.erriter, A.q1, A.q2, A.q3};
+        const long long fn = A.nflow;
+        const long long zn[] = {A.f1 * fn, A.f2 * fn, A.f3 * fn, (long long)iterNum, A.f1 * fn, A.f2 * fn, A.f3 * fn};
+        for (int i = 0; i < 7 && e == cudaSuccess; ++i)
             if (zn[i] > 0)
                 e = cudaMemsetAsync(zero[i], 0, sizeof(T) * zn[i], st);
         A.cs = cs;
@@ -1221,11 +1205,14 @@ asets_status mt_dispatch(int model, int dim, asets_context *ctx, int rows, int c
                          double beta, double cc, double steps, void *u, void *err, int *itNum)
 {
     if constexpr (sizeof(T) == 4)
-        if (model == MT_BINARY && dim == 3 && (long long)rows * cols * slices >= kOnePassMin)
-            return mt_binary3d_f32(ctx, rows, cols, slices, static_cast<const float *>(Cs),
-                                   static_cast<const float *>(Ct), static_cast<const float *>(alpha),
-                                   iterNum, beta, cc, steps, static_cast<float *>(u),
-                                   static_cast<float *>(err), itNum);
+        if (model == MT_BINARY && dim == 3 && (long long)rows * cols * slices >= kOnePassMin) {
+            const asets_status s =
+                mt_binary3d_f32(ctx, rows, cols, slices, static_cast<const float *>(Cs),
+                                static_cast<const float *>(Ct), static_cast<const float *>(alpha), iterNum, beta,
+                                cc, steps, static_cast<float *>(u), static_cast<float *>(err), itNum);
+            if (s != ASETS_ERR_OUT_OF_MEMORY)  // the two passes' rows are not padded
+                return s;
+        }
 #define MT_CASE(M, D)                                                                       \
     if (model == M && dim == D)                                                             \
         return mt_run<T, M, D>(ctx, rows, cols, slices, nlab, Cs, Ct, alpha, iterNum, beta, \

@@ -32,3 +32,4 @@ def test_special_values(what, dtype, shape, its):
     got = fn(cs, ct, al, [*shape, its, 1e-30, 0.3, steps])
     assert np.isnan(ref[0]).any() and got[2] == ref[2]
     assert np.array_equal(got[0], ref[0], equal_nan=True)
+
