@@ -351,14 +351,16 @@ __device__ __forceinline__ Rows<VEC> ld_rows(const float *p, bool ok)
 template <int VEC>
 __global__ void __launch_bounds__(32 * kAWarps)
     alpha_kernel(const float *img, int ny, int nx, int nz, const unsigned int *mm, float a, float b, float c,
-                 int squared, int L, int az, float *alpha)
+                 int squared, int L, int az, int per, float *alpha)
 {
-    const int lane = threadIdx.x & 31;
-    const int y = (blockIdx.x * 32 + lane) * VEC, x = blockIdx.y * kAWarps + (threadIdx.x >> 5);
-    if (x >= nx)
+    // `per` lanes have a column's rows; short columns share a warp
+    const int lane = threadIdx.x & 31, share = 32 / per, col = lane / per;
+    const int y = (blockIdx.x * per + lane - col * per) * VEC;
+    const int x0 = (blockIdx.y * kAWarps + (threadIdx.x >> 5)) * share, x = x0 + col;
+    if (x0 >= nx)
         return;  // a whole warp
     const int z0 = blockIdx.z * az, z1 = min(nz, z0 + az);
-    const bool in = y < ny;
+    const bool in = y < ny && x < nx && col < share;
     const long long plane = (long long)ny * nx, n = plane * nz;
     const float *p = img + (long long)x * ny + y;
     // 1/(max - min); a range whose reciprocal is not an ordinary number (and
@@ -377,8 +379,8 @@ __global__ void __launch_bounds__(32 * kAWarps)
     };
     const bool x_lo = x > 0, x_up = x + 1 < nx;
     const float sx = (x_lo && x_up) ? 0.5f : 1.f;
-    // the rows beyond the warp's 32*VEC
-    const bool edge_lo = lane == 0 && in && y > 0, edge_up = lane == 31 && y + VEC < ny;
+    // the rows beyond the warp's 32*VEC (a shared warp's columns are whole)
+    const bool edge_lo = lane == 0 && in && y > 0, edge_up = lane == 31 && in && y + VEC < ny;
     const long long z_off = (long long)z0 * plane;
     Rows<VEC> cur = ld_rows<VEC>(p + z_off, in), lo = z0 > 0 ? ld_rows<VEC>(p + z_off - plane, in) : cur;
     for (int z = z0; z < z1; ++z) {
@@ -642,8 +644,9 @@ extern "C" ASETS_API asets_status asets_alpha_contrast(asets_context *ctx, asets
     const int az = std::max(kAZ, (Nz + 65534) / 65535);  // planes per block: the grid's z extent
     auto launch = [&](auto vec) {
         constexpr int V = decltype(vec)::value;
-        const dim3 grid((Ny + 32 * V - 1) / (32 * V), (Nx + kAWarps - 1) / kAWarps, (Nz + az - 1) / az);
-        alpha_kernel<V><<<grid, 32 * kAWarps, 0, s.st>>>(vi.d, Ny, Nx, Nz, mm, a, b, c, squared, L, az, vo.d);
+        const int lanes = (Ny + V - 1) / V, per = lanes <= 16 ? lanes : 32, cols = kAWarps * (32 / per);
+        const dim3 grid((lanes + per - 1) / per, (Nx + cols - 1) / cols, (Nz + az - 1) / az);
+        alpha_kernel<V><<<grid, 32 * kAWarps, 0, s.st>>>(vi.d, Ny, Nx, Nz, mm, a, b, c, squared, L, az, per, vo.d);
     };
     const bool vec4 = (Ny & 3) == 0 && ((reinterpret_cast<uintptr_t>(vi.d) | reinterpret_cast<uintptr_t>(vo.d)) & 15) == 0;
     if (vec4)
