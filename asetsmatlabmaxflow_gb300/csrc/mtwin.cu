@@ -53,6 +53,7 @@ struct MTCtl {
 template <class T>
 struct MTArgs {
     int rows, cols, slices, nlab, nflow;
+    int step_rows, cell_rows;  // log2 of a tile's rows, where the kernel has no fixed count
     long long n, f1, f2, f3;  // cells and faces per flow label
     T cc, steps, half, one_over_cc, one_over_ccl, beta;
     DivConst<T> by_cc;
@@ -281,29 +282,38 @@ __device__ __forceinline__ T proj_factor(const MTArgs<T> &A, T a, T b, T d, T e,
 // buffer (q), the rescaled ones back to p, so that no pass reads a face
 // another thread of it writes.
 
-// A block steps the lower faces of a 32-row x 8-column tile of one flow label
-// and slice and those of the row and column past it, which the cells' norms
-// share through shared memory: a face costs one step (9/8 of one, with the
-// neighbouring tiles' faces), which in double is what the pass spends its
-// time on beside the norms at capacity.  The upper slice face is stepped
-// again by the cell below it.
+// A block steps the lower faces of a tile of one flow label and slice and
+// those of the row and column past it, which the cells' norms share through
+// shared memory: a face costs one step (9/8 of one, with the neighbouring tiles'
+// faces), which in double is what the pass spends its time on beside the
+// norms at capacity.  The upper slice face is stepped again by the cell below it.
+//
+// Tiles are 32 rows high (ROWS) where that leaves few lanes past the last row; a
+// kernel with ROWS = 0 takes 4 to 32 by the launch (tile_rows).
 constexpr int kTY = 32, kTX = 8;
 static_assert(kTY * kTX == kThreads, "one thread per cell of the tile");
+constexpr int kMinRows = 4;
 
-// Position of a block's tile, tiles running along rows, columns, then slices
-// (and labels).
-template <class T>
+// Rows (a power of two) and columns of a block's tile and its position, tiles
+// running along rows, columns, then slices (and labels).
+template <class T, int NT, int ROWS>
 struct Tile {
-    int y0, x0, pl;
-    __device__ explicit Tile(const MTArgs<T> &A, int tx = kTX, int ty = kTY)
+    int rows_log2, y0, x0, pl;
+    __device__ Tile(const MTArgs<T> &A, int log2) : rows_log2(log2)
     {
-        const unsigned int nty = (unsigned int)(A.rows + ty - 1) / ty;
-        const unsigned int ntx = (unsigned int)(A.cols + tx - 1) / tx;
+        const unsigned int nty = (unsigned int)(A.rows + ty() - 1) / ty();
+        const unsigned int ntx = (unsigned int)(A.cols + tx() - 1) / tx();
         const unsigned int q = blockIdx.x / nty;
-        y0 = (int)(blockIdx.x % nty) * ty;
-        x0 = (int)(q % ntx) * tx;
+        y0 = (int)(blockIdx.x % nty) * ty();
+        x0 = (int)(q % ntx) * tx();
         pl = (int)(q / ntx);
     }
+    __device__ __forceinline__ int ty() const { return ROWS ? ROWS : 1 << rows_log2; }
+    __device__ __forceinline__ int tx() const { return ROWS ? NT / (ROWS ? ROWS : 1) : NT >> rows_log2; }
+    // row and column of the tile's cell i
+    __device__ __forceinline__ int row(int i) const { return i & (ty() - 1); }
+    __device__ __forceinline__ int col(int i) const { return ROWS ? i / (ROWS ? ROWS : 1) : i >> rows_log2; }
+    static constexpr int kMostTX = NT / (ROWS ? ROWS : kMinRows), kMostTY = ROWS ? ROWS : 32;
 };
 
 // Slots in shared memory for the threads of the block that have a rare and
@@ -327,11 +337,13 @@ __device__ __forceinline__ int take_slots(int *count, int want)
     return base + before - want;
 }
 
-template <class T, int M, int D>
+template <class T, int M, int D, int ROWS>
 __global__ void __launch_bounds__(kThreads) mt_step_gk(const MTArgs<T> A)
 {
     constexpr bool QUEUE = sizeof(T) == 8;
-    __shared__ T s1[kTX + 1][kTY], s2[kTX][kTY + 1];
+    using Q = Tile<T, kThreads, ROWS>;
+    // column faces [x][y], row faces [x][y], one past the tile
+    __shared__ T s1[kThreads + Q::kMostTY], s2[kThreads + Q::kMostTX];
     __shared__ T s3[QUEUE && D == 3 ? 2 : 1][QUEUE && D == 3 ? kThreads : 1];
     __shared__ unsigned char s_q[kThreads];
     __shared__ int s_n;
@@ -339,8 +351,9 @@ __global__ void __launch_bounds__(kThreads) mt_step_gk(const MTArgs<T> A)
     grid_dependency_wait();
     if (finished(A))
         return;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const Tile<T> tile(A);
+    const Q tile(A, A.step_rows);
+    const int ty = tile.ty(), tx = tile.tx(), tid = threadIdx.x;
+    const int lane = tile.row(tid), w = tile.col(tid);
     const int k = tile.pl / A.slices, z = tile.pl % A.slices;
     const int y0 = tile.y0, x0 = tile.x0;
     if (threadIdx.x == 0)
@@ -379,18 +392,18 @@ __global__ void __launch_bounds__(kThreads) mt_step_gk(const MTArgs<T> A)
             q = face_step<T, M>(A, q0, A.ud[t + plane], v);
     }
     const T a = step1(y, x), d = step2(y, x);
-    s1[w][lane] = a;
-    s2[w][lane] = d;
-    if (w == 0)
-        s1[kTX][lane] = step1(y, x0 + kTX);
-    else if (w == 1 && lane < kTX)
-        s2[lane][kTY] = step2(y0 + kTY, x0 + lane);
+    s1[tid] = a;
+    s2[tid + w] = d;
+    if (tid < ty)
+        s1[kThreads + tid] = step1(y, x0 + tx);
+    else if (tid - ty < tx)
+        s2[(tid - ty) * (ty + 1) + ty] = step2(y0 + ty, x0 + tid - ty);
     if (in && x >= 1)
         A.q1[(long long)k * A.f1 + j1(A, y, x, z)] = a;
     if (in && y >= 1)
         A.q2[(long long)k * A.f2 + j2(A, y, x, z)] = d;
     __syncthreads();
-    const T b = s1[w + 1][lane], e = s2[w][lane + 1];
+    const T b = s1[tid + ty], e = s2[tid + w + 1];
     const bool inside = !in || surely_inside<T, D>(a, b, d, e, p, q, al);
     if constexpr (QUEUE) {
         if (in && inside)
@@ -405,11 +418,10 @@ __global__ void __launch_bounds__(kThreads) mt_step_gk(const MTArgs<T> A)
         }
         __syncthreads();
         if ((int)threadIdx.x < s_n) {  // at most one each
-            const int c = s_q[threadIdx.x], cl = c & 31, cw = c >> 5;
+            const int c = s_q[threadIdx.x], cl = tile.row(c), cw = tile.col(c);
             const long long tc = t + (long long)(cw - w) * A.rows + (cl - lane);
             const T pz = D == 3 ? s3[0][c] : (T)0, qz = D == 3 ? s3[D == 3 ? 1 : 0][c] : (T)0;
-            A.gk[tc] = proj_factor<T, D>(A, s1[cw][cl], s1[cw + 1][cl], s2[cw][cl], s2[cw][cl + 1], pz,
-                                         qz, A.alpha[tc]);
+            A.gk[tc] = proj_factor<T, D>(A, s1[c], s1[c + ty], s2[c + cw], s2[c + cw + 1], pz, qz, A.alpha[tc]);
         }
     } else if (in) {
         A.gk[t] = inside ? (T)1 : proj_factor<T, D>(A, a, b, d, e, p, q, al);
@@ -501,25 +513,26 @@ __device__ __forceinline__ T rescaled_divergence(const MTArgs<T> &A, int k, cons
 // and of the row and column past it is rescaled once, into shared memory, and
 // the faces with a factor below 1 by full warps together.  Called by every
 // thread of the block.
-template <class T, int D, int TX, int TY>
+template <class T, int D, int NT, int ROWS>
 struct FaceTile {
-    static constexpr int NT = TX * TY;
-    static_assert(TY >= TX && NT % 32 == 0, "the row past the tile is its second column's");
-    static constexpr int kFaces = (TX + 1) * TY + TX * (TY + 1) + (D == 3 ? 2 * NT : 0);
-    static constexpr int kRow = (TX + 1) * TY, kSlice = kRow + TX * (TY + 1);
-    T f[kFaces];               // column faces [x][y], row faces [x][y], slice faces (lower, upper)
+    using Q = Tile<T, NT, ROWS>;
+    static_assert(NT % 32 == 0 && Q::kMostTX + Q::kMostTY <= NT, "a thread has one face past the tile at most");
+    // column faces [x][y], row faces [x][y], one past the tile, slice faces (lower, upper)
+    static constexpr int kRow = NT + Q::kMostTY, kSlice = kRow + NT + Q::kMostTX;
+    static constexpr int kFaces = kSlice + (D == 3 ? 2 * NT : 0);
+    T f[kFaces];
     T g[kFaces][2];            // factors of the faces in the queue
     unsigned short q[kFaces];  // their places in f
     int n;
 
     // `in`: the thread's cell (y, x, z) is in the volume
-    __device__ T divergence(const MTArgs<T> &A, int k, int y, int x, int z, bool in)
+    __device__ T divergence(const MTArgs<T> &A, const Q &tile, int k, int y, int x, int z, bool in)
     {
-        const int lane = threadIdx.x % TY, w = threadIdx.x / TY;  // row and column in the tile
+        const int ty = tile.ty(), tx = tile.tx(), tid = threadIdx.x;
         const long long plane = (long long)A.rows * A.cols;
         const T *gk = A.gk + (long long)k * A.n + z * plane;
         const T *q1 = A.q1 + (long long)k * A.f1, *q2 = A.q2 + (long long)k * A.f2;
-        const int my1 = w * TY + lane, my2 = kRow + w * (TY + 1) + lane;
+        const int my1 = tid, my2 = kRow + tid + tile.col(tid);
         // up to five faces a thread: (place, factors), not yet in the queue
         int want = 0, at[5];
         T gu[5], gl[5];
@@ -547,10 +560,10 @@ struct FaceTile {
         col(0, my1, y, x);
         row(1, my2, y, x);
         at[2] = at[3] = at[4] = -1;
-        if (w == 0)
-            col(2, TX * TY + lane, y, x + TX);
-        else if (w == 1 && lane < TX)
-            row(2, kRow + lane * (TY + 1) + TY, y - lane + TY, x - w + lane);
+        if (tid < ty)
+            col(2, NT + tid, y, x + tx);
+        else if (tid - ty < tx)
+            row(2, kRow + (tid - ty) * (ty + 1) + ty, tile.y0 + ty, tile.x0 + tid - ty);
         if (D == 3) {
             const T *q3 = A.q3 + (long long)k * A.f3;
             const T *g0 = gk + (long long)x * A.rows + y;
@@ -575,7 +588,7 @@ struct FaceTile {
         for (int i = threadIdx.x; i < m; i += NT)
             f[q[i]] = mul(mul(A.half, add(g[i][0], g[i][1])), f[q[i]]);
         __syncthreads();
-        const T a = f[my1], b = f[my1 + TY], d = f[my2], e = f[my2 + 1];
+        const T a = f[my1], b = f[my1 + ty], d = f[my2], e = f[my2 + 1];
         if (in && x >= 1)
             A.p1[(long long)k * A.f1 + j1(A, y, x, z)] = a;
         if (in && y >= 1)
@@ -711,10 +724,9 @@ __device__ __forceinline__ double ishikawa_update(const MTArgs<T> &A, long long 
 // Per cell: divp of every flow label with the rescale of the stepped flows,
 // the cell update; the last block records erriter and the break.  Single
 // precision strides over the cells; in double a block has a tile (FaceTile).
-template <class T, int M, int D, int LFIX, int TX, int TY>
-__global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mt_cell(const MTArgs<T> A)
+template <class T, int M, int D, int LFIX, int NT, int ROWS>
+__global__ void __launch_bounds__(NT, 1024 / NT) mt_cell(const MTArgs<T> A)
 {
-    constexpr int NT = TX * TY;
     __shared__ double s_red[NT / 32];
     __shared__ int s_last;
     grid_launch_dependents();
@@ -738,12 +750,12 @@ __global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mt_cell(const MTArg
         }
     };
     if constexpr (sizeof(T) == 8) {
-        __shared__ FaceTile<T, D, TX, TY> faces;
-        const Tile<T> tile(A, TX, TY);
-        const int y = tile.y0 + threadIdx.x % TY, x = tile.x0 + threadIdx.x / TY, z = tile.pl;
+        __shared__ FaceTile<T, D, NT, ROWS> faces;
+        const Tile<T, NT, ROWS> tile(A, A.cell_rows);
+        const int y = tile.y0 + tile.row(threadIdx.x), x = tile.x0 + tile.col(threadIdx.x), z = tile.pl;
         const bool in = y < A.rows && x < A.cols;
         update(((long long)z * A.cols + x) * A.rows + y, in,
-               [&](int k) { return faces.divergence(A, k, y, x, z, in); });
+               [&](int k) { return faces.divergence(A, tile, k, y, x, z, in); });
     } else {
         MT_LOOP(A.n)
         {
@@ -844,21 +856,21 @@ int mt_grid(long long n, int sms)
 // Label counts with a Potts update of their own, which needs no divp
 constexpr bool potts_kernel_labels(int nlab) { return nlab >= 2 && nlab <= 6; }
 
-template <class T, int M, int D, int TX, int TY>
+template <class T, int M, int D, int NT, int ROWS>
 void launch_cell(const MTArgs<T> &A, int grid, cudaStream_t st)
 {
-    auto launch = [&](auto kernel) { launch_chained(kernel, dim3(grid), TX * TY, 0, st, A); };
+    auto launch = [&](auto kernel) { launch_chained(kernel, dim3(grid), NT, 0, st, A); };
     if constexpr (M == MT_POTTS) {
         switch (A.nlab) {
-        case 2: launch(mt_cell<T, M, D, 2, TX, TY>); return;
-        case 3: launch(mt_cell<T, M, D, 3, TX, TY>); return;
-        case 4: launch(mt_cell<T, M, D, 4, TX, TY>); return;
-        case 5: launch(mt_cell<T, M, D, 5, TX, TY>); return;
-        case 6: launch(mt_cell<T, M, D, 6, TX, TY>); return;
+        case 2: launch(mt_cell<T, M, D, 2, NT, ROWS>); return;
+        case 3: launch(mt_cell<T, M, D, 3, NT, ROWS>); return;
+        case 4: launch(mt_cell<T, M, D, 4, NT, ROWS>); return;
+        case 5: launch(mt_cell<T, M, D, 5, NT, ROWS>); return;
+        case 6: launch(mt_cell<T, M, D, 6, NT, ROWS>); return;
         default: break;
         }
     }
-    launch(mt_cell<T, M, D, 0, TX, TY>);
+    launch(mt_cell<T, M, D, 0, NT, ROWS>);
 }
 
 template <class T, int M, int D>
@@ -903,21 +915,40 @@ asets_status mt_run(asets_context *ctx, int rows, int cols, int slices, int nlab
     T *cs = nullptr, *ct = nullptr, *al = nullptr;
     asets_status status = ASETS_OK;
     const int grid = mt_grid(n * A.nflow, sms);
-    const long long tiles = (long long)((rows + kTY - 1) / kTY) * ((cols + kTX - 1) / kTX) * slices;
+    // Tiles of a slice's cells, and the rows of a tile of nt threads (as log2)
+    // that leaves the fewest lanes past the last row and column.
+    const auto tiles_of = [&](int ty, int tx) {
+        return (long long)((rows + ty - 1) / ty) * ((cols + tx - 1) / tx) * slices;
+    };
+    const auto best_rows = [&](int nt) {
+        int best = 5;
+        for (int l = 4; 1 << l >= kMinRows; --l)
+            if (tiles_of(1 << l, nt >> l) < tiles_of(1 << best, nt >> best))
+                best = l;
+        return best;
+    };
+    // A fixed 32 rows unless others save a seventh of the lanes.
+    const long long tiles = tiles_of(kTY, kTX);
+    A.step_rows = best_rows(kThreads);
+    const long long fitted = tiles_of(1 << A.step_rows, kThreads >> A.step_rows);
+    const bool fit_step = 7 * fitted <= 6 * tiles;
+    const long long step_tiles = fit_step ? fitted : tiles;
     // The cell update's tiles in double, 32 x 8; a tile's time is its chain of
     // labels and its FP64 operations on one SM, so that small volumes take half
     // ones: with less than a tile an SM 32 x 4 (us an iteration, 8 | 4 columns: 27 x
     // 28 x 21 Potts L = 3, 84 tiles, 41.6 | 31.1; 181 x 64 L = 5, 48 tiles, 31.1 |
     // 27.9), with less than four 16 x 8 where these leave a fifth fewer lanes
     // past the last row (35 x 30 x 19 L = 3: 47.8 | 38.8).
-    const auto tiles_of = [&](int ty, int tx) {
-        return (long long)((rows + ty - 1) / ty) * ((cols + tx - 1) / tx) * slices;
-    };
     const int rows32 = (rows + 31) / 32 * 32, rows16 = (rows + 15) / 16 * 16;
     const bool short_tiles = sizeof(T) == 8 && tiles < 4 * sms && 5 * rows16 <= 4 * rows32;
     const bool half_tiles = sizeof(T) == 8 && tiles < sms && !short_tiles;
     const long long cell_tiles = short_tiles ? tiles_of(16, kTX) : half_tiles ? tiles_of(kTY, kTX / 2) : tiles;
-    const int gcell = sizeof(T) == 8 ? (int)cell_tiles : mt_grid(n, sms), ginit = mt_grid(n, sms);
+    A.cell_rows = best_rows(kThreads / 2);
+    const long long fitted_cells = tiles_of(1 << A.cell_rows, (kThreads / 2) >> A.cell_rows);
+    const bool fit_cell =
+        sizeof(T) == 8 && 7 * fitted_cells <= 6 * cell_tiles * (short_tiles || half_tiles ? 1 : 2);
+    const int gcell = sizeof(T) == 8 ? (int)(fit_cell ? fitted_cells : cell_tiles) : mt_grid(n, sms),
+              ginit = mt_grid(n, sms);
     bool ok = get(&ct, n * nct) && get(&al, n * A.nflow) && get(&A.u, n * nu) &&
               get(&A.ud, n * A.nflow) &&
               get(&A.q1, A.f1 * A.nflow) && get(&A.q2, A.f2 * A.nflow) && get(&A.q3, A.f3 * A.nflow) &&
@@ -972,17 +1003,23 @@ asets_status mt_run(asets_context *ctx, int rows, int cols, int slices, int nlab
         int h_done = 0;
         for (int done_it = 0; e == cudaSuccess && done_it < iterNum; done_it += kChunk) {
             for (int i = 0; i < kChunk && done_it + i < iterNum; ++i) {
-                launch_chained(mt_step_gk<T, M, D>, dim3((unsigned int)(tiles * A.nflow)), kThreads, 0, st, A);
+                const dim3 gstep((unsigned int)(step_tiles * A.nflow));
+                if (fit_step)
+                    launch_chained(mt_step_gk<T, M, D, 0>, gstep, kThreads, 0, st, A);
+                else
+                    launch_chained(mt_step_gk<T, M, D, kTY>, gstep, kThreads, 0, st, A);
                 if constexpr (sizeof(T) == 8) {
-                    if (short_tiles || half_tiles) {
-                        if (short_tiles)
-                            launch_cell<T, M, D, kTX, 16>(A, gcell, st);
-                        else
-                            launch_cell<T, M, D, kTX / 2, kTY>(A, gcell, st);
-                        continue;
-                    }
+                    if (fit_cell)
+                        launch_cell<T, M, D, kThreads / 2, 0>(A, gcell, st);
+                    else if (short_tiles)
+                        launch_cell<T, M, D, kThreads / 2, 16>(A, gcell, st);
+                    else if (half_tiles)
+                        launch_cell<T, M, D, kThreads / 2, kTY>(A, gcell, st);
+                    else
+                        launch_cell<T, M, D, kThreads, kTY>(A, gcell, st);
+                } else {
+                    launch_cell<T, M, D, kThreads, kTY>(A, gcell, st);
                 }
-                launch_cell<T, M, D, kTX, kTY>(A, gcell, st);
             }
             e = cudaGetLastError();
             if (e == cudaSuccess)
@@ -1198,6 +1235,9 @@ asets_status mt_binary3d_f32(asets_context *ctx, int rows, int cols, int slices,
 // pass against two: 48^3 25.5 / 20.0, 128 x 128 x 10 25.3 / 24.2, 64^3
 // 23.5 / 29.3, 128 x 100 x 60 29.7 / 43.0).
 constexpr long long kOnePassMin = 200000;
+// and rows: its tiles have 64 (4 x 400 x 300 103.6 / 33.1, 8 x 300 x 200 62.2 / 33.4, 16
+// x 300 x 100 41.3 / 33.1).
+constexpr int kOnePassRows = 24;
 
 template <class T>
 asets_status mt_dispatch(int model, int dim, asets_context *ctx, int rows, int cols, int slices,
@@ -1205,7 +1245,7 @@ asets_status mt_dispatch(int model, int dim, asets_context *ctx, int rows, int c
                          double beta, double cc, double steps, void *u, void *err, int *itNum)
 {
     if constexpr (sizeof(T) == 4)
-        if (model == MT_BINARY && dim == 3 && (long long)rows * cols * slices >= kOnePassMin) {
+        if (model == MT_BINARY && dim == 3 && rows >= kOnePassRows && (long long)rows * cols * slices >= kOnePassMin) {
             const asets_status s =
                 mt_binary3d_f32(ctx, rows, cols, slices, static_cast<const float *>(Cs),
                                 static_cast<const float *>(Ct), static_cast<const float *>(alpha), iterNum, beta,
