@@ -10,6 +10,10 @@ static const StencilVariant kVariants[] = {
     make_variant3<14, 2, 3, EPI_DIV, true>(),
     make_variant3<13, 2, 4, EPI_DIV, true>(),
     make_variant3<12, 2, 4, EPI_DIV, true>(),
+    // 32-row tiles for volumes of up to 32 rows (step_cost3)
+    make_variant3<16, 1, 4, EPI_DIV, true>(),
+    make_variant3<12, 1, 4, EPI_DIV, true>(),
+    make_variant3<10, 1, 4, EPI_DIV, true>(),
 };
 
 const StencilVariant *flow3d_exact_variants(int *count)

@@ -75,6 +75,10 @@ double choose_split3(const StencilProblem &p, const StencilVariant &v, long long
 // time a column takes: measured at 64^3 to 256^3, the fast forms' steps take
 // (4 + TC) and the EXACT ones' (10 + TC) to within a few percent (binary
 // fast TC = 12, 13, 16 at 256^3: 0.94, 1.00, 1.21 us; EXACT 1.65, 1.77, 2.02).
+// A 32-row tile's step (one row a lane, labelled models) takes 0.7 of a 64-row
+// one's: the better tile up to 32 rows (28 x 200 x 200 Potts L = 4 78 us per iteration
+// against 90, EXACT 143 against 189), the worse from 33 on (90 x 150 x 150, three
+// tiles for two: 136 against 127, EXACT 222 against 221).
 double step_cost3(const StencilVariant &v);
 // The variant whose split takes the least time.  Fast 256^3 is split evenly
 // by 14 columns (19 x 4 tiles x 2 chunks = 152 blocks: 141 us per iteration

@@ -149,7 +149,10 @@ double choose_split3(const StencilProblem &p, const StencilVariant &v, long long
     return best;
 }
 
-double step_cost3(const StencilVariant &v) { return (v.exact ? 10.0 : 4.0) + v.tc; }
+double step_cost3(const StencilVariant &v)
+{
+    return ((v.exact ? 10.0 : 4.0) + v.tc) * (v.tr == 32 ? 0.7 : 1.0);
+}
 
 const StencilVariant *pick_split3(const StencilProblem &p, const StencilVariant *const *v, int n,
                                   int num_sms)
