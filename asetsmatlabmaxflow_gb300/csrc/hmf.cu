@@ -12,7 +12,8 @@
 //      memory when they fit, k1_staged);
 //   K2 gradient step of the spatial flows, K3 flow magnitude and projection
 //   factor, K4 flow rescale, K5 divergence (the rest of UpdateSpatialFlows);
-//   without direction fields in one kernel (2D) or two (3D).
+//   in single precision without direction fields in one kernel (2D) or two
+//   (3D).
 // Costs (CalculateCostsFullFlow) are summed on the device in double.
 //
 // The DAG solver (maxflow/asetsDAGMF2D.m / 3D, nodes may have several
@@ -920,7 +921,10 @@ __global__ void __launch_bounds__(kThreads) k_dag_point_staged(const HArgs<T> A)
 // within alpha^2 have factor 1 without the square root and the division.  The
 // factor is stored (to A.f) on the last pass only: nothing else reads it.
 // 768 x 640, six nodes: 20 us (28 x 32 tiles in shared memory, four phases
-// with barriers between them, factors stored each time: 26).
+// with barriers between them, factors stored each time: 26).  Single precision
+// only: in double, bound by its operations, the rows and columns that a warp
+// forms beside its own cost more than the passes' traffic (seven nodes, 40 iterations:
+// 512 x 512 16.0 ms against 12.8, 20 x 900 4.4 against 2.6).
 constexpr int kSweepThreads = 128, kSweepRows = 28;
 
 template <class T>
@@ -1166,31 +1170,33 @@ int h_grid(long long n, int sms)
 template <class T>
 void spatial_passes(HArgs<T> &A, int gn, int sms, cudaStream_t st, bool dirs, bool last)
 {
-    if (A.q1 && A.dim == 3 && A.m > 1) {
-        const dim3 grid((unsigned int)((A.n + kThreads - 1) / kThreads), A.m - 1);
-        launch_chained(k_step_factor3d<T>, grid, kThreads, 0, st, A);
-        launch_chained(k_rescale_div3d<T>, grid, kThreads, 0, st, A);
-        if (last)
-            std::swap(A.g, A.f);
-        return;
-    }
-    if (A.q1 && A.m > 1) {
-        // columns a warp: six warps for each of an SM's four schedulers if the
-        // image has them, no fewer than six columns (three more are read on
-        // either side), in whole groups of four steps
-        const int strips = (A.d1 + kSweepRows - 1) / kSweepRows;
-        const long long rows = (long long)strips * (A.m - 1);
-        long long chunks = (sms * 24LL + rows - 1) / rows;
-        chunks = std::max(1LL, std::min(chunks, (long long)(A.d2 + 5) / 6));
-        const int S = ((int)((A.d2 + chunks - 1) / chunks) + 2 + 3) / 4 * 4 - 2;
-        const int total = strips * ((A.d2 + S - 1) / S), per = kSweepThreads / 32;
-        launch_chained(k_spatial_sweep2d<T>, dim3((total + per - 1) / per, A.m - 1), kSweepThreads, 0, st, A,
-                       last ? 1 : 0, strips, total, S);
-        std::swap(A.p1, A.q1);
-        std::swap(A.p2, A.q2);
-        if (last)
-            std::swap(A.g, A.f);
-        return;
+    if constexpr (sizeof(T) == 4) {  // the second copy is single precision's
+        if (A.q1 && A.dim == 3) {
+            const dim3 grid((unsigned int)((A.n + kThreads - 1) / kThreads), A.m - 1);
+            launch_chained(k_step_factor3d<T>, grid, kThreads, 0, st, A);
+            launch_chained(k_rescale_div3d<T>, grid, kThreads, 0, st, A);
+            if (last)
+                std::swap(A.g, A.f);
+            return;
+        }
+        if (A.q1) {
+            // columns a warp: six warps for each of an SM's four schedulers if
+            // the image has them, no fewer than six columns (three more are read
+            // on either side), in whole groups of four steps
+            const int strips = (A.d1 + kSweepRows - 1) / kSweepRows;
+            const long long rows = (long long)strips * (A.m - 1);
+            long long chunks = (sms * 24LL + rows - 1) / rows;
+            chunks = std::max(1LL, std::min(chunks, (long long)(A.d2 + 5) / 6));
+            const int S = ((int)((A.d2 + chunks - 1) / chunks) + 2 + 3) / 4 * 4 - 2;
+            const int total = strips * ((A.d2 + S - 1) / S), per = kSweepThreads / 32;
+            launch_chained(k_spatial_sweep2d<T>, dim3((total + per - 1) / per, A.m - 1), kSweepThreads, 0, st, A,
+                           last ? 1 : 0, strips, total, S);
+            std::swap(A.p1, A.q1);
+            std::swap(A.p2, A.q2);
+            if (last)
+                std::swap(A.g, A.f);
+            return;
+        }
     }
     k2_gradient<T><<<gn, kThreads, 0, st>>>(A);
     if (dirs) {
@@ -1234,13 +1240,13 @@ bool setup_dirs(Get &get, cudaStream_t st, int dim, int m, void *const *const ld
 }
 
 // The second copy of the flows, and the factors; the root has no flows and no
-// factor.  Without them the four passes run, in place: where they are not used,
-// where they cannot be had, and in 3D for more nodes than a grid's second
-// dimension has blocks.
+// factor.  Without them the four passes run, in place: where they are not used
+// (direction fields; double precision), where they cannot be had, and in 3D for
+// more nodes than a grid's second dimension has blocks.
 template <class T, class Get>
 void setup_copies(Get &get, cudaStream_t st, HArgs<T> &A, bool dirs, cudaError_t &e)
 {
-    if (dirs || (A.dim == 3 && (sizeof(T) == 8 || A.m > 65536)))
+    if (dirs || sizeof(T) == 8 || A.m < 2 || (A.dim == 3 && A.m > 65536))
         return;
     void *vp = nullptr;
     if (!get(&vp, sizeof(T) * (A.f1 + A.f2 + A.f3 + A.ns) * A.m)) {
