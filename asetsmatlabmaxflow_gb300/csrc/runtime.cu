@@ -465,57 +465,70 @@ static double persistent_load(const asets_solver *s, const StencilVariant *v)
 // Default forms of a single multi-label 2D solve.  An image whose 16 x 16 tiles
 // are at most two per resident block runs as one whole-solve launch, and with
 // few flow labels fl also some more: r tiles a block (rounded up) with r*(fl + 2)
-// up to 16 in fast mode below 300,000 pixels, up to 21 in EXACT, whose sweeps
-// are slower.  Measured (us per iteration, tiles | best other form or default):
+// up to 16 in fast mode below 300,000 pixels, up to 20 in EXACT, whose sweeps
+// are slower, and 21 where three tiles a block are nearly full and the image is
+// no strip.  Measured (us per iteration, tiles | best other form or default):
 // fast Potts 512^2 L = 2 (16) 20.0 | 21.5, 440^2 L = 3 (15) 19.4 | 21.2, L = 4
 // (18) 22.8 | 21.7; EXACT 512^2 L = 3 (20) 26.9 | 28.7, 440^2 L = 5 (21) 33.0 |
-// 36.3, L = 6 (24) 36.8 | 34.7.
-static constexpr double kTileLabelsLoad = 2.0, kTileLabelsWork = 16.0, kTileLabelsWorkExact = 21.0;
+// 36.3, L = 6 (24) 36.8 | 34.7, 442 x 339 L = 5 (21) 36.5 | 34.3, Ishikawa 1006 x 457
+// L = 2 (21, seven tiles a block) 34.2 | 30.8.
+static constexpr double kTileLabelsLoad = 2.0, kTileLabelsWork = 16.0, kTileLabelsWorkExact = 20.0;
 static constexpr long long kFusedMinPx = 300000, kFusedMinPxExact = 1LL << 17;
-// Then one of the one-pass sweeps (0 in-step update, 1 one label warp, 2 two)
-// or the two-pass form (-1), by pixels: each from its line on, the last one
-// that is reached.  A sweep's time depends on how many warps its flow and
-// label updates make and what they wait for, so the lines are those of
-// measurements at 131,000 to 7.8 million pixels (as 362^2, 640 x 600, 800 x
-// 820, 1024^2, 1450 x 1300, 2048^2, 3000 x 2600) for each label count; the
-// choice wins 5 to 25 % at most sizes, e.g. fast Potts 800 x 820 L = 4 33.9 |
-// 37.6 two-pass, Ishikawa 1024^2 L = 6 49.9 | 65.3, Potts 2048^2 L = 7 235 | 350
-// (one label warp 498).
-struct FusedLine {
-    long long from;
-    int form;
-};
-static constexpr FusedLine kFusedForms[2][2][8][3] = {
-    {{// fast Potts, 1 .. 8 flow labels
-      {{0, 0}}, {{0, 0}, {450000, -1}, {2000000, 1}}, {{0, 2}}, {{0, 0}, {1200000, 1}},
-      {{0, 0}, {4000000, 2}}, {{0, 0}, {4000000, 2}}, {{0, 0}, {1500000, 2}}, {{0, 2}}},
-     {// fast Ishikawa
-      {{0, 0}}, {{0, 0}, {600000, -1}, {2000000, 1}}, {{0, 0}, {2000000, 2}}, {{0, 0}, {2000000, 1}},
-      {{0, 0}, {5000000, 2}}, {{0, 0}, {4000000, 2}}, {{0, 0}}, {{0, 0}, {5000000, 2}}}},
-    {{// EXACT Potts
-      {{0, -1}, {2200000, 0}}, {{0, -1}}, {{0, -1}, {1500000, 0}}, {{0, 1}},
-      {{0, 2}, {350000, 1}, {1200000, 0}}, {{0, -1}, {250000, 1}}, {{0, 2}, {700000, 1}}, {{0, 2}}},
-     {// EXACT Ishikawa
-      {{0, 1}, {900000, -1}, {1500000, 0}}, {{0, 1}}, {{0, 2}, {900000, 0}}, {{0, 1}},
-      {{0, 2}, {500000, 0}}, {{0, 2}}, {{0, 2}, {4000000, 0}}, {{0, 2}}}}};
+// Then the two-pass form ('-') or one of the one-pass sweeps (0 in-step update, 1
+// one label warp, 2 two), by the image's pixels (from 2^17 EXACT, from 300,000
+// fast; from 250,000 EXACT, 300,000 fast; from 500,000; one million; two million)
+// and its shape (more than four times as wide as tall; between; more than
+// twice as tall as wide), a letter for each number of flow labels, 1 to 8.  A
+// sweep's time depends on how many warps its flow and label updates make, what
+// they wait for and how many runs its chunks of the width are cut into, so the
+// letters are those of measurements: 135 shapes of 0.13 to 7.8 million pixels,
+// 16 : 1 to 1 : 16, each label count.  A letter is the form with the least mean
+// time over its class among those that are within 2.5 % of the plain rule's form
+// (two passes; in-step from 500,000 pixels with six flow labels or more; label
+// warps from two million, two up to three flow labels) at every shape of it.
+// Over all, 9 % less time than that rule: fast Potts 1378 x 1379 L = 4 68 us per
+// iteration against 86 with two passes, Ishikawa 2049 x 2050 L = 8 234 against 306
+// with one label warp, EXACT Potts 1025 x 1024 L = 7 120 against 140 in-step.
+// (One exception: EXACT Potts L = 6 from 250,000, 0.95 to 1.09 times as fast.)
+static const char *const kFusedForms[2][2][5][3] = {
+    // fast Potts
+    {{{"--------", "--------", "--------"},
+      {"--2---22", "--210-22", "-021-002"},
+      {"--2--022", "--210022", "----0002"},
+      {"--210022", "--210022", "---00000"},
+      {"22212222", "21211222", "21211222"}},
+     // fast Ishikawa
+     {{"--------", "--------", "--------"},
+      {"222-----", "00200000", "00200000"},
+      {"222--000", "--200000", "--200000"},
+      {"22200000", "--200000", "--000000"},
+      {"22222202", "22220200", "21220000"}}},
+    // EXACT Potts
+    {{{"--21---2", "-1212-22", "-1212122"},
+      {"--------", "--212112", "--21--12"},
+      {"------22", "---1-112", "---1--12"},
+      {"--212122", "---11112", "------12"},
+      {"2-211112", "2--11112", "2--11-12"}},
+     // EXACT Ishikawa
+     {{"1222222-", "12212222", "12212222"},
+      {"1-2-----", "22212-22", "222122-2"},
+      {"1-222222", "2-212222", "--210222"},
+      {"22212222", "--210222", "--010002"},
+      {"21212222", "21210222", "-1010022"}}}};
 
-// Below two million pixels only images at most four times as wide as tall (the
-// sweep runs along the width: 181 x 2000 fast Potts L = 6 43.0 | 38.7 two-pass,
-// 333 x 1100 L = 4 28.7 | 30.4) and, with fewer than six flow labels, at most
-// twice as tall as wide (1383 x 555 Ishikawa L = 3 31.5 | 29.0; 3000 x 130 Potts
-// L = 6 31.8 | 33.0).
 static int fused_form(bool ishikawa, int flow_labels, int exact, int nr, int ns)
 {
     const long long px = (long long)nr * ns;
-    if (px < (exact ? kFusedMinPxExact : kFusedMinPx) || flow_labels > 8)
+    const long long from[5] = {exact ? kFusedMinPxExact : kFusedMinPx, exact ? 250000 : kFusedMinPx, 500000,
+                               1000000, 2000000};
+    if (px < from[0] || flow_labels > 8)
         return -1;
-    if (px < 2000000 && (ns > 4LL * nr || (flow_labels < 6 && nr > 2LL * ns)))
-        return -1;
-    const FusedLine *line = kFusedForms[exact ? 1 : 0][ishikawa ? 1 : 0][flow_labels - 1];
-    int form = line[0].form;
-    for (int k = 1; k < 3 && line[k].from > 0 && px >= line[k].from; ++k)
-        form = line[k].form;
-    return form;
+    int size = 4;
+    while (px < from[size])
+        --size;
+    const int shape = ns > 4LL * nr ? 0 : nr > 2LL * ns ? 2 : 1;
+    const char form = kFusedForms[exact ? 1 : 0][ishikawa ? 1 : 0][size][shape][flow_labels - 1];
+    return form == '-' ? -1 : form - '0';
 }
 // Most 32 x 32 tiles per resident block the binary whole-solve kernel takes
 // by default: fast, every tile resident at once (beyond that the
@@ -559,8 +572,10 @@ static const StencilVariant *pick_variant(asets_solver *s, int exact, int tile_c
         const long long px = (long long)s->nr * s->ns;
         const int fl = s->flow_labels;
         const double load = persistent_load(s, match[4]), work = std::ceil(load) * (fl + 2);
-        if (load > 0.0 && (load <= kTileLabelsLoad ||
-                           (exact ? work <= kTileLabelsWorkExact : work <= kTileLabelsWork && px < kFusedMinPx)))
+        const bool nearly_full = fl == 5 && load > 2.5 && load <= 3.0 && s->nr <= 2LL * s->ns && s->ns <= 4LL * s->nr;
+        if (load > 0.0 &&
+            (load <= kTileLabelsLoad || (exact ? work <= kTileLabelsWorkExact || nearly_full
+                                               : work <= kTileLabelsWork && px < kFusedMinPx)))
             return match[4];
         const int form = fused_form(s->model == ASETS_ISHIKAWA, fl, exact, s->nr, s->ns);
         if (form >= 0)
