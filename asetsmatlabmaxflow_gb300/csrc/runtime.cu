@@ -438,17 +438,18 @@ static int attr_smem(const StencilVariant *v)
 static long long persistent_slots(const asets_solver *s, const StencilVariant *v)
 {
     const int smem = launch_smem(s, v);
-    if (cudaFuncSetAttribute(v->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, attr_smem(v)) !=
-        cudaSuccess) {
-        cudaGetLastError();
-        return 0;
+    int least = 1 << 20;
+    for (const void *fn : {v->fn, v->fn_many}) {
+        int per_sm = 0;
+        if (fn && (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, attr_smem(v)) != cudaSuccess ||
+                   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, v->nt, smem) != cudaSuccess)) {
+            cudaGetLastError();
+            return 0;
+        }
+        if (fn)
+            least = std::min(least, per_sm);
     }
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v->fn, v->nt, smem) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return (long long)per_sm * s->ctx->num_sms;
+    return (long long)least * s->ctx->num_sms;
 }
 
 // Tiles of the solver's problem per resident block in a whole-solve launch
@@ -532,9 +533,10 @@ static int fused_form(bool ishikawa, int flow_labels, int exact, int nr, int ns)
 }
 // Most 32 x 32 tiles per resident block the binary whole-solve kernel takes
 // by default: fast, every tile resident at once (beyond that the
-// two-iteration sweep wins); EXACT, up to eight (about 1600^2 pixels: the
-// EXACT sweep runs one iteration per pass)
-static constexpr double kTileBinaryMaxLoad = 1.0, kTileBinaryMaxLoadExact = 8.0;
+// two-iteration sweep wins); EXACT, up to six (about 1340^2 pixels: the EXACT
+// sweep runs one iteration per pass; 1300^2 50.5 us per iteration against 52.0,
+// 1400^2 59.9 against 54.8)
+static constexpr double kTileBinaryMaxLoad = 1.0, kTileBinaryMaxLoadExact = 6.0;
 
 // What the work split of a problem depends on.
 static StencilProblem item_geometry(const asets_solver *s)
@@ -718,7 +720,7 @@ static asets_status setup_kernel(asets_solver *s, int exact, int tile_config, bo
     CU_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v->fn, v->nt, smem));
     if (per_sm < 1)
         return fail(ASETS_ERR_UNSUPPORTED, "stencil kernel does not fit on an SM");
-    const long long slots = (long long)s->ctx->num_sms * per_sm;
+    const long long slots = v->persistent ? persistent_slots(s, v) : (long long)s->ctx->num_sms * per_sm;
     if (s->dim == 3)
         choose_split3(p, *v, slots, &A);
     else
@@ -1402,7 +1404,8 @@ static cudaError_t launch_persistent(asets_solver *s)
 {
     const StencilVariant *v = s->variant;
     void *params[] = {&s->bargs};
-    return cudaLaunchCooperativeKernel(v->fn, dim3(s->grid), dim3(v->nt), params, launch_smem(s, v),
+    const void *fn = v->fn_many && s->grid < s->bargs.total_items ? v->fn_many : v->fn;
+    return cudaLaunchCooperativeKernel(fn, dim3(s->grid), dim3(v->nt), params, launch_smem(s, v),
                                        s->ctx->stream);
 }
 

@@ -89,17 +89,19 @@ struct Tile2Loads {
             ct[k] = in ? __ldcg(P.ct + g) : 0.f;
         }
     }
-    // into the frame arrays (BR BS PS PT U AL)
+    // into the frame arrays (BR BS PS PT U AL); ALL: they were not issued with keep
+    template <bool ALL>
     __device__ void store(float *fsm) const
     {
+        const bool around = !ALL && kept;
 #pragma unroll
         for (int k = 0; k < PER; ++k) {
             const int i = threadIdx.x + k * NT;
-            if (wanted(i, kept)) {
+            if (wanted(i, around)) {
 #pragma unroll
                 for (int a = 0; a < 5; ++a)
                     fsm[a * G::F + i] = v[a][k];
-                if (!kept)
+                if (!around)
                     fsm[5 * G::F + i] = v[5][k];
             }
         }
@@ -108,9 +110,9 @@ struct Tile2Loads {
 
 // One ALM iteration of tile li of problem P from parity par, in the frame
 // `fsm` (Tile2Geom::NARR arrays): the loads' arrival, the phases, the stores
-// of the new flows and state, which stay in the frame as well.  Returns the
-// thread's share of erriter.
-template <int R, int S, int NT, bool EXACT>
+// of the new flows and (with KEEP) the state, which stay in the frame as well.
+// Returns the thread's share of erriter.
+template <int R, int S, int NT, bool EXACT, bool KEEP = false>
 __device__ __forceinline__ float tile2_iteration(const ProblemDesc &P, int par, int li, float *fsm,
                                                  const Tile2Loads<R, S, NT> &in)
 {
@@ -127,7 +129,7 @@ __device__ __forceinline__ float tile2_iteration(const ProblemDesc &P, int par, 
     const unsigned int pitch = (unsigned int)P.plane_stride;  // one row of Matlab x
     constexpr int PIX = Tile2Loads<R, S, NT>::PIX;
     float erru = 0.0f;
-    in.store(fsm);
+    in.template store<!KEEP>(fsm);
     __syncthreads();
 
     // gk on rows r0-2 .. r0+R+1, columns s0-2 .. s0+S+1
@@ -222,9 +224,14 @@ __device__ __forceinline__ float tile2_iteration(const ProblemDesc &P, int par, 
         pt_n = min_sel<EXACT>(pt_n, in.ct[k]);
         const float e = cc * ((pt_n + dv) - ps_n);
         erru += abs_ref(e);
-        d_ps[g] = PS[f] = ps_n;
-        d_pt[g] = PT[f] = pt_n;
-        d_u[g] = U[f] = u - e;
+        d_ps[g] = ps_n;
+        d_pt[g] = pt_n;
+        d_u[g] = u - e;
+        if (KEEP) {
+            PS[f] = ps_n;
+            PT[f] = pt_n;
+            U[f] = u - e;
+        }
     }
     __syncthreads();  // the frame is reused by the next item or iteration
     return erru;
@@ -300,7 +307,13 @@ __global__ void __launch_bounds__(NT, MINB) stencil2d_tile_kernel(const __grid_c
 // decision beside the loads and its partials in flight together, 301 x 170
 // with four labels takes 8.7 us an iteration (11.9 before), binary 256 x 256
 // 5.5 (6.3).
-template <int NT, class Load, class Iteration>
+//
+// TILES: one tile a block, several, or (TILES_ANY) whichever the launch has.  The
+// binary kernels are compiled for each apart: with both loops in one kernel
+// several tiles a block took 2 to 4 % longer (EXACT 1100 x 1100 38.6 us an iteration
+// against 37.6).
+enum Tiles { TILES_ONE, TILES_MANY, TILES_ANY };
+template <int NT, int TILES, class Load, class Iteration>
 __device__ __forceinline__ void tile_solve_loop(const ProblemDesc &P, unsigned int *arrivals,
                                                 double *s_red, int *s_stop, Load load, Iteration iteration)
 {
@@ -314,14 +327,16 @@ __device__ __forceinline__ void tile_solve_loop(const ProblemDesc &P, unsigned i
     const int max_it = ctl->max_it;
     const int break_lt = ctl->break_lt;
     const float err_bound = ctl->err_bound, denom = ctl->denom;
-    const bool one = P.n_items <= nb;
-    load(it, li, false);
+    const bool one = TILES == TILES_ANY ? P.n_items <= nb : TILES == TILES_ONE;
+    if (TILES != TILES_MANY)
+        load(it, li, false);
     for (unsigned int gen = 1;; ++gen) {
-        float erru = iteration(it, li);
-        for (int tile = li + nb; tile < P.n_items; tile += nb) {
-            load(it, tile, false);
-            erru += iteration(it, tile);
-        }
+        float erru = TILES != TILES_MANY ? iteration(it, li) : 0.0f;
+        if (TILES != TILES_ONE)
+            for (int tile = TILES == TILES_MANY ? li : li + nb; tile < P.n_items; tile += nb) {
+                load(it, tile, false);
+                erru += iteration(it, tile);
+            }
         const double part = block_sum<NT>(erru, s_red);
         if (tid == 0) {
             P.item_partials[(it & 1) * nb + li] = part;
@@ -347,7 +362,8 @@ __device__ __forceinline__ void tile_solve_loop(const ProblemDesc &P, unsigned i
         if (*s_stop == 2)
             break;  // a block did not arrive
         // the loads of the next iteration cover warp 0's decision
-        load(it + 1, li, one);
+        if (TILES != TILES_MANY)
+            load(it + 1, li, one);
         if (tid < 32) {
             double acc = lane_partials(P.item_partials + (it & 1) * nb, nb);
 #pragma unroll
@@ -377,7 +393,7 @@ __device__ __forceinline__ void tile_solve_loop(const ProblemDesc &P, unsigned i
     }
 }
 
-template <int R, int S, int NT, bool EXACT, int MINB>
+template <int R, int S, int NT, bool EXACT, int MINB, int TILES>
 __global__ void __launch_bounds__(NT, MINB)
     stencil2d_tile_persistent_kernel(const __grid_constant__ BatchArgs B)
 {
@@ -386,10 +402,12 @@ __global__ void __launch_bounds__(NT, MINB)
     __shared__ int s_stop;
     const ProblemDesc &P = B.probs[0];
     Tile2Loads<R, S, NT> in;
-    tile_solve_loop<NT>(
+    tile_solve_loop<NT, TILES>(
         P, B.queue, s_red, &s_stop,
         [&](int it, int tile, bool keep) { in.issue(P, it & 1, tile, keep); },
-        [&](int it, int tile) { return tile2_iteration<R, S, NT, EXACT>(P, it & 1, tile, fsm, in); });
+        [&](int it, int tile) {
+            return tile2_iteration<R, S, NT, EXACT, TILES == TILES_ONE>(P, it & 1, tile, fsm, in);
+        });
 }
 
 }  // namespace asets

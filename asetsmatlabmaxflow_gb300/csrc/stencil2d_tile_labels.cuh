@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(NT, 2)
     __shared__ double s_red[NT / 32];
     __shared__ int s_stop;
     const ProblemDesc &P = B.probs[0];
-    tile_solve_loop<NT>(
+    tile_solve_loop<NT, TILES_ANY>(
         P, B.queue, s_red, &s_stop,
         [&](int it, int tile, bool keep) { ltile_load<MODEL, NT>(P, it & 1, tile, fsm, keep); },
         [&](int it, int tile) { return ltile_iteration<MODEL, NT, EXACT>(P, it & 1, tile, fsm); });

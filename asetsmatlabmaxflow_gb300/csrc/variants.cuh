@@ -102,10 +102,13 @@ StencilVariant make_variant_tile()
     v.box_cols_bc = 1;
     v.tile_box_rows = R;
     v.temporal = 1;
-    if constexpr (PERSISTENT)
-        v.fn = reinterpret_cast<const void *>(&stencil2d_tile_persistent_kernel<R, S, NT, EXACT, MINB>);
-    else
+    if constexpr (PERSISTENT) {
+        v.fn = reinterpret_cast<const void *>(&stencil2d_tile_persistent_kernel<R, S, NT, EXACT, MINB, TILES_ONE>);
+        v.fn_many =
+            reinterpret_cast<const void *>(&stencil2d_tile_persistent_kernel<R, S, NT, EXACT, MINB, TILES_MANY>);
+    } else {
         v.fn = reinterpret_cast<const void *>(&stencil2d_tile_kernel<R, S, NT, EXACT, MINB>);
+    }
     v.s_tile = S;
     v.persistent = PERSISTENT ? 1 : 0;
     return v;
