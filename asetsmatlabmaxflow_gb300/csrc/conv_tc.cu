@@ -17,7 +17,9 @@
 // when the volume is small and by the MMAs when it is large (27 at 28 ns a
 // tile): 8.3 us at 32^3 and 12 us at 128 x 32 x 32, where a tile of 128 along y
 // at one x, loaded in runs of 128 bytes, took 24 and 22.  Two blocks an SM
-// overlap one's start and end with the other's work.
+// overlap one's start and end with the other's work.  Where that fills them
+// better, a tile's 16 rows are those of z at one x instead (`along_z`): a call of
+// 512 x 1 x 128 39 us against 64.
 //
 // The same kernel computes the data gradient: with `flip` the taps are
 // mirrored and the weight matrix transposed.  The weight gradient is a
@@ -51,13 +53,15 @@ struct ConvTcArgs {
     const float *addend;       // [v][16] FP32 or null: added before ReLU and mask
     void *out;                 // [v][16] BF16 or FP32
     int *err;
-    int ny, nx, nz;
-    int ytiles, xtiles;        // tiles of 8 x 16 voxels
+    int ny, nx;                // nx: of the tiles' second axis (x, or z along_z)
+    int ytiles, xtiles, ntiles;  // tiles of 8 x 16 voxels
+    int step_x, step_r;        // rows of the volume per step of the second axis and of the other
+    int tap_z, tap_x;          // bytes per step of a tap's dz and dx in a stage
     int relu, out_fp32, flip;
     int hp_in, hp_out;         // half-planar BF16 input (and mask) / output
     int ypad;                  // half-planar row length (ny rounded up to 8)
     int stages_log2;           // TMA ring depth of this launch
-    int stage_bytes, plane_bytes;  // of the staged [z][x][half][voxel][8], of one z of it
+    int stage_bytes;           // of the staged [other axis][second axis][half][voxel][8]
 };
 
 // Chained launches (ConvLaunch::chained) start while the layer before still
@@ -109,7 +113,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3_tc_kernel(const __grid_
         grid_launch_dependents();  // not before the allocation (above)
     }
 
-    const int ntiles = A.ytiles * A.xtiles * A.nz;
+    const int ntiles = A.ntiles;
     const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     auto issue = [&](int j) {
         const int st = j & smask, tile = blockIdx.x + j * gridDim.x;
@@ -183,7 +187,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3_tc_kernel(const __grid_
                 const uint32_t a0 = smem_addr(smem + st * kConvStageStride);
                 for (int t = 0; t < 27; ++t) {
                     const int dz = t / 9, dx = (t / 3) % 3, dy = t % 3;
-                    const uint32_t a = a0 + dz * A.plane_bytes + dx * kConvRowBytes + dy * 16;
+                    const uint32_t a = a0 + dz * A.tap_z + dx * A.tap_x + dy * 16;
                     const uint64_t ad = umma_smem_desc(a, kConvHalfBytes, kConvRowBytes);
                     const uint64_t bd = umma_smem_desc(b0 + t * kConvTapBytes, 256, 128);
                     umma_bf16(tmem + slot * 16, ad, bd, idesc, t > 0 ? 1u : 0u);
@@ -223,7 +227,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3_tc_kernel(const __grid_
             const int m = 32 * q + lane, z = rest / A.xtiles;
             const int x = rest % A.xtiles * 16 + (m >> 3), y = yt * 8 + (m & 7);
             if (y < A.ny && x < A.nx) {
-                const long long v = ((long long)z * A.nx + x) * A.ny + y;
+                const long long zx = (long long)z * A.step_r + (long long)x * A.step_x, v = zx * A.ny + y;
                 float o[16];
 #pragma unroll
                 for (int c = 0; c < 16; ++c)
@@ -245,7 +249,6 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3_tc_kernel(const __grid_
                         o[c] = fmaxf(o[c], 0.f);
                 }
                 // element offsets of the voxel's two channel halves in the input layout
-                const long long zx = (long long)z * A.nx + x;
                 const long long h0 = A.hp_in ? (zx * 2) * A.ypad * 8 + (long long)y * 8 : v * 16;
                 const long long h1 = A.hp_in ? h0 + (long long)A.ypad * 8 : v * 16 + 8;
                 if (A.mask) {
@@ -296,25 +299,30 @@ cudaError_t launch_conv3_tc(EncodeTiledFn encode, const ConvLaunch &c, int num_s
 {
     ConvTcArgs A;
     memset(&A, 0, sizeof A);
-    // The BF16 input as (8 ch, y, half, x, z) for channels-last
+    // The tiles' second axis (the one of 16 rows) and the other: x and z, or z
+    // and x where that makes fewer tiles.
+    const bool along_z = (long long)((c.nz + 15) / 16) * c.nx < (long long)((c.nx + 15) / 16) * c.nz;
+    const int n2 = along_z ? c.nz : c.nx, n3 = along_z ? c.nx : c.nz;
+    // The BF16 input as (8 ch, y, half, second, other) for channels-last
     // [z][x][y][16]; half-planar [z][x][half][ypad][8] as (ypad voxels of two
-    // 8-byte elements, 1, half, x, z), so that a box row is one run of memory.
-    // No more rows than a narrow volume has: what stays in the stage from
-    // another tile meets only outputs past the volume.
-    const int ypad = (c.ny + 7) / 8 * 8, xrows = c.nx < 16 ? c.nx + 2 : 18;
+    // 8-byte elements, 1, half, second, other), so that a box row is one run of
+    // memory.  No more rows than a narrow volume has: what stays in the stage
+    // from another tile meets only outputs past the volume.
+    const int ypad = (c.ny + 7) / 8 * 8, xrows = n2 < 16 ? n2 + 2 : 18;
+    const cuuint64_t row = (cuuint64_t)32 * (c.hp_in ? ypad : c.ny);  // bytes of a row of the volume
+    const cuuint64_t step2 = along_z ? row * c.nx : row, step3 = along_z ? row : row * c.nx;
     cuuint64_t dims[5], strides[4];
     cuuint32_t box[5];
     if (c.hp_in) {
-        const cuuint64_t d[5] = {(cuuint64_t)ypad * 2, 1, 2, (cuuint64_t)c.nx, (cuuint64_t)c.nz};
-        const cuuint64_t s[4] = {(cuuint64_t)16 * ypad, (cuuint64_t)16 * ypad, (cuuint64_t)32 * ypad,
-                                 (cuuint64_t)32 * ypad * c.nx};
+        const cuuint64_t d[5] = {(cuuint64_t)ypad * 2, 1, 2, (cuuint64_t)n2, (cuuint64_t)n3};
+        const cuuint64_t s[4] = {(cuuint64_t)16 * ypad, (cuuint64_t)16 * ypad, step2, step3};
         const cuuint32_t b[5] = {20, 1, 2, (cuuint32_t)xrows, 3};
         memcpy(dims, d, sizeof d);
         memcpy(strides, s, sizeof s);
         memcpy(box, b, sizeof b);
     } else {
-        const cuuint64_t d[5] = {8, (cuuint64_t)c.ny, 2, (cuuint64_t)c.nx, (cuuint64_t)c.nz};
-        const cuuint64_t s[4] = {32, 16, (cuuint64_t)32 * c.ny, (cuuint64_t)32 * c.ny * c.nx};
+        const cuuint64_t d[5] = {8, (cuuint64_t)c.ny, 2, (cuuint64_t)n2, (cuuint64_t)n3};
+        const cuuint64_t s[4] = {32, 16, step2, step3};
         const cuuint32_t b[5] = {8, 10, 2, (cuuint32_t)xrows, 3};
         memcpy(dims, d, sizeof d);
         memcpy(strides, s, sizeof s);
@@ -335,24 +343,27 @@ cudaError_t launch_conv3_tc(EncodeTiledFn encode, const ConvLaunch &c, int num_s
     A.out = c.y;
     A.err = d_err;
     A.ny = c.ny;
-    A.nx = c.nx;
-    A.nz = c.nz;
+    A.nx = n2;
     A.ytiles = ypad / 8;
-    A.xtiles = (c.nx + 15) / 16;
+    A.xtiles = (n2 + 15) / 16;
+    A.ntiles = A.ytiles * A.xtiles * n3;
+    A.step_x = along_z ? c.nx : 1;
+    A.step_r = along_z ? 1 : c.nx;
     A.relu = c.relu;
     A.out_fp32 = c.out_fp32;
     A.flip = c.flip;
     A.hp_in = c.hp_in;
     A.hp_out = c.hp_out;
     A.ypad = ypad;
-    A.plane_bytes = xrows * kConvRowBytes;
-    A.stage_bytes = 3 * A.plane_bytes;
+    const int other_bytes = xrows * kConvRowBytes;
+    A.tap_z = along_z ? kConvRowBytes : other_bytes;
+    A.tap_x = along_z ? other_bytes : kConvRowBytes;
+    A.stage_bytes = 3 * other_bytes;
     cudaError_t e = cudaFuncSetAttribute(conv3_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kConvSmem);
     if (e != cudaSuccess)
         return e;
-    const int tiles = A.ytiles * A.xtiles * c.nz;
-    const int grid = tiles < 2 * num_sms ? tiles : 2 * num_sms;
+    const int tiles = A.ntiles, grid = tiles < 2 * num_sms ? tiles : 2 * num_sms;
     while (A.stages_log2 < kConvStagesLog2 && (grid << A.stages_log2) < tiles)
         ++A.stages_log2;
     cudaLaunchAttribute attr{};
