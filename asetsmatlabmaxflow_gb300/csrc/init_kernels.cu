@@ -66,8 +66,9 @@ __device__ __forceinline__ void init_ishikawa(const InitArgs &A, long long g)
     A.pt[g + (A.nlab - 1) * S] = 0.0f;
 }
 
-// MODEL 0-2: the model's state; kPrepareCold: the binary state as v (cold_v)
-// with its gradient source; kPrepareNone: nothing
+// MODEL 0-2: the model's state (binary: with gk not null the gradient source of
+// it and zero flows too); kPrepareCold: the binary state as v (cold_v) with its
+// gradient source; kPrepareNone: nothing
 template <int MODEL>
 __device__ __forceinline__ void init_cells(const InitArgs &A, float *gk, float *v, float inv_cc)
 {
@@ -79,6 +80,10 @@ __device__ __forceinline__ void init_cells(const InitArgs &A, float *gk, float *
             continue;
         if (MODEL == 0) {
             init_binary(A, g);
+            if (gk) {  // u is 0 or 1: u/cc is u * inv_cc, rounded alike
+                const float m = A.pt[g];
+                gk[g] = 0.0f - ((m - m) + A.u[g] * inv_cc);
+            }
         } else if (MODEL == 1) {
             init_potts(A, g);
         } else if (MODEL == 2) {
@@ -92,10 +97,9 @@ __device__ __forceinline__ void init_cells(const InitArgs &A, float *gk, float *
     }
 }
 
-template <int MODEL>
-__global__ void init_kernel(const InitArgs A, float *gk, float *v, float inv_cc)
+__global__ void init_source_kernel(const InitArgs A, float *gk, float inv_cc)
 {
-    init_cells<MODEL>(A, gk, v, inv_cc);
+    init_cells<0>(A, gk, nullptr, inv_cc);
 }
 
 template <int MODEL>
@@ -165,22 +169,9 @@ static int grid_for(long long n, int num_sms)
     return (int)(b < cap ? b : cap);
 }
 
-cudaError_t launch_init(int model, const InitArgs &a, int num_sms, cudaStream_t st)
+cudaError_t launch_init_source(const InitArgs &a, float *gk, float inv_cc, int num_sms, cudaStream_t st)
 {
-    const int grid = grid_for(a.cells, num_sms);
-    switch (model) {
-    case 0: init_kernel<0><<<grid, kInitThreads, 0, st>>>(a, nullptr, nullptr, 0.f); break;
-    case 1: init_kernel<1><<<grid, kInitThreads, 0, st>>>(a, nullptr, nullptr, 0.f); break;
-    case 2: init_kernel<2><<<grid, kInitThreads, 0, st>>>(a, nullptr, nullptr, 0.f); break;
-    default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_cold_init(const InitArgs &a, float *gk, float *v, float inv_cc, int num_sms,
-                             cudaStream_t st)
-{
-    init_kernel<kPrepareCold><<<grid_for(a.cells, num_sms), kInitThreads, 0, st>>>(a, gk, v, inv_cc);
+    init_source_kernel<<<grid_for(a.cells, num_sms), kInitThreads, 0, st>>>(a, gk, inv_cc);
     return cudaGetLastError();
 }
 

@@ -189,10 +189,8 @@ struct PrepareArgs {
 };
 cudaError_t launch_prepare(const PrepareArgs &a, int num_sms, cudaStream_t st);
 
-// The cold binary start's v and gk (as launch_prepare with kPrepareCold).
-cudaError_t launch_cold_init(const InitArgs &a, float *gk, float *v, float inv_cc, int num_sms,
-                             cudaStream_t st);
-cudaError_t launch_init(int model, const InitArgs &a, int num_sms, cudaStream_t st);
+// The binary model's initial state and its gradient source gk with zero flows.
+cudaError_t launch_init_source(const InitArgs &a, float *gk, float inv_cc, int num_sms, cudaStream_t st);
 // The cold start's state (device_common.cuh) holds pt and u in one float for
 // costs and capacities below the limit and 0 < cc <= 1.
 constexpr float kColdInputLimit = 0x1p34f;

@@ -245,7 +245,7 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     ia.ct = ct;
     ia.alpha = al;
     ia.u = uu[0];
-    ia.ps = gk[1];  // used to form the source only; the first iteration overwrites it
+    ia.ps = gk[1];  // not read: the first iteration overwrites it
     ia.pt = pt[0];
     ia.ctl = ctl;
     ia.cells = cells;
@@ -262,43 +262,17 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     const StencilVariant *v = nv > 0 ? &tab[0] : nullptr;
     if (!v)
         return na_fail(ASETS_ERR_UNSUPPORTED, "no kernel variant");
-    if (maxIt >= 1) {
-        const bool check_alpha = !(flags & ASETS_FLAG_NO_ALPHA_CHECK);
-        IterControl checked;
-        memset(&checked, 0, sizeof checked);
-        if (check_alpha)
-            NA_TRY(launch_validate_alpha(ia, d->num_sms, sm));
-        if (v->cold)
-            NA_TRY(launch_check_range(ia, d->num_sms, sm));
-        if (check_alpha || v->cold) {
-            NA_TRY(cudaMemcpyAsync(&checked, ctl, sizeof checked, cudaMemcpyDeviceToHost, sm));
-            NA_TRY(cudaStreamSynchronize(sm));
-        }
-        if (checked.alpha_bad)
+    if (maxIt >= 1 && !(flags & ASETS_FLAG_NO_ALPHA_CHECK)) {
+        NA_TRY(launch_validate_alpha(ia, d->num_sms, sm));
+        int bad = 0;
+        NA_TRY(cudaMemcpyAsync(&bad, &ctl->alpha_bad, sizeof bad, cudaMemcpyDeviceToHost, sm));
+        NA_TRY(cudaStreamSynchronize(sm));
+        if (bad)
             return na_fail(ASETS_ERR_ALPHA, "alpha(x) must be positive. Exiting...");
-        if (v->cold && !checked.wide && cold_cc(cc))
-            v = v->cold;
     }
-    const bool cold = (v->epi == EPI_COLD && maxIt > 0);
-    CarryArgs ca;
-    memset(&ca, 0, sizeof ca);  // zero flows
-    ca.g = GridGeom{Ny, Nx, Nz, pitch, pitch * Nx, cells};
-    ca.flow_labels = 1;
-    ca.exact = exact;
-    ca.cc = cc;
-    ca.inv_cc = 1.0f / cc;
-    ca.ps = gk[1];
-    ca.pt = pt[0];
-    ca.u = uu[0];
-    ca.cs = cs;
-    ca.ct = ct;
-    ca.gk = gk[0];
-    if (cold) {
-        NA_TRY(launch_cold_init(ia, gk[0], pt[0], ca.inv_cc, d->num_sms, sm));
-    } else {
-        NA_TRY(launch_init(0, ia, d->num_sms, sm));
-        NA_TRY(launch_source(0, ca, d->num_sms, sm));
-    }
+    // (the cold start's joint state needs a check of the inputs that costs a
+    // call of a few iterations more than it gains at these sizes)
+    NA_TRY(launch_init_source(ia, gk[0], 1.0f / cc, d->num_sms, sm));
     StencilProblem p;
     memset(&p, 0, sizeof p);
     p.nr = Ny;
@@ -387,11 +361,6 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     if (out.error & DEV_ERR_TIMEOUT)
         return na_fail(ASETS_ERR_TIMEOUT, "a device-side wait timed out");
     const int final_par = (maxIt == 0) ? 0 : ((out.last_iter + 1) & 1);
-    if (cold) {
-        ca.v = pt[final_par];
-        ca.u_out = uu[final_par];
-        NA_TRY(launch_cold_state(ca, d->num_sms, sm));
-    }
     NA_TRY(cudaMemcpy2DAsync(u, (size_t)Ny * 4, uu[final_par], pitch * 4, (size_t)Ny * 4, rows,
                              cudaMemcpyDeviceToDevice, sm));
     NA_TRY(cudaStreamSynchronize(sm));
