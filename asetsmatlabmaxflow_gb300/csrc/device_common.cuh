@@ -102,36 +102,48 @@ __device__ __forceinline__ void tma_load_4d(void *smem_dst, const CUtensorMap *m
         : "memory");
 }
 
-// Tensor maps in global memory are read through a proxy of their own, which
-// neither an earlier copy nor an earlier kernel's stores to the same place
-// reach by themselves: the writer releases them, and the thread that issues
-// the loads acquires each map it uses before the first.  A launch that finds
-// other maps at the address of the one before (another variant's) would else
-// be free to load through the old ones.
-__device__ __forceinline__ void tensormap_release()
-{
-    asm volatile("fence.proxy.tensormap::generic.release.sys;" ::: "memory");
-}
+// Tensor maps in global memory (a batch's) are read through a proxy of their
+// own, which an earlier copy to the same place does not reach by itself: each
+// block acquires a map it uses before its first load through it.  A launch that
+// finds other maps at the address of the one before (another layout's) would
+// else be free to load through the old ones.  Maps among a launch's parameters
+// (BatchArgs::maps) need no fence.
 __device__ __forceinline__ void tensormap_acquire(const CUtensorMap *map)
 {
     asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(
         reinterpret_cast<uint64_t>(map)));
 }
-// The maps of parity par whose bits are set (HALO: Slot, TILE: TileSlot), one
-// a lane of the producer's warp.  Called between the two barriers that hand out
-// an item, before any of its values is held: further down, the fence cost
-// registers (100 iterations of Ishikawa 1024^2 L = 8 took 7.6 ms, 6.7 here;
-// binary 256^3 16.0, 14.8).
+// The maps of parity par of an item's problem whose bits are set (HALO: Slot,
+// TILE: TileSlot), one a lane of the producer's warp.  Nothing writes maps while a
+// launch runs, so a block acquires those of its first item, and again only where
+// the problem is another one (s_maps: the last acquired, -1 none).  Called between
+// the two barriers that hand out an item, before any of its values is held:
+// further down, the fence cost registers (100 iterations of Ishikawa 1024^2 L = 8
+// took 7.6 ms, 6.7 here; binary 256^3 16.0, 14.8).
 constexpr unsigned int kHaloMaps2D =
     1u << SL_BR | 1u << SL_BS | 1u << SL_S0 | 1u << SL_S1 | 1u << SL_S2 | 1u << SL_ALPHA;
 constexpr unsigned int kTileMapsBinary = 1u << TS_S1 | 1u << TS_S2 | 1u << TS_CS | 1u << TS_CT;
 template <unsigned int HALO, unsigned int TILE>
-__device__ __forceinline__ void tensormaps_acquire(const ProblemDesc &P, int par)
+__device__ __forceinline__ void tensormaps_acquire(const BatchArgs &B, int item, int par, int *s_maps)
 {
+    if (B.own_maps)
+        return;
+    const int problem = B.item_problem[item], maps = 2 * problem + par;
+    if (*s_maps == maps)
+        return;
+    const ProblemDesc &P = B.probs[problem];
     const unsigned int lane = threadIdx.x & 31;
     if ((HALO | TILE << NUM_SLOTS) >> lane & 1u)
         tensormap_acquire(lane < NUM_SLOTS ? &P.halo[par][lane] : &P.tile[par][lane - NUM_SLOTS]);
     __syncwarp();
+    if (lane == 0)
+        *s_maps = maps;
+}
+
+// The maps through which a problem of the launch is loaded.
+__device__ __forceinline__ const TensorMaps &tensormaps(const BatchArgs &B, const ProblemDesc &P)
+{
+    return B.own_maps ? B.maps : P;
 }
 
 // ---------------------------------------------------------------- arithmetic

@@ -108,10 +108,10 @@ __global__ void __launch_bounds__(kInitThreads) prepare_kernel(const __grid_cons
     const long long t0 = blockIdx.x * (long long)kInitThreads + threadIdx.x;
     const long long step = (long long)gridDim.x * kInitThreads;
     if (blockIdx.x == 0) {
+        // what follows the maps, which the launches have among their parameters
         const int *src = reinterpret_cast<const int *>(&A.desc);
-        for (int i = threadIdx.x; i < (int)(sizeof(ProblemDesc) / 4); i += kInitThreads)
+        for (int i = sizeof(TensorMaps) / 4 + threadIdx.x; i < (int)(sizeof(ProblemDesc) / 4); i += kInitThreads)
             reinterpret_cast<int *>(A.d_desc)[i] = src[i];
-        tensormap_release();
         if (threadIdx.x == 0)
             *A.d_ctl = A.ctl;
         if (threadIdx.x < 4)

@@ -60,12 +60,16 @@ enum Epilogue : int {
 // new ps needs no old ps).
 enum TileSlot : int { TS_S1 = 0, TS_S2 = 1, TS_CS = 2, TS_CT = 3, NUM_TILE_SLOTS = 4 };
 
-// One problem of a launch, in device memory.  Each TMA descriptor is one
-// 128-byte unit of the fence that orders its use (tensormap_acquire).
-struct alignas(128) ProblemDesc {
+// Each TMA descriptor is one 128-byte unit of the fence that orders its use
+// where it lies in device memory (tensormap_acquire).
+struct alignas(128) TensorMaps {
     CUtensorMap halo[2][NUM_SLOTS];        // [source parity][slot]
     CUtensorMap tile[2][NUM_TILE_SLOTS];   // binary; EPI_FUSED: [.][TS_CT] = Ct, all labels,
                                            // halo rows (the same map for both parities)
+};
+
+// One problem of a launch, in device memory.
+struct ProblemDesc : TensorMaps {
     float *dst_b[2][3];                    // [source parity][SL_BC, SL_BR, SL_BS]
     float *dst_s[2][3];                    // binary: ps (3D: gk), pt, u; EPI_DIV: [.][0] = divergence;
                                            // EPI_FUSED: Potts ps, pt, u; Ishikawa pt, -, u
@@ -98,6 +102,18 @@ struct BatchArgs {
     int total_items;
     unsigned int *queue;       // [0] next item, [1] blocks that left
     unsigned int *done_count;  // problems that have finished (shared by the launches of a batch)
+    // A launch over one problem has its maps here, with the launch's other
+    // parameters, which needs no fence: acquiring them from device memory takes an
+    // SM about 0.23 us for each map and block (Ishikawa 2048^2 L = 2 in step,
+    // sixteen blocks an SM: 78 us an iteration, 52 from here).  own_maps 0: those of
+    // the problems' descriptors.
+    int own_maps;
+    TensorMaps maps;
+    void use_maps(const ProblemDesc &d)
+    {
+        own_maps = 1;
+        maps = d;
+    }
 };
 
 }  // namespace asets

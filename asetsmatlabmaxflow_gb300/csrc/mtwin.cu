@@ -1160,6 +1160,7 @@ asets_status mt_binary3d_f32(asets_context *ctx, int rows, int cols, int slices,
         B.total_items = items;
         B.queue = static_cast<unsigned int *>(get(4 * sizeof(unsigned int)));
         B.done_count = B.queue + 2;
+        B.use_maps(D);
         auto tr = [&](cudaError_t r) {
             if (e == cudaSuccess)
                 e = r;

@@ -330,6 +330,7 @@ asets_status noalloc_solve(DeviceSetup &dv, const asets_options *opt, const floa
     bargs.total_items = items;
     bargs.queue = queue;
     bargs.done_count = queue + 2;
+    bargs.use_maps(A);
     long long grid = items;
     if (grid > slots)
         grid = slots;

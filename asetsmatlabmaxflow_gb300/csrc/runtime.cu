@@ -757,6 +757,7 @@ static asets_status setup_kernel(asets_solver *s, int exact, int tile_config, bo
     s->bargs.total_items = items;
     s->bargs.queue = s->d_queue;
     s->bargs.done_count = s->d_queue + 2;
+    s->bargs.use_maps(A);
     if (v->persistent)
         s->grid = (int)std::min<long long>(items, slots);  // all resident, one or more tiles each
     // erriter partials of the label kernels (labelled models)
@@ -1578,6 +1579,7 @@ static asets_status replay_first_of_pass(asets_solver *s, const IterControl &out
     ba.total_items = items;
     ba.queue = s->d_queue;
     ba.done_count = s->d_queue + 2;
+    ba.use_maps(D);
     void *params[] = {&ba};
     const long long grid = std::max<long long>(1, std::min<long long>(items, slots));
     CU_TRY(cudaLaunchKernel(v->fn, dim3((unsigned)grid), dim3(v->nt), params, v->smem_bytes, stm));
@@ -2226,6 +2228,7 @@ static asets_status batch_layout(asets_batch *b, asets_batch::Group &g)
     g.bargs.total_items = (int)item_problem.size();
     g.bargs.queue = g.d_queue;
     g.bargs.done_count = b->d_done;
+    g.bargs.own_maps = 0;
     return ASETS_OK;
 }
 

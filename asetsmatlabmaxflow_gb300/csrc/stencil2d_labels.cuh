@@ -70,13 +70,14 @@ struct Lab2Geom {
     static constexpr int XSYNC = ((MODEL == 1) ? FL : 2 * FL + L) * 64;
 };
 
-// The TMA loads of one stage (its plane; Ct three planes behind).
+// The TMA loads of one stage (its plane; Ct three planes behind).  These kernels
+// serve one problem a launch, whose maps are among its parameters.
 template <int MODEL, int L>
-__device__ __forceinline__ void lab2_issue(float *base, const ProblemDesc &P, int par, int r0,
+__device__ __forceinline__ void lab2_issue(float *base, const TensorMaps &M, int par, int r0,
                                            int plane, uint64_t *bar)
 {
     using G = Lab2Geom<MODEL, L>;
-    const CUtensorMap *hmaps = P.halo[par];
+    const CUtensorMap *hmaps = M.halo[par];
     mbar_arrive_expect_tx(bar, G::TX);
     tma_load_4d(base + G::OFF_BR, &hmaps[SL_BR], r0 - 4, 0, plane, 0, bar);
     tma_load_4d(base + G::OFF_BS, &hmaps[SL_BS], r0 - 4, 0, plane, 0, bar);
@@ -88,7 +89,7 @@ __device__ __forceinline__ void lab2_issue(float *base, const ProblemDesc &P, in
     }
     tma_load_4d(base + G::OFF_U, &hmaps[SL_S2], r0 - 4, 0, plane, 0, bar);
     tma_load_4d(base + G::OFF_AL, &hmaps[SL_ALPHA], r0 - 4, 0, plane, 0, bar);
-    tma_load_4d(base + G::OFF_CT, &P.tile[par][TS_CT], r0 - 4, 0, plane - 3, 0, bar);
+    tma_load_4d(base + G::OFF_CT, &M.tile[par][TS_CT], r0 - 4, 0, plane - 3, 0, bar);
 }
 
 // A flow thread: rows r, r+1 of flow label k, swept along the stream axis.
@@ -279,7 +280,7 @@ __device__ __forceinline__ float ishikawa_layer(int l, float dv_l, float ucc_l, 
 // Claim the next item of the launch: thread 0 reads its problem's iteration
 // once for the block.  Returns false when the launch has no items left.
 __device__ __forceinline__ bool lab2_next_item(const BatchArgs &B, int *s_item, int *s_iter,
-                                               int &item, int &it, bool producer_warp)
+                                               int &item, int &it)
 {
     if (threadIdx.x == 0) {
         const int itm = (int)atomicAdd(&B.queue[0], 1u);
@@ -294,8 +295,6 @@ __device__ __forceinline__ bool lab2_next_item(const BatchArgs &B, int *s_item, 
     __syncthreads();
     item = *s_item;
     it = *s_iter;
-    if (producer_warp && it >= 0)
-        tensormaps_acquire<kHaloMaps2D, 1u << TS_CT>(B.probs[B.item_problem[item]], it & 1);
     __syncthreads();  // s_item/s_iter are rewritten by the next fetch
     return item < B.total_items;
 }
@@ -363,7 +362,7 @@ __global__ void __launch_bounds__(32 * Lab2WarpsGeom<MODEL, L, LW>::NW, MINB)
     __syncthreads();
 
     const int lane_row = C * lane;                  // a flow thread's rows within the 64
-    const bool producer_warp = (k == FL), producer = producer_warp && lane == 0;  // the first label warp
+    const bool producer = (tid == FL * 32);         // lane 0 of the first label warp
     // a label-warp thread's rows within the 64: two (one label warp) or one
     const int lab_row = (LW == 1) ? lane_row : (k - FL) * 32 + lane;
     // hand-over entry (value v, label l) of buffer b at row `row`
@@ -372,7 +371,7 @@ __global__ void __launch_bounds__(32 * Lab2WarpsGeom<MODEL, L, LW>::NW, MINB)
     unsigned int q0 = 0;
     bool aborted = false;
     int item, it;
-    while (!aborted && lab2_next_item(B, &s_item, &s_iter, item, it, producer_warp)) {
+    while (!aborted && lab2_next_item(B, &s_item, &s_iter, item, it)) {
         if (it < 0)
             continue;  // the problem has converged
         const ProblemDesc &P = B.probs[B.item_problem[item]];
@@ -393,7 +392,7 @@ __global__ void __launch_bounds__(32 * Lab2WarpsGeom<MODEL, L, LW>::NW, MINB)
 
         auto issue_load = [&](int j) {
             const unsigned int q = q0 + j;
-            lab2_issue<MODEL, L>(stages + (q % NSTAGE) * G::STAGE, P, par, r0, p_first + j,
+            lab2_issue<MODEL, L>(stages + (q % NSTAGE) * G::STAGE, B.maps, par, r0, p_first + j,
                                  &bars[q % NSTAGE]);
         };
         if (producer)
@@ -632,12 +631,12 @@ __global__ void __launch_bounds__(32 * Lab2Geom<MODEL, L>::FL, MINB)
     __syncthreads();
 
     const int lane_row = C * lane;                  // the thread's rows within the 64
-    const bool producer = (tid == NT - 32), producer_warp = (tid >= NT - 32);
+    const bool producer = (k == FL - 1 && lane == 0);
 
     unsigned int q0 = 0;
     bool aborted = false;
     int item, it;
-    while (!aborted && lab2_next_item(B, &s_item, &s_iter, item, it, producer_warp)) {
+    while (!aborted && lab2_next_item(B, &s_item, &s_iter, item, it)) {
         if (it < 0)
             continue;  // the problem has converged
         const ProblemDesc &P = B.probs[B.item_problem[item]];
@@ -657,7 +656,7 @@ __global__ void __launch_bounds__(32 * Lab2Geom<MODEL, L>::FL, MINB)
 
         auto issue_load = [&](int j) {
             const unsigned int q = q0 + j;
-            lab2_issue<MODEL, L>(stages + (q % NSTAGE) * G::STAGE, P, par, r0, p_first + j,
+            lab2_issue<MODEL, L>(stages + (q % NSTAGE) * G::STAGE, B.maps, par, r0, p_first + j,
                                  &bars[q % NSTAGE]);
         };
         if (producer)

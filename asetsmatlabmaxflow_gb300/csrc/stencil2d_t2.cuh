@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(32 * NW, MINB)
     __shared__ int s_is_last;
     __shared__ int s_item;
     __shared__ int s_iter;
+    __shared__ int s_maps;
 
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     unsigned char *smem = reinterpret_cast<unsigned char *>(
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(32 * NW, MINB)
 
     if (tid == 0) {
         s_abort = 0;
+        s_maps = -1;
         for (int i = 0; i < NSTAGE; ++i)
             mbar_init(&bars[i], 1);
         mbar_fence_init();
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(32 * NW, MINB)
         const int item = s_item;
         const int it = s_iter;
         if (producer_warp && it >= 0)
-            tensormaps_acquire<kHaloMaps2D, kTileMapsBinary>(B.probs[B.item_problem[item]], (it >> 1) & 1);
+            tensormaps_acquire<kHaloMaps2D, kTileMapsBinary>(B, item, (it >> 1) & 1, &s_maps);
         __syncthreads();
         if (item >= B.total_items)
             break;
@@ -185,8 +187,8 @@ __global__ void __launch_bounds__(32 * NW, MINB)
             continue;
         const ProblemDesc &P = B.probs[B.item_problem[item]];
         const int par = (it >> 1) & 1;   // one parity flip per pass
-        const CUtensorMap *hmaps = P.halo[par];
-        const CUtensorMap *tmaps = P.tile[par];
+        const CUtensorMap *hmaps = tensormaps(B, P).halo[par];
+        const CUtensorMap *tmaps = tensormaps(B, P).tile[par];
         const int nr = P.nr, ns = P.ns;
         const float cc = P.cc, inv_cc = P.inv_cc, steps = P.steps;
         const int li = item - P.item_begin;

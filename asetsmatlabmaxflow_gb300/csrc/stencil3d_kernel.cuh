@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
     __shared__ int s_abort;
     __shared__ double s_red[NT / 32];
     __shared__ int s_is_last;
-    __shared__ int s_item, s_iter;
+    __shared__ int s_item, s_iter, s_maps;
 
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
 
@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
 
     if (tid == 0) {
         s_abort = 0;
+        s_maps = -1;
         for (int i = 0; i < NSTAGE; ++i)
             mbar_init(&bars[i], 1);
         mbar_fence_init();
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
         const int item = s_item;
         const int it = s_iter;
         if (producer_warp && it >= 0)
-            tensormaps_acquire<kHaloMaps, kTileMaps>(B.probs[B.item_problem[item]], it & 1);
+            tensormaps_acquire<kHaloMaps, kTileMaps>(B, item, it & 1, &s_maps);
         __syncthreads();  // s_item/s_iter are rewritten by the next fetch
         if (item >= B.total_items)
             break;
@@ -259,8 +260,8 @@ __global__ void __launch_bounds__(Geom3<TC, CELLS, EPI>::NT, 1)
         const ProblemDesc &P = B.probs[B.item_problem[item]];
         IterControl *ctl = P.ctl;
         const int par = it & 1;
-        const CUtensorMap *hmaps = P.halo[par];
-        const CUtensorMap *tmaps = P.tile[par];
+        const CUtensorMap *hmaps = tensormaps(B, P).halo[par];
+        const CUtensorMap *tmaps = tensormaps(B, P).tile[par];
         const int nr = P.nr, nc = P.nc, ns = P.ns;
         const float cc = P.cc, inv_cc = P.inv_cc, steps = P.steps;
         const int tiles = P.tiles_r * P.tiles_c;

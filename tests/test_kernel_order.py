@@ -44,8 +44,7 @@ def test_dependents_start_after_the_tensor_memory_is_held(name, kernel):
         assert "}" not in between or "__syncthreads()" in between
 
 
-@pytest.mark.parametrize("name", ["stencil2_kernel.cuh", "stencil2d_t2.cuh", "stencil2d_labels.cuh",
-                                  "stencil3d_kernel.cuh"])
+@pytest.mark.parametrize("name", ["stencil2_kernel.cuh", "stencil2d_t2.cuh", "stencil3d_kernel.cuh"])
 def test_tensor_maps_are_acquired_before_the_first_load(name):
     text = _code(name)
     found = 0
@@ -54,16 +53,34 @@ def test_tensor_maps_are_acquired_before_the_first_load(name):
             continue
         found += 1
         head = body[:body.index("issue_load")]
-        if "lab2_next_item(" in head:
-            head = _body(text, text.index("bool lab2_next_item("))
         at = re.search(r"if \(producer_warp && it >= 0\)\s*tensormaps_acquire<", head)
         assert at, kernel
         # a barrier between the warp's fences and the producer's loads
         assert "__syncthreads()" in head[at.end():], kernel
+        maps = re.findall(r"(\S+)\.(?:halo|tile)\[", body)
+        assert maps and all(m.endswith("P)") for m in maps) and "tensormaps(B, P)" in body, kernel
     assert found
 
 
-def test_tensor_maps_written_by_a_kernel_are_released():
+def test_one_problem_kernels_load_through_the_launchs_maps():
+    """The multi-label 2D kernels acquire nothing: every map they use is among
+    their launch's parameters."""
+    text = _code("stencil2d_labels.cuh")
+    assert re.findall(r"lab2_issue<MODEL, L>\([^;]*", text)
+    assert all(" B.maps, par" in c for c in re.findall(r"lab2_issue<MODEL, L>\([^;]*", text))
+    assert set(re.findall(r"(\w+)\.(?:halo|tile)\[", text)) == {"M"}
+
+
+def test_no_kernel_writes_tensor_maps():
+    """Launches over one problem have their maps among their parameters; the
+    kernel that writes the rest of a descriptor leaves those in it alone."""
     text = _code("init_kernels.cu")
     body = _body(text, text.index("prepare_kernel(const"))
-    assert body.index("tensormap_release()") > body.index("A.d_desc)[i]")
+    assert "int i = sizeof(TensorMaps) / 4 + threadIdx.x" in body and "A.d_desc)[i]" in body
+
+
+@pytest.mark.parametrize("name,launches", [("runtime.cu", 2), ("noalloc.cu", 1), ("mtwin.cu", 1)])
+def test_launches_say_where_their_maps_are(name, launches):
+    text = _code(name)
+    own, shared = text.count(".use_maps("), text.count(".own_maps = 0;")
+    assert own == launches and own + shared == text.count(".total_items = ")
