@@ -477,54 +477,64 @@ static constexpr double kTileLabelsLoad = 2.0, kTileLabelsWork = 16.0, kTileLabe
 static constexpr long long kFusedMinPx = 300000, kFusedMinPxExact = 1LL << 17;
 // Then the two-pass form ('-') or one of the one-pass sweeps (0 in-step update, 1
 // one label warp, 2 two), by the image's pixels (from 2^17 EXACT, from 300,000
-// fast; from 250,000 EXACT, 300,000 fast; from 500,000; one million; two million)
-// and its shape (more than four times as wide as tall; between; more than
-// twice as tall as wide), a letter for each number of flow labels, 1 to 8.  A
-// sweep's time depends on how many warps its flow and label updates make, what
+// fast; from 250,000 EXACT, 300,000 fast; from 500,000; one million; two million;
+// 3.5 million) and its shape (more than four times as wide as tall; between; more
+// than twice as tall as wide), a letter for each number of flow labels, 1 to 8.
+// A sweep's time depends on how many warps its flow and label updates make, what
 // they wait for and how many runs its chunks of the width are cut into, so the
 // letters are those of measurements: 135 shapes of 0.13 to 7.8 million pixels,
-// 16 : 1 to 1 : 16, each label count.  A letter is the form with the least mean
-// time over its class among those that are within 2.5 % of the plain rule's form
-// (two passes; in-step from 500,000 pixels with six flow labels or more; label
-// warps from two million, two up to three flow labels) at every shape of it.
-// Over all, 9 % less time than that rule: fast Potts 1378 x 1379 L = 4 68 us per
-// iteration against 86 with two passes, Ishikawa 2049 x 2050 L = 8 234 against 306
-// with one label warp, EXACT Potts 1025 x 1024 L = 7 120 against 140 in-step.
-// (One exception: EXACT Potts L = 6 from 250,000, 0.95 to 1.09 times as fast.)
-static const char *const kFusedForms[2][2][5][3] = {
+// 16 : 1 to 1 : 16, each label count (Potts L = 1: six shapes).  A letter is the
+// form of least mean time over its class among those that at every shape of it
+// are within 3 % of the plain rule's form (two passes; in-step from 500,000
+// pixels with six flow labels or more; label warps from two million, two up to
+// three flow labels), and of a rule of lines by pixels alone, fitted to a dozen
+// sizes; where there is none, the one least far behind.  Over all, 8 % less time than the plain
+// rule (0.9 to 2.4 times as fast, 0.96 and more at all but 12 of 3,614), 2.5 %
+// less than those lines, 1.3 % more than the best form of each: fast Potts 1378
+// x 1379 L = 4 66 us per iteration against 86 with two passes, Ishikawa 2049 x
+// 2050 L = 2 52 in-step against 58 to 64 otherwise, EXACT Potts 1025 x 1024 L = 7
+// 117 against 136 in-step.
+// Fast images below 300,000 pixels that are no whole solve keep two passes as
+// the plain rule does, though from four labels on a sweep may be ahead (440 x 440
+// Potts L = 4 23.8 us against 21.1 in step, Ishikawa L = 6 25.0 against 20.8).
+static const char *const kFusedForms[2][2][6][3] = {
     // fast Potts
     {{{"--------", "--------", "--------"},
-      {"--2---22", "--210-22", "-021-002"},
-      {"--2--022", "--210022", "----0002"},
-      {"--210022", "--210022", "---00000"},
-      {"22212222", "21211222", "21211222"}},
-     // fast Ishikawa
+      {"2-2---22", "0-210022", "0021-022"},
+      {"2-2--222", "0-210022", "0-210002"},
+      {"2-210022", "0-210022", "0-010022"},
+      {"22212222", "00210222", "00210022"},
+      {"22212222", "01212222", "01212222"}},
+    // fast Ishikawa
      {{"--------", "--------", "--------"},
       {"222-----", "00200000", "00200000"},
-      {"222--000", "--200000", "--200000"},
-      {"22200000", "--200000", "--000000"},
-      {"22222202", "22220200", "21220000"}}},
+      {"222--002", "00000000", "0-200000"},
+      {"22200000", "0-000000", "--000000"},
+      {"22200002", "02210000", "01210000"},
+      {"22212202", "01212202", "01210200"}}},
     // EXACT Potts
-    {{{"--21---2", "-1212-22", "-1212122"},
-      {"--------", "--212112", "--21--12"},
-      {"------22", "---1-112", "---1--12"},
-      {"--212122", "---11112", "------12"},
-      {"2-211112", "2--11112", "2--11-12"}},
-     // EXACT Ishikawa
-     {{"1222222-", "12212222", "12212222"},
-      {"1-2-----", "22212-22", "222122-2"},
-      {"1-222222", "2-212222", "--210222"},
-      {"22212222", "--210222", "--010002"},
-      {"21212222", "21210222", "-1010022"}}}};
+    {{{"--21--22", "-2212-22", "-1212222"},
+      {"------2-", "--212222", "--21--12"},
+      {"------2-", "---12212", "---1-212"},
+      {"--212222", "---11212", "---1-212"},
+      {"2-211212", "0--11212", "0--10-12"},
+      {"2-211212", "0--10-12", "0-010-12"}},
+    // EXACT Ishikawa
+     {{"21222222", "22212222", "22212222"},
+      {"2-2-----", "22212222", "22212222"},
+      {"2-2-2--2", "21212222", "0-212222"},
+      {"22212222", "01210222", "--010222"},
+      {"22212222", "01010022", "01010222"},
+      {"21212222", "01010022", "01010022"}}}};
 
 static int fused_form(bool ishikawa, int flow_labels, int exact, int nr, int ns)
 {
     const long long px = (long long)nr * ns;
-    const long long from[5] = {exact ? kFusedMinPxExact : kFusedMinPx, exact ? 250000 : kFusedMinPx, 500000,
-                               1000000, 2000000};
+    const long long from[6] = {exact ? kFusedMinPxExact : kFusedMinPx, exact ? 250000 : kFusedMinPx, 500000,
+                               1000000, 2000000, 3500000};
     if (px < from[0] || flow_labels > 8)
         return -1;
-    int size = 4;
+    int size = 5;
     while (px < from[size])
         --size;
     const int shape = ns > 4LL * nr ? 0 : nr > 2LL * ns ? 2 : 1;

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("model,dims,L,exact,launches", [
-    ("ishikawa", (1300, 810), 2, False, 32), ("ishikawa", (2480, 827), 2, False, 16), ("potts", (300, 2000), 7, False, 16),
+    ("ishikawa", (144, 2292), 8, False, 32), ("ishikawa", (2048, 2050), 2, False, 16), ("potts", (300, 2000), 7, False, 16),
     ("potts", (420, 2510), 7, True, 16), ("ishikawa", (400, 1700), 8, False, 16), ("potts", (585, 3504), 3, True, 16),
     ("potts", (442, 339), 5, True, 16), ("ishikawa", (1006, 457), 2, True, 16)])
 def test_class_and_result(model, dims, L, exact, launches):
