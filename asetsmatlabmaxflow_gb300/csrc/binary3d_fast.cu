@@ -7,7 +7,8 @@ namespace asets {
 
 // One kernel per tile width, for the cold start (pt and u in one array) and
 // for a given start; the widths whose items and waves fit a volume best differ
-// (pick_variant3), the ring depth is the one that measured fastest.
+// (pick_split3; for a batch's group batch_width3), the ring depth is the one
+// that measured fastest.
 static const StencilVariant kCold[] = {
     make_variant3<14, 2, 3, EPI_COLD, false>(),
     make_variant3<16, 2, 3, EPI_COLD, false>(),

@@ -51,7 +51,7 @@
 //
 // Measured (binary 256^3, us per iteration, beside the form that recomputed gk
 // from seven halo boxes with two barriers per step): fast 142 (3.5 TB/s on
-// the old form's 60 B, 6.1 on the 52 B) against 206, EXACT 268 against 390;
+// the old form's 60 B, 6.1 on the 52 B) against 206, EXACT 253 against 390;
 // the flow pass and label kernel of Potts 192^3 L = 4: 270 against 378.
 // Three stages, not the five or six that fit: the ring then holds what the
 // blocks need and they stay near one another in s, so that the halos are

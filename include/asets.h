@@ -49,7 +49,12 @@ typedef enum asets_memory { ASETS_HOST = 0, ASETS_DEVICE = 1 } asets_memory;
 /* Solve options; pass NULL for the defaults. */
 typedef struct asets_options {
     int flags;       /* ASETS_FLAG_* */
-    int tile_config; /* 0 = default; k >= 1 selects the k-th tile variant of the kernel */
+    /* 0 = default; k >= 1 selects the k-th tile variant of the kernel.  Which
+     * tiles there are depends on dimension, model and mode, and may change from
+     * version to version: 3D binary 4 (EXACT 3), labelled 7; 2D binary 9 (EXACT
+     * 8), labelled 9 (4 in a batch, where binary has 7, EXACT 6).  A k past the
+     * end selects the default.  EXACT results are the same for all. */
+    int tile_config;
     int reserved[6];
 } asets_options;
 
